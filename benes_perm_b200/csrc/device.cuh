@@ -273,132 +273,69 @@ __device__ __forceinline__ void emit_bit(uint32_t* blob, uint64_t abs_bit, bool 
 }
 
 // ------------------------------------------------------------------------
-// 128-bit helpers for the factoradic rank.
+// Factoradic ranks of the middle groups.
 // ------------------------------------------------------------------------
 struct U128 {
     unsigned long long lo, hi;
 };
 
-__device__ __forceinline__ U128 mul128(U128 a, U128 b) {
-    U128 r;
-    r.lo = a.lo * b.lo;
-    r.hi = __umul64hi(a.lo, b.lo) + a.lo * b.hi + a.hi * b.lo;
+// Factoradic rank of one middle group of `count` <= 32 entries v[0..count)
+// (encode_factoradic, src/internal.hpp:148-167), by one thread: digit j =
+// #{k < j : v[k] < v[j]} is a popc on the mask of values seen so far, and
+// Horner's rule rank = rank * (j + 1) + digit_j sums digit_j * count!/(j+1)!.
+// The rank stays below 20! < 2^62 through the first 20 entries, so those
+// steps are 64-bit.  A thread per group costs about 10 instructions per
+// entry; the earlier warp-per-group form (ballots, prefix-OR and a 128-bit
+// shuffle tree) cost about 7 warp instructions per entry, 20 times more per
+// group.  *valid is false when a value is out of range or repeated.
+__device__ __forceinline__ U128 thread_factoradic_rank(const uint16_t* v, uint32_t count,
+    bool* valid) {
+    uint32_t seen = 0;
+    bool ok = true;
+    auto digit = [&](uint32_t j) {
+        const uint32_t value = v[j];
+        ok = ok && value < count;
+        const uint32_t bit = 1u << (value & 31u);
+        const uint32_t d = (uint32_t)__popc(seen & (bit - 1u));
+        seen |= bit;
+        return d;
+    };
+    U128 r = {0ull, 0ull};
+    const uint32_t narrow = count < 20 ? count : 20;
+    for (uint32_t j = 0; j < narrow; ++j) {
+        r.lo = r.lo * (j + 1) + digit(j);
+    }
+    for (uint32_t j = 20; j < count; ++j) {
+        const unsigned long long f = j + 1;
+        const unsigned long long lo = r.lo * f;
+        r.hi = __umul64hi(r.lo, f) + r.hi * f;
+        r.lo = lo + digit(j);
+        r.hi += r.lo < lo ? 1ull : 0ull;
+    }
+    *valid = ok && (uint32_t)__popc(seen) == count;
     return r;
 }
 
-__device__ __forceinline__ U128 add128(U128 a, U128 b) {
-    U128 r;
-    r.lo = a.lo + b.lo;
-    r.hi = a.hi + b.hi + (r.lo < a.lo ? 1ull : 0ull);
-    return r;
-}
-
-__device__ __forceinline__ U128 shfl_down128(U128 v, int d) {
-    U128 r;
-    r.lo = __shfl_down_sync(0xffffffffu, v.lo, d);
-    r.hi = __shfl_down_sync(0xffffffffu, v.hi, d);
-    return r;
-}
-
-// Factoradic rank of one middle group held one entry per lane (lanes
-// >= count are idle), as in encode_factoradic (src/internal.hpp:148-167):
-// digit j = #{k < j : v[k] < v[j]} and rank = sum_j digit_j * count!/(j+1)!.
-// Digits come from five ballots (a one-hot lane mask per value) and a
-// prefix-OR over values; the mixed-radix sum is an order-preserving tree
-// reduction of (rank, radix product) pairs: (r1,m1)+(r2,m2) = (r1*m2+r2, m1*m2).
-// Must be called by all 32 lanes.  Result valid in lane 0.  *distinct is
-// false (in every lane) when two lanes hold the same value.
-__device__ __forceinline__ U128 warp_factoradic_rank(uint32_t value, uint32_t count,
-    bool* distinct) {
-    const unsigned lane = threadIdx.x & 31;
-    const bool live = lane < count;
-    const unsigned active = __ballot_sync(0xffffffffu, live);
-    unsigned onehot = active;
-    for (int b = 0; b < 5; ++b) {
-        const unsigned bits = __ballot_sync(0xffffffffu, live && ((value >> b) & 1));
-        onehot &= ((lane >> b) & 1) ? bits : ~bits;
-    }
-    // with count values below count, every value has exactly one lane iff
-    // no value is missing
-    *distinct = __ballot_sync(0xffffffffu, live && __popc(onehot) != 1) == 0;
-    // onehot (in lane L) = the lane holding value L.  Exclusive prefix OR
-    // over values gives the lanes holding a smaller value.
-    unsigned below = onehot;
-    for (int d = 1; d < 32; d <<= 1) {
-        const unsigned t = __shfl_up_sync(0xffffffffu, below, d);
-        if ((int)lane >= d) {
-            below |= t;
-        }
-    }
-    below = __shfl_up_sync(0xffffffffu, below, 1);
-    if (lane == 0) {
-        below = 0;
-    }
-    const unsigned smaller = __shfl_sync(0xffffffffu, below, live ? value : 0);
-    const uint32_t digit = live ? (uint32_t)__popc(smaller & ((1u << lane) - 1u)) : 0u;
-    // The first three tree levels combine blocks of at most 8 radices, whose
-    // product stays below 25 * 26 * ... * 32 < 2^39: 64-bit arithmetic
-    // suffices there (and the partial rank is below the product).
-    unsigned long long r64 = digit;
-    unsigned long long m64 = live ? (unsigned long long)(lane + 1) : 1ull;
-    for (int d = 1; d < 8; d <<= 1) {
-        const unsigned long long r2 = __shfl_down_sync(0xffffffffu, r64, d);
-        const unsigned long long m2 = __shfl_down_sync(0xffffffffu, m64, d);
-        if ((lane & (2 * d - 1)) == 0) {
-            r64 = r64 * m2 + r2;
-            m64 *= m2;
-        }
-    }
-    U128 r = {r64, 0ull};
-    U128 m = {m64, 0ull};
-    for (int d = 8; d < 32; d <<= 1) {
-        const U128 r2 = shfl_down128(r, d);
-        const U128 m2 = shfl_down128(m, d);
-        if ((lane & (2 * d - 1)) == 0) {
-            r = add128(mul128(r, m2), r2);
-            m = mul128(m, m2);
-        }
-    }
-    return r;
-}
-
-// OR `nbits` (<= 118) bits of `rank` into the blob at absolute bit `abs`.
-// Lanes 0..4 each handle one destination word.  All lanes call.
-__device__ __forceinline__ void emit_rank(uint32_t* blob, uint64_t abs, uint32_t nbits,
+// ORs the `nbits` (<= 118) bits of `rank` into the blob at absolute bit
+// `abs`; rank < count! <= 2^nbits, so no bit at or above nbits is set.
+__device__ __forceinline__ void thread_emit_rank(uint32_t* blob, uint64_t abs, uint32_t nbits,
     U128 rank) {
-    const unsigned lane = threadIdx.x & 31;
-    rank.lo = __shfl_sync(0xffffffffu, rank.lo, 0);
-    rank.hi = __shfl_sync(0xffffffffu, rank.hi, 0);
-    if (nbits == 0 || lane >= 5) {
+    if (nbits == 0) {
         return;
     }
+    uint32_t* word = blob + (abs >> 5);
     const uint32_t shift = (uint32_t)(abs & 31);
-    const uint64_t word0 = abs >> 5;
-    const uint32_t last = (uint32_t)((shift + nbits - 1) >> 5);
-    if (lane > last) {
-        return;
-    }
-    // bits of the rank that land in destination word `lane`
-    const int lo_bit = (int)lane * 32 - (int)shift; // rank bit at dest bit 0 of this word
-    // rank < count! < 2^nbits, so no rank bit at or above nbits is set and
-    // the word is a plain 32-bit window of the 128-bit rank
-    uint32_t v;
-    if (lo_bit < 0) {
-        v = (uint32_t)(rank.lo << (uint32_t)(-lo_bit));
-    } else {
-        const uint32_t sh = (uint32_t)lo_bit; // < 128
-        unsigned long long x;
-        if (sh >= 64) {
-            x = rank.hi >> (sh - 64);
-        } else if (sh == 0) {
-            x = rank.lo;
-        } else {
-            x = (rank.lo >> sh) | (rank.hi << (64 - sh));
+    const uint32_t last = (shift + nbits - 1) >> 5; // destination words 0..last
+    uint32_t w[5] = {(uint32_t)rank.lo, (uint32_t)(rank.lo >> 32), (uint32_t)rank.hi,
+        (uint32_t)(rank.hi >> 32), 0u};
+    uint32_t below = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < 5; ++i) {
+        const uint32_t v = __funnelshift_l(below, w[i], shift);
+        below = w[i];
+        if (i <= last && v != 0) {
+            atomicOr(word + i, v);
         }
-        v = (uint32_t)x;
-    }
-    if (v != 0) {
-        atomicOr(blob + word0 + lane, v);
     }
 }
 

@@ -263,7 +263,7 @@ TileShape tile_shape(const Plan& p, uint32_t t0) {
     TileShape s;
     s.slots = (uint32_t)std::min<uint64_t>(slots, 1u << 30);
     s.pairs = (uint32_t)std::min<uint64_t>(pairs, 1u << 30);
-    uint32_t off[9];
+    uint32_t off[8];
     s.smem = tile_smem_layout(s.slots, s.pairs, off);
     if (slots >= 65536 || pairs >= (1u << 30)) {
         s.smem = UINT32_MAX;

@@ -36,7 +36,7 @@
 
 namespace bpb200 {
 
-constexpr uint32_t kNodeWaveLog2 = 6;
+constexpr uint32_t kNodeWaveLog2 = 7;
 constexpr uint32_t kNodeWave = 1u << kNodeWaveLog2; // tile node descriptors held in shared memory at once
 constexpr uint32_t kTileThreads = 512;
 // 4 slots per thread measured fastest on B200 at 2^30 uniform entries

@@ -40,8 +40,7 @@ __host__ __device__ inline uint32_t tile_smem_layout(uint32_t slots, uint32_t pa
     off[4] = o; o = align_up(o + words * 4, 16);           // xbits (input switches)
     off[5] = o; o = align_up(o + words * 4, 16);           // ybits (output switches)
     off[6] = o; o = align_up(o + 2 * kNodeWave * (uint32_t)sizeof(NodeAddress), 16);
-    off[7] = o; o = align_up(o + kNodeWave * 8, 16);       // leafbit
-    off[8] = o; o = align_up(o + slots * 2, 16);           // inv[1]
+    off[7] = o; o = align_up(o + slots * 2, 16);           // inv[1]
     return o;
 }
 
@@ -120,15 +119,14 @@ template <typename T>
 __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
     const T* __restrict__ src, uint32_t* __restrict__ blob, uint32_t* status, uint32_t slots,
     uint32_t pairs, uint32_t tile, unsigned char* smem) {
-    uint32_t off[9];
+    uint32_t off[8];
     tile_smem_layout(slots, pairs, off);
     uint16_t* vals[2] = {(uint16_t*)(smem + off[0]), (uint16_t*)(smem + off[1])};
-    uint16_t* invs[2] = {(uint16_t*)(smem + off[2]), (uint16_t*)(smem + off[8])};
+    uint16_t* invs[2] = {(uint16_t*)(smem + off[2]), (uint16_t*)(smem + off[7])};
     uint32_t* uf = (uint32_t*)(smem + off[3]);
     uint32_t* xbits = (uint32_t*)(smem + off[4]);
     uint32_t* ybits = (uint32_t*)(smem + off[5]);
     NodeAddress* desc = (NodeAddress*)(smem + off[6]);
-    uint64_t* leafbit = (uint64_t*)(smem + off[7]);
 
     const Plan& plan = *plan_ptr;
     const uint32_t tid = threadIdx.x;
@@ -384,9 +382,9 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
             const uint32_t wave_log2 = t < kNodeWaveLog2 ? t : kNodeWaveLog2; // log2(min(nodes, kNodeWave))
             const uint32_t wn = 1u << wave_log2;
             for (uint32_t w0 = 0; w0 < nodes; w0 += wn) {
-                if (tid < 2 * wn) {
-                    const uint32_t slot = tid >> 1;
-                    const int side = (int)(tid & 1);
+                for (uint32_t e = tid; e < 2 * wn; e += blockDim.x) {
+                    const uint32_t slot = e >> 1;
+                    const int side = (int)(e & 1);
                     const uint32_t node = first + w0 + slot;
                     const uint32_t s = node_size(node);
                     if (internal_node(w0 + slot, s)) {
@@ -505,42 +503,26 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
         }
 
         // leaves at this level (all of level D, and the size-`leaf` nodes of a
-        // mixed level D - 1)
+        // mixed level D - 1): one thread per leaf (see thread_factoradic_rank)
         if (lv.q <= leaf) {
-            for (uint32_t w0 = 0; w0 < nodes; w0 += kNodeWave) {
-                const uint32_t wn = nodes - w0 < kNodeWave ? nodes - w0 : kNodeWave;
-                if (tid < wn) {
-                    const uint32_t node = first + w0 + tid;
-                    uint64_t v = ~0ull;
-                    const bool exists = all_exist ||
-                        size_at(plan.levels[level - 1], level - 1, node >> 1) > leaf;
-                    if (node_size(node) <= leaf && exists) {
-                        int section = 0;
-                        const uint64_t bit = leaf_rank_bit(plan, level, node, &section);
-                        v = plan.section_offset[section] * 8 + bit;
-                    }
-                    leafbit[tid] = v;
+            for (uint32_t path = tid; path < nodes; path += blockDim.x) {
+                const uint32_t node = first + path;
+                const uint32_t s = node_size(node);
+                const bool exists = all_exist ||
+                    size_at(plan.levels[level - 1], level - 1, node >> 1) > leaf;
+                if (s > leaf || !exists) {
+                    continue;
                 }
-                __syncthreads();
-                for (uint32_t li = warp; li < wn; li += nwarps) {
-                    const uint64_t at = leafbit[li];
-                    if (at == ~0ull) {
-                        continue;
-                    }
-                    const uint32_t path = w0 + li;
-                    const uint32_t s = node_size(first + path);
-                    const uint32_t v = lane < s ? (uint32_t)cur[path * cap + lane] : 0u;
-                    if (lane < s && v >= s) {
-                        atomicOr(status, kErrNotPermutation);
-                    }
-                    bool distinct = true;
-                    const U128 rank = warp_factoradic_rank(v < s ? v : 0u, s, &distinct);
-                    if (!distinct && lane == 0) {
-                        atomicOr(status, kErrNotPermutation);
-                    }
-                    emit_rank(blob, at, plan.fact_bits[s], rank);
+                int section = 0;
+                const uint64_t bit = leaf_rank_bit(plan, level, node, &section);
+                bool valid = true;
+                const U128 rank = thread_factoradic_rank(cur + path * cap, s, &valid);
+                if (!valid) {
+                    atomicOr(status, kErrNotPermutation);
+                    continue;
                 }
-                __syncthreads();
+                thread_emit_rank(blob, plan.section_offset[section] * 8 + bit,
+                    plan.fact_bits[s], rank);
             }
         }
         if (level >= D) {

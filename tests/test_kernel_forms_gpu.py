@@ -1,0 +1,26 @@
+# SPDX-License-Identifier: Apache-2.0
+"""Byte parity with the oracle at the edges of the kernels' forms (tile and
+node sizes, group sizes, word boundaries); the bar is byte equality."""
+import numpy as np
+import pytest
+
+from helpers import b200_format, oracle_format
+
+pytestmark = pytest.mark.gpu
+
+
+def check(gpu, oracle, n, seed, kind=None, dtype=np.uint32, **kw):
+    perm = gpu.fill_permutation(kind if kind is not None else gpu.PermutationKind.uniform, seed,
+                                n, dtype)
+    got = gpu.compress(perm, gpu.CompressOptions(format=b200_format(gpu, kw)))
+    assert got == oracle.compress(perm, oracle_format(kw))
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 19, 20, 21, 22, 31, 32, 33, 39, 40, 41, 63, 64, 65,
+                               32 * 128 - 1, 32 * 128 + 1])
+@pytest.mark.parametrize("placement", [0, 1, 2])
+def test_middle_group_ranks(gpu, oracle, n, placement):
+    """Groups of 1..32 entries: the 64-bit and the 128-bit Horner steps meet
+    at 20 entries; ranks start at every bit offset of a word."""
+    for m in (4, 5):
+        check(gpu, oracle, n, 7 * n + m, middle_group_log2=m, middle_placement=placement)
