@@ -254,21 +254,28 @@ __global__ void prologue(uint32_t* status, uint32_t* blob, Header h) {
 // ------------------------------------------------------------ tile sizing
 
 TileShape tile_shape(const Plan& p, uint32_t t0) {
-    uint64_t slots = 0, pairs = 0;
+    uint64_t slots = 0;
     for (uint32_t l = t0; l <= p.depth; ++l) {
-        const uint64_t n = 1ull << (l - t0);
-        slots = std::max<uint64_t>(slots, n * p.levels[l].cap);
-        pairs = std::max<uint64_t>(pairs, n * p.levels[l].pcap);
+        const uint64_t stride = 2 * ((p.levels[l].pcap + 1) / 2 * 2);
+        slots = std::max<uint64_t>(slots, stride << (l - t0));
     }
     TileShape s;
     s.slots = (uint32_t)std::min<uint64_t>(slots, 1u << 30);
-    s.pairs = (uint32_t)std::min<uint64_t>(pairs, 1u << 30);
-    uint32_t off[8];
-    s.smem = tile_smem_layout(s.slots, s.pairs, off);
-    if (slots >= 65536 || pairs >= (1u << 30)) {
+    uint32_t off[7];
+    s.smem = tile_smem_layout(s.slots, off);
+    if (slots >= 65536) {
         s.smem = UINT32_MAX;
     }
     return s;
+}
+
+// Threads per tile.  With more tiles than two per SM, 256: the tile is bound
+// by instruction issue and by its barriers, and three small CTAs per SM wait
+// less at theirs (tiles of 100,000,007 entries: 6.1 ms against 7.7 ms with
+// 512).  Fewer tiles than that leave SMs idle, and one tile ends sooner with
+// 512 (8192 entries: 107 us against 140 us).  Wide tiles fill an SM each.
+unsigned tile_threads(uint64_t tiles, bool wide) {
+    return wide ? 2 * kTileThreads : (tiles > 2 * 148 ? kTileThreads / 2 : kTileThreads);
 }
 
 // Picks the tile level: the first level whose nodes fit `tile_max` entries
@@ -787,7 +794,8 @@ void launch_levels(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p,
         throw CudaFail{cudaErrorInvalidValue, "too many tiles"};
     }
     const bool wide = shape.smem > kTileSmemTwoPerSm;
-    auto launch_tile = [&](auto kernel, const auto* src, unsigned threads) {
+    const unsigned threads = tile_threads(tiles, wide);
+    auto launch_tile = [&](auto kernel, const auto* src) {
         allow_tile_smem((const void*)kernel);
         uint64_t lo = 0;
         const size_t count = parts != nullptr ? parts->cuts.size() : 1;
@@ -796,7 +804,7 @@ void launch_levels(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p,
             if (hi > lo) {
                 rec.launch(kKindTile, [&] {
                     kernel<<<(unsigned)(hi - lo), threads, shape.smem, st>>>(dp, src, d_blob,
-                        w.d_status, shape.slots, shape.pairs, (uint32_t)lo);
+                        w.d_status, shape.slots, (uint32_t)lo);
                 });
             }
             if (parts != nullptr && parts->after_part) {
@@ -807,15 +815,15 @@ void launch_levels(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p,
     };
     if (t0 == 0) {
         if (wide) {
-            launch_tile(tile_encode_wide<T>, d_in, 2 * kTileThreads);
+            launch_tile(tile_encode_wide<T>, d_in);
         } else {
-            launch_tile(tile_encode<T>, d_in, kTileThreads);
+            launch_tile(tile_encode<T>, d_in);
         }
     } else {
         if (wide) {
-            launch_tile(tile_encode_wide<uint32_t>, cur32, 2 * kTileThreads);
+            launch_tile(tile_encode_wide<uint32_t>, cur32);
         } else {
-            launch_tile(tile_encode<uint32_t>, cur32, kTileThreads);
+            launch_tile(tile_encode<uint32_t>, cur32);
         }
     }
     check(cudaGetLastError(), "tile kernel launch");

@@ -36,7 +36,7 @@
 
 namespace bpb200 {
 
-constexpr uint32_t kNodeWaveLog2 = 7;
+constexpr uint32_t kNodeWaveLog2 = 8;
 constexpr uint32_t kNodeWave = 1u << kNodeWaveLog2; // tile node descriptors held in shared memory at once
 constexpr uint32_t kTileThreads = 512;
 // 4 slots per thread measured fastest on B200 at 2^30 uniform entries
@@ -75,7 +75,6 @@ static_assert(kResolveItems == 1 || kResolveItems == 2 || kResolveItems == 4 ||
 
 struct TileShape {
     uint32_t slots;   // padded entry slots needed at the deepest level
-    uint32_t pairs;   // padded pair-node slots needed
     uint32_t smem;    // dynamic shared memory bytes
 };
 

@@ -2,8 +2,27 @@
 //
 // Tile kernel: one CTA per node of the tile level; the node's whole subtree
 // (every remaining routing level plus the middle-group ranks) is encoded in
-// shared memory.  Node-local values fit 16 bits (a tile holds at most a few
-// thousand entries), union-find words are 32-bit shared-memory words.
+// shared memory, on 16-bit node-local indexes.
+//
+// A node is held as its inverse (inv[o] = the input routed to output o) and
+// as its output edges: edge[u] is the input that shares input u's output
+// pair, edge[inv[2k]] = inv[2k+1] and back.  With pair-node k = inputs
+// {2k, 2k+1}, one 32-bit word per pair-node holds both edges, and the
+// constraint graph (src/benes.cpp:238-252) is a set of cycles over
+// pair-nodes: a path that enters pair-node k at input w leaves it at w^1 and
+// goes on to edge[w^1].  The inputs at which a path enters all have one
+// colour, and walked backwards the path enters at their partners, which have
+// the other.  An odd node's unpaired input t = s-1 gets a virtual partner s,
+// and its unpaired output a virtual partner output fed by s, which closes
+// the tail's path into a cycle as well.  The canonical rule (the odd tail
+// has colour 0, else the component's smallest input has) is then: with
+// key(v) = v, or (v - t) mod 2^16 in an odd node (which puts t and s first),
+// the colour of input v is the low bit of the smallest key on the directed
+// cycle through v, because that cycle passes the component's smallest
+// pair-node at exactly one of its two inputs.
+//
+// What bounds it: shared-memory latency and instruction issue; nothing
+// leaves the SM between the input load and the switch bits.
 #pragma once
 
 #include "device.cuh"
@@ -22,111 +41,104 @@ __host__ __device__ inline uint32_t align_up(uint32_t x, uint32_t a) { return (x
 struct FastDiv {
     uint32_t d, m;
     __device__ explicit FastDiv(uint32_t div)
-        : d(div), m(div > 1 ? (uint32_t)((0x100000000ull + div - 1) / div) : 0u) {}
+        : d(div), m(div > 1 ? 0xffffffffu / div + 1u : 0u) {}
     __device__ __forceinline__ uint32_t operator()(uint32_t n) const {
         return d > 1 ? __umulhi(n, m) : n;
     }
 };
 
-// Byte offsets of the smem arrays; identical on host (sizing) and device.
-__host__ __device__ inline uint32_t tile_smem_layout(uint32_t slots, uint32_t pairs,
-    uint32_t* off) {
-    const uint32_t words = (pairs + 31) / 32 + 1;
-    uint32_t o = 0;
-    off[0] = o; o = align_up(o + slots * 2, 16);           // vals[0]
-    off[1] = o; o = align_up(o + slots * 2, 16);           // vals[1]
-    off[2] = o; o = align_up(o + slots * 2, 16);           // inv[0]
-    off[3] = o; o = align_up(o + pairs * 4, 16);           // uf
-    off[4] = o; o = align_up(o + words * 4, 16);           // xbits (input switches)
-    off[5] = o; o = align_up(o + words * 4, 16);           // ybits (output switches)
-    off[6] = o; o = align_up(o + 2 * kNodeWave * (uint32_t)sizeof(NodeAddress), 16);
-    off[7] = o; o = align_up(o + slots * 2, 16);           // inv[1]
-    return o;
+// Pair-nodes per node in the tile's arrays: the level's pair-nodes rounded
+// up to an even number, so that a node's inverse starts on an 8-byte
+// boundary and four outputs (two output pairs) are one 64-bit load.
+__host__ __device__ inline uint32_t tile_pair_stride(uint64_t pcap) {
+    return ((uint32_t)pcap + 1u) & ~1u;
 }
 
-// Uniform-level fast path for node sizes in the tile (1) or size_at everywhere (0).
-#ifndef BPB200_TILE_UNIFORM
-#define BPB200_TILE_UNIFORM 1
-#endif
-
-// Tile input through one bulk asynchronous copy (1) or batched plain loads (0).
-#ifndef BPB200_TILE_BULK_LOAD
-#define BPB200_TILE_BULK_LOAD 0
-#endif
-constexpr uint32_t kBulkWaitCap = 1u << 22; // mbarrier polls before giving up
+// One pair-node in 2^kTileRulerLog2 is a ruler (see the walk below).
+constexpr uint32_t kTileRulerLog2 = 3;
+// Nodes of at most this many pair-nodes are coloured by one thread each.
+constexpr uint32_t kTileSerialPairs = 64;
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
 
-// Bounded wait for phase 0 of `mbar`; true once the phase has completed.
-__device__ __forceinline__ bool bulk_wait(uint32_t mbar) {
-    for (uint32_t it = 0; it < kBulkWaitCap; ++it) {
-        uint32_t done = 0;
-        asm volatile("{\n\t.reg .pred p;\n\t"
-                     "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                     "selp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(done) : "r"(mbar), "r"(0u) : "memory");
-        if (done) return true;
-    }
-    return false;
+// Shared-memory accesses of the walks, by 32-bit address: words that other
+// threads of the block rewrite meanwhile, and a store without a branch.
+__device__ __forceinline__ uint32_t shared_load(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
 }
 
-// Copies the s0 32-bit input values at `in` into `stage` (16-byte aligned,
-// at least s0 * 4 + 16 bytes, free until the caller is done with it): the
-// 16-byte-aligned interior of the range with one cp.async.bulk counted on an
-// mbarrier, the ragged ends (at most three values each) with plain loads, so
-// nothing outside the range is read.  Value i lands at stage[lead + i];
-// returns lead, or ~0u when the copy did not complete within the poll bound
-// (the status word then says so).  Every thread of the block calls it.
-__device__ __forceinline__ uint32_t tile_bulk_stage(const uint32_t* in, uint32_t s0,
-    uint32_t* stage, uint64_t* mbar, uint32_t* status) {
-    const uint64_t g0 = (uint64_t)in;
-    const uint64_t g1 = g0 + (uint64_t)s0 * 4;
-    const uint64_t a0 = (g0 + 15) & ~15ull;
-    const uint64_t a1 = g1 & ~15ull;
-    const uint32_t lead = (uint32_t)((g0 & 15) >> 2);
-    const bool bulk = a1 > a0;
-    const uint32_t mb = smem_addr(mbar);
-    if (threadIdx.x == 0 && bulk) {
-        const uint32_t bytes = (uint32_t)(a1 - a0);
-        const uint32_t dst = smem_addr(stage) + (uint32_t)(a0 - (g0 & ~15ull));
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(mb) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-                     :: "r"(mb), "r"(bytes) : "memory");
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes "
-                     "[%0], [%1], %2, [%3];"
-                     :: "r"(dst), "l"(a0), "r"(bytes), "r"(mb) : "memory");
+__device__ __forceinline__ void shared_store16_if(bool yes, uint32_t addr, uint32_t v) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\t"
+                 "@p st.volatile.shared.u16 [%1], %2;\n\t}"
+                 :: "r"((uint32_t)yes), "r"(addr), "h"((uint16_t)v) : "memory");
+}
+
+// Where one node's switches of one section go: first bits of its run in
+// packet 0 and in its tail packet, packets of the section's cluster apart.
+struct TileAddress {
+    uint64_t full; // top bit: the cluster root is a large node
+    uint64_t tail;
+};
+constexpr uint64_t kTileRootLarge = 1ull << 63;
+
+// Byte offsets of the smem arrays; identical on host (sizing) and device.
+// `slots`: 2 * tile_pair_stride * nodes at the level that needs most.
+__host__ __device__ inline uint32_t tile_smem_layout(uint32_t slots, uint32_t* off) {
+    const uint32_t words = slots / 64 + 2;
+    const uint32_t rulers = (slots >> (kTileRulerLog2 + 1)) + 1;
+    uint32_t o = 0;
+    off[0] = o; o = align_up(o + slots * 2, 16);           // inverse, even levels
+    off[1] = o; o = align_up(o + slots * 2, 16);           // inverse, odd levels
+    off[2] = o; o = align_up(o + slots * 2, 16);           // edges, one word per pair-node
+    off[3] = o; o = align_up(o + rulers * 8, 16);          // directed ruler states
+    off[4] = o; o = align_up(o + words * 4, 16);           // xbits (input switches)
+    off[5] = o; o = align_up(o + words * 4, 16);           // ybits (output switches)
+    off[6] = o; o = align_up(o + 2 * kNodeWave * (uint32_t)sizeof(TileAddress), 16);
+    return o;
+}
+
+// Colours one node of at most 64 pair-nodes (Mask: 32 or 64 bits) with one
+// thread: cycle after cycle from the smallest unvisited pair-node, the odd
+// tail's first, exactly the canonical order, so every cycle's first input
+// has colour 0 and no minimum is needed.  One dependent shared-memory load
+// per pair-node.  Returns bit k = colour of input 2k.
+template <typename Mask>
+__device__ __forceinline__ Mask tile_colour_node(const uint32_t* edge, uint32_t s) {
+    const uint32_t np = s - s / 2;
+    Mask todo = np >= sizeof(Mask) * 8 ? ~(Mask)0 : (((Mask)1 << np) - 1);
+    Mask x = 0;
+    uint32_t w = (s & 1u) != 0 ? s - 1 : 0u;
+    for (uint32_t i = 0; i < np; ++i) {
+        const uint32_t k = w >> 1;
+        const uint32_t v = edge[k];
+        todo &= ~((Mask)1 << k);
+        x |= (Mask)(w & 1u) << k;
+        w = (w & 1u) != 0 ? v & 0xffffu : v >> 16;
+        if (((todo >> (w >> 1)) & 1u) == 0) { // cycle closed
+            w = 2u * (uint32_t)(sizeof(Mask) == 8 ? __ffsll((long long)todo) : __ffs((int)todo)) - 2u;
+        }
     }
-    // ragged ends: values before a0 and from a1 on (all of them without bulk)
-    const uint32_t head = bulk ? (uint32_t)((a0 - g0) >> 2) : s0;
-    const uint32_t tail = bulk ? (uint32_t)((a1 - g0) >> 2) : s0;
-    for (uint32_t i = threadIdx.x; i < head; i += blockDim.x) stage[lead + i] = in[i];
-    for (uint32_t i = tail + threadIdx.x; i < s0; i += blockDim.x) stage[lead + i] = in[i];
-    __syncthreads(); // the mbarrier is initialised before anyone polls it
-    const bool ok = !bulk || bulk_wait(mb);
-    if (__syncthreads_or(!ok)) {
-        if (threadIdx.x == 0) atomicOr(status, kErrIterationCap);
-        bulk_wait(mb); // give the copy in flight one more bounded chance
-        __syncthreads();
-        return ~0u;
-    }
-    return lead;
+    return x;
 }
 
 template <typename T>
 __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
     const T* __restrict__ src, uint32_t* __restrict__ blob, uint32_t* status, uint32_t slots,
-    uint32_t pairs, uint32_t tile, unsigned char* smem) {
-    uint32_t off[8];
-    tile_smem_layout(slots, pairs, off);
-    uint16_t* vals[2] = {(uint16_t*)(smem + off[0]), (uint16_t*)(smem + off[1])};
-    uint16_t* invs[2] = {(uint16_t*)(smem + off[2]), (uint16_t*)(smem + off[7])};
-    uint32_t* uf = (uint32_t*)(smem + off[3]);
+    uint32_t tile, unsigned char* smem) {
+    uint32_t off[7];
+    tile_smem_layout(slots, off);
+    uint16_t* invs[2] = {(uint16_t*)(smem + off[0]), (uint16_t*)(smem + off[1])};
+    uint32_t* edge = (uint32_t*)(smem + off[2]);
+    uint16_t* edge16 = (uint16_t*)edge;
+    uint32_t* state = (uint32_t*)(smem + off[3]);
+    volatile uint32_t* vstate = state;
     uint32_t* xbits = (uint32_t*)(smem + off[4]);
     uint32_t* ybits = (uint32_t*)(smem + off[5]);
-    NodeAddress* desc = (NodeAddress*)(smem + off[6]);
+    TileAddress* desc = (TileAddress*)(smem + off[6]);
 
     const Plan& plan = *plan_ptr;
     const uint32_t tid = threadIdx.x;
@@ -141,39 +153,41 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
     if (T0 > 0 && size_at(plan.levels[T0 - 1], T0 - 1, J >> 1) <= leaf) {
         return; // child of a leaf: not part of the tree
     }
+    // The levels and groups the tile works on, into L1: their first uses would
+    // otherwise be chains of dependent L2 reads at every level.
+    {
+        uint32_t sum = 0;
+        const char* lo = reinterpret_cast<const char*>(&plan);
+        auto touch = [&](const void* from, const void* to) {
+            const uint32_t a = (uint32_t)((const char*)from - lo) & ~127u;
+            const uint32_t b = (uint32_t)((const char*)to - lo);
+            for (uint32_t at = a + 128 * tid; at < b; at += 128 * blockDim.x) {
+                sum += *reinterpret_cast<const uint32_t*>(lo + at);
+            }
+        };
+        touch(&plan, &plan.groups[0][plan.group_count[0]]);
+        touch(&plan.groups[1][0], &plan.groups[1][plan.group_count[1]]);
+        touch(&plan.levels[0], &plan.levels[D + 1]);
+        asm volatile("" :: "r"(sum));
+    }
+    // The tile's own node: its inverse and edges, or, when it is a leaf, its
+    // values.  Never-written inverse slots mean a repeated value; a tile
+    // that is not a permutation ends here, so everything below runs on valid
+    // indexes.
     {
         const LevelInfo& l0 = plan.levels[T0];
         const uint32_t s0 = size_at(l0, T0, J);
         const T* in = src + (uint64_t)J * l0.cap;
-        bool loaded = false;
-#if BPB200_TILE_BULK_LOAD
-        if (sizeof(T) == 4 && s0 >= 256) {
-            // staged over vals[1], inv[0] and the union-find words, which
-            // phase A fills only after the conversion below
-            __shared__ uint64_t bulk_bar;
-            uint32_t* stage = (uint32_t*)(smem + off[1]);
-            const uint32_t lead = tile_bulk_stage((const uint32_t*)in, s0, stage, &bulk_bar,
-                status);
-            if (lead == ~0u) {
-                return;
-            }
-            for (uint32_t i = tid; i < s0; i += blockDim.x) {
-                const uint32_t v = stage[lead + i];
-                if (v >= s0) {
-                    atomicOr(status, kErrNotPermutation);
-                    vals[0][i] = 0;
-                } else {
-                    vals[0][i] = (uint16_t)v;
-                }
-            }
-            loaded = true;
+        uint16_t* inv = invs[0];
+        const bool is_leaf = s0 <= leaf;
+        bool bad = false;
+        for (uint32_t e = tid; e < tile_pair_stride(l0.pcap); e += blockDim.x) {
+            reinterpret_cast<uint32_t*>(inv)[e] = ~0u;
         }
-#endif
-        // every load of a batch is issued before any is used: the error
-        // atomic below may alias the input as far as the compiler knows, so
-        // a plain loop would wait out one HBM round trip per element
+        __syncthreads();
+        // every load of a batch is issued before any is used
         constexpr int kBatch = 8;
-        for (uint32_t i0 = tid; !loaded && i0 < s0; i0 += kBatch * blockDim.x) {
+        for (uint32_t i0 = tid; i0 < s0; i0 += kBatch * blockDim.x) {
             uint64_t v[kBatch];
 #pragma unroll
             for (int q = 0; q < kBatch; ++q) {
@@ -187,218 +201,309 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
                     break;
                 }
                 if (v[q] >= s0) {
-                    atomicOr(status, kErrNotPermutation);
-                    vals[0][i] = 0;
+                    bad = true;
                 } else {
-                    vals[0][i] = (uint16_t)v[q];
+                    inv[is_leaf ? i : (uint32_t)v[q]] = (uint16_t)(is_leaf ? v[q] : i);
                 }
             }
         }
+        __syncthreads();
+        if (!is_leaf) {
+            for (uint32_t k = tid; k < s0 - s0 / 2; k += blockDim.x) {
+                const uint32_t both = reinterpret_cast<const uint32_t*>(inv)[k];
+                const uint32_t u = both & 0xffffu;
+                const uint32_t w = 2 * k + 1 < s0 ? both >> 16 : s0; // virtual partner
+                if (u >= s0 || (2 * k + 1 < s0 && w >= s0)) {
+                    bad = true;
+                } else {
+                    edge16[u] = (uint16_t)w;
+                    edge16[w] = (uint16_t)u;
+                }
+            }
+        }
+        if (__syncthreads_or(bad)) {
+            if (tid == 0) atomicOr(status, kErrNotPermutation);
+            return;
+        }
     }
-    __syncthreads();
 
     for (uint32_t t = 0;; ++t) {
         const uint32_t level = T0 + t;
         const LevelInfo& lv = plan.levels[level];
-        const uint32_t cap = (uint32_t)lv.cap;
-        const uint32_t pcap = (uint32_t)lv.pcap;
-        const FastDiv by_cap(cap), by_pcap(pcap);
         const uint32_t nodes = 1u << t;
         const uint32_t first = J << t;
-        uint16_t* cur = vals[t & 1];
-        uint16_t* nxt = vals[(t + 1) & 1];
-        uint16_t* inv = invs[t & 1];        // this level's inverse
-        uint16_t* child_inv = invs[(t + 1) & 1];
+        const uint32_t q32 = (uint32_t)lv.q;
+        const uint32_t r32 = (uint32_t)lv.r;
+        const uint32_t ps = tile_pair_stride(lv.pcap);
+        const uint32_t stride = 2 * ps;
+        const FastDiv by_ps(ps);
+        uint16_t* cur = invs[t & 1]; // this level's inverse (values, for leaves)
+        uint16_t* nxt = invs[(t + 1) & 1];
         // uniform per level: whether every node here exists / is internal
         const bool all_exist = level == 0 || plan.levels[level - 1].q > leaf;
-        const bool all_internal = lv.q > leaf && all_exist;
-        // node sizes: every node of a level without large nodes (r = 0, all
-        // levels of a power-of-two count) has q entries
-#if BPB200_TILE_UNIFORM
-        const uint32_t q32 = (uint32_t)lv.q;
-        const bool uniform = lv.r == 0;
-        auto node_size = [&](uint32_t node) {
-            return uniform ? q32 : size_at(lv, level, node);
+        const bool all_internal = q32 > leaf && all_exist;
+        auto node_size = [&](uint32_t path) {
+            // levels without large nodes (all of a power-of-two count): q
+            if (r32 == 0) return q32;
+            return q32 + ((__brev(first + path) >> (32 - level)) < r32 ? 1u : 0u);
         };
-#else
-        auto node_size = [&](uint32_t node) { return size_at(lv, level, node); };
-#endif
+        auto exists = [&](uint32_t path) {
+            return all_exist ||
+                size_at(plan.levels[level - 1], level - 1, (first + path) >> 1) > leaf;
+        };
         auto internal_node = [&](uint32_t path, uint32_t s) {
-            if (all_internal) return true;
-            if (s <= leaf) return false;
-            return all_exist || size_at(plan.levels[level - 1], level - 1, (first + path) >> 1) > leaf;
+            return all_internal || (s > leaf && exists(path));
         };
 
+        // key(w) = (w + bias) mod 2^16 (see the top of this file)
+        auto key_bias = [](uint32_t s) { return (s & 1u) != 0 ? 0u - (s - 1u) : 0u; };
+
         if (level < D) {
-            if (t == 0 && T0 == 0) {
-                // the whole permutation is in this tile: mark inverse slots so
-                // duplicates show up as never-written entries
-                for (uint32_t e = tid; e < cap; e += blockDim.x) {
-                    inv[e] = 0xffffu;
+            // ---- input switch bits: the colour of input 2k of every pair-node
+            if (ps <= kTileSerialPairs) {
+                for (uint32_t e = tid; e < (nodes * ps + 31) / 32 + 1; e += blockDim.x) xbits[e] = 0;
+                __syncthreads();
+                for (uint32_t path = tid; path < nodes; path += blockDim.x) {
+                    const uint32_t s = node_size(path);
+                    if (!internal_node(path, s)) {
+                        continue;
+                    }
+                    const uint32_t at = path * ps;
+                    uint64_t x;
+                    if (ps <= 32) {
+                        x = tile_colour_node<uint32_t>(edge + at, s);
+                    } else {
+                        x = tile_colour_node<uint64_t>(edge + at, s);
+                    }
+                    const uint32_t sh = at & 31;
+                    const uint64_t lo = x << sh;
+                    uint32_t* word = xbits + (at >> 5);
+                    if ((uint32_t)lo != 0) atomicOr(word, (uint32_t)lo);
+                    if ((lo >> 32) != 0) atomicOr(word + 1, (uint32_t)(lo >> 32));
+                    if (sh != 0 && (x >> (64 - sh)) != 0) {
+                        atomicOr(word + 2, (uint32_t)(x >> (64 - sh)));
+                    }
+                }
+            } else {
+                // Ruler walks.  One pair-node in 8 (at a hashed position) is
+                // a ruler; a thread walks both directions away from it until
+                // each meets a ruler or a pair-node stamped by a walk coming
+                // the other way, so every pair-node is passed about once.  A
+                // passed pair-node's edge word becomes the stamp 0x8000 |
+                // ruler << 1 | (direction ^ side of entry): each pair-node
+                // needs its edges once only.  Rulers are stamped first, as
+                // passed by their own direction 0.  A walk that enters a
+                // stamped pair-node at input w goes on as directed ruler
+                // stamp ^ (w & 1); two walks crossing may both stamp the
+                // pair-nodes where they cross, with stamps that say the same.
+                const uint32_t rulers = (nodes * ps + (1u << kTileRulerLog2) - 1) >> kTileRulerLog2;
+                const uint32_t edge_addr = smem_addr(edge);
+                for (uint32_t r = tid; r < rulers; r += blockDim.x) {
+                    const uint32_t at = (r << kTileRulerLog2) +
+                        ((r * 0x9E3779B1u) >> (32 - kTileRulerLog2));
+                    const uint32_t path = by_ps(at);
+                    const uint32_t s = path < nodes ? node_size(path) : 0;
+                    const bool real = at - path * ps < s - s / 2 && internal_node(path, s);
+                    state[2 * r] = real ? edge[at] : 0x80000000u; // no input index: padding
+                    if (real) edge16[2 * at] = (uint16_t)(0x8000u | (r << 1));
                 }
                 __syncthreads();
-            }
-            // A (first tile level only; every later level's inverse and
-            // union-find roots come from its parent's phase E0): inverse
-            // and union-find init
-            for (uint32_t e = tid; t == 0 && e < nodes * cap; e += blockDim.x) {
-                const uint32_t path = by_cap(e);
-                const uint32_t i = e - path * cap;
-                const uint32_t s = node_size(first + path);
-                if (i >= s || !internal_node(path, s)) {
-                    continue;
+                for (uint32_t r = tid; r < rulers; r += blockDim.x) {
+                    const uint32_t mine = state[2 * r];
+                    if (mine == 0x80000000u) {
+                        state[2 * r] = 0xffff0000u | (2 * r);
+                        state[2 * r + 1] = 0xffff0000u | (2 * r + 1);
+                        continue;
+                    }
+                    const uint32_t at = (r << kTileRulerLog2) +
+                        ((r * 0x9E3779B1u) >> (32 - kTileRulerLog2));
+                    const uint32_t path = by_ps(at);
+                    const uint32_t base = path * ps;
+                    const uint32_t bias = key_bias(node_size(path));
+                    const uint32_t v0 = 2 * (at - base);
+                    // both walks advance together, two loads in flight
+                    uint32_t wa = mine >> 16, wb = mine & 0xffffu;
+                    uint32_t ma = (v0 + bias) & 0xffffu, mb = (v0 + 1 + bias) & 0xffffu;
+                    const uint32_t mark = 0x8000u | (r << 1);
+                    const uint32_t at0 = edge_addr + 4 * base;
+                    uint32_t pa, pb; // 0 while the walk goes on
+                    uint32_t qa, qb;
+                    do {
+                        qa = at0 + ((wa << 1) & ~3u);
+                        qb = at0 + ((wb << 1) & ~3u);
+                        const uint32_t va = shared_load(qa), vb = shared_load(qb);
+                        pa = va & 0x8000u;
+                        pb = vb & 0x8000u;
+                        shared_store16_if(pa == 0, qa, mark | (wa & 1u));
+                        shared_store16_if(pb == 0, qb, mark | (~wb & 1u));
+                        ma = pa == 0 ? min(ma, (wa + bias) & 0xffffu) : ma;
+                        mb = pb == 0 ? min(mb, (wb + bias) & 0xffffu) : mb;
+                        wa = pa == 0 ? (va >> ((~wa & 1u) << 4)) & 0xffffu : wa;
+                        wb = pb == 0 ? (vb >> ((~wb & 1u) << 4)) & 0xffffu : wb;
+                    } while ((pa & pb) == 0);
+                    // the stamps the walks ended at are still there: stamps
+                    // are only ever replaced by ones that say the same
+                    const uint32_t na = (shared_load(qa) & 0x7fffu) ^ (wa & 1u);
+                    const uint32_t nb = (shared_load(qb) & 0x7fffu) ^ (wb & 1u);
+                    const uint32_t m = min(ma, mb ^ 1u);
+                    state[2 * r] = (m << 16) | na;
+                    state[2 * r + 1] = ((m ^ 1u) << 16) | nb;
                 }
-                if ((i & 1u) == 0) { // every pair-node is a root, whatever its values
-                    const uint32_t id = path * pcap + (i >> 1);
-                    uf[id] = id << 1;
+                __syncthreads();
+                // Each directed ruler state holds the smallest key of the
+                // stretch up to `next` (both half-walks of every ruler in
+                // it): three hops a round at least quadruple the stretch.
+                // States change in place: a state read early or late is a
+                // shorter or a longer stretch, both true.
+                for (uint32_t reach = 1; reach < (ps >> kTileRulerLog2) + 2; reach *= 4) {
+                    for (uint32_t i = tid; i < 2 * rulers; i += blockDim.x) {
+                        uint32_t me = vstate[i];
+#pragma unroll
+                        for (uint32_t hop = 0; hop < 3; ++hop) {
+                            const uint32_t far = vstate[me & 0xffffu];
+                            me = (min(me, far) & 0xffff0000u) | (far & 0xffffu);
+                        }
+                        vstate[i] = me;
+                    }
+                    __syncthreads();
                 }
-                const uint32_t v = cur[e];
-                if (v >= s) {
-                    atomicOr(status, kErrNotPermutation);
-                    continue;
+                const uint32_t total = nodes * ps;
+                for (uint32_t base = warp * 32; base < total; base += nwarps * 32) {
+                    const uint32_t q = base + lane;
+                    const uint32_t v = q < total ? edge[q] : 0x8000u;
+                    // padding pair-nodes hold anything: their bits are
+                    // never used, but the ruler must stay in range
+                    uint32_t x = (state[min(v & 0x7ffeu, 2 * rulers - 2)] >> 16) ^ v;
+                    if ((v & 0x8000u) == 0) { // a cycle without rulers, or padding
+                        const uint32_t path = by_ps(q);
+                        const uint32_t k = q - path * ps;
+                        const uint32_t s = node_size(path);
+                        if (k < s - s / 2 && internal_node(path, s)) {
+                            const uint32_t bias = key_bias(s);
+                            uint32_t w = 2 * k, word = v;
+                            x = ~0u; // the smallest key: walk the cycle whole
+                            for (uint32_t step = 0; step < ps; ++step) {
+                                x = min(x, (w + bias) & 0xffffu);
+                                w = (w & 1u) != 0 ? word & 0xffffu : word >> 16;
+                                if (w == 2 * k) break;
+                                word = edge[path * ps + (w >> 1)];
+                            }
+                        }
+                    }
+                    const unsigned word = __ballot_sync(0xffffffffu, (x & 1u) != 0);
+                    if (lane == 0) {
+                        xbits[base >> 5] = word;
+                    }
                 }
-                inv[path * cap + v] = (uint16_t)i;
             }
             __syncthreads();
-            // B: one union per output pair.  Consecutive threads take the
-            // same pair of consecutive nodes, so the unions running at once
-            // spread over all nodes of the level instead of crowding one
-            // node's few roots (with 16 nodes of 256 pair-nodes, node-major
-            // order ran all 256 unions of a node at once; tile time at 2^30
-            // entries 157 -> 145 ms).
-            for (uint32_t idx = tid; idx < nodes * pcap; idx += blockDim.x) {
-                const uint32_t path = idx & (nodes - 1);
-                const uint32_t k = idx >> t;
-                const uint32_t s = node_size(first + path);
-                if (k >= s / 2 || !internal_node(path, s)) {
-                    continue;
-                }
-                const uint32_t u = inv[path * cap + 2 * k];
-                const uint32_t w = inv[path * cap + 2 * k + 1];
-                if (u >= s || w >= s) {
-                    atomicOr(status, kErrNotPermutation);
-                    continue;
-                }
-                const uint32_t base = path * pcap;
-                uf_union(uf, base + (u >> 1), base + (w >> 1), 1u ^ (u & 1u) ^ (w & 1u), status);
-            }
-            __syncthreads();
-            // C: orient odd nodes so the unpaired tail gets colour 0
-            for (uint32_t path = tid; path < nodes; path += blockDim.x) {
-                const uint32_t s = node_size(first + path);
-                if ((s & 1u) == 0 || !internal_node(path, s)) {
-                    continue;
-                }
-                if (inv[path * cap + s - 1] >= s) {
-                    atomicOr(status, kErrNotPermutation);
-                    continue;
-                }
-                const Found f = uf_find(uf, path * pcap + (s >> 1), status);
-                if (f.bit) {
-                    atomicOr(uf + f.root, 1u);
-                }
-            }
-            __syncthreads();
-            // D: colours, child scatter
-            const uint32_t ccap = (uint32_t)plan.levels[level + 1].cap;
-            const uint32_t ptotal = nodes * pcap;
-            for (uint32_t base = warp * 32; base < ptotal; base += nwarps * 32) {
-                const uint32_t p = base + lane;
-                uint32_t x = 0;
-                if (p < ptotal) {
-                    const uint32_t path = by_pcap(p);
-                    const uint32_t k = p - path * pcap;
-                    const uint32_t s = node_size(first + path);
-                    if (k < s - s / 2 && internal_node(path, s)) {
-                        const Found f = uf_find(uf, p, status);
-                        x = f.bit ^ (uf_load(uf, f.root) & 1u);
-                        const uint32_t node = path * cap;
+            // ---- output switch bits, and the children: output pair k's
+            // colour-0 input inv[2k + y] goes left with value k, the other
+            // right (as level_outputs does for the global levels).  A thread
+            // takes two output pairs, which make one output pair of each
+            // child: it writes that pair of the children's inverses and both
+            // of its edges, or a leaf child's values.
+            {
+                const LevelInfo& cl = plan.levels[level + 1];
+                const uint32_t cstride = 2 * tile_pair_stride(cl.pcap);
+                const uint32_t hs = ps / 2;
+                const FastDiv by_hs(hs);
+                const uint32_t total = nodes * hs;
+                for (uint32_t base = warp * 32; base < total; base += nwarps * 32) {
+                    const uint32_t idx = base + lane;
+                    bool y[2] = {false, false};
+                    if (idx < total) {
+                        const uint32_t path = by_hs(idx);
+                        const uint32_t k0 = 2 * (idx - path * hs);
+                        const uint32_t s = node_size(path);
                         const uint32_t half = s / 2;
-                        if (k < half) {
-                            nxt[2 * path * ccap + k] = (uint16_t)(cur[node + 2 * k + x] >> 1);
-                            nxt[(2 * path + 1) * ccap + k] = (uint16_t)(cur[node + 2 * k + 1 - x] >> 1);
-                        } else {
-                            nxt[2 * path * ccap + k] = (uint16_t)(cur[node + s - 1] >> 1);
+                        const uint32_t sl = s - half;
+                        if (k0 < sl && internal_node(path, s)) {
+                            const uint2 four = *reinterpret_cast<const uint2*>(cur + path * stride + 2 * k0);
+                            uint32_t left[2], right[2];
+#pragma unroll
+                            for (uint32_t i = 0; i < 2; ++i) {
+                                const uint32_t both = i == 0 ? four.x : four.y;
+                                const uint32_t u = both & 0xffffu;
+                                if (k0 + i < half) {
+                                    const uint32_t q = path * ps + (u >> 1);
+                                    y[i] = (((xbits[q >> 5] >> (q & 31)) ^ u) & 1u) != 0;
+                                }
+                                // the odd tail output (k = half) goes left: y stays 0
+                                left[i] = (y[i] ? both >> 16 : u) >> 1;
+                                right[i] = (y[i] ? u : both >> 16) >> 1;
+                            }
+                            auto child = [&](uint32_t cpath, uint32_t cs, const uint32_t (&v)[2]) {
+                                if (k0 >= cs) return;
+                                uint16_t* to = nxt + cpath * cstride;
+                                const bool two = k0 + 1 < cs;
+                                if (cs > leaf) {
+                                    const uint32_t w = two ? v[1] : cs; // virtual partner
+                                    *reinterpret_cast<uint32_t*>(to + k0) = v[0] | (w << 16);
+                                    edge16[cpath * cstride + v[0]] = (uint16_t)w;
+                                    edge16[cpath * cstride + w] = (uint16_t)v[0];
+                                } else {
+                                    to[v[0]] = (uint16_t)k0;
+                                    if (two) to[v[1]] = (uint16_t)(k0 + 1);
+                                }
+                            };
+                            child(2 * path, sl, left);
+                            child(2 * path + 1, half, right);
                         }
                     }
-                }
-                const unsigned word = __ballot_sync(0xffffffffu, x != 0);
-                if (lane == 0) {
-                    xbits[base >> 5] = word;
-                }
-            }
-            __syncthreads();
-            // E0: output switch bits in natural order, and the children's
-            // inverse and union-find roots (as level_outputs does for the
-            // global levels: output pair k's colour-0 input inv[2k + y]
-            // goes left with value k, the other right)
-            const uint32_t ccpcap = (uint32_t)plan.levels[level + 1].pcap;
-            for (uint32_t base = warp * 32; base < ptotal; base += nwarps * 32) {
-                const uint32_t p = base + lane;
-                bool y = false;
-                if (p < ptotal) {
-                    const uint32_t path = by_pcap(p);
-                    const uint32_t k = p - path * pcap;
-                    const uint32_t s = node_size(first + path);
-                    const uint32_t half = s / 2;
-                    if (k <= half && internal_node(path, s)) {
-                        const uint32_t lb = 2 * path * ccap;
-                        const uint32_t rb = lb + ccap;
-                        if (k < half) {
-                            const uint32_t u = inv[path * cap + 2 * k];
-                            const uint32_t w = inv[path * cap + 2 * k + 1];
-                            uint16_t to_left = 0xffffu, to_right = 0xffffu;
-                            if (u < s && w < s) { // an unwritten slot (repeated value) holds anything
-                                const uint32_t q = path * pcap + (u >> 1);
-                                y = (((xbits[q >> 5] >> (q & 31)) ^ u) & 1u) != 0;
-                                to_left = (uint16_t)((y ? w : u) >> 1);
-                                to_right = (uint16_t)((y ? u : w) >> 1);
-                            }
-                            child_inv[lb + k] = to_left;
-                            child_inv[rb + k] = to_right;
-                        } else if ((s & 1u) != 0) {
-                            const uint32_t u = inv[path * cap + s - 1];
-                            child_inv[lb + half] = u < s ? (uint16_t)(u >> 1) : (uint16_t)0xffffu;
-                        }
-                        if ((k & 1u) == 0) {
-                            if (k < s - half) {
-                                const uint32_t id = 2 * path * ccpcap + (k >> 1);
-                                uf[id] = id << 1;
-                            }
-                            if (k < half) {
-                                const uint32_t id = (2 * path + 1) * ccpcap + (k >> 1);
-                                uf[id] = id << 1;
-                            }
-                        }
+                    // lane i holds bits 2i and 2i + 1 of the 64 from 2 * base
+                    const uint32_t two = ((y[0] ? 1u : 0u) | (y[1] ? 2u : 0u)) << (2 * (lane & 15));
+                    const uint32_t low = __reduce_or_sync(0xffffffffu, lane < 16 ? two : 0u);
+                    const uint32_t high = __reduce_or_sync(0xffffffffu, lane < 16 ? 0u : two);
+                    if (lane < 2) {
+                        ybits[(base >> 4) + lane] = lane == 0 ? low : high;
                     }
                 }
-                const unsigned word = __ballot_sync(0xffffffffu, y);
-                if (lane == 0) {
-                    ybits[base >> 5] = word;
-                }
             }
-            __syncthreads();
-            // E: switch bits, packet-major over a wave of node descriptors
+            // ---- switch bits out, packet-major over a wave of node addresses
             const uint32_t wave_log2 = t < kNodeWaveLog2 ? t : kNodeWaveLog2; // log2(min(nodes, kNodeWave))
             const uint32_t wn = 1u << wave_log2;
             for (uint32_t w0 = 0; w0 < nodes; w0 += wn) {
                 for (uint32_t e = tid; e < 2 * wn; e += blockDim.x) {
                     const uint32_t slot = e >> 1;
                     const int side = (int)(e & 1);
-                    const uint32_t node = first + w0 + slot;
-                    const uint32_t s = node_size(node);
+                    const uint32_t s = node_size(w0 + slot);
                     if (internal_node(w0 + slot, s)) {
-                        desc[side * kNodeWave + slot] = node_address(plan, side, level, node);
+                        const NodeAddress a = node_address(plan, side, level, first + w0 + slot);
+                        const GroupInfo& gi = plan.groups[side][lv.side[side].group];
+                        const bool large = a.packet_bits == gi.packet_bits[1] &&
+                            gi.packet_bits[0] != gi.packet_bits[1];
+                        const uint64_t at = plan.section_offset[side] * 8 + a.base;
+                        desc[side * kNodeWave + slot] = TileAddress{
+                            (at + a.full_prefix) | (large ? kTileRootLarge : 0ull),
+                            at + a.tail_prefix};
                     }
                 }
                 __syncthreads();
                 for (int side = 0; side < 2; ++side) {
                     const LevelSide& ls = lv.side[side];
-                    const uint32_t span_log2 = plan.groups[side][ls.group].depth - ls.rel - 1;
+                    const GroupInfo& gi = plan.groups[side][ls.group];
+                    const uint32_t span_log2 = gi.depth - ls.rel - 1;
                     const uint32_t shift = wave_log2 + span_log2;
-                    const uint32_t packets = (cap / 2 + (1u << span_log2) - 1) >> span_log2;
+                    const uint32_t packets =
+                        ((uint32_t)lv.cap / 2 + (1u << span_log2) - 1) >> span_log2;
                     const uint32_t* bits = side == 0 ? xbits : ybits;
-                    const uint64_t sec = plan.section_offset[side] * 8;
+                    const uint64_t packet_bits[2] = {gi.packet_bits[0], gi.packet_bits[1]};
+                    // blob bit of switch `pair` of a node with `half` switches
+                    auto bit_of = [&](uint32_t slot, uint32_t pair, uint32_t half) {
+                        const TileAddress& a = desc[side * kNodeWave + slot];
+                        const uint32_t packet = pair >> span_log2;
+                        const uint64_t full = a.full;
+                        return (packet == (half - 1) >> span_log2 ? a.tail : full & ~kTileRootLarge) +
+                            packet * packet_bits[full >> 63] + (pair & ((1u << span_log2) - 1));
+                    };
+                    auto put = [&](uint64_t dest, uint32_t v) {
+                        const uint32_t sh = (uint32_t)(dest & 31);
+                        atomicOr(blob + (dest >> 5), v << sh);
+                        if (sh != 0 && (v >> (32 - sh)) != 0) {
+                            atomicOr(blob + (dest >> 5) + 1, v >> (32 - sh));
+                        }
+                    };
                     if (span_log2 >= 5) {
                         // runs of at least 32 switches: word-wise copies as in
                         // level_emit_words (the bit arrays keep a spare word)
@@ -412,24 +517,17 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
                             const uint32_t pair0 =
                                 (packet << span_log2) + ((rem & ((1u << cshift) - 1)) << 5);
                             const uint32_t path = w0 + slot;
-                            const uint32_t s = node_size(first + path);
+                            const uint32_t s = node_size(path);
                             if (pair0 >= s / 2 || !internal_node(path, s)) {
                                 continue;
                             }
-                            const uint32_t q = path * pcap + pair0;
+                            const uint32_t q = path * ps + pair0;
                             uint32_t v = __funnelshift_r(bits[q >> 5], bits[(q >> 5) + 1], q & 31);
                             if (s / 2 - pair0 < 32) {
                                 v &= (1u << (s / 2 - pair0)) - 1u;
                             }
-                            if (v == 0) {
-                                continue;
-                            }
-                            const uint64_t dest =
-                                sec + switch_bit(desc[side * kNodeWave + slot], pair0);
-                            const uint32_t off = (uint32_t)(dest & 31);
-                            atomicOr(blob + (dest >> 5), v << off);
-                            if (off != 0 && (v >> (32 - off)) != 0) {
-                                atomicOr(blob + (dest >> 5) + 1, v >> (32 - off));
+                            if (v != 0) {
+                                put(bit_of(slot, pair0, s / 2), v);
                             }
                         }
                         continue;
@@ -437,8 +535,8 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
                     // short runs: the packets every node fills go out as
                     // word blocks (see level_emit_blocks), the rest bit by bit
                     uint32_t full = 0;
-                    if (all_internal && lv.q / 2 >= 1) {
-                        full = (uint32_t)(((lv.q / 2) - 1) >> span_log2);
+                    if (all_internal && q32 / 2 >= 1) {
+                        full = ((q32 / 2) - 1) >> span_log2;
                     }
                     if (full > packets) {
                         full = packets;
@@ -457,21 +555,14 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
                             const uint32_t slot0 = (c & ((1u << groups_log2) - 1)) << g_log2;
                             uint32_t v = 0;
                             for (uint32_t i = 0; i < (1u << g_log2); ++i) {
-                                const uint32_t q = (w0 + slot0 + i) * pcap + (packet << span_log2);
+                                const uint32_t q = (w0 + slot0 + i) * ps + (packet << span_log2);
                                 const uint32_t field =
                                     __funnelshift_r(bits[q >> 5], bits[(q >> 5) + 1], q & 31) &
                                     span_mask;
                                 v |= field << (i << span_log2);
                             }
-                            if (v == 0) {
-                                continue;
-                            }
-                            const uint64_t dest = sec +
-                                switch_bit(desc[side * kNodeWave + slot0], packet << span_log2);
-                            const uint32_t off = (uint32_t)(dest & 31);
-                            atomicOr(blob + (dest >> 5), v << off);
-                            if (off != 0 && (v >> (32 - off)) != 0) {
-                                atomicOr(blob + (dest >> 5) + 1, v >> (32 - off));
+                            if (v != 0) { // below every node's tail packet
+                                put(bit_of(slot0, packet << span_log2, node_size(w0 + slot0) / 2), v);
                             }
                         }
                     }
@@ -486,12 +577,12 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
                             const uint32_t slot = rem >> span_log2;
                             const uint32_t pair = (packet << span_log2) + (rem & ((1u << span_log2) - 1));
                             const uint32_t path = w0 + slot;
-                            const uint32_t s = node_size(first + path);
+                            const uint32_t s = node_size(path);
                             if (pair < s / 2 && internal_node(path, s)) {
-                                const uint32_t q = path * pcap + pair;
+                                const uint32_t q = path * ps + pair;
                                 set = ((bits[q >> 5] >> (q & 31)) & 1u) != 0;
                                 if (set) {
-                                    dest = sec + switch_bit(desc[side * kNodeWave + slot], pair);
+                                    dest = bit_of(slot, pair, s / 2);
                                 }
                             }
                         }
@@ -504,19 +595,16 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
 
         // leaves at this level (all of level D, and the size-`leaf` nodes of a
         // mixed level D - 1): one thread per leaf (see thread_factoradic_rank)
-        if (lv.q <= leaf) {
+        if (q32 <= leaf) {
             for (uint32_t path = tid; path < nodes; path += blockDim.x) {
-                const uint32_t node = first + path;
-                const uint32_t s = node_size(node);
-                const bool exists = all_exist ||
-                    size_at(plan.levels[level - 1], level - 1, node >> 1) > leaf;
-                if (s > leaf || !exists) {
+                const uint32_t s = node_size(path);
+                if (s > leaf || !exists(path)) {
                     continue;
                 }
                 int section = 0;
-                const uint64_t bit = leaf_rank_bit(plan, level, node, &section);
+                const uint64_t bit = leaf_rank_bit(plan, level, first + path, &section);
                 bool valid = true;
-                const U128 rank = thread_factoradic_rank(cur + path * cap, s, &valid);
+                const U128 rank = thread_factoradic_rank(cur + path * stride, s, &valid);
                 if (!valid) {
                     atomicOr(status, kErrNotPermutation);
                     continue;
@@ -535,12 +623,12 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
 template <typename T>
 __global__ void __launch_bounds__(kTileThreads, 2) tile_encode(const Plan* __restrict__ plan,
     const T* __restrict__ src, uint32_t* __restrict__ blob, uint32_t* status, uint32_t slots,
-    uint32_t pairs, uint32_t part_first) {
+    uint32_t part_first) {
     extern __shared__ __align__(16) unsigned char smem[];
     // a sharded call encodes only its own tiles (level_nodes); a launch may
     // cover a part of them, from tile part_first on
     const uint32_t first = (uint32_t)level_nodes(*plan, plan->tile_level).lo + part_first;
-    tile_body<T>(plan, src, blob, status, slots, pairs, first + blockIdx.x, smem);
+    tile_body<T>(plan, src, blob, status, slots, first + blockIdx.x, smem);
 }
 
 // Tiles too large for two CTAs per SM (nodes of 16384 entries, up to about
@@ -549,10 +637,10 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_encode(const Plan* __res
 template <typename T>
 __global__ void __launch_bounds__(2 * kTileThreads, 1) tile_encode_wide(
     const Plan* __restrict__ plan, const T* __restrict__ src, uint32_t* __restrict__ blob,
-    uint32_t* status, uint32_t slots, uint32_t pairs, uint32_t part_first) {
+    uint32_t* status, uint32_t slots, uint32_t part_first) {
     extern __shared__ __align__(16) unsigned char smem[];
     const uint32_t first = (uint32_t)level_nodes(*plan, plan->tile_level).lo + part_first;
-    tile_body<T>(plan, src, blob, status, slots, pairs, first + blockIdx.x, smem);
+    tile_body<T>(plan, src, blob, status, slots, first + blockIdx.x, smem);
 }
 
 // Tiles of many permutations in one launch (the batched and serving forms):
@@ -567,7 +655,7 @@ struct TileJob {
     uint32_t* blob;
     uint32_t* status;
     uint32_t slots;
-    uint32_t pairs;
+    uint32_t pad_;
     uint32_t first_block;
     uint32_t tiles;
     uint32_t blob_words;   // words to clear (single-tile jobs)
@@ -593,7 +681,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_encode_batch(
         if (threadIdx.x == 0) *job.status = 0;
         __syncthreads();
     }
-    tile_body<T>(job.plan, (const T*)job.src, job.blob, job.status, job.slots, job.pairs,
+    tile_body<T>(job.plan, (const T*)job.src, job.blob, job.status, job.slots,
         blockIdx.x - job.first_block, smem);
 }
 

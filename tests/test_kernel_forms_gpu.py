@@ -24,3 +24,15 @@ def test_middle_group_ranks(gpu, oracle, n, placement):
     at 20 entries; ranks start at every bit offset of a word."""
     for m in (4, 5):
         check(gpu, oracle, n, 7 * n + m, middle_group_log2=m, middle_placement=placement)
+
+
+@pytest.mark.parametrize("n", [34, 63, 64, 65, 66, 127, 128, 129, 130, 131, 255, 257, 258, 259,
+                               1023, 1025, 2049, 4097, 8191, 8192])
+def test_tile_nodes(gpu, oracle, n):
+    """Odd and even nodes around the one-thread colouring's limits (32 and 64
+    pair-nodes) and around the ruler walks' buckets, random and structured."""
+    kinds = gpu.PermutationKind
+    for m in (1, 2, 5):
+        for kind in (kinds.uniform, kinds.single_cycle, kinds.identity, kinds.reverse):
+            check(gpu, oracle, n, n + m, kind, np.uint64 if m == 2 else np.uint32,
+                  middle_group_log2=m)
