@@ -27,48 +27,42 @@
 namespace bpb200 {
 
 enum BatchKind : int {
-    kBReset = 0,
+    kBInit = 0,
     kBInverse,
-    kBDescriptors,
+    kBEdges,
     kBWalk,
-    kBWalkShort,
-    kBSuperWalk,
-    kBSuperShort,
-    kBJumpBlock,
-    kBJump,
-    kBCheck,
-    kBColour,
+    kBRank,
+    kBColours,
     kBUnion,
     kBOrient,
-    kBFinalize,
+    kBRoots,
     kBOutputs,
-    kBatchKinds
+    kBContract,                         // list e -> e + 1: kBContract + e - 1
+    kBExpand = kBContract + kMaxLists,  // list e + 1 -> e: kBExpand + e - 1
+    kBatchKinds = kBExpand + kMaxLists
 };
 
 // One permutation at one routing level of a batched launch sequence.
 struct LevelJob {
     const Plan* plan;
-    const void* src;         // this level's values (the caller's input at level 0)
-    uint32_t* dst;           // children's values
+    const void* src;         // level 0: the caller's input
     uint32_t* inv;           // this level's inverse
-    uint32_t* child_inv;     // children's inverse (null when the children are tiles)
-    uint32_t* owner;
-    uint32_t* uf;
+    uint32_t* child_inv;     // children's inverse
+    uint32_t* edge;          // edges, or union-find words, of this level and then the next
     uint32_t* xbits;
     uint32_t* ybits;
-    uint4* state;            // ruler states
-    uint4* sstate;           // super-ruler states: two buffers of `supers`
-    uint32_t* super_of;
-    uint32_t* control;       // the permutation's per-level control words
+    uint4* state[kMaxLists + 1];
+    uint32_t* mark[kMaxLists + 1];
+    uint8_t* colour[kMaxLists + 1];
+    uint32_t* control;       // the level's control words
     uint32_t* status;
     NodeAddress* addr[2];
-    uint32_t* blob;          // level 0 only: the blob whose header the reset writes
+    uint32_t* blob;          // level 0: the blob whose header is written
     uint32_t level;
-    uint32_t src_bytes;      // 8 only at level 0 of a uint64 input
-    uint32_t buckets;        // rulers
-    uint32_t supers;         // super-rulers
-    uint32_t rounds;         // jumping rounds (multi-launch form)
-    uint32_t force_union_find;
+    uint32_t src_bytes;
+    uint32_t top;            // list that list_rank colours
+    uint32_t walks;          // 1: coloured by walks, 0: by union-find
+    uint32_t child_walks;    // the next global level: 1 walks, 0 union-find, 2 none
     uint32_t header_bytes;   // level 0 only
     uint8_t header[84];
     uint32_t first[kBatchKinds];
@@ -132,114 +126,77 @@ __global__ void __launch_bounds__(256) batch_fill(const FillJob* jobs, uint32_t 
     }
 }
 
-// Control words of the level; at level 0 also the status word and the
-// blob header (after the blob was cleared by batch_fill).
-__global__ void __launch_bounds__(32) batch_reset(const LevelJob* jobs, uint32_t n) {
+// Status word, blob header (after the blob was cleared by batch_fill) and
+// switch addresses of every level.
+__global__ void __launch_bounds__(256) batch_init(const LevelJob* jobs, uint32_t n) {
     Grid g;
-    const LevelJob* j = level_job(jobs, n, kBReset, &g);
+    const LevelJob* j = level_job(jobs, n, kBInit, &g);
     if (g.bid >= g.nblk) return;
-    control_reset_run(g, j->control, j->force_union_find);
-    if (j->blob != nullptr) {
+    if (g.bid == 0) {
         if (threadIdx.x == 0) *j->status = 0;
         uint8_t* b = reinterpret_cast<uint8_t*>(j->blob);
         for (uint32_t i = threadIdx.x; i < j->header_bytes; i += blockDim.x) b[i] = j->header[i];
     }
+    level_descriptors_run(g, j->plan, j->addr[0], j->addr[1]);
 }
 
 __global__ void __launch_bounds__(256) batch_inverse(const LevelJob* jobs, uint32_t n) {
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBInverse, &g);
     if (g.bid >= g.nblk) return;
+    uint32_t* uf = j->walks ? nullptr : j->edge;
+    uint32_t* claims = j->control + kCtlClaimInverse;
     if (j->src_bytes == 8) {
-        level_inverse_run<uint64_t>(g, j->plan, j->level, (const uint64_t*)j->src, j->inv, j->uf,
-            j->owner, j->control + kCtlClaimInverse, j->status);
+        level_inverse_run<uint64_t>(g, j->plan, (const uint64_t*)j->src, j->inv, uf, claims, j->status);
     } else {
-        level_inverse_run<uint32_t>(g, j->plan, j->level, (const uint32_t*)j->src, j->inv, j->uf,
-            j->owner, j->control + kCtlClaimInverse, j->status);
+        level_inverse_run<uint32_t>(g, j->plan, (const uint32_t*)j->src, j->inv, uf, claims, j->status);
     }
 }
 
-__global__ void __launch_bounds__(256) batch_descriptors(const LevelJob* jobs, uint32_t n) {
+__global__ void __launch_bounds__(256) batch_edges(const LevelJob* jobs, uint32_t n) {
     Grid g;
-    const LevelJob* j = level_job(jobs, n, kBDescriptors, &g);
+    const LevelJob* j = level_job(jobs, n, kBEdges, &g);
     if (g.bid >= g.nblk) return;
-    level_descriptors_run(g, j->plan, j->level, j->addr[0], j->addr[1]);
+    level_edges_run(g, j->plan, j->inv, j->edge, j->status);
 }
 
 __global__ void __launch_bounds__(256) batch_walk(const LevelJob* jobs, uint32_t n) {
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBWalk, &g);
     if (g.bid >= g.nblk) return;
-    if (j->src_bytes == 8) {
-        level_walk_run<uint64_t>(g, j->plan, j->level, (const uint64_t*)j->src, j->inv, j->owner,
-            j->state, j->control);
-    } else {
-        level_walk_run<uint32_t>(g, j->plan, j->level, (const uint32_t*)j->src, j->inv, j->owner,
-            j->state, j->control);
-    }
+    level_walk_run(g, j->plan, j->level, j->edge, j->state[1], j->mark[1], j->status);
 }
 
-__global__ void __launch_bounds__(256) batch_walk_short(const LevelJob* jobs, uint32_t n) {
+__global__ void __launch_bounds__(256) batch_contract(const LevelJob* jobs, uint32_t n, uint32_t e) {
     Grid g;
-    const LevelJob* j = level_job(jobs, n, kBWalkShort, &g);
+    const LevelJob* j = level_job(jobs, n, kBContract + (int)e - 1, &g);
     if (g.bid >= g.nblk) return;
-    if (j->src_bytes == 8) {
-        level_walk_short_run<uint64_t>(g, j->plan, j->level, (const uint64_t*)j->src, j->inv,
-            j->owner, j->control);
-    } else {
-        level_walk_short_run<uint32_t>(g, j->plan, j->level, (const uint32_t*)j->src, j->inv,
-            j->owner, j->control);
-    }
+    list_contract_run(g, j->plan, j->level, e, j->state[e], j->mark[e], j->state[e + 1],
+        j->mark[e + 1], j->status);
 }
 
-__global__ void __launch_bounds__(256) batch_super_walk(const LevelJob* jobs, uint32_t n) {
+__global__ void __launch_bounds__(kRankThreads, 1) batch_rank(const LevelJob* jobs, uint32_t n) {
+    extern __shared__ __align__(16) uint32_t rank_shared[];
     Grid g;
-    const LevelJob* j = level_job(jobs, n, kBSuperWalk, &g);
+    const LevelJob* j = level_job(jobs, n, kBRank, &g);
     if (g.bid >= g.nblk) return;
-    ruler_super_walk_run(g, j->state, 0u, j->buckets, j->sstate, j->super_of, j->control);
+    list_rank_run(g, j->plan, j->level, j->top, j->state[j->top], j->colour[j->top], j->status,
+        rank_shared);
 }
 
-__global__ void __launch_bounds__(256) batch_super_short(const LevelJob* jobs, uint32_t n) {
+__global__ void __launch_bounds__(256) batch_expand(const LevelJob* jobs, uint32_t n, uint32_t e) {
     Grid g;
-    const LevelJob* j = level_job(jobs, n, kBSuperShort, &g);
+    const LevelJob* j = level_job(jobs, n, kBExpand + (int)e - 1, &g);
     if (g.bid >= g.nblk) return;
-    ruler_super_short_run(g, j->state, 0u, j->buckets, j->super_of, j->control);
+    list_expand_run(g, j->plan, j->level, e, j->state[e], j->mark[e], j->colour[e + 1],
+        j->colour[e], j->status);
 }
 
-__global__ void __launch_bounds__(kJumpBlockThreads, 1) batch_jump_block(const LevelJob* jobs,
-    uint32_t n) {
+__global__ void __launch_bounds__(256) batch_colours(const LevelJob* jobs, uint32_t n) {
     Grid g;
-    const LevelJob* j = level_job(jobs, n, kBJumpBlock, &g);
+    const LevelJob* j = level_job(jobs, n, kBColours, &g);
     if (g.bid >= g.nblk) return;
-    ruler_jump_block_run(g, j->sstate, j->sstate + j->supers, 0u, j->supers, j->rounds,
-        j->control);
-}
-
-__global__ void __launch_bounds__(256) batch_jump(const LevelJob* jobs, uint32_t n,
-    uint32_t round) {
-    Grid g;
-    const LevelJob* j = level_job(jobs, n, kBJump, &g);
-    if (g.bid >= g.nblk || round > j->rounds) return;
-    uint4* s0 = j->sstate;
-    uint4* s1 = j->sstate + j->supers;
-    ruler_jump_run(g, (round & 1u) ? s1 : s0, (round & 1u) ? s0 : s1, 0u, j->supers, round,
-        j->control);
-}
-
-__global__ void __launch_bounds__(32) batch_check(const LevelJob* jobs, uint32_t n,
-    uint32_t round) {
-    Grid g;
-    const LevelJob* j = level_job(jobs, n, kBCheck, &g);
-    if (g.bid >= g.nblk || round > j->rounds || threadIdx.x != 0) return;
-    ruler_check_run(g, round, j->control);
-}
-
-__global__ void __launch_bounds__(256) batch_colour(const LevelJob* jobs, uint32_t n) {
-    Grid g;
-    const LevelJob* j = level_job(jobs, n, kBColour, &g);
-    if (g.bid >= g.nblk) return;
-    ruler_colour_run(g, 0u, j->buckets, j->super_of, j->sstate, j->sstate + j->supers,
-        j->control);
+    level_colours_run(g, j->plan, j->level, j->edge, j->colour[1], j->xbits, j->status);
 }
 
 __global__ void __launch_bounds__(256, BPB200_UNION_MIN_BLOCKS) batch_union(const LevelJob* jobs,
@@ -247,45 +204,30 @@ __global__ void __launch_bounds__(256, BPB200_UNION_MIN_BLOCKS) batch_union(cons
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBUnion, &g);
     if (g.bid >= g.nblk) return;
-    level_union_run(g, j->plan, j->level, j->inv, j->uf, j->control + kCtlHard,
-        j->control + kCtlClaimUnion, j->status);
+    level_union_run(g, j->plan, j->level, j->inv, j->edge, j->control + kCtlClaimUnion, j->status);
 }
 
 __global__ void __launch_bounds__(256) batch_orient(const LevelJob* jobs, uint32_t n) {
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBOrient, &g);
     if (g.bid >= g.nblk) return;
-    level_orient_run(g, j->plan, j->level, j->inv, j->uf, j->control + kCtlHard, j->status);
+    level_orient_run(g, j->plan, j->level, j->inv, j->edge, j->status);
 }
 
-// Resident blocks per SM of batch_finalize (its job lookup costs registers
-// that level_finalize does not need).
-#ifndef BPB200_BATCH_FINAL_MIN_BLOCKS
-#define BPB200_BATCH_FINAL_MIN_BLOCKS 4
-#endif
-
-__global__ void __launch_bounds__(256, BPB200_BATCH_FINAL_MIN_BLOCKS) batch_finalize(const LevelJob* jobs, uint32_t n) {
+__global__ void __launch_bounds__(256, 4) batch_roots(const LevelJob* jobs, uint32_t n) {
     Grid g;
-    const LevelJob* j = level_job(jobs, n, kBFinalize, &g);
+    const LevelJob* j = level_job(jobs, n, kBRoots, &g);
     if (g.bid >= g.nblk) return;
-    if (j->src_bytes == 8) {
-        level_finalize_run<uint64_t>(g, j->plan, j->level, (const uint64_t*)j->src, j->owner,
-            j->super_of, j->sstate, j->sstate + j->supers, j->uf, j->xbits, j->dst, j->control,
-            j->status);
-    } else {
-        level_finalize_run<uint32_t>(g, j->plan, j->level, (const uint32_t*)j->src, j->owner,
-            j->super_of, j->sstate, j->sstate + j->supers, j->uf, j->xbits, j->dst, j->control,
-            j->status);
-    }
+    level_roots_run(g, j->plan, j->level, j->edge, j->xbits, j->control + kCtlClaimRoots, j->status);
 }
 
 __global__ void __launch_bounds__(256) batch_outputs(const LevelJob* jobs, uint32_t n) {
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBOutputs, &g);
     if (g.bid >= g.nblk) return;
-    const bool global_child = j->child_inv != nullptr;
     level_outputs_run(g, j->plan, j->level, j->inv, j->xbits, j->ybits, j->child_inv,
-        global_child ? j->owner : nullptr, global_child ? j->uf : nullptr);
+        j->child_walks == 1 ? j->edge : nullptr, j->child_walks == 0 ? j->edge : nullptr,
+        j->control + kCtlClaimOutputs);
 }
 
 // Emission forms (kernels.cuh), one launch per form over every (permutation,

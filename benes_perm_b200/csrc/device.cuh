@@ -26,6 +26,7 @@ __device__ __forceinline__ Grid launch_grid() { return Grid{blockIdx.x, gridDim.
 constexpr uint32_t kErrNotPermutation = 1u;  // value out of range or duplicated
 constexpr uint32_t kErrIterationCap = 2u;    // a bounded retry loop gave up
 constexpr uint32_t kErrInconsistent = 4u;    // colouring constraint violated
+constexpr uint32_t kErrGaveUp = 8u;          // a walk ran too long: encode again with union-find
 
 // Retry bound for every lock-free loop; far above what a valid input needs.
 // Parents strictly decrease along every union-find chain (links go to the

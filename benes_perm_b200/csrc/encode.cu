@@ -71,6 +71,35 @@ void check(cudaError_t e, const char* what) {
 
 // ------------------------------------------------------------ workspace
 
+// Device arrays of the ruler lists 1..kMaxLists (walk.cuh); index 0 unused.
+struct WalkLists {
+    uint4* state[kMaxLists + 1] = {};
+    uint32_t* mark[kMaxLists + 1] = {};
+    uint8_t* colour[kMaxLists + 1] = {};
+};
+
+constexpr uint64_t up256(uint64_t x) { return (x + 255) & ~255ull; }
+
+// Elements of list e over `pairs` pair-nodes.
+constexpr uint64_t list_elements(uint64_t pairs, uint32_t e) {
+    return (pairs >> (kRulerLog2 * e)) + 2;
+}
+
+// Bytes of the lists over `pairs` pair-nodes; with `base`, places them there.
+constexpr uint64_t place_lists(uint64_t pairs, unsigned char* base, WalkLists* out) {
+    uint64_t at = 0;
+    for (uint32_t e = 1; e <= kMaxLists; ++e) {
+        const uint64_t n = list_elements(pairs, e);
+        if (out != nullptr) {
+            out->state[e] = reinterpret_cast<uint4*>(base + at);
+            out->mark[e] = reinterpret_cast<uint32_t*>(base + at + up256(n * 16));
+            out->colour[e] = reinterpret_cast<uint8_t*>(base + at + up256(n * 16) + up256(n * 4));
+        }
+        at += up256(n * 16) + up256(n * 4) + up256(n);
+    }
+    return at;
+}
+
 struct Workspace {
     int device = -1;
     cudaStream_t stream = nullptr;
@@ -83,16 +112,14 @@ struct Workspace {
     Plan* h_plan = nullptr;       // pinned staging for the plan upload
     uint32_t* d_status = nullptr;
     uint32_t* h_status = nullptr; // pinned
-    uint32_t* vals[2] = {nullptr, nullptr};
-    uint32_t* inv = nullptr;
-    uint32_t* inv2 = nullptr;     // next level's inverse (levels alternate the two)
-    uint32_t* uf = nullptr;
+    uint32_t* inv[2] = {nullptr, nullptr}; // levels alternate the two
+    uint32_t* edge = nullptr;              // output edges of a walk level, or a
+                                           // union-find level's words (one per pair-node)
     uint32_t* xbits = nullptr;
     uint32_t* ybits = nullptr;
-    uint32_t* owner = nullptr;             // ruler id stamped on each walked even vertex, per pair-node
-    uint4* state[2] = {nullptr, nullptr};  // ruler states; [1] holds the super-ruler states
-    uint32_t* super_of = nullptr;          // super-ruler (or stamped colour) of each ruler
-    uint32_t* control = nullptr;           // per-level control words (walk.cuh)
+    WalkLists lists;                       // ruler lists of the walk levels
+    void* lists_mem = nullptr;
+    uint32_t* control = nullptr;           // per-level control words
     uint2* records = nullptr;              // partitioned-inverse records (kernels.cuh)
     uint32_t* cursor = nullptr;            // fill level of each destination window
     NodeAddress* addr[2] = {nullptr, nullptr};
@@ -105,17 +132,15 @@ struct Workspace {
     bool busy = false;
 
     void release_scratch() {
-        for (void* p : {(void*)vals[0], (void*)vals[1], (void*)inv, (void*)inv2, (void*)uf,
-                 (void*)xbits,
-                 (void*)ybits, (void*)owner, (void*)state[0], (void*)state[1], (void*)super_of,
-                 (void*)control,
-                 (void*)records, (void*)cursor, (void*)addr[0], (void*)addr[1]}) {
+        for (void* p : {(void*)inv[0], (void*)inv[1], (void*)edge, (void*)xbits, (void*)ybits,
+                 lists_mem, (void*)control, (void*)records, (void*)cursor, (void*)addr[0],
+                 (void*)addr[1]}) {
             if (p) cudaFree(p);
         }
-        vals[0] = vals[1] = inv = inv2 = uf = xbits = ybits = owner = control = cursor = nullptr;
-        super_of = nullptr;
+        inv[0] = inv[1] = edge = xbits = ybits = control = cursor = nullptr;
+        lists = WalkLists();
+        lists_mem = nullptr;
         records = nullptr;
-        state[0] = state[1] = nullptr;
         addr[0] = addr[1] = nullptr;
         slot_cap = pair_cap = node_cap = 0;
     }
@@ -194,7 +219,7 @@ struct Lease {
 void ensure_scratch(Workspace& w, const Plan& p) {
     uint64_t slots = p.tile_level > 0 ? p.max_slots : 0;
     uint64_t pairs = p.tile_level > 0 ? p.max_pairs : 0;
-    uint64_t nodes = p.tile_level > 0 ? (1ull << (p.tile_level - 1)) : 0;
+    uint64_t nodes = p.tile_level > 0 ? (1ull << p.tile_level) : 0;
     const bool need_records = p.levels[0].cap > kWalkMaxNode;
     if (slots <= w.slot_cap && pairs <= w.pair_cap && nodes <= w.node_cap &&
         (w.records != nullptr || !need_records)) {
@@ -207,19 +232,14 @@ void ensure_scratch(Workspace& w, const Plan& p) {
     pairs = std::max(pairs, 2 * w.pair_cap);
     nodes = std::max(nodes, 2 * w.node_cap);
     w.release_scratch();
-    check(cudaMalloc(&w.vals[0], slots * 4), "cudaMalloc(level array)");
-    check(cudaMalloc(&w.vals[1], slots * 4), "cudaMalloc(level array)");
-    check(cudaMalloc(&w.inv, slots * 4), "cudaMalloc(inverse)");
-    check(cudaMalloc(&w.inv2, slots * 4), "cudaMalloc(inverse)");
-    check(cudaMalloc(&w.uf, pairs * 4), "cudaMalloc(union-find)");
-    check(cudaMalloc(&w.xbits, ((pairs + 31) / 32 + 1) * 4), "cudaMalloc(colour bits)");
-    check(cudaMalloc(&w.ybits, ((pairs + 31) / 32 + 1) * 4), "cudaMalloc(output bits)");
-    check(cudaMalloc(&w.owner, pairs * 4), "cudaMalloc(owners)"); // one per pair-node
-    const uint64_t buckets = (slots >> kRulerLog2) + 1;
-    check(cudaMalloc(&w.state[0], buckets * sizeof(uint4)), "cudaMalloc(ruler state)");
-    check(cudaMalloc(&w.state[1], buckets * sizeof(uint4)), "cudaMalloc(ruler state)");
-    check(cudaMalloc(&w.super_of, buckets * 4), "cudaMalloc(super rulers)");
-    check(cudaMalloc(&w.control, kCtlWords * 4), "cudaMalloc(control)");
+    check(cudaMalloc(&w.inv[0], slots * 4), "cudaMalloc(inverse)");
+    check(cudaMalloc(&w.inv[1], slots * 4), "cudaMalloc(inverse)");
+    check(cudaMalloc(&w.edge, slots * 4), "cudaMalloc(edges)");
+    check(cudaMalloc(&w.xbits, (pairs / 32 + 4) * 4), "cudaMalloc(colour bits)");
+    check(cudaMalloc(&w.ybits, (pairs / 32 + 4) * 4), "cudaMalloc(output bits)");
+    check(cudaMalloc(&w.lists_mem, place_lists(pairs, nullptr, nullptr)), "cudaMalloc(ruler lists)");
+    place_lists(pairs, (unsigned char*)w.lists_mem, &w.lists);
+    check(cudaMalloc(&w.control, kMaxLevels * kCtlWords * 4), "cudaMalloc(control)");
     if (p.levels[0].cap > kWalkMaxNode) {
         // only levels with nodes above L2 size use the partitioned inverse
         check(cudaMalloc(&w.records, slots * sizeof(uint2)), "cudaMalloc(records)");
@@ -293,7 +313,7 @@ void choose_tile(Plan& p, TileShape* shape, uint64_t tile_max = kTileMaxEntries)
     p.tile_level = t0;
     uint64_t slots = 0, pairs = 0;
     for (uint32_t l = 0; l <= t0; ++l) {
-        slots = std::max<uint64_t>(slots, (1ull << l) * p.levels[l].cap);
+        slots = std::max<uint64_t>(slots, (1ull << l) * 2 * p.levels[l].pcap);
         pairs = std::max<uint64_t>(pairs, (1ull << l) * p.levels[l].pcap);
     }
     p.max_slots = slots;
@@ -333,7 +353,7 @@ Tuning default_tuning() {
         const char* env = std::getenv("BPB200_WALK_BLOCKS_PER_SM");
         const int v = env ? std::atoi(env) : 4;
         return Tuning{(uint32_t)(v < 1 ? 1 : (v > 8 ? 8 : v)), BPB200_WALK_MAX_LOG2,
-            BPB200_JUMP_BLOCK_LOG2, 13};
+            kRankMaxLog2, 13};
     }();
     return t;
 }
@@ -533,12 +553,6 @@ void emission_launches(const Plan& p, uint32_t l, int side, F&& f) {
         grid_for((packets - std::min(packets, full)) << (nr.shift + span_log2), kLevelThreads));
 }
 
-// One global routing level: inverse (level 0 only; every later level's
-// inverse comes from its parent's output pass), orbit-walk colouring
-// (union-find only when the walks give up), children, then both sections'
-// switch bits and the children's inverses.  `inv` holds this level's
-// inverse; `child_inv` receives the next level's (null when the next level
-// is the tile's, which builds its own in shared memory).
 // Level 0's input still arriving from the host in parts: after wait(k) the
 // stream has waited for part k, and entries [0, ends[k]) are on the device.
 struct InputParts {
@@ -546,42 +560,62 @@ struct InputParts {
     std::function<void(uint32_t part)> wait;
 };
 
-template <typename TV>
+// How the elements of one walk level's nodes are ranked: lists 1..top are
+// built, list `top` by list_rank with `threads` and `smem`.
+struct RankShape {
+    uint32_t top;
+    uint32_t threads;
+    uint32_t smem;
+};
+
+RankShape rank_shape(const LevelInfo& lv, const Tuning& tune) {
+    const uint32_t limit = 1u << std::min(kRankMaxLog2, std::max(kRankMinLog2, tune.jump_block_log2));
+    RankShape r{1, 0, 0};
+    while (r.top < kMaxLists && list_node_max(lv.pcap, r.top) > limit) ++r.top;
+    const uint32_t count = list_node_max(lv.pcap, r.top);
+    r.threads = rank_threads(count);
+    r.smem = rank_smem(count);
+    return r;
+}
+
+// Whether a level is coloured by walks (else by union-find).
+bool walk_level(const LevelInfo& lv, const Tuning& tune, bool union_find_only) {
+    return lv.cap <= (1ull << tune.walk_max_log2) && !union_find_only;
+}
+
+int device_sms() {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
+void allow_smem(const void* kernel);
+
+// One global routing level: level 0 builds its inverse; then the colouring
+// (walks, or union-find for nodes above L2 size), and the output pass, which
+// writes the children; then both sections' switch bits.  `inv` holds this
+// level's inverse; `child_inv` receives the next level's.
+template <typename T>
 void run_level(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p, const Tuning& tune,
-    uint32_t l, const TV* src, uint32_t* dst, uint32_t* d_blob, uint32_t* inv,
-    uint32_t* child_inv, const InputParts* input = nullptr) {
+    uint32_t l, const T* src, uint32_t* d_blob, uint32_t* inv, uint32_t* child_inv,
+    bool union_find_only, const InputParts* input = nullptr) {
     const Plan* dp = w.d_plan;
     const LevelInfo& lv = p.levels[l];
-    // the whole level's extent (array layout), and this call's share of it
-    const uint64_t slots = lv.cap << l;
-    const uint32_t buckets = (uint32_t)((slots + (1u << kRulerLog2) - 1) >> kRulerLog2);
     const NodeRange nr = level_nodes(p, l);
-    const RulerRange rr = ruler_range(p, l);
-    const uint32_t slo = (rr.lo + (1u << kSuperLog2) - 1) >> kSuperLog2;
-    const uint32_t shi = (rr.hi + (1u << kSuperLog2) - 1) >> kSuperLog2;
-    const uint64_t prs = lv.pcap << nr.shift;
+    const uint64_t prs = lv.pcap << nr.shift; // this call's pair-nodes
+    const uint64_t pair_lo = nr.lo * lv.pcap;
     const uint64_t nodes = 1ull << nr.shift;
-    const uint32_t my_buckets = rr.hi - rr.lo;
-    const int gs = grid_for((slots + kInverseItems - 1) / kInverseItems, kLevelThreads);
-    const int gu = grid_for((prs + kUnionItems - 1) / kUnionItems, kLevelThreads);
-    const int gr = grid_for((prs + kResolveItems - 1) / kResolveItems, kLevelThreads);
     const int gp = grid_for(prs, kLevelThreads);
-    const int gn = grid_for(nodes, kLevelThreads);
-    const int gw = grid_for(my_buckets, kLevelThreads);
-    uint32_t* ctl = w.control;
-    // nodes whose arrays do not fit in L2 are coloured by union-find
-    // 0: walks where they pay; 1: union-find everywhere; 2: walks, then the
-    // union-find fallback as if they had given up (test hooks)
-    const int colouring = g_force_union_find.load();
-    const bool walks = lv.cap <= (1ull << tune.walk_max_log2) && colouring != 1;
-    control_reset<<<1, 32, 0, st>>>(ctl, walks ? 0u : 1u);
-    rec.launches += 1;
+    uint32_t* ctl = w.control + l * kCtlWords;
+    const bool walks = walk_level(lv, tune, union_find_only);
     if (l == 0 && lv.cap > kWalkMaxNode && w.records != nullptr) {
+        const uint64_t slots = lv.cap;
         const uint32_t windows = (uint32_t)((slots + (1ull << kPlaceLog2) - 1) >> kPlaceLog2);
         check(cudaMemsetAsync(w.cursor, 0, windows * 4, st), "cudaMemsetAsync(cursors)");
         auto bucket = [&](uint64_t lo, uint64_t hi) {
             const int gb = grid_for((hi - lo + kBucketItems - 1) / kBucketItems, kBucketThreads);
-            level_bucket<TV><<<gb, kBucketThreads, 0, st>>>(dp, l, src, w.records, w.cursor, w.uf,
+            level_bucket<T><<<gb, kBucketThreads, 0, st>>>(dp, l, src, w.records, w.cursor, w.edge,
                 w.d_status, lo, hi);
         };
         const uint32_t parts = input != nullptr ? (uint32_t)input->ends.size() : 0;
@@ -607,115 +641,92 @@ void run_level(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p, cons
             for (uint32_t k = 0; k < (uint32_t)input->ends.size(); ++k) input->wait(k);
         }
         rec.launch(kKindInverse, [&] {
-            level_inverse<TV><<<gs, kLevelThreads, 0, st>>>(dp, l, src, inv, w.uf, w.owner,
+            level_inverse<T><<<grid_for((lv.cap + kInverseItems - 1) / kInverseItems, kLevelThreads),
+                kLevelThreads, 0, st>>>(dp, src, inv, walks ? nullptr : w.edge,
                 ctl + kCtlClaimInverse, w.d_status);
         });
     }
-    rec.launch(kKindDescriptors, [&] {
-        level_descriptors<<<gn, kLevelThreads, 0, st>>>(dp, l, w.addr[0], w.addr[1]);
-    });
     if (walks) {
+        const RankShape shape = rank_shape(lv, tune);
+        const ListRange rr = list_range(pair_lo, pair_lo + prs, 1);
+        if (l == 0) {
+            rec.launch(kKindInverse, [&] {
+                level_edges<<<gp, kLevelThreads, 0, st>>>(dp, inv, w.edge, w.d_status);
+            });
+        }
         rec.launch(kKindWalk, [&] {
-            // persistent warps claiming ruler chunks in address order
-            int dev = 0, sms = 148;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            const uint64_t want = ((uint64_t)my_buckets + kWalkChunk - 1) / kWalkChunk * 32;
-            const int gwalk = (int)std::max<uint64_t>(1,
-                std::min<uint64_t>((uint64_t)sms * tune.walk_blocks_per_sm,
-                    (want + kLevelThreads - 1) / kLevelThreads));
-            level_walk<TV><<<gwalk, kLevelThreads, 0, st>>>(dp, l, src, inv, w.owner,
-                w.state[0], ctl);
-            level_walk_short<TV><<<gp, kLevelThreads, 0, st>>>(dp, l, src, inv, w.owner, ctl);
-        }, 2);
-        // super-rulers of one orbit lie in one node: at most
-        // (cap >> (kRulerLog2 + kSuperLog2)) + 2 of them
-        const uint32_t supers = (buckets + (1u << kSuperLog2) - 1) >> kSuperLog2;
-        uint32_t rounds = 1;
-        while ((1ull << rounds) < (lv.cap >> (kRulerLog2 + kSuperLog2)) + 2) {
-            ++rounds;
-        }
-        uint4* sstate[2] = {w.state[1], w.state[1] + supers};
-        // few super-rulers: every round in one CTA; otherwise one launch pair per round
-        const bool one_block = shi - slo <= (1u << tune.jump_block_log2);
+            level_walk<<<(rr.hi - rr.lo + kLevelThreads - 1) / kLevelThreads, kLevelThreads, 0,
+                st>>>(dp, l, w.edge, w.lists.state[1], w.lists.mark[1], w.d_status);
+        });
         rec.launch(kKindJump, [&] {
-            check(cudaMemsetAsync(w.super_of, 0xff, (uint64_t)buckets * 4, st),
-                "cudaMemsetAsync(super rulers)");
-            ruler_super_walk<<<grid_for(shi - slo, kLevelThreads), kLevelThreads, 0, st>>>(
-                w.state[0], rr.lo, rr.hi, sstate[0], w.super_of, ctl);
-            ruler_super_short<<<gw, kLevelThreads, 0, st>>>(w.state[0], rr.lo, rr.hi, w.super_of,
-                ctl);
-            if (one_block) {
-                ruler_jump_block<<<1, kJumpBlockThreads, 0, st>>>(sstate[0], sstate[1], slo, shi,
-                    rounds, ctl);
-            } else {
-                const int gj = grid_for(shi - slo, kLevelThreads);
-                for (uint32_t r = 0; r <= rounds; ++r) {
-                    ruler_jump<<<gj, kLevelThreads, 0, st>>>(sstate[r & 1], sstate[(r + 1) & 1],
-                        slo, shi, r, ctl);
-                    ruler_check<<<1, 1, 0, st>>>(r, ctl);
-                }
+            for (uint32_t e = 1; e < shape.top; ++e) {
+                const ListRange to = list_range(pair_lo, pair_lo + prs, e + 1);
+                list_contract<<<grid_for(2ull * (to.hi - to.lo), kLevelThreads), kLevelThreads, 0,
+                    st>>>(dp, l, e, w.lists.state[e], w.lists.mark[e], w.lists.state[e + 1],
+                    w.lists.mark[e + 1], w.d_status);
             }
-            ruler_colour<<<gw, kLevelThreads, 0, st>>>(rr.lo, rr.hi, w.super_of, sstate[0],
-                sstate[1], ctl);
-        }, one_block ? 4 : 3 + 2 * (rounds + 1));
-        if (colouring == 2) {
-            level_force_fallback<<<1, 1, 0, st>>>(ctl + kCtlHard);
-            rec.launches += 1;
-        }
+            allow_smem((const void*)list_rank);
+            list_rank<<<(unsigned)std::min<uint64_t>(nodes, 1u << 20), shape.threads, shape.smem,
+                st>>>(dp, l, shape.top, w.lists.state[shape.top], w.lists.colour[shape.top],
+                w.d_status);
+            for (uint32_t e = shape.top; e-- > 1;) {
+                const ListRange to = list_range(pair_lo, pair_lo + prs, e);
+                list_expand<<<grid_for(to.hi - to.lo, kLevelThreads), kLevelThreads, 0, st>>>(dp, l,
+                    e, w.lists.state[e], w.lists.mark[e], w.lists.colour[e + 1],
+                    w.lists.colour[e], w.d_status);
+            }
+        }, 2 * shape.top - 1);
+        rec.launch(kKindResolve, [&] {
+            level_colours<<<gp, kLevelThreads, 0, st>>>(dp, l, w.edge, w.lists.colour[1], w.xbits,
+                w.d_status);
+        });
+    } else {
+        rec.launch(kKindUnion, [&] {
+            level_union<<<grid_for((prs + kUnionItems - 1) / kUnionItems, kLevelThreads),
+                kLevelThreads, 0, st>>>(dp, l, inv, w.edge, ctl + kCtlClaimUnion, w.d_status);
+        });
+        rec.launch(kKindOrient, [&] {
+            level_orient<<<grid_for(nodes, kLevelThreads), kLevelThreads, 0, st>>>(dp, l, inv, w.edge,
+                w.d_status);
+        });
+        rec.launch(kKindResolve, [&] {
+            level_roots<<<grid_for((prs + kResolveItems - 1) / kResolveItems, kLevelThreads),
+                kLevelThreads, 0, st>>>(dp, l, w.edge, w.xbits, ctl + kCtlClaimRoots, w.d_status);
+        });
     }
-    // a walk level's union-find words are set up only if it falls back
-    const bool reset_uf = walks && l > 0;
-    rec.launch(kKindUnion, [&] {
-        if (reset_uf) {
-            level_uf_reset<<<gp, kLevelThreads, 0, st>>>(dp, l, w.uf, ctl + kCtlHard);
-        }
-        level_union<<<gu, kLevelThreads, 0, st>>>(dp, l, inv, w.uf, ctl + kCtlHard,
-            ctl + kCtlClaimUnion, w.d_status);
-    }, reset_uf ? 2 : 1);
-    rec.launch(kKindOrient, [&] {
-        level_orient<<<gn, kLevelThreads, 0, st>>>(dp, l, inv, w.uf, ctl + kCtlHard, w.d_status);
-    });
-    rec.launch(kKindResolve, [&] {
-        const uint32_t supers = (buckets + (1u << kSuperLog2) - 1) >> kSuperLog2;
-        level_finalize<TV><<<gr, kLevelThreads, 0, st>>>(dp, l, src, w.owner, w.super_of,
-            w.state[1], w.state[1] + supers, w.uf, w.xbits, dst, ctl, w.d_status);
-    });
     rec.launch(kKindOutputBits, [&] {
-        // the next level's walk owners start unset and its pair-nodes as
-        // roots; the tile level keeps its own state in shared memory
-        const bool global_child = child_inv != nullptr;
-        // owners only matter where the orbit walks run
-        const bool child_walks = global_child && p.levels[l + 1].cap <= (1ull << tune.walk_max_log2)
-            && colouring != 1;
-        // union-find roots only for children coloured by union-find; a walk
-        // child sets them up itself if it falls back (level_uf_reset)
-        level_outputs<<<gp, kLevelThreads, 0, st>>>(dp, l, inv, w.xbits, w.ybits, child_inv,
-            child_walks ? w.owner : nullptr, global_child && !child_walks ? w.uf : nullptr);
+        // the colours are all in xbits: the child level's edges or union-find
+        // words take the place of this level's; the tile builds its own
+        const bool global_child = l + 1 < p.tile_level;
+        const bool child_walks = global_child && walk_level(p.levels[l + 1], tune, union_find_only);
+        level_outputs<<<grid_for(prs / 2, kLevelThreads), kLevelThreads, 0, st>>>(dp, l, inv,
+            w.xbits, w.ybits, child_inv, child_walks ? w.edge : nullptr,
+            global_child && !child_walks ? w.edge : nullptr, ctl + kCtlClaimOutputs);
     });
     // above the shard level every shard computes the level, shard 0 alone
     // writes its switches
     const bool emit = p.shards <= 1 || l >= p.shard_level || p.shard == 0;
     for (int side = 0; side < 2 && emit; ++side) {
         const uint32_t* bits = side == 0 ? w.xbits : w.ybits;
+        const NodeAddress* addr = w.addr[side] + (1ull << l);
         emission_launches(p, l, side, [&](int form, uint64_t full, int blocks) {
             rec.launch(kKindEmit, [&] {
                 switch (form) {
                 case kEmitWords:
-                    level_emit_words<<<blocks, kLevelThreads, 0, st>>>(dp, l, side, bits,
-                        w.addr[side], d_blob);
+                    level_emit_words<<<blocks, kLevelThreads, 0, st>>>(dp, l, side, bits, addr,
+                        d_blob);
                     break;
                 case kEmitTranspose:
                     level_emit_transpose<<<blocks, kLevelThreads, 0, st>>>(dp, l, side, bits,
-                        w.addr[side], d_blob, full);
+                        addr, d_blob, full);
                     break;
                 case kEmitBlocks:
-                    level_emit_blocks<<<blocks, kLevelThreads, 0, st>>>(dp, l, side, bits,
-                        w.addr[side], d_blob, full);
+                    level_emit_blocks<<<blocks, kLevelThreads, 0, st>>>(dp, l, side, bits, addr,
+                        d_blob, full);
                     break;
                 default:
-                    level_emit<<<blocks, kLevelThreads, 0, st>>>(dp, l, side, bits, w.addr[side],
-                        d_blob, full);
+                    level_emit<<<blocks, kLevelThreads, 0, st>>>(dp, l, side, bits, addr, d_blob,
+                        full);
                     break;
                 }
             });
@@ -724,13 +735,13 @@ void run_level(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p, cons
     check(cudaGetLastError(), "level kernel launch");
 }
 
-// Raises a tile kernel's dynamic shared memory limit to the whole tile
+// Raises a kernel's dynamic shared memory limit to the whole shared-memory
 // budget, once per kernel and device.  Setting it per call to the call's own
 // size raced between concurrent callers: the limit is per function, and a
 // caller that lowered it between another caller's set and launch made that
 // launch fail ("too many resources requested").  The limit only bounds what
 // a launch may ask for; occupancy follows each launch's actual request.
-void allow_tile_smem(const void* kernel) {
+void allow_smem(const void* kernel) {
     static std::mutex m;
     static std::vector<std::pair<const void*, int>> done;
     int dev = 0;
@@ -758,32 +769,30 @@ struct TileParts {
 template <typename T>
 void launch_levels(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p,
     const TileShape& shape, const Tuning& tune, const T* d_in, uint32_t* d_blob,
-    const LevelHook* after_level = nullptr, const TileParts* parts = nullptr,
-    const InputParts* input = nullptr) {
+    bool union_find_only, const LevelHook* after_level = nullptr,
+    const TileParts* parts = nullptr, const InputParts* input = nullptr) {
     const Plan* dp = w.d_plan;
     const uint32_t t0 = p.tile_level;
     if (t0 > 0) {
         // level 0 validation: inverse slots start as 0xffffffff so a
         // duplicated value leaves a never-written slot behind
-        check(cudaMemsetAsync(w.inv, 0xff, p.levels[0].cap * 4, st), "cudaMemsetAsync");
+        check(cudaMemsetAsync(w.inv[0], 0xff, p.levels[0].cap * 4, st), "cudaMemsetAsync");
+        check(cudaMemsetAsync(w.control, 0, t0 * kCtlWords * 4, st), "cudaMemsetAsync(control)");
+        rec.launch(kKindDescriptors, [&] {
+            level_descriptors<<<grid_for(1ull << t0, kLevelThreads), kLevelThreads, 0, st>>>(dp,
+                w.addr[0], w.addr[1]);
+        });
     }
-    const uint32_t* cur32 = nullptr;
-    uint32_t* invs[2] = {w.inv, w.inv2};
     for (uint32_t l = 0; l < t0; ++l) {
         rec.level = (int)l;
-        uint32_t* dst = w.vals[l & 1];
-        uint32_t* child_inv = l + 1 < t0 ? invs[(l + 1) & 1] : nullptr;
-        if (l == 0) {
-            run_level<T>(w, rec, st, p, tune, l, d_in, dst, d_blob, invs[0], child_inv, input);
-        } else {
-            run_level<uint32_t>(w, rec, st, p, tune, l, cur32, dst, d_blob, invs[l & 1],
-                child_inv);
-        }
-        cur32 = dst;
+        uint32_t* inv = w.inv[l & 1];
+        uint32_t* child_inv = w.inv[(l + 1) & 1];
+        run_level<T>(w, rec, st, p, tune, l, d_in, d_blob, inv, child_inv, union_find_only, input);
         if (after_level != nullptr) {
             (*after_level)(l);
         }
     }
+    const uint32_t* tile_inv = w.inv[t0 & 1];
     if (t0 == 0 && input != nullptr) {
         // the tile reads the input directly: all of it first
         for (uint32_t k = 0; k < (uint32_t)input->ends.size(); ++k) input->wait(k);
@@ -796,7 +805,7 @@ void launch_levels(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p,
     const bool wide = shape.smem > kTileSmemTwoPerSm;
     const unsigned threads = tile_threads(tiles, wide);
     auto launch_tile = [&](auto kernel, const auto* src) {
-        allow_tile_smem((const void*)kernel);
+        allow_smem((const void*)kernel);
         uint64_t lo = 0;
         const size_t count = parts != nullptr ? parts->cuts.size() : 1;
         for (size_t k = 0; k < count; ++k) {
@@ -821,9 +830,9 @@ void launch_levels(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p,
         }
     } else {
         if (wide) {
-            launch_tile(tile_encode_wide<uint32_t>, cur32);
+            launch_tile(tile_encode_wide<uint32_t>, tile_inv);
         } else {
-            launch_tile(tile_encode<uint32_t>, cur32);
+            launch_tile(tile_encode<uint32_t>, tile_inv);
         }
     }
     check(cudaGetLastError(), "tile kernel launch");
@@ -928,11 +937,27 @@ thread_local std::vector<Recorder::Mark> t_marks;
 thread_local std::vector<double> t_mark_seconds;
 std::atomic<int> g_profiling{0};
 
-// Queues the whole encode on `st` and waits for it.
+// Return code of a finished encode's status word.
+int status_code(uint32_t status, char* err, size_t err_len) {
+    if (status & kErrNotPermutation) {
+        set_error(err, err_len, "input must contain every value from zero through size minus one");
+        return kInvalidArgument;
+    }
+    if (status & (kErrIterationCap | kErrInconsistent | kErrGaveUp)) {
+        set_error(err, err_len, "b200 device status reported a failed colouring");
+        return kRuntime;
+    }
+    return kOk;
+}
+
+// Queues the whole encode on `st` and waits for it.  When a walk gave up
+// (contrived inputs only), or the test hook asks for it, the permutation is
+// encoded a second time with union-find on every level; `again` (may be
+// null) then says so: what the hooks handed out earlier is stale.
 int run(Workspace& w, Call& call, cudaStream_t st, const void* d_in, uint32_t entry_bytes,
     uint32_t* d_blob, double* device_seconds, char* err, size_t err_len,
     const LevelHook* after_level = nullptr, const TileParts* parts = nullptr,
-    const InputParts* input = nullptr) {
+    const InputParts* input = nullptr, bool* again = nullptr) {
     const Plan& p = *call.plan;
     ensure_scratch(w, p);
     Recorder rec;
@@ -946,18 +971,33 @@ int run(Workspace& w, Call& call, cudaStream_t st, const void* d_in, uint32_t en
     h.bytes = p.shards > 1 && p.shard != 0 ? 0u : (uint32_t)call.layout.header_bytes;
     write_header(call.layout, h.data);
     check(cudaEventRecord(w.start, st), "cudaEventRecord");
-    check(cudaMemsetAsync(d_blob, 0, (p.end_offset + 3) / 4 * 4, st), "cudaMemsetAsync(blob)");
-    rec.launch(kKindPrologue, [&] { prologue<<<1, 128, 0, st>>>(w.d_status, d_blob, h); });
-    if (entry_bytes == 4) {
-        launch_levels<uint32_t>(w, rec, st, p, call.shape, call.tune, (const uint32_t*)d_in,
-            d_blob, after_level, parts, input);
-    } else {
-        launch_levels<uint64_t>(w, rec, st, p, call.shape, call.tune, (const uint64_t*)d_in,
-            d_blob, after_level, parts, input);
+    const int colouring = g_force_union_find.load();
+    bool union_find_only = colouring == 1;
+    uint32_t status = 0;
+    for (int pass = 0; pass < 2; ++pass) {
+        check(cudaMemsetAsync(d_blob, 0, (p.end_offset + 3) / 4 * 4, st), "cudaMemsetAsync(blob)");
+        rec.launch(kKindPrologue, [&] { prologue<<<1, 128, 0, st>>>(w.d_status, d_blob, h); });
+        if (entry_bytes == 4) {
+            launch_levels<uint32_t>(w, rec, st, p, call.shape, call.tune, (const uint32_t*)d_in,
+                d_blob, union_find_only, after_level, parts, input);
+        } else {
+            launch_levels<uint64_t>(w, rec, st, p, call.shape, call.tune, (const uint64_t*)d_in,
+                d_blob, union_find_only, after_level, parts, input);
+        }
+        check(cudaEventRecord(w.stop, st), "cudaEventRecord");
+        check(cudaMemcpyAsync(w.h_status, w.d_status, 4, cudaMemcpyDeviceToHost, st), "status");
+        check(cudaStreamSynchronize(st), "cudaStreamSynchronize");
+        status = *w.h_status;
+        if (union_find_only || p.tile_level == 0 ||
+            ((status & kErrGaveUp) == 0 && colouring != 2)) {
+            break;
+        }
+        union_find_only = true;
+        after_level = nullptr;
+        parts = nullptr;
+        input = nullptr; // all of it is on the device by now
+        if (again != nullptr) *again = true;
     }
-    check(cudaEventRecord(w.stop, st), "cudaEventRecord");
-    check(cudaMemcpyAsync(w.h_status, w.d_status, 4, cudaMemcpyDeviceToHost, st), "status");
-    check(cudaStreamSynchronize(st), "cudaStreamSynchronize");
     float ms = 0;
     check(cudaEventElapsedTime(&ms, w.start, w.stop), "cudaEventElapsedTime");
     if (device_seconds) {
@@ -969,16 +1009,7 @@ int run(Workspace& w, Call& call, cudaStream_t st, const void* d_in, uint32_t en
     }
     rec.collect(t_kernel_seconds, t_kernel_counts, &t_marks, &t_mark_seconds);
     t_launches = rec.launches;
-    const uint32_t status = *w.h_status;
-    if (status & kErrNotPermutation) {
-        set_error(err, err_len, "input must contain every value from zero through size minus one");
-        return kInvalidArgument;
-    }
-    if (status & (kErrIterationCap | kErrInconsistent)) {
-        set_error(err, err_len, "b200 device status reported a failed colouring");
-        return kRuntime;
-    }
-    return kOk;
+    return status_code(status, err, err_len);
 }
 
 // Whether the current device is an sm_100 part, cached per device: the
@@ -1430,9 +1461,10 @@ int compress_host(const void* entries, uint64_t count, uint32_t entry_bytes,
             hand_out(w.parts[k], to);
         }
     };
+    bool again = false;
     rc = run(w, call, w.stream, w.input, device_width, w.blob, device_seconds, err, err_len,
         early.levels ? &level_hook : nullptr, early.cuts.empty() ? nullptr : &parts,
-        overlap ? &input : nullptr);
+        overlap ? &input : nullptr, &again);
     if (uploader.joinable()) {
         uploader.join();
     }
@@ -1454,6 +1486,10 @@ int compress_host(const void* entries, uint64_t count, uint32_t entry_bytes,
     }
     if (helper_failed.load()) {
         throw CudaFail{cudaErrorUnknown, "staged blob download"};
+    }
+    if (again) { // the pieces handed out belong to the first attempt
+        done[0] = 0;
+        done[1] = call.plan->section_offset[1];
     }
     // the rest: the tail of each section and whatever follows the output
     // section (the separate middle section)
@@ -1706,24 +1742,18 @@ constexpr uint64_t kSlots = kMaxEntries + (1ull << 14); // level slots incl. pad
 constexpr uint64_t kPairs = kSlots / 2 + (1ull << 13);
 constexpr uint64_t kNodes = 1ull << 10;               // descriptors per global level
 
-constexpr size_t up256(size_t x) { return (x + 255) / 256 * 256; }
 constexpr size_t kOffPlan = 0;
 constexpr size_t kOffStatus = kOffPlan + up256(sizeof(Plan));
-constexpr size_t kOffVals0 = kOffStatus + 256;
-constexpr size_t kOffVals1 = kOffVals0 + up256(kSlots * 4);
-constexpr size_t kOffInv = kOffVals1 + up256(kSlots * 4);
+constexpr size_t kOffControl = kOffStatus + 256;
+constexpr size_t kOffInv = kOffControl + up256(kMaxLevels * kCtlWords * 4);
 constexpr size_t kOffInv2 = kOffInv + up256(kSlots * 4);
-constexpr size_t kOffUf = kOffInv2 + up256(kSlots * 4);
-constexpr size_t kOffXbits = kOffUf + up256(kPairs * 4);
-constexpr size_t kOffYbits = kOffXbits + up256((kPairs / 32 + 1) * 4);
-constexpr size_t kOffAddr0 = kOffYbits + up256((kPairs / 32 + 1) * 4);
+constexpr size_t kOffEdge = kOffInv2 + up256(kSlots * 4);
+constexpr size_t kOffXbits = kOffEdge + up256(kSlots * 4);
+constexpr size_t kOffYbits = kOffXbits + up256((kPairs / 32 + 4) * 4);
+constexpr size_t kOffAddr0 = kOffYbits + up256((kPairs / 32 + 4) * 4);
 constexpr size_t kOffAddr1 = kOffAddr0 + up256(kNodes * sizeof(NodeAddress));
-constexpr size_t kOffOwner = kOffAddr1 + up256(kNodes * sizeof(NodeAddress));
-constexpr size_t kOffState0 = kOffOwner + up256(kPairs * 4);
-constexpr size_t kOffState1 = kOffState0 + up256(((kSlots >> kRulerLog2) + 1) * sizeof(uint4));
-constexpr size_t kOffSuper = kOffState1 + up256(((kSlots >> kRulerLog2) + 1) * sizeof(uint4));
-constexpr size_t kOffControl = kOffSuper + up256(((kSlots >> kRulerLog2) + 1) * 4);
-constexpr size_t kBytes = kOffControl + 256; // under 8 MB
+constexpr size_t kOffLists = kOffAddr1 + up256(kNodes * sizeof(NodeAddress));
+constexpr size_t kBytes = kOffLists + place_lists(kPairs, nullptr, nullptr); // under 8 MB
 static_assert(kBytes < (8u << 20), "allocation-free scratch stays under 8 MB");
 
 } // namespace noalloc
@@ -1791,7 +1821,7 @@ extern "C" int bpb200_compress_device_noalloc(const void* d_entries, uint64_t co
             return rc;
         }
         const Plan& p = *call.plan;
-        const uint64_t nodes = p.tile_level > 0 ? (1ull << (p.tile_level - 1)) : 0;
+        const uint64_t nodes = p.tile_level > 0 ? (1ull << p.tile_level) : 0;
         if ((p.tile_level > 0 && (p.max_slots > noalloc::kSlots || p.max_pairs > noalloc::kPairs)) ||
             nodes > noalloc::kNodes) {
             set_error(err, err_len, "format needs more scratch than the allocation-free entry point holds");
@@ -1799,20 +1829,15 @@ extern "C" int bpb200_compress_device_noalloc(const void* d_entries, uint64_t co
         }
         w.d_plan = reinterpret_cast<Plan*>(base + noalloc::kOffPlan);
         w.d_status = reinterpret_cast<uint32_t*>(base + noalloc::kOffStatus);
-        w.vals[0] = reinterpret_cast<uint32_t*>(base + noalloc::kOffVals0);
-        w.vals[1] = reinterpret_cast<uint32_t*>(base + noalloc::kOffVals1);
-        w.inv = reinterpret_cast<uint32_t*>(base + noalloc::kOffInv);
-        w.inv2 = reinterpret_cast<uint32_t*>(base + noalloc::kOffInv2);
-        w.uf = reinterpret_cast<uint32_t*>(base + noalloc::kOffUf);
+        w.control = reinterpret_cast<uint32_t*>(base + noalloc::kOffControl);
+        w.inv[0] = reinterpret_cast<uint32_t*>(base + noalloc::kOffInv);
+        w.inv[1] = reinterpret_cast<uint32_t*>(base + noalloc::kOffInv2);
+        w.edge = reinterpret_cast<uint32_t*>(base + noalloc::kOffEdge);
         w.xbits = reinterpret_cast<uint32_t*>(base + noalloc::kOffXbits);
         w.ybits = reinterpret_cast<uint32_t*>(base + noalloc::kOffYbits);
         w.addr[0] = reinterpret_cast<NodeAddress*>(base + noalloc::kOffAddr0);
         w.addr[1] = reinterpret_cast<NodeAddress*>(base + noalloc::kOffAddr1);
-        w.owner = reinterpret_cast<uint32_t*>(base + noalloc::kOffOwner);
-        w.state[0] = reinterpret_cast<uint4*>(base + noalloc::kOffState0);
-        w.state[1] = reinterpret_cast<uint4*>(base + noalloc::kOffState1);
-        w.super_of = reinterpret_cast<uint32_t*>(base + noalloc::kOffSuper);
-        w.control = reinterpret_cast<uint32_t*>(base + noalloc::kOffControl);
+        place_lists(noalloc::kPairs, base + noalloc::kOffLists, &w.lists);
         cudaStream_t st = (cudaStream_t)stream;
         // The plan source is ordinary host memory: the copy is staged before
         // cudaMemcpyAsync returns, so g_plan can be reused by the next call.
@@ -1823,28 +1848,33 @@ extern "C" int bpb200_compress_device_noalloc(const void* d_entries, uint64_t co
         write_header(call.layout, h.data);
         // Everything that must start cleared is cleared by the call itself:
         // the blob (memset), the status word (prologue) and, when level
-        // kernels run, the inverse sentinels used for validation.
-        check(cudaMemsetAsync(d_blob, 0, (p.end_offset + 3) / 4 * 4, st), "cudaMemsetAsync(blob)");
-        Recorder rec; // timing disabled: no events are created
-        rec.st = st;
-        rec.launch(kKindPrologue, [&] { prologue<<<1, 128, 0, st>>>(w.d_status, (uint32_t*)d_blob, h); });
-        if (entry_bytes == 4) {
-            launch_levels<uint32_t>(w, rec, st, p, call.shape, call.tune, (const uint32_t*)d_entries,
-                (uint32_t*)d_blob);
-        } else {
-            launch_levels<uint64_t>(w, rec, st, p, call.shape, call.tune, (const uint64_t*)d_entries,
-                (uint32_t*)d_blob);
-        }
+        // kernels run, their counters and the inverse sentinels used for
+        // validation.  A second pass as in run().
+        const int colouring = g_force_union_find.load();
+        bool union_find_only = colouring == 1;
         uint32_t status = 0;
-        check(cudaMemcpyAsync(&status, w.d_status, 4, cudaMemcpyDeviceToHost, st), "status");
-        check(cudaStreamSynchronize(st), "cudaStreamSynchronize");
-        if (status & kErrNotPermutation) {
-            set_error(err, err_len, "input must contain every value from zero through size minus one");
-            return kInvalidArgument;
+        for (int pass = 0; pass < 2; ++pass) {
+            check(cudaMemsetAsync(d_blob, 0, (p.end_offset + 3) / 4 * 4, st), "cudaMemsetAsync(blob)");
+            Recorder rec; // timing disabled: no events are created
+            rec.st = st;
+            rec.launch(kKindPrologue, [&] { prologue<<<1, 128, 0, st>>>(w.d_status, (uint32_t*)d_blob, h); });
+            if (entry_bytes == 4) {
+                launch_levels<uint32_t>(w, rec, st, p, call.shape, call.tune,
+                    (const uint32_t*)d_entries, (uint32_t*)d_blob, union_find_only);
+            } else {
+                launch_levels<uint64_t>(w, rec, st, p, call.shape, call.tune,
+                    (const uint64_t*)d_entries, (uint32_t*)d_blob, union_find_only);
+            }
+            check(cudaMemcpyAsync(&status, w.d_status, 4, cudaMemcpyDeviceToHost, st), "status");
+            check(cudaStreamSynchronize(st), "cudaStreamSynchronize");
+            if (union_find_only || p.tile_level == 0 ||
+                ((status & kErrGaveUp) == 0 && colouring != 2)) {
+                break;
+            }
+            union_find_only = true;
         }
-        if (status & (kErrIterationCap | kErrInconsistent)) {
-            set_error(err, err_len, "b200 device status reported a failed colouring");
-            return kRuntime;
+        if (const int bad = status_code(status, err, err_len)) {
+            return bad;
         }
         return kOk;
     });

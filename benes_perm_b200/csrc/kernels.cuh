@@ -13,13 +13,13 @@
 //                pair-nodes: colour(u) != colour(w) becomes
 //                x(u/2) ^ x(w/2) = 1 ^ (u&1) ^ (w&1), x(k) = colour(2k)
 //   orient       odd nodes: flip the tail's component so the tail is colour 0
-//   finalize     (walk.cuh) x(k) = parity to the component minimum (the
-//                canonical colouring: each component's smallest vertex gets
-//                colour 0), or the orbit-walk colour on walk levels;
-//                children left[k] = p[2k+x]/2, right[k] = p[2k+1-x]/2; the
-//                input switch of pair k is x(k)
+//   roots        x(k) = parity to the component minimum (the canonical
+//                colouring: each component's smallest vertex gets colour
+//                0); the input switch of pair k is x(k).  Nodes that fit L2
+//                are coloured by walks instead (walk.cuh)
 //   outputs      output switch of output pair k is colour(inv[2k]); the
-//                children's inverses follow from the same two reads
+//                children's inverses follow from the same two reads (the
+//                values p are read at level 0 only)
 //   emit         switch bits into the clustered blob layout: word copies of
 //                long packet runs, word blocks of short ones, bits for the
 //                rest
@@ -57,12 +57,12 @@ constexpr int kInverseItems = BPB200_INVERSE_ITEMS; // slots per thread in level
 #define BPB200_UNION_MIN_BLOCKS 4
 #endif
 constexpr int kUnionItems = BPB200_UNION_ITEMS; // output pairs per thread in level_union
-// level_finalize shape: pair-nodes per thread (1, 2, 4 or 8; 32 / items lanes
+// level_roots shape: pair-nodes per thread (1, 2, 4 or 8; 32 / items lanes
 // assemble one colour word) and the minimum resident blocks of 256 per SM.
 // 2 pair-nodes at 8 blocks measured fastest on B200 at 2^30 uniform entries
-// (finalize 115 ms per compress; 2 at 6 blocks: 120; 4 at 6 blocks: 144;
-// 4 at the compiler's choice of 4 blocks: 134; 8: 286): the finds are
-// latency-bound, so more resident warps beat more finds per thread.
+// (115 ms per compress while the pass also moved values; 2 at 6 blocks: 120;
+// 4 at 6 blocks: 144; 8: 286): the finds are latency-bound, so more resident
+// warps beat more finds per thread.
 #ifndef BPB200_RESOLVE_ITEMS
 #define BPB200_RESOLVE_ITEMS 2
 #endif
@@ -71,7 +71,25 @@ constexpr int kUnionItems = BPB200_UNION_ITEMS; // output pairs per thread in le
 #endif
 constexpr int kResolveItems = BPB200_RESOLVE_ITEMS;
 static_assert(kResolveItems == 1 || kResolveItems == 2 || kResolveItems == 4 ||
-    kResolveItems == 8, "level_finalize assembles colour words from 1, 2, 4 or 8 bits per lane");
+    kResolveItems == 8, "level_roots assembles colour words from 1, 2, 4 or 8 bits per lane");
+// Levels whose nodes have at most 2^BPB200_FINAL_STRIDE_LOG2 entries resolve
+// in grid-stride order, larger ones in claimed order (see level_roots);
+// measured on B200 at 2^30 uniform entries (105 ms per compress with values;
+// limit 2^24: 110 ms; 2^23: 119 ms).
+#ifndef BPB200_FINAL_STRIDE_LOG2
+#define BPB200_FINAL_STRIDE_LOG2 26
+#endif
+
+// Control words of a level: work counters of its claiming kernels, zeroed
+// for every level at once before the first launch.
+enum : int {
+    kCtlClaimInverse = 0, // level_inverse
+    kCtlClaimPlace = 1,   // level_place
+    kCtlClaimUnion = 3,   // level_union
+    kCtlClaimRoots = 4,   // level_roots
+    kCtlClaimOutputs = 5, // level_outputs
+    kCtlWords = 8
+};
 
 struct TileShape {
     uint32_t slots;   // padded entry slots needed at the deepest level
@@ -86,23 +104,22 @@ __device__ __forceinline__ uint32_t size_at(const LevelInfo& lv, uint32_t level,
 
 // ------------------------------------------------------------ level kernels
 
+// Inverse of level 0: inv[p[i]] = i.  With `uf`, every pair-node also starts
+// as its own root, whatever its values: a stale word could point outside.
 template <typename T>
 __device__ __forceinline__ void level_inverse_run(Grid grid, const Plan* __restrict__ plan,
-    uint32_t level, const T* __restrict__ src, uint32_t* __restrict__ inv,
-    uint32_t* __restrict__ uf, uint32_t* __restrict__ owner, uint32_t* claims, uint32_t* status) {
-    const LevelInfo& lv = plan->levels[level];
-    const uint32_t cap = (uint32_t)lv.cap;
-    const uint32_t pcap = (uint32_t)lv.pcap;
-    const uint64_t total = (uint64_t)cap << level;
+    const T* __restrict__ src, uint32_t* __restrict__ inv, uint32_t* __restrict__ uf,
+    uint32_t* claims, uint32_t* status) {
+    const uint32_t s = (uint32_t)plan->levels[0].q;
     const bool aligned = ((uintptr_t)src & 15u) == 0;
     uint64_t first;
-    while (claim_chunk(claims, (uint64_t)blockDim.x * kInverseItems, total, &first)) {
+    while (claim_chunk(claims, (uint64_t)blockDim.x * kInverseItems, s, &first)) {
         const uint64_t e0 = first + (uint64_t)threadIdx.x * kInverseItems;
-        if (e0 >= total) {
+        if (e0 >= s) {
             continue;
         }
         T v[kInverseItems];
-        if (aligned && e0 + kInverseItems <= total) {
+        if (aligned && e0 + kInverseItems <= s) {
             constexpr int kVec = 16 / sizeof(T);
 #pragma unroll
             for (int q = 0; q < kInverseItems / kVec; ++q) {
@@ -114,33 +131,23 @@ __device__ __forceinline__ void level_inverse_run(Grid grid, const Plan* __restr
         } else {
 #pragma unroll
             for (int q = 0; q < kInverseItems; ++q) {
-                v[q] = e0 + q < total ? src[e0 + q] : (T)0;
+                v[q] = e0 + q < s ? src[e0 + q] : (T)0;
             }
         }
-        uint32_t j = (uint32_t)(e0 / cap);
-        uint32_t i = (uint32_t)(e0 - (uint64_t)j * cap);
-        uint32_t s = size_at(lv, level, j);
+        const uint32_t i0 = (uint32_t)e0;
 #pragma unroll
         for (int q = 0; q < kInverseItems; ++q) {
-            if (e0 + q < total && i < s) {
-                // every pair-node starts as its own root, whatever its values:
-                // a stale word could point outside the array; and unowned
-                if ((i & 1u) == 0) {
-                    const uint32_t id = j * pcap + (i >> 1);
-                    uf[id] = id << 1;
-                    owner[id] = ~0u;
+            if (e0 + q < s) {
+                const uint32_t i = i0 + q;
+                if (uf != nullptr && (i & 1u) == 0) {
+                    uf[i >> 1] = i & ~1u;
                 }
                 const uint64_t val = (uint64_t)v[q];
                 if (val >= s) {
                     atomicOr(status, kErrNotPermutation);
                 } else {
-                    inv[(uint64_t)j * cap + val] = i;
+                    inv[val] = i;
                 }
-            }
-            if (++i == cap) {
-                i = 0;
-                ++j;
-                s = size_at(lv, level, j);
             }
         }
     }
@@ -148,9 +155,9 @@ __device__ __forceinline__ void level_inverse_run(Grid grid, const Plan* __restr
 
 template <typename T>
 __global__ void __launch_bounds__(256) level_inverse(const Plan* __restrict__ plan,
-    uint32_t level, const T* __restrict__ src, uint32_t* __restrict__ inv,
-    uint32_t* __restrict__ uf, uint32_t* __restrict__ owner, uint32_t* claims, uint32_t* status) {
-    level_inverse_run<T>(launch_grid(), plan, level, src, inv, uf, owner, claims, status);
+    const T* __restrict__ src, uint32_t* __restrict__ inv, uint32_t* __restrict__ uf,
+    uint32_t* claims, uint32_t* status) {
+    level_inverse_run<T>(launch_grid(), plan, src, inv, uf, claims, status);
 }
 
 // ---------------------------------------------------------------------------
@@ -194,7 +201,7 @@ __device__ __forceinline__ void level_bucket_run(Grid grid, const Plan* __restri
     const LevelInfo& lv = plan->levels[level];
     const uint32_t cap = (uint32_t)lv.cap;
     const uint32_t pcap = (uint32_t)lv.pcap;
-    const uint64_t slots = (uint64_t)cap << level;
+    const uint64_t slots = cap;
     const uint64_t total = e_hi < slots ? e_hi : slots;
     const uint32_t windows = (uint32_t)((slots + (1ull << kPlaceLog2) - 1) >> kPlaceLog2);
     const uint64_t chunk = (uint64_t)blockDim.x * kBucketItems;
@@ -306,15 +313,10 @@ __global__ void __launch_bounds__(256) level_place(const Plan* __restrict__ plan
 // Blocks claim chunks of output pairs in address order (claim_chunk), so the
 // union-find words being linked at any time belong to the few nodes those
 // chunks cover: once a node's words fit in L2 the random finds hit there.
-// `hard` was written by earlier launches: all threads see the same value.
 __device__ __forceinline__ void level_union_run(Grid grid, const Plan* __restrict__ plan,
-    uint32_t level, const uint32_t* __restrict__ inv, uint32_t* uf, const uint32_t* hard,
-    uint32_t* claims, uint32_t* status) {
-    if (hard != nullptr && *hard == 0) {
-        return; // the orbit walks coloured this level
-    }
+    uint32_t level, const uint32_t* __restrict__ inv, uint32_t* uf, uint32_t* claims,
+    uint32_t* status) {
     const LevelInfo& lv = plan->levels[level];
-    const uint32_t cap = (uint32_t)lv.cap;
     const uint32_t pcap = (uint32_t)lv.pcap;
     const NodeRange nr = level_nodes(*plan, level);
     const uint64_t begin = nr.lo * pcap;
@@ -339,9 +341,9 @@ __device__ __forceinline__ void level_union_run(Grid grid, const Plan* __restric
         for (int q = 0; q < kUnionItems; ++q) {
             if (p0 + q < end && k < s / 2) {
                 pending |= 1u << q;
-                const uint64_t at = (uint64_t)j * cap + 2 * k;
-                u[q] = inv[at];
-                w[q] = inv[at + 1];
+                const uint2 both = *reinterpret_cast<const uint2*>(inv + 2 * ((uint64_t)j * pcap + k));
+                u[q] = both.x;
+                w[q] = both.y;
                 base[q] = j * pcap;
                 rel[q] = s; // stash the node size for the range check below
             }
@@ -369,42 +371,14 @@ __device__ __forceinline__ void level_union_run(Grid grid, const Plan* __restric
 }
 
 __global__ void __launch_bounds__(256, BPB200_UNION_MIN_BLOCKS) level_union(const Plan* __restrict__ plan,
-    uint32_t level, const uint32_t* __restrict__ inv, uint32_t* uf, const uint32_t* hard,
-    uint32_t* claims, uint32_t* status) {
-    level_union_run(launch_grid(), plan, level, inv, uf, hard, claims, status);
-}
-
-// Walk levels: their pair-nodes start as union-find roots only when the
-// walks gave up (the `hard` flag) and the level falls back to union-find;
-// the parent's output pass does not set them up for walk levels.
-__global__ void __launch_bounds__(256) level_uf_reset(const Plan* __restrict__ plan,
-    uint32_t level, uint32_t* __restrict__ uf, const uint32_t* hard) {
-    if (*hard == 0) {
-        return;
-    }
-    const LevelInfo& lv = plan->levels[level];
-    const NodeRange nr = level_nodes(*plan, level);
-    const uint64_t lo = nr.lo * lv.pcap;
-    const uint64_t hi = lo + (lv.pcap << nr.shift);
-    for (uint64_t id = lo + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; id < hi;
-         id += (uint64_t)gridDim.x * blockDim.x) {
-        uf[id] = (uint32_t)id << 1;
-    }
-}
-
-// Test hook: the walks of the level ran, but the level is coloured by the
-// union-find fallback anyway, as if a walk had given up.
-__global__ void level_force_fallback(uint32_t* hard) {
-    *hard = 1;
+    uint32_t level, const uint32_t* __restrict__ inv, uint32_t* uf, uint32_t* claims,
+    uint32_t* status) {
+    level_union_run(launch_grid(), plan, level, inv, uf, claims, status);
 }
 
 __device__ __forceinline__ void level_orient_run(Grid grid, const Plan* __restrict__ plan, uint32_t level,
-    const uint32_t* __restrict__ inv, uint32_t* uf, const uint32_t* hard, uint32_t* status) {
-    if (hard != nullptr && *hard == 0) {
-        return;
-    }
+    const uint32_t* __restrict__ inv, uint32_t* uf, uint32_t* status) {
     const LevelInfo& lv = plan->levels[level];
-    const uint32_t cap = (uint32_t)lv.cap;
     const uint32_t pcap = (uint32_t)lv.pcap;
     const NodeRange nr = level_nodes(*plan, level);
     const uint64_t nodes_end = nr.lo + (1ull << nr.shift);
@@ -414,7 +388,7 @@ __device__ __forceinline__ void level_orient_run(Grid grid, const Plan* __restri
         if ((s & 1u) == 0) {
             continue;
         }
-        if (inv[j * cap + s - 1] >= s) {
+        if (inv[2 * j * pcap + s - 1] >= s) {
             atomicOr(status, kErrNotPermutation);
             continue;
         }
@@ -426,112 +400,216 @@ __device__ __forceinline__ void level_orient_run(Grid grid, const Plan* __restri
 }
 
 __global__ void level_orient(const Plan* __restrict__ plan, uint32_t level,
-    const uint32_t* __restrict__ inv, uint32_t* uf, const uint32_t* hard, uint32_t* status) {
-    level_orient_run(launch_grid(), plan, level, inv, uf, hard, status);
+    const uint32_t* __restrict__ inv, uint32_t* uf, uint32_t* status) {
+    level_orient_run(launch_grid(), plan, level, inv, uf, status);
 }
 
-__device__ __forceinline__ void level_descriptors_run(Grid grid, const Plan* __restrict__ plan, uint32_t level,
+// Switch addresses of every node of the levels above the tile's: level l's
+// nodes start at element 2^l of in_addr / out_addr.
+__device__ __forceinline__ void level_descriptors_run(Grid grid, const Plan* __restrict__ plan,
     NodeAddress* __restrict__ in_addr, NodeAddress* __restrict__ out_addr) {
-    const NodeRange nr = level_nodes(*plan, level);
-    const uint64_t nodes_end = nr.lo + (1ull << nr.shift);
-    for (uint64_t j = nr.lo + (uint64_t)grid.bid * blockDim.x + threadIdx.x; j < nodes_end;
-         j += (uint64_t)grid.nblk * blockDim.x) {
-        in_addr[j] = node_address(*plan, 0, level, j);
-        out_addr[j] = node_address(*plan, 1, level, j);
+    const uint64_t end = 1ull << plan->tile_level;
+    for (uint64_t i = 1 + (uint64_t)grid.bid * blockDim.x + threadIdx.x; i < end;
+         i += (uint64_t)grid.nblk * blockDim.x) {
+        const uint32_t level = high_bit(i);
+        const uint64_t j = i - (1ull << level);
+        const NodeRange nr = level_nodes(*plan, level);
+        if (j >= nr.lo && j < nr.lo + (1ull << nr.shift)) {
+            in_addr[i] = node_address(*plan, 0, level, j);
+            out_addr[i] = node_address(*plan, 1, level, j);
+        }
     }
 }
 
-__global__ void level_descriptors(const Plan* __restrict__ plan, uint32_t level,
+__global__ void __launch_bounds__(256) level_descriptors(const Plan* __restrict__ plan,
     NodeAddress* __restrict__ in_addr, NodeAddress* __restrict__ out_addr) {
-    level_descriptors_run(launch_grid(), plan, level, in_addr, out_addr);
+    level_descriptors_run(launch_grid(), plan, in_addr, out_addr);
+}
+
+// Input switch bits of a union-find level: bit k = colour of input 2k = the
+// pair-node's parity to its root, flipped by the root's orientation flag;
+// kResolveItems pair-nodes per thread.
+__device__ __forceinline__ void level_roots_run(Grid grid, const Plan* __restrict__ plan,
+    uint32_t level, uint32_t* uf, uint32_t* __restrict__ xbits, uint32_t* claims,
+    uint32_t* status) {
+    const LevelInfo& lv = plan->levels[level];
+    const uint32_t pcap = (uint32_t)lv.pcap;
+    // this call's pair-nodes [lo_pair, end); chunks start at a 32-pair
+    // boundary at or below lo_pair so colour words are written whole
+    const NodeRange nr = level_nodes(*plan, level);
+    const uint64_t lo_pair = nr.lo * pcap;
+    const uint64_t end = lo_pair + ((uint64_t)pcap << nr.shift);
+    const uint64_t begin = lo_pair & ~31ull;
+    const uint64_t total = end - begin;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t chunk = (uint64_t)blockDim.x * kResolveItems;
+    // Levels with nodes far above L2 size claim chunks in order (the finds of
+    // neighbouring chunks share the top of their trees).  With nodes near L2
+    // size, claimed chunks would crowd every find in flight onto the root
+    // chains of one or two nodes' large components, which then serialise:
+    // those stride over the whole level (at 2^30 uniform entries, claimed
+    // order took 18.5 -> 12.5 ms on the 2^30-slot level but 14 -> 19 ms on
+    // 2^24-slot nodes).
+    uint64_t first = (uint64_t)grid.bid * chunk;
+    bool started = false;
+    const bool claimed = lv.cap > (1ull << BPB200_FINAL_STRIDE_LOG2);
+    auto next_chunk = [&]() -> bool {
+        if (claimed) {
+            return claim_chunk(claims, chunk, total, &first);
+        }
+        if (started) {
+            first += (uint64_t)grid.nblk * chunk;
+        }
+        started = true;
+        return first < total;
+    };
+    while (next_chunk()) {
+        const uint64_t p0 = begin + first + (uint64_t)threadIdx.x * kResolveItems;
+        uint32_t j = (uint32_t)(p0 / pcap);
+        uint32_t k = (uint32_t)(p0 - (uint64_t)j * pcap);
+        uint32_t s = size_at(lv, level, j);
+        uint32_t live = 0;
+        uint32_t x[kResolveItems];
+#pragma unroll
+        for (int q = 0; q < kResolveItems; ++q) {
+            x[q] = (uint32_t)(p0 + q);
+            if (p0 + q >= lo_pair && p0 + q < end && k < s - s / 2) live |= 1u << q;
+            if (++k == pcap) {
+                k = 0;
+                ++j;
+                s = size_at(lv, level, j);
+            }
+        }
+        Found f[kResolveItems];
+        uf_find_many<kResolveItems>(uf, x, f, live, status, true);
+        uint32_t mine = 0; // this lane's kResolveItems colour bits
+#pragma unroll
+        for (int q = 0; q < kResolveItems; ++q) {
+            if (!(live & (1u << q))) continue;
+            mine |= (f[q].bit ^ (uf[f[q].root] & 1u)) << q;
+            // point the pair-node at its root (a true fact), so the finds of
+            // the pair-nodes below it end one step later (105.0 ms per
+            // compress at 2^30 entries against 106.2 without)
+            if (f[q].root != x[q]) {
+                uf[x[q]] = (f[q].root << 1) | f[q].bit;
+            }
+        }
+        // 32 / kResolveItems lanes hold one 32-pair colour word
+        constexpr uint32_t kWordLanes = 32 / kResolveItems;
+        uint32_t v = mine << ((lane & (kWordLanes - 1)) * kResolveItems);
+#pragma unroll
+        for (uint32_t d = 1; d < kWordLanes; d <<= 1) {
+            v |= __shfl_xor_sync(0xffffffffu, v, d);
+        }
+        if ((lane & (kWordLanes - 1)) == 0 && p0 < end) {
+            xbits[p0 >> 5] = v;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(256, BPB200_FINAL_MIN_BLOCKS) level_roots(
+    const Plan* __restrict__ plan, uint32_t level, uint32_t* uf, uint32_t* __restrict__ xbits,
+    uint32_t* claims, uint32_t* status) {
+    level_roots_run(launch_grid(), plan, level, uf, xbits, claims, status);
 }
 
 // Output side of a level, in natural (node, output pair) order: the output
-// switch bits and the children's inverses, so no level below the first
-// scatters an inverse.  Output pair k of node j joins outputs 2k and 2k+1,
-// fed by inputs u0 = inv[2k] and u1 = inv[2k+1], whose colours differ.  Its
-// switch bit is y = colour(u0) (src/benes.cpp:306-310: the output bit of
-// input i is colour(i) ^ (p[i] & 1), and p[u0] = 2k).  Of the two, the
-// colour-0 input inv[2k + y] is routed to the left child, where it sits at
-// input pair inv[2k + y] >> 1 and carries value k (src/benes.cpp:313-314);
-// the other goes right with the same value.  So
+// switch bits and the children, so no level below the first scatters an
+// inverse.  Output pair k of node j joins outputs 2k and 2k+1, fed by inputs
+// u0 = inv[2k] and u1 = inv[2k+1], whose colours differ.  Its switch bit is
+// y = colour(u0) (src/benes.cpp:306-310: the output bit of input i is
+// colour(i) ^ (p[i] & 1), and p[u0] = 2k).  Of the two, the colour-0 input
+// inv[2k + y] is routed to the left child, where it sits at input pair
+// inv[2k + y] >> 1 and carries value k (src/benes.cpp:313-314); the other
+// goes right with the same value.  So
 //     left_inv[k] = inv[2k + y] >> 1,  right_inv[k] = inv[2k + 1 - y] >> 1,
 // and an odd node's tail output s - 1, whose input is coloured 0, gives
-// left_inv[s / 2] = inv[s - 1] >> 1.  The pass reads inv sequentially and
-// one colour bit per output pair, and writes the children's inverse
-// sequentially.  It also resets the children's walk owners (one word per
-// pair-node: the stamp of its even vertex, the only one the walks read) and
-// pair-node union-find roots (`child_owner` / `child_uf`, may be null), the
-// state the next level's colouring starts from.  A value out of range (only
-// possible when the input was not a permutation, which level 0 reports)
-// leaves 0xffffffff, which every user range-checks.
+// left_inv[s / 2] = inv[s - 1] >> 1.  A thread takes two output pairs, which
+// make one output pair of each child: one 16-byte load of inv, one 8-byte
+// store per child inverse, and, for a child level coloured by walks
+// (`child_edge`), that pair's edges; for one coloured by union-find
+// (`child_uf`), its pair-node's root.  An odd child's tail is stored with
+// its virtual partner.  The edges are the only random writes (their node
+// fits L2); xbits gathers one bit per output pair.  A value out of range
+// (only possible when the input was not a permutation, which level 0
+// reports, or after a walk gave up) leaves 0xffffffff, which every user
+// range-checks.
 __device__ __forceinline__ void level_outputs_run(Grid grid, const Plan* __restrict__ plan,
     uint32_t level, const uint32_t* __restrict__ inv, const uint32_t* __restrict__ xbits,
     uint32_t* __restrict__ ybits, uint32_t* __restrict__ child_inv,
-    uint32_t* __restrict__ child_owner, uint32_t* __restrict__ child_uf) {
+    uint32_t* __restrict__ child_edge, uint32_t* __restrict__ child_uf, uint32_t* claims) {
     const LevelInfo& lv = plan->levels[level];
     const LevelInfo& cl = plan->levels[level + 1];
-    const uint32_t cap = (uint32_t)lv.cap;
-    const uint32_t pcap = (uint32_t)lv.pcap;
-    const uint32_t ccap = (uint32_t)cl.cap;
-    const uint32_t cpcap = (uint32_t)cl.pcap;
-    // this call's output pairs; the loop starts at a 32-pair boundary so
-    // each warp assembles whole bit words (bits before `first` stay zero)
+    const uint32_t ps = (uint32_t)lv.pcap;
+    const uint32_t hs = ps / 2; // quads of outputs per node
+    const uint32_t cps = (uint32_t)cl.pcap;
+    // this call's quads; the loop starts at a 32-quad boundary so each warp
+    // assembles whole bit words (bits before `first` stay zero)
     const NodeRange nr = level_nodes(*plan, level);
-    const uint64_t first = nr.lo * pcap;
-    const uint64_t end = first + ((uint64_t)pcap << nr.shift);
+    const uint64_t first = nr.lo * hs;
+    const uint64_t end = first + ((uint64_t)hs << nr.shift);
     const uint64_t begin = first & ~31ull;
-    const uint64_t stride = (uint64_t)grid.nblk * blockDim.x;
-    for (uint64_t p = begin + (uint64_t)grid.bid * blockDim.x + threadIdx.x;
-         p - (threadIdx.x & 31) < end; p += stride) {
-        bool y = false;
-        if (p >= first && p < end) {
-            const uint32_t j = (uint32_t)(p / pcap);
-            const uint32_t k = (uint32_t)(p - (uint64_t)j * pcap);
+    const uint32_t lane = threadIdx.x & 31;
+    uint64_t chunk = 0;
+    // claimed in address order (claim_chunk), 4 outputs a thread: the child
+    // nodes being scattered to at any time fit L2 (in grid-stride order the
+    // output pass took 407 ms per compress at 2^30 entries, claimed 100 ms;
+    // 4 and 16 quads a claim 111 and 152 ms)
+    while (claim_chunk(claims, blockDim.x, end - begin, &chunk)) {
+        const uint64_t g = begin + chunk + threadIdx.x;
+        if (g - lane >= end) continue;
+        uint32_t ys = 0;
+        if (g >= first && g < end) {
+            const uint32_t j = (uint32_t)g / hs;
+            const uint32_t k0 = 2 * ((uint32_t)g - j * hs);
             const uint32_t s = size_at(lv, level, j);
             const uint32_t half = s / 2;
-            const uint64_t node = (uint64_t)j * cap;
-            const uint64_t lb = (uint64_t)(2 * j) * ccap;
-            const uint64_t rb = lb + ccap;
-            if (k < half) {
-                const uint32_t u0 = inv[node + 2 * k];
-                const uint32_t u1 = inv[node + 2 * k + 1];
-                uint32_t to_left = ~0u, to_right = ~0u;
-                if (u0 < s && u1 < s) {
-                    const uint64_t q = (uint64_t)j * pcap + (u0 >> 1);
-                    y = (((xbits[q >> 5] >> (q & 31)) ^ u0) & 1u) != 0;
-                    to_left = (y ? u1 : u0) >> 1;
-                    to_right = (y ? u0 : u1) >> 1;
+            if (k0 < s - half) {
+                const uint4 four = __ldcs(reinterpret_cast<const uint4*>(inv) + g);
+                uint32_t left[2], right[2];
+#pragma unroll
+                for (uint32_t i = 0; i < 2; ++i) {
+                    const uint32_t u = i == 0 ? four.x : four.z;
+                    const uint32_t w = i == 0 ? four.y : four.w;
+                    bool y = false;
+                    left[i] = right[i] = ~0u;
+                    if (k0 + i < half) {
+                        if (u < s && w < s) {
+                            const uint32_t q = j * ps + (u >> 1);
+                            y = (((xbits[q >> 5] >> (q & 31)) ^ u) & 1u) != 0;
+                            left[i] = (y ? w : u) >> 1;
+                            right[i] = (y ? u : w) >> 1;
+                        }
+                    } else if (k0 + i == half && u < s) { // the odd tail
+                        left[i] = u >> 1;
+                    }
+                    ys |= (y ? 1u : 0u) << i;
                 }
-                if (child_inv != nullptr) {
-                    child_inv[lb + k] = to_left;
-                    child_inv[rb + k] = to_right;
-                }
-            } else if (k == half && (s & 1u) != 0) {
-                const uint32_t u = inv[node + s - 1];
-                if (child_inv != nullptr) child_inv[lb + half] = u < s ? u >> 1 : ~0u;
-            }
-            // children's pair-nodes start as their own roots: left child of
-            // s - s/2 entries, right of s/2; pair-node k/2 for even k
-            if (child_uf != nullptr && (k & 1u) == 0) {
-                if (k < s - half) {
-                    const uint32_t id = 2 * j * cpcap + (k >> 1);
-                    child_uf[id] = id << 1;
-                }
-                if (k < half) {
-                    const uint32_t id = (2 * j + 1) * cpcap + (k >> 1);
-                    child_uf[id] = id << 1;
-                }
-            }
-            // children's walk owners, one per pair-node, start unset
-            if (child_owner != nullptr && (k & 1u) == 0) {
-                if (k < s - half) child_owner[2 * j * cpcap + (k >> 1)] = ~0u;
-                if (k < half) child_owner[(2 * j + 1) * cpcap + (k >> 1)] = ~0u;
+                auto child = [&](uint32_t node, uint32_t cs, const uint32_t (&v)[2]) {
+                    if (k0 >= cs) return;
+                    const uint64_t at = 2ull * node * cps;
+                    const uint32_t w = k0 + 1 < cs ? v[1] : cs; // virtual partner
+                    __stcs(reinterpret_cast<uint2*>(child_inv + at + k0), make_uint2(v[0], w));
+                    if (child_edge != nullptr) {
+                        if (v[0] < cs && w < cs + (cs & 1u)) {
+                            child_edge[at + v[0]] = w;
+                            child_edge[at + w] = v[0];
+                        }
+                    } else if (child_uf != nullptr) {
+                        const uint32_t id = node * cps + (k0 >> 1);
+                        child_uf[id] = id << 1;
+                    }
+                };
+                child(2 * j, s - half, left);
+                child(2 * j + 1, half, right);
             }
         }
-        const unsigned word = __ballot_sync(0xffffffffu, y);
-        if ((threadIdx.x & 31) == 0) {
-            ybits[p >> 5] = word;
+        // lane i holds bits 2i and 2i + 1 of the 64 from quad g - lane
+        const uint32_t two = ys << (2 * (lane & 15));
+        const uint32_t low = __reduce_or_sync(0xffffffffu, lane < 16 ? two : 0u);
+        const uint32_t high = __reduce_or_sync(0xffffffffu, lane < 16 ? 0u : two);
+        if (lane < 2) {
+            ybits[((g - lane) >> 4) + lane] = lane == 0 ? low : high;
         }
     }
 }
@@ -539,8 +617,9 @@ __device__ __forceinline__ void level_outputs_run(Grid grid, const Plan* __restr
 __global__ void __launch_bounds__(256) level_outputs(const Plan* __restrict__ plan,
     uint32_t level, const uint32_t* __restrict__ inv, const uint32_t* __restrict__ xbits,
     uint32_t* __restrict__ ybits, uint32_t* __restrict__ child_inv,
-    uint32_t* __restrict__ child_owner, uint32_t* __restrict__ child_uf) {
-    level_outputs_run(launch_grid(), plan, level, inv, xbits, ybits, child_inv, child_owner, child_uf);
+    uint32_t* __restrict__ child_edge, uint32_t* __restrict__ child_uf, uint32_t* claims) {
+    level_outputs_run(launch_grid(), plan, level, inv, xbits, ybits, child_inv, child_edge,
+        child_uf, claims);
 }
 
 // Switch bits of one section at one level, packet-major: thread t maps to

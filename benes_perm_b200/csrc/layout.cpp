@@ -220,7 +220,7 @@ Error make_plan(const Layout& L, uint64_t tile_max, Plan* out) {
             lv.q = n >> l;
             lv.r = n & ((1ull << l) - 1);
             lv.cap = lv.q + (lv.r != 0 ? 1 : 0);
-            lv.pcap = (lv.cap + 1) / 2;
+            lv.pcap = ((lv.cap + 1) / 2 + 1) & ~1ull;
             for (int big = 0; big < 2; ++big) {
                 const uint64_t c = lv.q + (uint64_t)big;
                 lv.middle[big] = sizes.middle(c);
@@ -290,7 +290,7 @@ Error make_plan(const Layout& L, uint64_t tile_max, Plan* out) {
         p.tile_level = tile;
         uint64_t slots = 0, pairs = 0;
         for (uint32_t l = 0; l <= tile; ++l) {
-            const uint64_t s = (1ull << l) * p.levels[l].cap;
+            const uint64_t s = (1ull << l) * 2 * p.levels[l].pcap;
             const uint64_t q = (1ull << l) * p.levels[l].pcap;
             slots = s > slots ? s : slots;
             pairs = q > pairs ? q : pairs;

@@ -13,11 +13,12 @@
 // descriptor tree (the reference's make_compact_tree64,
 // src/internal.hpp:908-1003) is ever built.
 //
-// In device memory a level is stored "padded": node j occupies slots
-// [j * cap_l, j * cap_l + size), cap_l = ceil(N / 2^l); its pair-nodes
-// (one per input pair, plus the odd tail) occupy [j * pcap_l, ...),
-// pcap_l = ceil(cap_l / 2).  Children of node j are nodes 2j and 2j+1 of
-// level l+1, so padded offsets need no prefix sums.
+// In device memory a level is stored "padded": the pair-nodes of node j (one
+// per input pair, plus the odd tail) occupy [j * pcap_l, ...), pcap_l =
+// ceil(cap_l / 2) rounded up to even, cap_l = ceil(N / 2^l), and its slots
+// (inputs or outputs) [2 * j * pcap_l, ...).  Even strides put four outputs,
+// which two output pairs share, on a 16-byte boundary.  Children of node j
+// are nodes 2j and 2j+1 of level l+1, so padded offsets need no prefix sums.
 #pragma once
 
 #include <cstddef>
@@ -54,8 +55,8 @@ struct LevelSide {
 struct LevelInfo {
     uint64_t q;            // small node size
     uint64_t r;            // number of large (q + 1) nodes
-    uint64_t cap;          // padded slots per node = ceil(N / 2^l)
-    uint64_t pcap;         // padded pair-nodes per node = ceil(cap / 2)
+    uint64_t cap;          // entries of the largest node = ceil(N / 2^l)
+    uint64_t pcap;         // padded pair-nodes per node: ceil(cap / 2), rounded up to even
     uint64_t middle[2];    // middle bits of a small / large node's subtree
     uint64_t section[2][2];// [section][small/large]: switch bits + embedded middle bits
     LevelSide side[2];     // 0 = input section, 1 = output section
@@ -73,7 +74,7 @@ struct Plan {
     uint64_t end_offset;
     uint64_t switch_bits;
     uint64_t middle_bits;
-    uint64_t max_slots;         // max over levels of 2^l * cap_l
+    uint64_t max_slots;         // max over levels of 2^l * 2 * pcap_l
     uint64_t max_pairs;         // max over levels of 2^l * pcap_l
     uint32_t fact_bits[33];     // ceil(log2(c!)) for c = 0..32
     // Subtree sharding: with shards = 2^shard_level > 1 this call encodes

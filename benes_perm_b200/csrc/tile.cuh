@@ -171,46 +171,47 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
         asm volatile("" :: "r"(sum));
     }
     // The tile's own node: its inverse and edges, or, when it is a leaf, its
-    // values.  Never-written inverse slots mean a repeated value; a tile
-    // that is not a permutation ends here, so everything below runs on valid
-    // indexes.
+    // values.  A whole permutation (tile level 0) is given by its values, a
+    // node of a later level by its inverse.  A tile that is not a permutation
+    // ends here, so everything below runs on valid indexes.
     {
         const LevelInfo& l0 = plan.levels[T0];
         const uint32_t s0 = size_at(l0, T0, J);
-        const T* in = src + (uint64_t)J * l0.cap;
+        const uint32_t np = s0 - s0 / 2;
+        const uint32_t ps0 = tile_pair_stride(l0.pcap);
         uint16_t* inv = invs[0];
+        uint32_t* inv32 = reinterpret_cast<uint32_t*>(inv);
         const bool is_leaf = s0 <= leaf;
         bool bad = false;
-        for (uint32_t e = tid; e < tile_pair_stride(l0.pcap); e += blockDim.x) {
-            reinterpret_cast<uint32_t*>(inv)[e] = ~0u;
-        }
-        __syncthreads();
         // every load of a batch is issued before any is used
         constexpr int kBatch = 8;
-        for (uint32_t i0 = tid; i0 < s0; i0 += kBatch * blockDim.x) {
-            uint64_t v[kBatch];
+        if (T0 == 0) {
+            // never-written inverse slots mean a repeated value
+            for (uint32_t e = tid; e < ps0; e += blockDim.x) inv32[e] = ~0u;
+            __syncthreads();
+            for (uint32_t i0 = tid; i0 < s0; i0 += kBatch * blockDim.x) {
+                uint64_t v[kBatch];
 #pragma unroll
-            for (int q = 0; q < kBatch; ++q) {
-                const uint32_t i = i0 + q * blockDim.x;
-                v[q] = i < s0 ? (uint64_t)__ldcs(in + i) : 0;
-            }
+                for (int q = 0; q < kBatch; ++q) {
+                    const uint32_t i = i0 + q * blockDim.x;
+                    v[q] = i < s0 ? (uint64_t)__ldcs(src + i) : 0;
+                }
 #pragma unroll
-            for (int q = 0; q < kBatch; ++q) {
-                const uint32_t i = i0 + q * blockDim.x;
-                if (i >= s0) {
-                    break;
-                }
-                if (v[q] >= s0) {
-                    bad = true;
-                } else {
-                    inv[is_leaf ? i : (uint32_t)v[q]] = (uint16_t)(is_leaf ? v[q] : i);
+                for (int q = 0; q < kBatch; ++q) {
+                    const uint32_t i = i0 + q * blockDim.x;
+                    if (i >= s0) {
+                        break;
+                    }
+                    if (v[q] >= s0) {
+                        bad = true;
+                    } else {
+                        inv[is_leaf ? i : (uint32_t)v[q]] = (uint16_t)(is_leaf ? v[q] : i);
+                    }
                 }
             }
-        }
-        __syncthreads();
-        if (!is_leaf) {
-            for (uint32_t k = tid; k < s0 - s0 / 2; k += blockDim.x) {
-                const uint32_t both = reinterpret_cast<const uint32_t*>(inv)[k];
+            __syncthreads();
+            for (uint32_t k = tid; k < np && !is_leaf; k += blockDim.x) {
+                const uint32_t both = inv32[k];
                 const uint32_t u = both & 0xffffu;
                 const uint32_t w = 2 * k + 1 < s0 ? both >> 16 : s0; // virtual partner
                 if (u >= s0 || (2 * k + 1 < s0 && w >= s0)) {
@@ -219,6 +220,40 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
                     edge16[u] = (uint16_t)w;
                     edge16[w] = (uint16_t)u;
                 }
+            }
+        } else {
+            // never-written edges mean a repeated value
+            for (uint32_t k = tid; k < np; k += blockDim.x) edge[k] = ~0u;
+            __syncthreads();
+            const uint2* in = reinterpret_cast<const uint2*>(src) + (uint64_t)J * l0.pcap;
+            for (uint32_t k0 = tid; k0 < np; k0 += kBatch * blockDim.x) {
+                uint2 v[kBatch];
+#pragma unroll
+                for (int q = 0; q < kBatch; ++q) {
+                    const uint32_t k = k0 + q * blockDim.x;
+                    v[q] = k < np ? __ldcs(in + k) : make_uint2(0u, 0u);
+                }
+#pragma unroll
+                for (int q = 0; q < kBatch; ++q) {
+                    const uint32_t k = k0 + q * blockDim.x;
+                    if (k >= np) {
+                        break;
+                    }
+                    const uint32_t u = v[q].x;
+                    const uint32_t w = 2 * k + 1 < s0 ? v[q].y : s0; // virtual partner
+                    if (u >= s0 || (2 * k + 1 < s0 && w >= s0)) {
+                        bad = true;
+                    } else {
+                        inv32[k] = u | (w << 16);
+                        edge16[u] = (uint16_t)w;
+                        edge16[w] = (uint16_t)u;
+                    }
+                }
+            }
+            __syncthreads();
+            for (uint32_t k = tid; k < np; k += blockDim.x) {
+                const uint32_t both = edge[k];
+                bad |= (both & 0xffffu) == 0xffffu || (both >> 16) == 0xffffu;
             }
         }
         if (__syncthreads_or(bad)) {

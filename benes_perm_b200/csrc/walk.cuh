@@ -1,37 +1,50 @@
 // SPDX-License-Identifier: Apache-2.0
 //
-// Canonical colouring of the global levels by orbit walks.
+// Canonical colouring of the global levels by two-way walks over contracted
+// lists.
 //
-// Within a node of s entries let A(v) = v^1 (input pair partner) and
-// B(u) = inv[p[u]^1] (the input whose output is paired with u's output).
-// The constraint graph (src/benes.cpp:238-252) alternates A and B edges, so
-// each component is a cycle that splits into two orbits of f = B o A,
-// f(v) = inv[p[v^1]^1], mirrors of each other (O and O^1); all vertices of
-// one orbit share a colour and the mirror has the other.  An odd node gets
-// one virtual vertex s with p[s] = s (so inv[s] = s): the reference's tail
-// path then closes into a cycle through s, and giving the tail t = s-1 the
-// smallest key makes "orbit holding the smallest key gets colour 0" exactly
-// the reference's canonical rule (odd tail first, then each component's
-// smallest vertex, src/benes.cpp:253-297):
-//     colour(v) = [min key(O(v)) > min key(O(v^1))],  key(t) = 0, key(v) = v+1.
+// A node's constraint graph (src/benes.cpp:238-252) is held as its output
+// edges: edge[u] is the input that shares input u's output pair, two words
+// per pair-node k = inputs {2k, 2k+1}.  The graph is a set of cycles over
+// pair-nodes: a path that enters pair-node k at input w leaves it at w^1 and
+// goes on to edge[w^1].  All inputs at which a directed path enters have one
+// colour; the path walked backwards enters at their partners, which have the
+// other.  An odd node's unpaired input t = s-1 gets a virtual partner s, and
+// its unpaired output a virtual partner output fed by s, so the tail's path
+// closes into a cycle too.  With key(w) = w, or (w - t) mod 2^32 in an odd
+// node (which puts t and s first), the canonical rule (odd tail colour 0,
+// else the component's smallest input, src/benes.cpp:253-297) says: the
+// colour of input w is the low bit of the smallest key on the directed cycle
+// through w, because that cycle passes the component's smallest pair-node at
+// exactly one of its two inputs.
 //
-// Orbits are long for random inputs, so one vertex in every bucket of
-// 2^kRulerLog2 slots (at a hashed position) is a ruler.  A ruler walks its
-// orbit up to the next ruler, stamping each even vertex it passes with its
-// id and keeping the minimum key of the segment and of the segment's
-// mirror.  Only even vertices are stamped, into one owner word per
-// pair-node: the colour of pair-node k is the colour of vertex 2k, and
-// halving the stamps halves the walk's random writes and its owner array.
-// Pointer jumping over rulers (stopping after the first round that changes
-// nothing, which implies convergence on cycles) turns segment minima into
-// orbit minima.  No atomics, no shared roots: every step is two independent
-// gathers.  Cycles without any ruler are short for all but contrived inputs
-// and are walked whole (level_walk_short); a walk longer than kWalkCap sets
-// the `hard` flag and the level falls back to the union-find kernels.
+// List 0 is the pair-nodes.  One element of a list in 8, at a hashed place
+// (ruler_slot), is an element of the next list.  Two walks leave it, one per
+// direction, each up to the next such element or to an element stamped by a
+// walk that came the other way, so every element is passed about once: that
+// is half the steps of one-way walks, and the stamp overwrites edge words
+// that nobody needs again, so the walks touch 4 bytes per entry and make one
+// dependent access per step.  A stamp names the walk that passed: kStamp |
+// ruler << 1 | (direction ^ side of entry); a walk that enters a stamped
+// element at side b goes on as directed ruler (stamp ^ b).  Walks that cross
+// may both stamp the elements where they cross, with stamps that say the
+// same.  Each directed ruler keeps its successor and the smallest key its
+// own walk saw; a ruler's two walks together cover the stretches around it,
+// so folding min(m0, m1 ^ 1) over the rulers of a cycle (^ 1 mirrors a key
+// to the other direction) covers the whole cycle.  Lists are contracted
+// (list_contract) until a node's elements fit one CTA, which colours them in
+// shared memory (list_rank); the colours then go back down the lists
+// (list_expand) and to the pair-nodes (level_colours).
 //
-// Walks pay off while a node's arrays fit in L2 (random access there is
-// 6-8x faster than in HBM on B200); nodes above kWalkMaxNode entries are
-// coloured by union-find, which needs fewer HBM round trips per entry.
+// Cycles without any ruler are short for all but contrived inputs: each of
+// their elements walks them whole.  A walk longer than its cap sets
+// kErrGaveUp and the host encodes the permutation again with union-find on
+// every level.  Indexes read from memory are range-checked throughout: an
+// input that is not a permutation, or a level after a walk that gave up,
+// leaves arbitrary words behind.
+//
+// What bounds the walks: random L2 accesses (a node's edges fit L2 up to
+// kWalkMaxNode entries); larger nodes are coloured by union-find.
 #pragma once
 
 #include "device.cuh"
@@ -42,784 +55,512 @@
 
 namespace bpb200 {
 
-// Tuning knobs, overridable at build time.  Measured on B200 over uniform
-// 2^30-entry inputs with super-ruler jumping: one ruler per 8 slots, walks
-// up to 2^23-entry nodes and 4 walk blocks per SM gave the lowest total
-// (1078 ms; rulers per 16 slots: 1094 at 3 blocks per SM; per 32: 1175;
-// per 4: 1132; walk limit 2^24: 1112).  Denser rulers give shorter,
-// more numerous walk chains, which hide the L2 latency of each step better.
-#ifndef BPB200_RULER_LOG2
-#define BPB200_RULER_LOG2 3
-#endif
 #ifndef BPB200_WALK_MAX_LOG2
 #define BPB200_WALK_MAX_LOG2 23
 #endif
-// Union-find levels whose nodes have at most 2^BPB200_FINAL_STRIDE_LOG2
-// slots finalize in grid-stride order, larger ones in claimed order (see
-// level_finalize); measured on B200 at 2^30 uniform entries (finalize 105 ms
-// per compress; limit 2^24: 110 ms; 2^23: 119 ms).
-#ifndef BPB200_FINAL_STRIDE_LOG2
-#define BPB200_FINAL_STRIDE_LOG2 26
-#endif
-// Union-find levels: level_finalize writes each pair-node's root back (1),
-// measured on B200 at 2^30 uniform entries: finalize 105.0 ms per compress
-// against 106.2 without.
-#ifndef BPB200_RESOLVE_WRITEBACK
-#define BPB200_RESOLVE_WRITEBACK 1
-#endif
-
-constexpr uint32_t kRulerLog2 = BPB200_RULER_LOG2; // one ruler per 2^kRulerLog2 slots
-constexpr uint32_t kWalkCap = 1u << 16;      // longest ruler walk before giving up
-#ifndef BPB200_WALK_CHUNK
-#define BPB200_WALK_CHUNK 32
-#endif
-// rulers claimed per warp at a time: 32 measured fastest on B200 at 2^30
-// uniform entries (walks 157 ms per compress; 16: 159 ms; 8: 176 ms)
-constexpr uint32_t kWalkChunk = BPB200_WALK_CHUNK;
-constexpr uint32_t kJumpItems = 8;           // rulers per thread in a claimed jump chunk
 constexpr uint64_t kWalkMaxNode = 1ull << BPB200_WALK_MAX_LOG2; // larger: union-find
-static_assert(BPB200_RULER_LOG2 >= 2 && BPB200_RULER_LOG2 <= 8, "ruler density out of range");
 static_assert(BPB200_WALK_MAX_LOG2 >= 13 && BPB200_WALK_MAX_LOG2 <= 28, "walk limit out of range");
-constexpr uint32_t kUnset = 0xffffffffu;     // owner of a vertex no walk reached
-// Walk owners are one word per pair-node: owner[j * pcap + k] is the stamp
-// of even vertex 2k of node j (the finalize reads only even vertices), half
-// the footprint of a word per slot, which keeps more of a node in L2.
-constexpr uint32_t kColourTag = 0x80000000u; // owner value carrying a colour directly
-constexpr uint32_t kNoRuler = 0xffffffffu;   // bucket whose hashed slot is padding
+constexpr uint32_t kRulerLog2 = 3;          // elements per element of the next list (log2)
+constexpr uint32_t kWalkCap = 1u << 16;     // longest walk between rulers
+constexpr uint32_t kShortCap = 1u << 10;    // longest cycle without rulers
+constexpr uint32_t kStamp = 0x80000000u;
+constexpr uint32_t kNone = 0xffffffffu;     // successor of an absent element
+constexpr uint32_t kMaxLists = 5;           // lists of rulers: 1..kMaxLists
+constexpr uint32_t kRankMaxLog2 = 14;       // most elements of a node list_rank takes (log2)
+constexpr uint32_t kRankMinLog2 = 10;
 
-// control words of a level
-enum : int {
-    kCtlHard = 0,
-    kCtlChanged = 1,
-    kCtlDone = 2,
-    kCtlFinal = 3,
-    kCtlClaim = 4,       // ruler chunks handed out by level_walk
-    kCtlClaimPlace = 5,  // chunks handed out by level_place
-    kCtlClaimInverse = 6, // chunks handed out by level_inverse
-    kCtlClaimJump = 7,   // ruler chunks handed out by ruler_jump (reset every round)
-    kCtlClaimUnion = 8,  // chunks handed out by level_union
-    kCtlClaimFinal = 9,  // chunks handed out by level_finalize
-    kCtlClaimSuper = 10, // super-ruler chunks handed out by ruler_super_walk
-    kCtlWords = 16       // control_reset clears them with one warp
-};
-
-__device__ __forceinline__ uint32_t ruler_position(uint32_t bucket) {
-    return (bucket * 0x9E3779B1u) >> (32 - kRulerLog2);
+// Element of list e that element i of list e + 1 stands for.
+__host__ __device__ __forceinline__ uint32_t ruler_slot(uint32_t i) {
+    return (i << kRulerLog2) + ((i * 0x9E3779B1u) >> (32 - kRulerLog2));
+}
+__host__ __device__ __forceinline__ bool is_ruler(uint32_t element) {
+    return element == ruler_slot(element >> kRulerLog2);
 }
 
-__device__ __forceinline__ bool is_ruler_slot(uint32_t slot) {
-    return (slot & ((1u << kRulerLog2) - 1)) == ruler_position(slot >> kRulerLog2);
-}
-
-// The rulers of this call's nodes (level_nodes): buckets [lo, hi) covering
-// slots [slot_lo, slot_end).  A bucket at either end may hash its ruler
-// into a neighbouring node outside the range; such rulers are marked absent.
-struct RulerRange {
+// This call's elements of list e (0: pair-nodes): those that stand for the
+// pair-nodes [pair_lo, pair_end) lie in [lo, hi); the first and the last may
+// stand for a pair-node outside and are absent then.
+struct ListRange {
     uint32_t lo, hi;
-    uint64_t slot_lo, slot_end;
 };
 
-BP_HD RulerRange ruler_range(const Plan& p, uint32_t level) {
-    const LevelInfo& lv = p.levels[level];
-    const NodeRange nr = level_nodes(p, level);
-    const uint64_t slot_lo = nr.lo * lv.cap;
-    const uint64_t slot_end = slot_lo + (lv.cap << nr.shift);
-    return RulerRange{(uint32_t)(slot_lo >> kRulerLog2),
-        (uint32_t)((slot_end + (1u << kRulerLog2) - 1) >> kRulerLog2), slot_lo, slot_end};
+BP_HD ListRange list_range(uint64_t pair_lo, uint64_t pair_end, uint32_t e) {
+    return ListRange{(uint32_t)(pair_lo >> (kRulerLog2 * e)),
+        (uint32_t)((pair_end - 1) >> (kRulerLog2 * e)) + 1};
 }
 
-// One node of one level, as seen by a walker.
-template <typename T>
-struct NodeView {
-    const T* p;            // node's values (node-local)
-    const uint32_t* inv;   // node's inverse
-    uint32_t s;            // entries
-    bool odd;
+// Pair-node that element i of list e stands for.
+__device__ __forceinline__ uint32_t pair_of(uint32_t i, uint32_t e) {
+    for (; e > 0; --e) {
+        i = ruler_slot(i);
+    }
+    return i;
+}
 
-    // f(v) = inv[p[v^1]^1] with the virtual vertex s of an odd node; returns
-    // 0xffffffff when a value is out of range (input is not a permutation)
-    __device__ __forceinline__ uint32_t f(uint32_t v) const {
-        const uint32_t a = v ^ 1u;
-        uint32_t o;
-        if (odd && a == s) {
-            o = s;
-        } else {
-            const uint64_t value = (uint64_t)p[a];
-            if (value >= s) {
-                return 0xffffffffu;
-            }
-            o = (uint32_t)value;
+// Words other blocks rewrite while the walks run: read past L1.
+__device__ __forceinline__ uint2 load_live(const uint2* p) {
+    uint2 v;
+    asm volatile("ld.volatile.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint32_t load_live(const uint32_t* p) {
+    return *(const volatile uint32_t*)p;
+}
+
+// Smallest key of the stretches around a ruler, for paths that enter it in
+// direction 0 (direction 1: ^ 1).
+__device__ __forceinline__ uint32_t around(uint4 state) { return min(state.y, state.w ^ 1u); }
+
+// The edges of level 0, from its inverse: one thread per output pair.  Every
+// later level's edges are written by its parent's output pass.  A slot no
+// value was routed to means a repeated value.
+__device__ __forceinline__ void level_edges_run(Grid grid, const Plan* __restrict__ plan,
+    const uint32_t* __restrict__ inv, uint32_t* __restrict__ edge, uint32_t* status) {
+    const uint32_t s = (uint32_t)plan->levels[0].q;
+    const uint32_t np = s - s / 2;
+    bool bad = false;
+    for (uint32_t k = grid.bid * blockDim.x + threadIdx.x; k < np; k += grid.nblk * blockDim.x) {
+        const uint2 both = reinterpret_cast<const uint2*>(inv)[k];
+        const uint32_t u = both.x;
+        const uint32_t w = 2 * k + 1 < s ? both.y : s;
+        if (u >= s || (2 * k + 1 < s && w >= s)) {
+            bad = true;
+            continue;
         }
-        const uint32_t b = o ^ 1u;
-        return (odd && b == s) ? s : inv[b];
+        edge[u] = w;
+        edge[w] = u;
     }
-    __device__ __forceinline__ uint32_t key(uint32_t v) const {
-        return (odd && v == s - 1) ? 0u : v + 1;
-    }
+    if (bad) atomicOr(status, kErrNotPermutation);
+}
+
+__global__ void __launch_bounds__(256) level_edges(const Plan* __restrict__ plan,
+    const uint32_t* __restrict__ inv, uint32_t* __restrict__ edge, uint32_t* status) {
+    level_edges_run(launch_grid(), plan, inv, edge, status);
+}
+
+// One direction of a walk, advanced one element at a time.  `enter` is the
+// side and element it enters next, `best` its smallest key so far.
+struct Walk {
+    uint32_t enter, best, next;
+    bool live;
 };
 
-// Ruler walks.  Warps claim chunks of kWalkChunk rulers in address order
-// from a per-level counter, so the walks in flight at any moment touch a
-// window of a few tens of MB that stays in L2; within a warp each lane takes
-// the next ruler of the chunk as soon as its current walk ends, so walk
-// lengths (geometric, mean 2^kRulerLog2) do not leave lanes idle behind the
-// longest walk.  state[r] = {next ruler, min key, min mirror key, 0};
-// owner[pair-node] = r for every real even vertex the walk passes.
-template <typename T>
-__device__ __forceinline__ void level_walk_run(Grid grid, const Plan* __restrict__ plan, uint32_t level,
-    const T* __restrict__ vals, const uint32_t* __restrict__ inv, uint32_t* __restrict__ owner,
-    uint4* __restrict__ state, uint32_t* control) {
-    const LevelInfo& lv = plan->levels[level];
-    const uint32_t cap = (uint32_t)lv.cap;
-    const RulerRange rr = ruler_range(*plan, level);
-    const uint32_t lane = threadIdx.x & 31;
-    const unsigned below = (1u << lane) - 1u;
-    uint32_t next_free = 0, hi = 0; // current chunk, warp-uniform
-    bool exhausted = false;
-    bool active = false;
-    uint32_t r = 0, base = 0, own = 0, s = 0, cur = 0, ma = 0, mb = 0, steps = 0;
-    bool odd = false;
-    for (;;) {
-        const unsigned idle = __ballot_sync(0xffffffffu, !active);
-        if (idle != 0 && next_free >= hi && !exhausted) {
-            uint32_t c = 0;
-            if (lane == 0) c = atomicAdd(control + kCtlClaim, 1u);
-            c = __shfl_sync(0xffffffffu, c, 0);
-            const uint64_t lo = rr.lo + (uint64_t)c * kWalkChunk;
-            if (lo >= rr.hi) {
-                exhausted = true;
-            } else {
-                next_free = (uint32_t)lo;
-                hi = (uint32_t)(lo + kWalkChunk < rr.hi ? lo + kWalkChunk : rr.hi);
-            }
-        }
-        if (!active) {
-            const uint32_t mine = next_free + (uint32_t)__popc(idle & below);
-            if (mine < hi) {
-                r = mine;
-                const uint32_t slot = (r << kRulerLog2) + ruler_position(r);
-                const bool in_range = slot >= rr.slot_lo && slot < rr.slot_end;
-                const uint32_t j = in_range ? slot / cap : 0u;
-                const uint32_t v0 = slot - j * cap;
-                s = in_range ? size_at(lv, level, j) : 0u;
-                if (!in_range || v0 >= s) {
-                    state[r] = make_uint4(kNoRuler, 0, 0, 0);
-                } else {
-                    base = j * cap;
-                    own = j * (uint32_t)lv.pcap;
-                    odd = (s & 1u) != 0;
-                    const NodeView<T> nv{vals + base, inv + base, s, odd};
-                    cur = v0;
-                    ma = nv.key(v0);
-                    mb = nv.key(v0 ^ 1u);
-                    steps = 0;
-                    active = true;
-                }
-            }
-        }
-        next_free = min(next_free + (uint32_t)__popc(idle), hi);
-        if (__ballot_sync(0xffffffffu, active) == 0) {
-            if (exhausted) break;
-            continue;
-        }
-        if (active) {
-            const NodeView<T> nv{vals + base, inv + base, s, odd};
-            const uint32_t w = nv.f(cur);
-            bool end = false;
-            uint32_t next = r;
-            if (w >= s + (odd ? 1u : 0u)) {
-                atomicOr(control + kCtlHard, 1u); // not a permutation
-                end = true;
-            } else if (w < s && is_ruler_slot(base + w)) {
-                next = (base + w) >> kRulerLog2;
-                end = true;
-            } else {
-                if (w < s && (w & 1u) == 0) owner[own + (w >> 1)] = r;
-                ma = min(ma, nv.key(w));
-                mb = min(mb, nv.key(w ^ 1u));
-                cur = w;
-                if (++steps == kWalkCap) {
-                    atomicOr(control + kCtlHard, 1u);
-                    end = true;
-                }
-            }
-            if (end) {
-                state[r] = make_uint4(next, ma, mb, 0);
-                active = false;
-            }
-        }
-    }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) level_walk(const Plan* __restrict__ plan, uint32_t level,
-    const T* __restrict__ vals, const uint32_t* __restrict__ inv, uint32_t* __restrict__ owner,
-    uint4* __restrict__ state, uint32_t* control) {
-    level_walk_run<T>(launch_grid(), plan, level, vals, inv, owner, state, control);
-}
-
-// Orbits no ruler reached: thread per pair-node whose even vertex is
-// neither a ruler nor stamped, i.e. lies in a ruler-free orbit (its
-// mirror orbit may have rulers; the walk folds the mirror's keys as it
-// goes, so it needs nothing from them).  Only the walker starting at the
-// smallest even vertex of its orbit walks the orbit whole (the others stop
-// at the first smaller even vertex, about log L steps), then stamps the
-// orbit's colour on every real vertex of it; the cost is O(L log L) per
-// orbit, and such orbits are short for all but contrived inputs.
-template <typename T>
-__device__ __forceinline__ void level_walk_short_run(Grid grid, const Plan* __restrict__ plan,
-    uint32_t level, const T* __restrict__ vals, const uint32_t* __restrict__ inv,
-    uint32_t* __restrict__ owner, uint32_t* control) {
-    const LevelInfo& lv = plan->levels[level];
-    const uint32_t cap = (uint32_t)lv.cap;
-    const uint32_t pcap = (uint32_t)lv.pcap;
-    const NodeRange nr = level_nodes(*plan, level);
-    const uint64_t end = (nr.lo + (1ull << nr.shift)) * pcap;
-    for (uint64_t pidx = nr.lo * pcap + (uint64_t)grid.bid * blockDim.x + threadIdx.x; pidx < end;
-         pidx += (uint64_t)grid.nblk * blockDim.x) {
-        const uint32_t j = (uint32_t)(pidx / pcap);
-        const uint32_t k = (uint32_t)(pidx - (uint64_t)j * pcap);
-        const uint32_t s = size_at(lv, level, j);
-        if (k >= s - s / 2) {
-            continue;
-        }
-        const uint32_t base = j * cap;
-        const uint32_t own = j * pcap;
-        const uint32_t v = 2 * k;
-        if (is_ruler_slot(base + v) || owner[own + k] != kUnset) {
-            continue;
-        }
-        const NodeView<T> nv{vals + base, inv + base, s, (s & 1u) != 0};
-        const uint32_t mine = nv.key(v);
-        uint32_t ma = mine, mb = nv.key(v ^ 1u);
-        uint32_t cur = v;
-        bool closed = false, smallest = true;
-        for (uint32_t step = 0; step < kWalkCap; ++step) {
-            const uint32_t w = nv.f(cur);
-            if (w >= s + (nv.odd ? 1u : 0u)) {
-                break;
-            }
-            if (w == v) {
-                closed = true;
-                break;
-            }
-            if ((w & 1u) == 0 && w < s && nv.key(w) < mine) {
-                smallest = false; // that vertex's walker covers this orbit
-                closed = true;
-                break;
-            }
-            ma = min(ma, nv.key(w));
-            mb = min(mb, nv.key(w ^ 1u));
-            cur = w;
-        }
-        if (!closed) {
-            atomicOr(control + kCtlHard, 1u);
-            continue;
-        }
-        if (!smallest) {
-            continue;
-        }
-        const uint32_t colour = kColourTag | (ma > mb ? 1u : 0u);
-        cur = v;
-        do {
-            if (cur < s && (cur & 1u) == 0) owner[own + (cur >> 1)] = colour;
-            cur = nv.f(cur);
-        } while (cur != v);
-    }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) level_walk_short(const Plan* __restrict__ plan,
-    uint32_t level, const T* __restrict__ vals, const uint32_t* __restrict__ inv,
-    uint32_t* __restrict__ owner, uint32_t* control) {
-    level_walk_short_run<T>(launch_grid(), plan, level, vals, inv, owner, control);
-}
-
-// One pointer-jumping round over ruler states (src -> dst).  Blocks claim
-// chunks of rulers in address order, so the rulers being jumped at any time
-// (and, early on, the near successors they read) stay close together.
-// The done/hard words were written by earlier launches, so every thread of
-// a block sees the same value and the block leaves together.
-// States [lo, hi) are this call's super-rulers (all of them unless the
-// level is sharded); a successor outside them can only come from a
-// non-permutation and sends the level to union-find.
-__device__ __forceinline__ void ruler_jump_run(Grid grid, const uint4* __restrict__ src,
-    uint4* __restrict__ dst, uint32_t lo, uint32_t hi, uint32_t round, uint32_t* control) {
-    if (*(volatile uint32_t*)(control + kCtlDone) != 0 ||
-        *(volatile uint32_t*)(control + kCtlHard) != 0) {
-        return;
-    }
-    bool changed = false;
-    const uint64_t chunk = (uint64_t)blockDim.x * kJumpItems;
-    uint64_t first = 0;
-    bool bad = false;
-    while (claim_chunk(control + kCtlClaimJump, chunk, hi - lo, &first)) {
-        for (uint32_t k = 0; k < kJumpItems; ++k) {
-            const uint64_t r = lo + first + (uint64_t)k * blockDim.x + threadIdx.x;
-            if (r >= hi) {
-                break;
-            }
-            const uint4 me = src[r];
-            if (me.x == kNoRuler || me.x < lo || me.x >= hi) {
-                bad |= me.x != kNoRuler;
-                dst[r] = me;
-                continue;
-            }
-            const uint4 nx = src[me.x];
-            const uint4 out = make_uint4(nx.x, min(me.y, nx.y), min(me.z, nx.z), 0);
-            changed |= (out.y != me.y) || (out.z != me.z);
-            dst[r] = out;
-        }
-    }
-    if (__any_sync(0xffffffffu, changed) && (threadIdx.x & 31) == 0) {
-        atomicOr(control + kCtlChanged, 1u);
-    }
-    if (bad) {
-        atomicOr(control + kCtlHard, 1u);
-    }
-    (void)round;
-}
-
-__global__ void __launch_bounds__(256) ruler_jump(const uint4* __restrict__ src,
-    uint4* __restrict__ dst, uint32_t lo, uint32_t hi, uint32_t round, uint32_t* control) {
-    ruler_jump_run(launch_grid(), src, dst, lo, hi, round, control);
-}
-
-// After a round: a round that changed nothing means every ruler holds its
-// orbit's minima; later rounds then return at once.
-__device__ __forceinline__ void ruler_check_run(Grid grid, uint32_t round, uint32_t* control) {
-    control[kCtlClaimJump] = 0; // the next round claims from the start again
-    if (control[kCtlDone] != 0 || control[kCtlHard] != 0) {
-        return;
-    }
-    control[kCtlFinal] = (round + 1) & 1u; // buffer the round just wrote
-    if (control[kCtlChanged] == 0) {
-        control[kCtlDone] = 1;
-    }
-    control[kCtlChanged] = 0;
-}
-
-__global__ void ruler_check(uint32_t round, uint32_t* control) {
-    ruler_check_run(launch_grid(), round, control);
-}
-
-// Levels with few super-rulers spend their jumping time on launches, not on
-// the rounds: a round over a few thousand states is shorter than the gap
-// between two launches.  ruler_jump_block runs all rounds of such a level in
-// one CTA, a block barrier between rounds, and leaves the control words as
-// the ruler_jump / ruler_check sequence would (kCtlFinal names the buffer
-// the last executed round wrote; kCtlDone is set when a round changed
-// nothing).  Each thread handles kJumpBlockBatch states at a time, loading
-// all of them before their successors so the gathers overlap.
-constexpr uint32_t kJumpBlockThreads = 1024;
-constexpr uint32_t kJumpBlockBatch = 4;
-#ifndef BPB200_JUMP_BLOCK_LOG2
-#define BPB200_JUMP_BLOCK_LOG2 14
-#endif
-constexpr uint32_t kJumpBlockMaxStates = 1u << BPB200_JUMP_BLOCK_LOG2;
-
-__device__ __forceinline__ void ruler_jump_block_run(Grid grid, uint4* s0, uint4* s1,
-    uint32_t lo, uint32_t hi, uint32_t rounds, uint32_t* control) {
-    // written by earlier launches: every thread reads the same values
-    if (*(volatile uint32_t*)(control + kCtlDone) != 0 ||
-        *(volatile uint32_t*)(control + kCtlHard) != 0) {
-        return;
-    }
-    __shared__ uint32_t changed[2];
-    if (threadIdx.x == 0) {
-        changed[0] = 0u;
-        changed[1] = 0u;
-    }
-    __syncthreads();
-    uint32_t final_buffer = 0;
-    bool done = false;
-    bool bad = false;
-    for (uint32_t r = 0; r <= rounds; ++r) {
-        const uint4* src = (r & 1u) ? s1 : s0;
-        uint4* dst = (r & 1u) ? s0 : s1;
-        bool ch = false;
-        for (uint32_t base = lo; base < hi; base += kJumpBlockThreads * kJumpBlockBatch) {
-            uint4 me[kJumpBlockBatch], nx[kJumpBlockBatch];
-#pragma unroll
-            for (uint32_t k = 0; k < kJumpBlockBatch; ++k) {
-                const uint32_t i = base + k * kJumpBlockThreads + threadIdx.x;
-                me[k] = i < hi ? __ldcg(src + i) : make_uint4(kNoRuler, 0u, 0u, 0u);
-            }
-#pragma unroll
-            for (uint32_t k = 0; k < kJumpBlockBatch; ++k) {
-                const bool inside = me[k].x >= lo && me[k].x < hi;
-                const bool live = me[k].x != kNoRuler && inside;
-                bad |= me[k].x != kNoRuler && !inside;
-                nx[k] = live ? __ldcg(src + me[k].x) : me[k];
-            }
-#pragma unroll
-            for (uint32_t k = 0; k < kJumpBlockBatch; ++k) {
-                const uint32_t i = base + k * kJumpBlockThreads + threadIdx.x;
-                if (i >= hi) {
-                    continue;
-                }
-                if (me[k].x == kNoRuler || me[k].x < lo || me[k].x >= hi) {
-                    dst[i] = me[k];
-                    continue;
-                }
-                const uint4 out = make_uint4(nx[k].x, min(me[k].y, nx[k].y),
-                    min(me[k].z, nx[k].z), 0u);
-                ch |= (out.y != me[k].y) || (out.z != me[k].z);
-                dst[i] = out;
-            }
-        }
-        if (ch) {
-            changed[r & 1u] = 1u;
-        }
-        __syncthreads(); // this round's states and flag are visible to the block
-        const bool any = changed[r & 1u] != 0u;
-        final_buffer = (r + 1u) & 1u;
-        if (threadIdx.x == 0) {
-            changed[(r + 1u) & 1u] = 0u; // every thread read it a round ago
-        }
-        __syncthreads();
-        if (!any) {
-            done = true;
-            break;
-        }
-    }
-    if (bad) {
-        atomicOr(control + kCtlHard, 1u); // a successor out of range: fall back to union-find
-    }
-    if (threadIdx.x == 0) {
-        control[kCtlFinal] = final_buffer;
-        if (done) {
-            control[kCtlDone] = 1u;
-        }
-        control[kCtlChanged] = 0u;
-        control[kCtlClaimJump] = 0u;
-    }
-}
-
-__global__ void __launch_bounds__(kJumpBlockThreads, 1) ruler_jump_block(uint4* s0, uint4* s1,
-    uint32_t lo, uint32_t hi, uint32_t rounds, uint32_t* control) {
-    ruler_jump_block_run(launch_grid(), s0, s1, lo, hi, rounds, control);
-}
-
-// ---------------------------------------------------------------------------
-// Super-rulers.  Jumping over all rulers costs a full pass over their states
-// per round (about log2 of the rulers in an orbit rounds).  Instead every
-// ruler whose id is a multiple of 2^kSuperLog2 is a super-ruler: it follows
-// the ruler chain to the next super-ruler once (ruler_super_walk), folding
-// the segment minima and stamping super_of[r] on the rulers it passes; the
-// jumping then runs over the 2^kSuperLog2 times smaller super states.  Ruler
-// cycles without a super-ruler are closed by ruler_super_short, which stamps
-// their colour directly (kColourTag).  super_of[] starts at kUnset.
-// ---------------------------------------------------------------------------
-constexpr uint32_t kSuperLog2 = 4;
-
-// Rulers [rlo, rhi) are this call's (ruler_range); their super-rulers are
-// the multiples of 2^kSuperLog2 among them.
-__device__ __forceinline__ void ruler_super_walk_run(Grid grid, const uint4* __restrict__ state,
-    uint32_t rlo, uint32_t rhi, uint4* __restrict__ sstate, uint32_t* __restrict__ super_of,
-    uint32_t* control) {
-    if (*(volatile uint32_t*)(control + kCtlHard) != 0) {
-        return; // the level is coloured by union-find
-    }
-    const uint32_t slo = (rlo + (1u << kSuperLog2) - 1) >> kSuperLog2;
-    const uint32_t shi = (rhi + (1u << kSuperLog2) - 1) >> kSuperLog2;
-    uint64_t first = 0;
-    while (claim_chunk(control + kCtlClaimSuper, blockDim.x, shi - slo, &first)) {
-        const uint64_t i = slo + first + threadIdx.x;
-        if (i >= shi) {
-            continue;
-        }
-        const uint32_t r = (uint32_t)i << kSuperLog2;
-        const uint4 me = state[r];
-        if (me.x == kNoRuler) {
-            sstate[i] = make_uint4(kNoRuler, 0, 0, 0);
-            continue;
-        }
-        super_of[r] = r;
-        uint32_t ma = me.y, mb = me.z, cur = me.x;
-        for (uint32_t hop = 0; (cur & ((1u << kSuperLog2) - 1)) != 0; ++hop) {
-            if (cur < rlo || cur >= rhi || hop == kWalkCap) {
-                atomicOr(control + kCtlHard, 1u);
-                break;
-            }
-            const uint4 st = state[cur];
-            super_of[cur] = r;
-            ma = min(ma, st.y);
-            mb = min(mb, st.z);
-            cur = st.x;
-        }
-        sstate[i] = make_uint4(cur >> kSuperLog2, ma, mb, 0);
-    }
-}
-
-__global__ void __launch_bounds__(256) ruler_super_walk(const uint4* __restrict__ state,
-    uint32_t rlo, uint32_t rhi, uint4* __restrict__ sstate, uint32_t* __restrict__ super_of,
-    uint32_t* control) {
-    ruler_super_walk_run(launch_grid(), state, rlo, rhi, sstate, super_of, control);
-}
-
-// Ruler cycles that contain no super-ruler: thread per ruler no super walk
-// reached; the ruler with the smallest id of its cycle folds the cycle's
-// minima and stamps the colour on every ruler of it.
-__device__ __forceinline__ void ruler_super_short_run(Grid grid, const uint4* __restrict__ state,
-    uint32_t rlo, uint32_t rhi, uint32_t* __restrict__ super_of, uint32_t* control) {
-    if (*(volatile uint32_t*)(control + kCtlHard) != 0) {
-        return;
-    }
-    for (uint32_t r = rlo + grid.bid * blockDim.x + threadIdx.x; r < rhi;
-         r += grid.nblk * blockDim.x) {
-        if (super_of[r] != kUnset) {
-            continue;
-        }
-        const uint4 me = state[r];
-        if (me.x == kNoRuler) {
-            continue;
-        }
-        uint32_t ma = me.y, mb = me.z, cur = me.x;
-        bool smallest = true, closed = false;
-        for (uint32_t hop = 0; hop < kWalkCap; ++hop) {
-            if (cur < rlo || cur >= rhi) {
-                break;
-            }
-            if (cur == r) {
-                closed = true;
-                break;
-            }
-            if (cur < r) {
-                smallest = false; // that ruler's thread closes this cycle
-                closed = true;
-                break;
-            }
-            const uint4 st = state[cur];
-            ma = min(ma, st.y);
-            mb = min(mb, st.z);
-            cur = st.x;
-        }
-        if (!closed) {
-            atomicOr(control + kCtlHard, 1u);
-            continue;
-        }
-        if (!smallest) {
-            continue;
-        }
-        const uint32_t colour = kColourTag | (ma > mb ? 1u : 0u);
-        cur = r;
-        for (uint32_t hop = 0; hop < kWalkCap; ++hop) {
-            super_of[cur] = colour;
-            cur = state[cur].x;
-            if (cur == r || cur < rlo || cur >= rhi) {
-                break;
-            }
-        }
-    }
-}
-
-__global__ void __launch_bounds__(256) ruler_super_short(const uint4* __restrict__ state,
-    uint32_t rlo, uint32_t rhi, uint32_t* __restrict__ super_of, uint32_t* control) {
-    ruler_super_short_run(launch_grid(), state, rlo, rhi, super_of, control);
-}
-
-// After the jumping: every ruler's colour, stamped into super_of in place
-// of its super-ruler (kColourTag | colour, the form ruler cycles without a
-// super-ruler already have), so level_finalize resolves a vertex's owner
-// with one dependent load instead of two.  The super-ruler states read here
-// are the buffer the last jumping round wrote (kCtlFinal).
-__device__ __forceinline__ void ruler_colour_run(Grid grid, uint32_t rlo, uint32_t rhi,
-    uint32_t* __restrict__ super_of, const uint4* __restrict__ s0, const uint4* __restrict__ s1,
-    const uint32_t* control) {
-    if (*(volatile const uint32_t*)(control + kCtlHard) != 0) {
-        return; // the level is coloured by union-find
-    }
-    const uint4* state = control[kCtlFinal] ? s1 : s0;
-    for (uint32_t r = rlo + grid.bid * blockDim.x + threadIdx.x; r < rhi;
-         r += grid.nblk * blockDim.x) {
-        const uint32_t so = super_of[r];
-        if (so == kUnset || (so & kColourTag) != 0) {
-            continue;
-        }
-        const uint4 st = state[so >> kSuperLog2];
-        super_of[r] = kColourTag | (st.y > st.z ? 1u : 0u);
-    }
-}
-
-__global__ void __launch_bounds__(256) ruler_colour(uint32_t rlo, uint32_t rhi,
-    uint32_t* super_of, const uint4* s0, const uint4* s1, const uint32_t* control) {
-    ruler_colour_run(launch_grid(), rlo, rhi, super_of, s0, s1, control);
-}
-
-// Clears the level's control words; `force_union_find` pre-sets the hard
-// flag so the level is coloured by union-find (a test hook for that path).
-__device__ __forceinline__ void control_reset_run(Grid grid, uint32_t* control, uint32_t force_union_find) {
-    if (threadIdx.x < kCtlWords) {
-        control[threadIdx.x] = threadIdx.x == kCtlHard ? force_union_find : 0u;
-    }
-}
-
-__global__ void control_reset(uint32_t* control, uint32_t force_union_find) {
-    control_reset_run(launch_grid(), control, force_union_find);
-}
-
-// Colours (from the walks, or from union-find when the level fell back),
-// children and the colour bitmap: kResolveItems pair-nodes per thread.
-// Blocks claim chunks in address order so the finds (or ruler-state reads)
-// of a chunk stay within the nodes it covers.  Every thread of a block runs
-// every claimed chunk (the colour bitmap is assembled with warp shuffles).
-template <typename T>
-__device__ __forceinline__ void level_finalize_run(Grid grid, const Plan* __restrict__ plan,
-    uint32_t level, const T* __restrict__ src, const uint32_t* __restrict__ owner,
-    const uint32_t* __restrict__ super_of, const uint4* __restrict__ state0,
-    const uint4* __restrict__ state1, uint32_t* uf,
-    uint32_t* __restrict__ xbits, uint32_t* __restrict__ dst, uint32_t* control,
+// Walks over the pair-nodes: state[r] = {successor, smallest key} of ruler
+// r's two directions.  One thread per ruler, both directions in lockstep, so
+// two loads are in flight; blocks start in address order, so the walks in
+// flight at any moment touch few nodes.  (Persistent warps that hand every
+// lane its next walk as soon as one ends took 11.8 ms per level at 2^30
+// entries: the hand-over cost more than the lanes idle behind the longest
+// walk of their warp.)  mark[r] = 0 resets the stamps of list_contract.
+__device__ __forceinline__ void level_walk_run(Grid grid, const Plan* __restrict__ plan,
+    uint32_t level, uint32_t* edge, uint4* __restrict__ state, uint32_t* __restrict__ mark,
     uint32_t* status) {
     const LevelInfo& lv = plan->levels[level];
-    const uint32_t cap = (uint32_t)lv.cap;
-    const uint32_t pcap = (uint32_t)lv.pcap;
-    const uint32_t ccap = (uint32_t)plan->levels[level + 1].cap;
-    // this call's pair-nodes [lo_pair, end); chunks start at a 32-pair
-    // boundary at or below lo_pair so colour words are written whole
+    const uint32_t ps = (uint32_t)lv.pcap;
     const NodeRange nr = level_nodes(*plan, level);
-    const uint64_t lo_pair = nr.lo * pcap;
-    const uint64_t end = lo_pair + ((uint64_t)pcap << nr.shift);
-    const uint64_t begin = lo_pair & ~31ull;
-    const uint64_t total = end - begin;
-    const bool hard = control[kCtlHard] != 0;
-    const uint4* state = control[kCtlFinal] ? state1 : state0;
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t chunk = (uint64_t)blockDim.x * kResolveItems;
-    // Walk levels claim chunks in order (ruler states of the nodes in flight
-    // stay in L2), and so do union-find levels with nodes far above L2 size
-    // (the finds of neighbouring chunks share the top of their trees).  On
-    // union-find levels with nodes near L2 size, claimed chunks would crowd
-    // every find in flight onto the root chains of one or two nodes' large
-    // components, which then serialise: those stride over the whole level
-    // (at 2^30 uniform entries, claimed order took 18.5 -> 12.5 ms on the
-    // 2^30-slot level but 14 -> 19 ms on 2^24-slot nodes).
-    uint64_t first = (uint64_t)grid.bid * chunk;
-    bool started = false;
-    const bool claimed = !hard || cap > (1ull << BPB200_FINAL_STRIDE_LOG2);
-    auto next_chunk = [&]() -> bool {
-        if (claimed) {
-            return claim_chunk(control + kCtlClaimFinal, chunk, total, &first);
+    const uint64_t pair_lo = nr.lo * ps;
+    const uint64_t pair_end = pair_lo + ((uint64_t)ps << nr.shift);
+    const ListRange rr = list_range(pair_lo, pair_end, 1);
+    bool bad = false;
+    for (uint32_t r = rr.lo + grid.bid * blockDim.x + threadIdx.x; r < rr.hi;
+         r += grid.nblk * blockDim.x) {
+        mark[r] = 0;
+        const uint32_t q = ruler_slot(r);
+        const bool in_range = q >= pair_lo && q < pair_end;
+        const uint32_t j = in_range ? q / ps : 0u;
+        const uint32_t base = j * ps;
+        const uint32_t s = in_range ? size_at(lv, level, j) : 0u;
+        const uint32_t limit = 2 * (s - s / 2);
+        const uint32_t own = 2 * (q - base);
+        if (own >= limit) {
+            state[r] = make_uint4(kNone, kNone, kNone, kNone);
+            continue;
         }
-        if (started) {
-            first += (uint64_t)grid.nblk * chunk;
-        }
-        started = true;
-        return first < total;
-    };
-    while (next_chunk()) {
-        const uint64_t p0 = begin + first + (uint64_t)threadIdx.x * kResolveItems;
-        uint32_t j = (uint32_t)(p0 / pcap);
-        uint32_t k = (uint32_t)(p0 - (uint64_t)j * pcap);
-        uint32_t s = size_at(lv, level, j);
-        uint32_t jj[kResolveItems], kk[kResolveItems], ss[kResolveItems], c[kResolveItems];
-        uint32_t live = 0;
+        uint2* node = reinterpret_cast<uint2*>(edge) + base;
+        const uint32_t bias = (s & 1u) != 0 ? 0u - (s - 1) : 0u;
+        const uint2 mine = load_live(node + (own >> 1));
+        Walk w[2] = {{mine.y, own + bias, 2 * r, mine.y < limit},
+            {mine.x, own + 1 + bias, 2 * r + 1, mine.x < limit}};
+        bad |= !w[0].live || !w[1].live;
+        for (uint32_t step = 0; (w[0].live || w[1].live) && step < kWalkCap; ++step) {
+            bool ruler[2];
+            uint2 v[2];
 #pragma unroll
-        for (int q = 0; q < kResolveItems; ++q) {
-            jj[q] = j;
-            kk[q] = k;
-            ss[q] = s;
-            c[q] = 0;
-            if (p0 + q >= lo_pair && p0 + q < end && k < s - s / 2) live |= 1u << q;
-            if (++k == pcap) {
-                k = 0;
-                ++j;
-                s = size_at(lv, level, j);
-            }
-        }
-        if (hard) {
-            uint32_t x[kResolveItems];
-            Found f[kResolveItems];
-#pragma unroll
-            for (int q = 0; q < kResolveItems; ++q) x[q] = (uint32_t)(p0 + q);
-            uf_find_many<kResolveItems>(uf, x, f, live, status, true);
-#pragma unroll
-            for (int q = 0; q < kResolveItems; ++q) {
-                if (live & (1u << q)) c[q] = f[q].bit ^ (uf[f[q].root] & 1u);
-#if BPB200_RESOLVE_WRITEBACK
-                // point the pair-node at its root (a true fact), so the
-                // finds of the pair-nodes below it end one step later
-                if ((live & (1u << q)) && f[q].root != x[q]) {
-                    uf[x[q]] = (f[q].root << 1) | f[q].bit;
-                }
-#endif
-            }
-        } else {
-            // ruler id (or direct colour) of vertex 2k: every even vertex is
-            // a ruler, stamped by the ruler walk that passes it, or stamped
-            // by the short walk of its ruler-free orbit
-            uint32_t id[kResolveItems];
-#pragma unroll
-            for (int q = 0; q < kResolveItems; ++q) {
-                if (!(live & (1u << q))) continue;
-                const uint32_t slot = jj[q] * cap + 2 * kk[q];
-                id[q] = is_ruler_slot(slot) ? slot >> kRulerLog2 : owner[jj[q] * pcap + kk[q]];
+            for (uint32_t d = 0; d < 2; ++d) {
+                ruler[d] = is_ruler(base + (w[d].enter >> 1));
+                v[d] = make_uint2(kStamp, 0u);
+                if (w[d].live && !ruler[d]) v[d] = load_live(node + (w[d].enter >> 1));
             }
 #pragma unroll
-            for (int q = 0; q < kResolveItems; ++q) {
-                if (!(live & (1u << q))) continue;
-                uint32_t colour;
-                if (id[q] == kUnset) {
-                    atomicOr(status, kErrInconsistent); // a walk must have reached it
-                    colour = 0;
-                } else if (id[q] & kColourTag) {
-                    colour = id[q] & 1u;
+            for (uint32_t d = 0; d < 2; ++d) {
+                if (!w[d].live) continue;
+                const uint32_t side = w[d].enter & 1u;
+                if ((v[d].x & kStamp) != 0) {
+                    w[d].next = side ^ (ruler[d]
+                        ? ((base + (w[d].enter >> 1)) >> kRulerLog2) << 1 : v[d].x & ~kStamp);
+                    w[d].live = false;
                 } else {
-                    // ruler -> its super-ruler's orbit minima (or a colour
-                    // stamped on a super-free ruler cycle)
-                    const uint32_t so = super_of[id[q]];
-                    if (so == kUnset) {
-                        atomicOr(status, kErrInconsistent);
-                        colour = 0;
-                    } else if (so & kColourTag) {
-                        colour = so & 1u;
-                    } else {
-                        const uint4 st = state[so >> kSuperLog2];
-                        colour = st.y > st.z ? 1u : 0u;
+                    *(volatile uint32_t*)&node[w[d].enter >> 1].x = kStamp | (r << 1) | (d ^ side);
+                    w[d].best = min(w[d].best, w[d].enter + bias);
+                    w[d].enter = side != 0 ? v[d].x : v[d].y;
+                    if (w[d].enter >= limit) {
+                        bad = true;
+                        w[d].live = false;
                     }
                 }
-                c[q] = colour;
             }
         }
-        uint32_t mine = 0; // this lane's kResolveItems colour bits
-#pragma unroll
-        for (int q = 0; q < kResolveItems; ++q) {
-            if (!(live & (1u << q))) continue;
-            mine |= c[q] << q;
-            const uint64_t node = (uint64_t)jj[q] * cap;
-            const uint64_t left = (uint64_t)(2 * jj[q]) * ccap;
-            const uint64_t right = (uint64_t)(2 * jj[q] + 1) * ccap;
-            const uint32_t half = ss[q] / 2;
-            if (kk[q] < half) {
-                const uint32_t va = (uint32_t)src[node + 2 * kk[q] + c[q]];
-                const uint32_t vb = (uint32_t)src[node + 2 * kk[q] + 1 - c[q]];
-                dst[left + kk[q]] = va >> 1;
-                dst[right + kk[q]] = vb >> 1;
-            } else {
-                dst[left + kk[q]] = (uint32_t)(src[node + ss[q] - 1] >> 1);
-            }
-        }
-        // 32 / kResolveItems lanes hold one 32-pair colour word
-        constexpr uint32_t kWordLanes = 32 / kResolveItems;
-        uint32_t v = mine << ((lane & (kWordLanes - 1)) * kResolveItems);
-#pragma unroll
-        for (uint32_t d = 1; d < kWordLanes; d <<= 1) {
-            v |= __shfl_xor_sync(0xffffffffu, v, d);
-        }
-        if ((lane & (kWordLanes - 1)) == 0 && p0 < end) {
-            xbits[p0 >> 5] = v;
-        }
+        bad |= w[0].live || w[1].live;
+        state[r] = make_uint4(w[0].next, w[0].best, w[1].next, w[1].best);
     }
+    if (bad) atomicOr(status, kErrGaveUp);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256, BPB200_FINAL_MIN_BLOCKS) level_finalize(const Plan* __restrict__ plan,
-    uint32_t level, const T* __restrict__ src, const uint32_t* __restrict__ owner,
-    const uint32_t* __restrict__ super_of, const uint4* __restrict__ state0,
-    const uint4* __restrict__ state1, uint32_t* uf,
-    uint32_t* __restrict__ xbits, uint32_t* __restrict__ dst, uint32_t* control,
+__global__ void __launch_bounds__(256, 8) level_walk(const Plan* __restrict__ plan, uint32_t level,
+    uint32_t* edge, uint4* __restrict__ state, uint32_t* __restrict__ mark, uint32_t* status) {
+    level_walk_run(launch_grid(), plan, level, edge, state, mark, status);
+}
+
+// Walks over list e (state, mark), giving list e + 1 (up_state, up_mark).
+// Same walks as level_walk with a list element's two successors in the place
+// of a pair-node's edges and its stamp in mark[]; one walk per thread, in
+// address order.
+__device__ __forceinline__ void list_contract_run(Grid grid, const Plan* __restrict__ plan,
+    uint32_t level, uint32_t e, const uint4* __restrict__ state, uint32_t* mark,
+    uint4* __restrict__ up_state, uint32_t* __restrict__ up_mark, uint32_t* status) {
+    const uint32_t ps = (uint32_t)plan->levels[level].pcap;
+    const NodeRange nr = level_nodes(*plan, level);
+    const uint64_t pair_lo = nr.lo * ps;
+    const uint64_t pair_end = pair_lo + ((uint64_t)ps << nr.shift);
+    const ListRange from = list_range(pair_lo, pair_end, e);
+    const ListRange to = list_range(pair_lo, pair_end, e + 1);
+    uint2* half = reinterpret_cast<uint2*>(up_state);
+    bool bad = false;
+    for (uint64_t unit = 2ull * to.lo + (uint64_t)grid.bid * blockDim.x + threadIdx.x;
+         unit < 2ull * to.hi; unit += (uint64_t)grid.nblk * blockDim.x) {
+        const uint32_t up = (uint32_t)(unit >> 1);
+        const uint32_t r = ruler_slot(up);
+        if ((unit & 1) == 0) up_mark[up] = 0;
+        uint4 st = make_uint4(kNone, kNone, kNone, kNone);
+        if (r >= from.lo && r < from.hi) st = state[r];
+        if (st.x == kNone) {
+            half[unit] = make_uint2(kNone, kNone);
+            continue;
+        }
+        uint32_t cur = (r << 1) | (uint32_t)(unit & 1);
+        uint32_t m = ~0u, next = kNone;
+        for (uint32_t step = 0; next == kNone; ++step) {
+            m = min(m, around(st) ^ (cur & 1u));
+            cur = (cur & 1u) != 0 ? st.z : st.x;
+            const uint32_t at = cur >> 1;
+            if (at < from.lo || at >= from.hi || step == kWalkCap) {
+                bad = true;
+                next = (uint32_t)unit;
+            } else if (is_ruler(at)) {
+                next = ((at >> kRulerLog2) << 1) | (cur & 1u);
+            } else {
+                st = state[at];
+                const uint32_t stamp = load_live(mark + at);
+                if ((stamp & kStamp) != 0) {
+                    next = (stamp & ~kStamp) ^ (cur & 1u);
+                } else {
+                    *(volatile uint32_t*)(mark + at) = kStamp | ((uint32_t)unit ^ (cur & 1u));
+                }
+            }
+        }
+        half[unit] = make_uint2(next, m);
+    }
+    if (bad) atomicOr(status, kErrGaveUp);
+}
+
+__global__ void __launch_bounds__(256) list_contract(const Plan* __restrict__ plan,
+    uint32_t level, uint32_t e, const uint4* __restrict__ state, uint32_t* mark,
+    uint4* __restrict__ up_state, uint32_t* __restrict__ up_mark, uint32_t* status) {
+    list_contract_run(launch_grid(), plan, level, e, state, mark, up_state, up_mark, status);
+}
+
+// Colours of list e's elements (colour[i]: the colour of paths that enter
+// element i in direction 0) from those of list e + 1.
+__device__ __forceinline__ void list_expand_run(Grid grid, const Plan* __restrict__ plan,
+    uint32_t level, uint32_t e, const uint4* __restrict__ state,
+    const uint32_t* __restrict__ mark, const uint8_t* __restrict__ up_colour,
+    uint8_t* __restrict__ colour, uint32_t* status) {
+    const uint32_t ps = (uint32_t)plan->levels[level].pcap;
+    const NodeRange nr = level_nodes(*plan, level);
+    const uint64_t pair_lo = nr.lo * ps;
+    const uint64_t pair_end = pair_lo + ((uint64_t)ps << nr.shift);
+    const ListRange from = list_range(pair_lo, pair_end, e);
+    const ListRange to = list_range(pair_lo, pair_end, e + 1);
+    bool bad = false;
+    for (uint32_t i = from.lo + grid.bid * blockDim.x + threadIdx.x; i < from.hi;
+         i += grid.nblk * blockDim.x) {
+        const uint32_t stamp = mark[i];
+        uint32_t c;
+        if (is_ruler(i)) {
+            c = up_colour[i >> kRulerLog2];
+        } else if ((stamp & kStamp) != 0) {
+            const uint32_t up = (stamp & ~kStamp) >> 1;
+            const bool in_range = up >= to.lo && up < to.hi;
+            bad |= !in_range;
+            c = in_range ? up_colour[up] ^ (stamp & 1u) : 0u;
+        } else {
+            uint4 st = state[i];
+            if (st.x == kNone) continue;
+            uint32_t cur = i << 1, m = ~0u, step = 0;
+            do {
+                m = min(m, around(st) ^ (cur & 1u));
+                cur = (cur & 1u) != 0 ? st.z : st.x;
+                const uint32_t at = cur >> 1;
+                if (at < from.lo || at >= from.hi || ++step == kShortCap) {
+                    bad = true;
+                    break;
+                }
+                st = state[at];
+            } while (cur != i << 1);
+            c = m & 1u;
+        }
+        colour[i] = (uint8_t)(c & 1u);
+    }
+    if (bad) atomicOr(status, kErrGaveUp);
+}
+
+__global__ void __launch_bounds__(256) list_expand(const Plan* __restrict__ plan, uint32_t level,
+    uint32_t e, const uint4* __restrict__ state, const uint32_t* __restrict__ mark,
+    const uint8_t* __restrict__ up_colour, uint8_t* __restrict__ colour, uint32_t* status) {
+    list_expand_run(launch_grid(), plan, level, e, state, mark, up_colour, colour, status);
+}
+
+// Most elements of one node in list e (one more at either end when nodes
+// start inside an element's bucket).
+BP_HD uint32_t list_node_max(uint64_t ps, uint32_t e) {
+    const uint32_t sh = kRulerLog2 * e;
+    return (ps & ((1ull << sh) - 1)) == 0 ? (uint32_t)(ps >> sh) : (uint32_t)((ps - 1) >> sh) + 2;
+}
+
+// Dynamic shared memory of list_rank for nodes of `count` elements.
+BP_HD uint32_t rank_smem(uint32_t count) {
+    const uint32_t rulers = ((count - 1) >> kRulerLog2) + 1;
+    return count * 8 + rulers * 16;
+}
+constexpr uint32_t kRankThreads = 1024;
+constexpr uint32_t kRankBatch = 5; // directed states per thread, at least 2 * rulers / threads
+
+// Threads of a list_rank launch: one per 4 elements, so a thread's loads of
+// list states are few; at most kRankBatch directed states each.
+BP_HD uint32_t rank_threads(uint32_t count) {
+    uint32_t t = 128;
+    while (t < kRankThreads && t * 4 < count) t *= 2;
+    return t;
+}
+
+// Colours of every element of list e, one CTA per node: the node's list is
+// contracted once more in shared memory by the tile's ruler walk and
+// finished by pointer tripling over the rulers.  Element i's word holds the
+// local directed successors: low half that of direction 1, high half that of
+// direction 0 (so a path entering at side b leaves through half b ^ 1, as
+// with a pair-node's edges), or a stamp.
+__device__ __forceinline__ void list_rank_run(Grid grid, const Plan* __restrict__ plan,
+    uint32_t level, uint32_t e, const uint4* __restrict__ state, uint8_t* __restrict__ colour,
+    uint32_t* status, uint32_t* smem) {
+    const uint32_t ps = (uint32_t)plan->levels[level].pcap;
+    const NodeRange nr = level_nodes(*plan, level);
+    const uint32_t tid = threadIdx.x;
+    bool bad = false;
+    for (uint64_t j = nr.lo + grid.bid; j < nr.lo + (1ull << nr.shift); j += grid.nblk) {
+        const uint64_t pair_lo = j * ps;
+        const ListRange range = list_range(pair_lo, pair_lo + ps, e);
+        const uint32_t count = range.hi - range.lo;
+        const uint32_t rulers = ((count - 1) >> kRulerLog2) + 1;
+        volatile uint32_t* link = smem;
+        volatile uint16_t* link16 = reinterpret_cast<volatile uint16_t*>(smem);
+        uint32_t* key = smem + count;
+        uint32_t* smin = key + count;      // 2 * rulers
+        uint32_t* snext = smin + 2 * rulers;
+        __syncthreads(); // the previous node's arrays are free
+        for (uint32_t i = tid; i < count; i += blockDim.x) {
+            const uint32_t q = pair_of(range.lo + i, e);
+            const bool mine = q >= pair_lo && q < pair_lo + ps;
+            const uint4 st = mine ? state[range.lo + i] : make_uint4(kNone, 0, 0, 0);
+            uint32_t word = 0x8000u; // not here: nothing leads to it
+            uint32_t k = ~0u;
+            if (st.x != kNone) {
+                uint32_t a = st.x - 2 * range.lo, b = st.z - 2 * range.lo;
+                if (a >= 2 * count || b >= 2 * count) {
+                    bad = true;
+                    a = 2 * i;
+                    b = 2 * i + 1;
+                }
+                word = b | (a << 16);
+                k = around(st);
+            }
+            key[i] = k;
+            link[i] = word;
+        }
+        __syncthreads();
+        // rulers first: their word moves to the state, a stamp takes its place
+        for (uint32_t r = tid; r < rulers; r += blockDim.x) {
+            const uint32_t i = ruler_slot(r);
+            const uint32_t word = i < count ? link[i] : 0x8000u;
+            snext[2 * r] = word;
+            if ((word & 0x8000u) == 0) link16[2 * i] = (uint16_t)(0x8000u | (r << 1));
+        }
+        __syncthreads();
+        for (uint32_t r = tid; r < rulers; r += blockDim.x) {
+            const uint32_t word = snext[2 * r];
+            if ((word & 0x8000u) != 0) {
+                snext[2 * r] = 2 * r;
+                snext[2 * r + 1] = 2 * r + 1;
+                smin[2 * r] = smin[2 * r + 1] = ~0u;
+                continue;
+            }
+            const uint32_t own = key[ruler_slot(r)];
+            uint32_t wa = word >> 16, wb = word & 0xffffu;
+            uint32_t ma = own, mb = own ^ 1u;
+            bool ga = true, gb = true;
+            uint32_t va = 0, vb = 0;
+            for (uint32_t step = 0; (ga || gb) && step <= count; ++step) {
+                va = link[wa >> 1];
+                vb = link[wb >> 1];
+                ga = (va & 0x8000u) == 0;
+                gb = (vb & 0x8000u) == 0;
+                if (ga) {
+                    link16[wa & ~1u] = (uint16_t)(0x8000u | (r << 1) | (wa & 1u));
+                    ma = min(ma, key[wa >> 1] ^ (wa & 1u));
+                    wa = (wa & 1u) != 0 ? va & 0xffffu : va >> 16;
+                }
+                if (gb) {
+                    link16[wb & ~1u] = (uint16_t)(0x8000u | (r << 1) | (~wb & 1u));
+                    mb = min(mb, key[wb >> 1] ^ (wb & 1u));
+                    wb = (wb & 1u) != 0 ? vb & 0xffffu : vb >> 16;
+                }
+            }
+            const uint32_t na = ga ? 2 * r : (va & 0x7fffu) ^ (wa & 1u);
+            const uint32_t nb = gb ? 2 * r + 1 : (vb & 0x7fffu) ^ (wb & 1u);
+            bad |= ga || gb || na >= 2 * rulers || nb >= 2 * rulers;
+            const uint32_t m = min(ma, mb ^ 1u);
+            smin[2 * r] = m;
+            smin[2 * r + 1] = m ^ 1u;
+            snext[2 * r] = na < 2 * rulers ? na : 2 * r;
+            snext[2 * r + 1] = nb < 2 * rulers ? nb : 2 * r + 1;
+        }
+        __syncthreads();
+        for (uint32_t reach = 1; reach < rulers + 1; reach *= 3) {
+            uint32_t om[kRankBatch], on[kRankBatch];
+#pragma unroll
+            for (uint32_t b = 0; b < kRankBatch; ++b) {
+                const uint32_t i = tid + b * blockDim.x;
+                if (i >= 2 * rulers) continue;
+                const uint32_t n1 = snext[i];
+                const uint32_t n2 = snext[n1];
+                om[b] = min(smin[i], min(smin[n1], smin[n2]));
+                on[b] = snext[n2];
+            }
+            __syncthreads();
+#pragma unroll
+            for (uint32_t b = 0; b < kRankBatch; ++b) {
+                const uint32_t i = tid + b * blockDim.x;
+                if (i >= 2 * rulers) continue;
+                smin[i] = om[b];
+                snext[i] = on[b];
+            }
+            __syncthreads();
+        }
+        for (uint32_t i = tid; i < count; i += blockDim.x) {
+            const uint32_t word = link[i];
+            uint32_t c;
+            if ((word & 0x8000u) != 0) {
+                if (key[i] == ~0u) continue; // another node's, or absent
+                const uint32_t r2 = word & 0x7ffeu;
+                c = r2 < 2 * rulers ? smin[r2] ^ word : 0u;
+            } else { // a cycle without rulers
+                uint32_t cur = 2 * i, v = word, m = ~0u, step = 0;
+                do {
+                    m = min(m, key[cur >> 1] ^ (cur & 1u));
+                    cur = (cur & 1u) != 0 ? v & 0xffffu : v >> 16;
+                    if (cur >= 2 * count || ++step == kShortCap) {
+                        bad = true;
+                        break;
+                    }
+                    v = link[cur >> 1];
+                } while (cur != 2 * i);
+                c = m;
+            }
+            colour[range.lo + i] = (uint8_t)(c & 1u);
+        }
+    }
+    if (bad) atomicOr(status, kErrGaveUp);
+}
+
+__global__ void __launch_bounds__(kRankThreads, 1) list_rank(const Plan* __restrict__ plan,
+    uint32_t level, uint32_t e, const uint4* __restrict__ state, uint8_t* __restrict__ colour,
     uint32_t* status) {
-    level_finalize_run<T>(launch_grid(), plan, level, src, owner, super_of, state0, state1, uf, xbits, dst, control, status);
+    extern __shared__ __align__(16) uint32_t rank_shared[];
+    list_rank_run(launch_grid(), plan, level, e, state, colour, status, rank_shared);
+}
+
+// Input switch bits of a walk level: the colour of input 2k of every
+// pair-node k, from the stamp of the walk that passed it and that ruler's
+// colour.  One thread per pair-node, in address order.
+__device__ __forceinline__ void level_colours_run(Grid grid, const Plan* __restrict__ plan,
+    uint32_t level, const uint32_t* __restrict__ edge, const uint8_t* __restrict__ colour,
+    uint32_t* __restrict__ xbits, uint32_t* status) {
+    const LevelInfo& lv = plan->levels[level];
+    const uint32_t ps = (uint32_t)lv.pcap;
+    // this call's pair-nodes; the loop starts at a 32-pair boundary so each
+    // warp assembles whole bit words (bits before `first` stay zero)
+    const NodeRange nr = level_nodes(*plan, level);
+    const uint64_t first = nr.lo * ps;
+    const uint64_t end = first + ((uint64_t)ps << nr.shift);
+    const ListRange rr = list_range(first, end, 1);
+    const uint2* pairs = reinterpret_cast<const uint2*>(edge);
+    bool bad = false;
+    for (uint64_t p = (first & ~31ull) + (uint64_t)grid.bid * blockDim.x + threadIdx.x;
+         p - (threadIdx.x & 31) < end; p += (uint64_t)grid.nblk * blockDim.x) {
+        uint32_t x = 0;
+        if (p >= first && p < end) {
+            const uint32_t q = (uint32_t)p;
+            const uint2 v = pairs[q];
+            if (is_ruler(q)) {
+                x = colour[q >> kRulerLog2];
+            } else if ((v.x & kStamp) != 0) {
+                const uint32_t r = (v.x & ~kStamp) >> 1;
+                // padding pair-nodes hold anything; their bits are not used
+                if (r >= rr.lo && r < rr.hi) x = colour[r] ^ v.x;
+            } else {
+                const uint32_t j = q / ps;
+                const uint32_t k = q - j * ps;
+                const uint32_t s = size_at(lv, level, j);
+                const uint32_t limit = 2 * (s - s / 2);
+                if (2 * k < limit) { // a cycle without rulers: walk it whole
+                    const uint2* node = pairs + (uint64_t)j * ps;
+                    const uint32_t bias = (s & 1u) != 0 ? 0u - (s - 1) : 0u;
+                    uint32_t cur = 2 * k, step = 0;
+                    uint2 word = v;
+                    x = ~0u;
+                    do {
+                        x = min(x, cur + bias);
+                        cur = (cur & 1u) != 0 ? word.x : word.y;
+                        if (cur >= limit || ++step == kShortCap) {
+                            bad = true;
+                            break;
+                        }
+                        word = node[cur >> 1];
+                    } while (cur != 2 * k);
+                }
+            }
+        }
+        const unsigned word = __ballot_sync(0xffffffffu, (x & 1u) != 0);
+        if ((threadIdx.x & 31) == 0) {
+            xbits[p >> 5] = word;
+        }
+    }
+    if (bad) atomicOr(status, kErrGaveUp);
+}
+
+__global__ void __launch_bounds__(256) level_colours(const Plan* __restrict__ plan,
+    uint32_t level, const uint32_t* __restrict__ edge, const uint8_t* __restrict__ colour,
+    uint32_t* __restrict__ xbits, uint32_t* status) {
+    level_colours_run(launch_grid(), plan, level, edge, colour, xbits, status);
 }
 
 } // namespace bpb200

@@ -36,3 +36,19 @@ def test_tile_nodes(gpu, oracle, n):
         for kind in (kinds.uniform, kinds.single_cycle, kinds.identity, kinds.reverse):
             check(gpu, oracle, n, n + m, kind, np.uint64 if m == 2 else np.uint32,
                   middle_group_log2=m)
+
+
+@pytest.mark.parametrize("n", [8193, 8194, 16385, 16386, 16387, 32771, (1 << 17) + 6, (1 << 18) - 1,
+                               1 << 18, (1 << 18) + 2, (1 << 18) + 3, (1 << 20) + 1])
+@pytest.mark.parametrize("jump", [10, 14])
+def test_walk_lists(gpu, oracle, n, jump):
+    """Global levels coloured by walks, with nodes ranked straight from their
+    rulers and after one to three contractions; random and structured."""
+    kinds = gpu.PermutationKind
+    gpu.set_tuning({"jump_block_log2": jump, "tile_max_log2": 13})
+    try:
+        for i, kind in enumerate((kinds.uniform, kinds.single_cycle, kinds.identity,
+                                  kinds.reverse)):
+            check(gpu, oracle, n, n + i, kind, np.uint64 if i & 1 else np.uint32)
+    finally:
+        gpu.set_tuning(None)
