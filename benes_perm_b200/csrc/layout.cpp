@@ -300,6 +300,15 @@ Error make_plan(const Layout& L, uint64_t tile_max, Plan* out) {
         for (uint32_t c = 0; c <= 32; ++c) {
             p.fact_bits[c] = factoradic_bits(c);
         }
+        for (uint32_t i = 1; i <= 32; ++i) {
+            p.digit_reciprocal[i] = i > 1 ? 0xffffffffu / i + 1u : 0u;
+            uint32_t product = i, digits = 1;
+            while (digits < i && (uint64_t)product * (i - digits) < (1u << 27)) {
+                product *= i - digits;
+                ++digits;
+            }
+            p.digit_groups[i] = {~0ull / product, product, digits};
+        }
         return {};
     } catch (const Fail& f) {
         return {f.code, f.message};

@@ -15,6 +15,8 @@
 
 #include "plan.hpp"
 
+#include <cstdint>
+
 namespace bpb200 {
 
 // Status bits of one lookup (ORed over a batch).
@@ -41,95 +43,190 @@ BP_HD uint32_t blob_bit(const BlobBits& b, uint64_t offset, uint64_t bit, uint32
     return (uint32_t)(b.data[byte] >> (bit & 7)) & 1u;
 }
 
-// `bits` (<= 128) bits from bit `first` of the section at byte `offset`,
-// LSB-first into lo/hi (read_rank, src/internal.hpp:1015-1033), a byte at
-// a time.
+// Bits [first, first + bits) (bits <= 128) of the section at byte `offset`,
+// LSB-first (read_rank, src/internal.hpp:1015-1033): 32-bit words from the
+// aligned word that holds the first bit; words that reach over either end of
+// the blob are put together from its bytes.
 BP_HD void blob_rank(const BlobBits& b, uint64_t offset, uint64_t first, uint32_t bits,
-    uint64_t* lo, uint64_t* hi, uint32_t* status) {
-    *lo = 0;
-    *hi = 0;
-    uint32_t i = 0;
-    while (i < bits) {
-        const uint64_t at = first + i;
-        const uint64_t byte = offset + (at >> 3);
-        if (byte >= b.len) {
-            *status |= kLookupTruncated;
-            return;
-        }
-        const uint32_t shift = (uint32_t)(at & 7);
-        uint32_t take = 8 - shift;
-        if (take > bits - i) {
-            take = bits - i;
-        }
-        const uint64_t v = (uint64_t)((b.data[byte] >> shift) & ((1u << take) - 1));
-        if (i < 64) {
-            *lo |= v << i;
-            if (i + take > 64) {
-                *hi |= v >> (64 - i);
+    uint32_t (&rank)[4], uint32_t* status) {
+    rank[0] = rank[1] = rank[2] = rank[3] = 0;
+    if (bits == 0) {
+        return;
+    }
+    if (offset + ((first + bits - 1) >> 3) >= b.len) {
+        *status |= kLookupTruncated;
+        return;
+    }
+    const uintptr_t base = (uintptr_t)b.data;
+    const uint64_t at = (uint64_t)(base & 3) * 8 + offset * 8 + first; // bit from the aligned base
+    const uint32_t shift = (uint32_t)(at & 31);
+    const uint64_t word0 = at >> 5;
+    const uint32_t words = (shift + bits + 31) >> 5; // 1..5
+    uint32_t below = 0;
+    for (uint32_t i = 0; i < 5; ++i) {
+        uint32_t w = 0;
+        if (i < words) {
+            // byte range of the word inside the blob
+            const int64_t lo = (int64_t)((word0 + i) * 4) - (int64_t)(base & 3);
+            if (lo >= 0 && (uint64_t)lo + 4 <= b.len) {
+                w = *reinterpret_cast<const uint32_t*>(b.data + lo);
+            } else {
+                for (int k = 0; k < 4; ++k) {
+                    if (lo + k >= 0 && (uint64_t)(lo + k) < b.len) {
+                        w |= (uint32_t)b.data[lo + k] << (8 * k);
+                    }
+                }
             }
-        } else {
-            *hi |= v << (i - 64);
         }
-        i += take;
+        if (i > 0) {
+            rank[i - 1] = shift == 0 ? below : (below >> shift) | (w << (32 - shift));
+        }
+        below = w;
+    }
+    for (uint32_t i = 0; i < 4; ++i) { // drop the bits of the next rank
+        const uint32_t keep = bits > 32 * i ? bits - 32 * i : 0;
+        if (keep < 32) rank[i] &= (1u << keep) - 1u;
     }
 }
 
-// (lo, hi) /= d in place for 1 <= d <= 32; returns the remainder.  Long
-// division over 32-bit limbs: the running remainder stays below d, so each
-// step's dividend fits in 37 bits.
-BP_HD uint32_t divide_small(uint64_t* lo, uint64_t* hi, uint32_t d) {
-    uint64_t rem = 0;
-    uint64_t limb[4] = {*hi >> 32, *hi & 0xffffffffull, *lo >> 32, *lo & 0xffffffffull};
-    for (int k = 0; k < 4; ++k) {
-        const uint64_t cur = (rem << 32) | limb[k];
-        limb[k] = cur / d;
-        rem = cur % d;
-    }
-    *hi = (limb[0] << 32) | limb[1];
-    *lo = (limb[2] << 32) | limb[3];
-    return (uint32_t)rem;
+BP_HD uint32_t mul_high(uint32_t a, uint32_t b) {
+    return (uint32_t)(((uint64_t)a * b) >> 32);
 }
-
-// Position of the (k+1)-th lowest set bit of `mask` (k < popcount(mask)).
-BP_HD uint32_t nth_set_bit(uint32_t mask, uint32_t k) {
-    for (uint32_t i = 0; i < k; ++i) {
-        mask &= mask - 1;
-    }
+BP_HD uint64_t mul_high(uint64_t a, uint64_t b) {
 #if defined(__CUDA_ARCH__)
-    return (uint32_t)__ffs(mask) - 1;
+    return __umul64hi(a, b);
 #else
-    return (uint32_t)__builtin_ctz(mask);
+    return (uint64_t)(((unsigned __int128)a * b) >> 64);
 #endif
 }
 
 // Leaf step of the lookup: the local permutation of `size` (<= 32) entries
-// encoded by the factoradic rank (lo, hi), applied forward to `index`
-// (p[index]) or inverted (the i with p[i] == index).
+// encoded by the factoradic rank, applied forward to `index` (p[index]) or
+// inverted (the i with p[i] == index).
 //
 // The rank is the mixed-radix number with digits d[i] = #{k < i : p[k] <
 // p[i]}, radix i + 1 (encode_factoradic, src/internal.hpp:148-167), so the
-// lowest digit is d[size-1].  Peeling digits from the top entry down, p[i]
-// is the d[i]-th smallest value not yet taken by an entry above i; the peel
-// stops as soon as the wanted entry is known.
-BP_HD uint32_t leaf_apply(uint64_t lo, uint64_t hi, uint32_t size, uint32_t index, bool inverse) {
-    uint32_t free_values = size >= 32 ? 0xffffffffu : ((1u << size) - 1);
-    for (uint32_t i = size; i-- > 0;) {
-        const uint32_t digit = divide_small(&lo, &hi, i + 1);
-        const uint32_t value = nth_set_bit(free_values, digit);
-        free_values &= ~(1u << value);
-        if (!inverse && i == index) {
-            return value;
+// lowest digit is d[size-1].  Digits come off from the top entry down: one
+// long division of the rank by the product of the next radices (below 2^27)
+// leaves a remainder whose digits are 32-bit divisions by a reciprocal,
+// floor(n / r) = mul_high(n, ceil(2^32 / r)), exact while n * r < 2^32.  The
+// long division's limbs are divided by a 64-bit reciprocal rounded down,
+// whose quotient is at most one too small.
+// Inverse: entry k has the d[k]-th smallest value of the entries up to k, so
+// the wanted value's rank t among them either is d[k], or loses one when
+// d[k] < t.  Forward: the same steps backwards, from entry `index` up:
+// p[index] starts as d[index] and gains one for every later entry whose
+// digit is not above it.
+BP_HD uint32_t leaf_apply(const Plan& p, uint32_t (&rank)[4], uint32_t size,
+    uint32_t index, bool inverse) {
+    uint8_t digits[32];
+    uint32_t t = index;
+    uint32_t i = size;
+    while (i > 0) {
+        const DigitGroup group = p.digit_groups[i];
+        uint64_t rem = 0;
+        for (int k = 3; k >= 0; --k) {
+            if (rem == 0 && rank[k] == 0) {
+                continue; // leading zero limbs
+            }
+            const uint64_t cur = (rem << 32) | rank[k];
+            uint64_t quot = mul_high(cur, group.reciprocal);
+            rem = cur - quot * group.product;
+            if (rem >= group.product) {
+                rem -= group.product;
+                ++quot;
+            }
+            rank[k] = (uint32_t)quot;
         }
-        if (inverse && value == index) {
-            return i;
+        uint32_t rest = (uint32_t)rem;
+        for (uint32_t g = 0; g < group.digits; ++g) {
+            const uint32_t radix = i--; // entry i's digit, after the decrement
+            uint32_t digit = 0;
+            if (radix > 1) {
+                const uint32_t q = mul_high(rest, p.digit_reciprocal[radix]);
+                digit = rest - q * radix;
+                rest = q;
+            }
+            if (inverse) {
+                if (digit == t) {
+                    return i;
+                }
+                t -= digit < t ? 1u : 0u;
+            } else if (i == index) {
+                uint32_t value = digit;
+                for (uint32_t k = index + 1; k < size; ++k) {
+                    value += digits[k] <= value ? 1u : 0u;
+                }
+                return value;
+            } else {
+                digits[i] = (uint8_t)digit;
+            }
         }
     }
     return 0; // unreachable for index < size
 }
 
+// Switch addresses along one query's path through one section.  All nodes of
+// the path inside one cluster group share the cluster root, so its base is
+// worked out once per group; below it only the packet that holds the wanted
+// pair is looked at (node_address works out both kinds).
+struct PathAddress {
+    uint64_t base = 0;  // blob bit of the cluster's packets
+    uint64_t root_count = 0;
+    uint64_t packet_bits = 0;
+    uint32_t group = ~0u;
+    uint32_t rs = 0;
+
+    template <typename Int>
+    BP_HD uint64_t bit(const Plan& p, int side, uint32_t level, Int node, Int size, Int pair) {
+        const LevelSide& ls = p.levels[level].side[side];
+        const GroupInfo& gi = p.groups[side][ls.group];
+        const uint32_t rel = ls.rel;
+        if (ls.group != group) {
+            group = ls.group;
+            base = p.section_offset[side] * 8 + cluster_base(p, side, group, level, node);
+            rs = node_is_large(p.levels[gi.start], gi.start, node >> rel) ? 1u : 0u;
+            root_count = p.levels[gi.start].q + rs;
+            packet_bits = gi.packet_bits[rs];
+        }
+        const Int path = node & (((Int)1 << rel) - 1);
+        const uint32_t span_log2 = gi.depth - rel - 1;
+        const Int packet = pair >> span_log2;
+        const uint64_t at = base + packet * packet_bits + (pair & (((Int)1 << span_log2) - 1));
+        if (packet == (size / 2 - 1) >> span_log2) {
+            return at + ls.prefix_tail[rs][size != (Int)p.levels[level].q ? 1 : 0] +
+                packet_path_bits(root_count, gi.depth, rel, packet, path, p.leaf);
+        }
+        // a node with a packet after this one fills it, and then so does
+        // every node of the level but for a short tail of the smallest
+        const Int span = (Int)1 << span_log2;
+        const Int small = (Int)(root_count >> rel);
+        if (small > p.leaf && small / 2 >= span) {
+            return at + ls.prefix0[rs] + ((uint64_t)path << span_log2);
+        }
+        return at + ls.prefix0[rs] +
+            packet_path_bits(root_count, gi.depth, rel, 0, path, p.leaf);
+    }
+};
+
+// node_size, in 32 bits where those hold every index.
+BP_HD uint64_t path_node_size(const LevelInfo& lv, uint32_t level, uint64_t node) {
+    return node_size(lv, level, node);
+}
+BP_HD uint32_t path_node_size(const LevelInfo& lv, uint32_t level, uint32_t node) {
+#if defined(__CUDA_ARCH__)
+    const uint32_t reversed = level == 0 ? 0u : __brev(node) >> (32 - level);
+#else
+    const uint32_t reversed = (uint32_t)reverse_bits(node, level);
+#endif
+    return (uint32_t)lv.q + (reversed < (uint32_t)lv.r ? 1u : 0u);
+}
+
 // Forward (p[value]) or inverse (p^-1[value]) lookup.  Returns a
-// LookupStatus; *out is valid when it is kLookupOk.
-BP_HD uint32_t lookup_one(const Plan& p, const BlobBits& blob, uint64_t value, bool inverse,
+// LookupStatus; *out is valid when it is kLookupOk.  Int holds every index
+// and node of the permutation: 32 bits up to 2^31 entries, else 64.
+template <typename Int>
+BP_HD uint32_t lookup_path(const Plan& p, const BlobBits& blob, uint64_t value, bool inverse,
     uint64_t* out) {
     if (value >= p.n) {
         return kLookupOutOfRange;
@@ -137,42 +234,50 @@ BP_HD uint32_t lookup_one(const Plan& p, const BlobBits& blob, uint64_t value, b
     uint32_t status = 0;
     const int down = inverse ? 1 : 0; // section read on the way down
     const int up = 1 - down;
-    uint64_t index = value;
-    uint64_t node = 0;
-    uint64_t size = p.n;
+    Int index = (Int)value;
+    Int node = 0;
+    Int size = (Int)p.n;
     uint32_t level = 0;
+    PathAddress way_down;
     while (size > p.leaf) {
         if (level >= p.depth) {
             return kLookupBadPlan;
         }
         bool right = false;
         if ((size & 1) == 0 || index != size - 1) { // the odd tail passes straight left
-            const uint64_t bit = switch_bit(node_address(p, down, level, node), index >> 1);
-            right = blob_bit(blob, p.section_offset[down], bit, &status) != (uint32_t)(index & 1);
+            const uint64_t bit = way_down.bit(p, down, level, node, size, index >> 1);
+            right = blob_bit(blob, 0, bit, &status) != (uint32_t)(index & 1);
         }
         index >>= 1;
         node = 2 * node + (right ? 1 : 0);
         ++level;
-        size = node_size(p.levels[level], level, node);
+        size = path_node_size(p.levels[level], level, node);
     }
     int section = 0;
     const uint64_t rank_bit = leaf_rank_bit(p, level, node, &section);
-    uint64_t lo = 0, hi = 0;
-    blob_rank(blob, p.section_offset[section], rank_bit, p.fact_bits[size], &lo, &hi, &status);
-    index = leaf_apply(lo, hi, (uint32_t)size, (uint32_t)index, inverse);
+    uint32_t rank[4];
+    blob_rank(blob, p.section_offset[section], rank_bit, p.fact_bits[size], rank, &status);
+    index = leaf_apply(p, rank, (uint32_t)size, (uint32_t)index, inverse);
+    PathAddress way_up;
     for (uint32_t l = level; l-- > 0;) {
-        const uint64_t at = node >> (level - l);
+        const Int at = node >> (level - l);
         const uint32_t right = (uint32_t)(node >> (level - 1 - l)) & 1u;
-        const uint64_t count = node_size(p.levels[l], l, at);
+        const Int count = path_node_size(p.levels[l], l, at);
         if (right == 0 && (count & 1) != 0 && index == count / 2) {
             index = count - 1; // back out through the odd tail
             continue;
         }
-        const uint64_t bit = switch_bit(node_address(p, up, l, at), index);
-        index = 2 * index + (right ^ blob_bit(blob, p.section_offset[up], bit, &status));
+        const uint64_t bit = way_up.bit(p, up, l, at, count, index);
+        index = 2 * index + (right ^ blob_bit(blob, 0, bit, &status));
     }
     *out = index;
     return status;
+}
+
+BP_HD uint32_t lookup_one(const Plan& p, const BlobBits& blob, uint64_t value, bool inverse,
+    uint64_t* out) {
+    return p.n <= (1ull << 31) ? lookup_path<uint32_t>(p, blob, value, inverse, out)
+                               : lookup_path<uint64_t>(p, blob, value, inverse, out);
 }
 
 } // namespace bpb200

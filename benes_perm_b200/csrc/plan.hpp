@@ -62,6 +62,14 @@ struct LevelInfo {
     LevelSide side[2];     // 0 = input section, 1 = output section
 };
 
+// Radices i, i - 1, ... of a factoradic rank whose product stays below 2^27,
+// taken off the rank with one long division (lookup.hpp).
+struct DigitGroup {
+    uint64_t reciprocal; // floor((2^64 - 1) / product)
+    uint32_t product;
+    uint32_t digits;
+};
+
 struct Plan {
     uint64_t n;
     uint32_t leaf;         // 2^middle_group_log2
@@ -77,6 +85,8 @@ struct Plan {
     uint64_t max_slots;         // max over levels of 2^l * 2 * pcap_l
     uint64_t max_pairs;         // max over levels of 2^l * pcap_l
     uint32_t fact_bits[33];     // ceil(log2(c!)) for c = 0..32
+    uint32_t digit_reciprocal[33]; // ceil(2^32 / r) for r = 2..32
+    DigitGroup digit_groups[33];   // from radix i down, i = 1..32
     // Subtree sharding: with shards = 2^shard_level > 1 this call encodes
     // every node of the levels above shard_level and, from shard_level on,
     // only the subtree of node `shard` of level shard_level (see
@@ -183,6 +193,9 @@ BP_HD uint64_t packet_path_bits(uint64_t root, uint32_t depth, uint32_t rel,
         } else {
             share[big] = pairs - first < span ? pairs - first : span;
         }
+    }
+    if (share[0] == share[1]) { // every packet but a short tail: no node sizes needed
+        return paths * share[0];
     }
     const uint64_t nl = count_large(paths, rel, large);
     return nl * share[1] + (paths - nl) * share[0];

@@ -52,3 +52,22 @@ def test_walk_lists(gpu, oracle, n, jump):
             check(gpu, oracle, n, n + i, kind, np.uint64 if i & 1 else np.uint32)
     finally:
         gpu.set_tuning(None)
+
+
+@pytest.mark.parametrize("n,m,placement", [(33, 5, 0), (4097, 1, 1), (70001, 4, 2), (65536, 5, 0)])
+@pytest.mark.parametrize("shift", [0, 1, 3])
+def test_lookup_words(gpu, oracle, n, m, placement, shift):
+    """Lookups of every entry in a blob at any byte alignment: ranks are read
+    as aligned words, the first and last of which reach over its ends."""
+    import torch
+    kw = dict(middle_group_log2=m, middle_placement=placement)
+    perm = gpu.fill_permutation(gpu.PermutationKind.uniform, n + m, n, np.uint64)
+    blob = oracle.compress(perm, oracle_format(kw))
+    room = torch.zeros(len(blob) + shift, dtype=torch.uint8, device="cuda")
+    room[shift:] = torch.frombuffer(bytearray(blob), dtype=torch.uint8).cuda()
+    out = torch.empty(n, dtype=torch.int64, device="cuda")
+    want = torch.from_numpy(perm.astype(np.int64))
+    for inverse in (False, True):
+        gpu.lookup_device(room.data_ptr() + shift, len(blob), n, b200_format(gpu, kw),
+                          out.data_ptr(), n, inverse=inverse)
+        assert torch.equal(out.cpu(), torch.argsort(want) if inverse else want)
