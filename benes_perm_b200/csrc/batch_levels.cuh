@@ -49,6 +49,7 @@ struct LevelJob {
     uint32_t* inv;           // this level's inverse
     uint32_t* child_inv;     // children's inverse
     uint32_t* edge;          // edges, or union-find words, of this level and then the next
+    uint32_t* stamp;
     uint32_t* xbits;
     uint32_t* ybits;
     uint4* state[kMaxLists + 1];
@@ -157,14 +158,14 @@ __global__ void __launch_bounds__(256) batch_edges(const LevelJob* jobs, uint32_
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBEdges, &g);
     if (g.bid >= g.nblk) return;
-    level_edges_run(g, j->plan, j->inv, j->edge, j->status);
+    level_edges_run(g, j->plan, j->inv, j->edge, j->stamp, j->status);
 }
 
 __global__ void __launch_bounds__(256) batch_walk(const LevelJob* jobs, uint32_t n) {
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBWalk, &g);
     if (g.bid >= g.nblk) return;
-    level_walk_run(g, j->plan, j->level, j->edge, j->state[1], j->mark[1], j->status);
+    level_walk_run(g, j->plan, j->level, j->edge, j->stamp, j->state[1], j->mark[1], j->status);
 }
 
 __global__ void __launch_bounds__(256) batch_contract(const LevelJob* jobs, uint32_t n, uint32_t e) {
@@ -196,7 +197,7 @@ __global__ void __launch_bounds__(256) batch_colours(const LevelJob* jobs, uint3
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBColours, &g);
     if (g.bid >= g.nblk) return;
-    level_colours_run(g, j->plan, j->level, j->edge, j->colour[1], j->xbits, j->status);
+    level_colours_run(g, j->plan, j->level, j->edge, j->stamp, j->colour[1], j->xbits, j->status);
 }
 
 __global__ void __launch_bounds__(256, BPB200_UNION_MIN_BLOCKS) batch_union(const LevelJob* jobs,
@@ -226,7 +227,7 @@ __global__ void __launch_bounds__(256) batch_outputs(const LevelJob* jobs, uint3
     const LevelJob* j = level_job(jobs, n, kBOutputs, &g);
     if (g.bid >= g.nblk) return;
     level_outputs_run(g, j->plan, j->level, j->inv, j->xbits, j->ybits, j->child_inv,
-        j->child_walks == 1 ? j->edge : nullptr, j->child_walks == 0 ? j->edge : nullptr,
+        j->child_walks == 1 ? j->edge : nullptr, j->stamp, j->child_walks == 0 ? j->edge : nullptr,
         j->control + kCtlClaimOutputs);
 }
 

@@ -115,6 +115,7 @@ struct Workspace {
     uint32_t* inv[2] = {nullptr, nullptr}; // levels alternate the two
     uint32_t* edge = nullptr;              // output edges of a walk level, or a
                                            // union-find level's words (one per pair-node)
+    uint32_t* stamp = nullptr;             // walk stamps, one per pair-node
     uint32_t* xbits = nullptr;
     uint32_t* ybits = nullptr;
     WalkLists lists;                       // ruler lists of the walk levels
@@ -132,12 +133,12 @@ struct Workspace {
     bool busy = false;
 
     void release_scratch() {
-        for (void* p : {(void*)inv[0], (void*)inv[1], (void*)edge, (void*)xbits, (void*)ybits,
+        for (void* p : {(void*)inv[0], (void*)inv[1], (void*)edge, (void*)stamp, (void*)xbits, (void*)ybits,
                  lists_mem, (void*)control, (void*)records, (void*)cursor, (void*)addr[0],
                  (void*)addr[1]}) {
             if (p) cudaFree(p);
         }
-        inv[0] = inv[1] = edge = xbits = ybits = control = cursor = nullptr;
+        inv[0] = inv[1] = edge = stamp = xbits = ybits = control = cursor = nullptr;
         lists = WalkLists();
         lists_mem = nullptr;
         records = nullptr;
@@ -235,6 +236,7 @@ void ensure_scratch(Workspace& w, const Plan& p) {
     check(cudaMalloc(&w.inv[0], slots * 4), "cudaMalloc(inverse)");
     check(cudaMalloc(&w.inv[1], slots * 4), "cudaMalloc(inverse)");
     check(cudaMalloc(&w.edge, slots * 4), "cudaMalloc(edges)");
+    check(cudaMalloc(&w.stamp, pairs * 4), "cudaMalloc(stamps)");
     check(cudaMalloc(&w.xbits, (pairs / 32 + 4) * 4), "cudaMalloc(colour bits)");
     check(cudaMalloc(&w.ybits, (pairs / 32 + 4) * 4), "cudaMalloc(output bits)");
     check(cudaMalloc(&w.lists_mem, place_lists(pairs, nullptr, nullptr)), "cudaMalloc(ruler lists)");
@@ -651,12 +653,12 @@ void run_level(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p, cons
         const ListRange rr = list_range(pair_lo, pair_lo + prs, 1);
         if (l == 0) {
             rec.launch(kKindInverse, [&] {
-                level_edges<<<gp, kLevelThreads, 0, st>>>(dp, inv, w.edge, w.d_status);
+                level_edges<<<gp, kLevelThreads, 0, st>>>(dp, inv, w.edge, w.stamp, w.d_status);
             });
         }
         rec.launch(kKindWalk, [&] {
             level_walk<<<(rr.hi - rr.lo + kLevelThreads - 1) / kLevelThreads, kLevelThreads, 0,
-                st>>>(dp, l, w.edge, w.lists.state[1], w.lists.mark[1], w.d_status);
+                st>>>(dp, l, w.edge, w.stamp, w.lists.state[1], w.lists.mark[1], w.d_status);
         });
         rec.launch(kKindJump, [&] {
             for (uint32_t e = 1; e < shape.top; ++e) {
@@ -677,8 +679,8 @@ void run_level(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p, cons
             }
         }, 2 * shape.top - 1);
         rec.launch(kKindResolve, [&] {
-            level_colours<<<gp, kLevelThreads, 0, st>>>(dp, l, w.edge, w.lists.colour[1], w.xbits,
-                w.d_status);
+            level_colours<<<gp, kLevelThreads, 0, st>>>(dp, l, w.edge, w.stamp, w.lists.colour[1],
+                w.xbits, w.d_status);
         });
     } else {
         rec.launch(kKindUnion, [&] {
@@ -700,7 +702,7 @@ void run_level(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p, cons
         const bool global_child = l + 1 < p.tile_level;
         const bool child_walks = global_child && walk_level(p.levels[l + 1], tune, union_find_only);
         level_outputs<<<grid_for(prs / 2, kLevelThreads), kLevelThreads, 0, st>>>(dp, l, inv,
-            w.xbits, w.ybits, child_inv, child_walks ? w.edge : nullptr,
+            w.xbits, w.ybits, child_inv, child_walks ? w.edge : nullptr, w.stamp,
             global_child && !child_walks ? w.edge : nullptr, ctl + kCtlClaimOutputs);
     });
     // above the shard level every shard computes the level, shard 0 alone
@@ -1748,7 +1750,8 @@ constexpr size_t kOffControl = kOffStatus + 256;
 constexpr size_t kOffInv = kOffControl + up256(kMaxLevels * kCtlWords * 4);
 constexpr size_t kOffInv2 = kOffInv + up256(kSlots * 4);
 constexpr size_t kOffEdge = kOffInv2 + up256(kSlots * 4);
-constexpr size_t kOffXbits = kOffEdge + up256(kSlots * 4);
+constexpr size_t kOffStamp = kOffEdge + up256(kSlots * 4);
+constexpr size_t kOffXbits = kOffStamp + up256(kPairs * 4);
 constexpr size_t kOffYbits = kOffXbits + up256((kPairs / 32 + 4) * 4);
 constexpr size_t kOffAddr0 = kOffYbits + up256((kPairs / 32 + 4) * 4);
 constexpr size_t kOffAddr1 = kOffAddr0 + up256(kNodes * sizeof(NodeAddress));
@@ -1833,6 +1836,7 @@ extern "C" int bpb200_compress_device_noalloc(const void* d_entries, uint64_t co
         w.inv[0] = reinterpret_cast<uint32_t*>(base + noalloc::kOffInv);
         w.inv[1] = reinterpret_cast<uint32_t*>(base + noalloc::kOffInv2);
         w.edge = reinterpret_cast<uint32_t*>(base + noalloc::kOffEdge);
+        w.stamp = reinterpret_cast<uint32_t*>(base + noalloc::kOffStamp);
         w.xbits = reinterpret_cast<uint32_t*>(base + noalloc::kOffXbits);
         w.ybits = reinterpret_cast<uint32_t*>(base + noalloc::kOffYbits);
         w.addr[0] = reinterpret_cast<NodeAddress*>(base + noalloc::kOffAddr0);

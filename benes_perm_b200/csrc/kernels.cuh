@@ -527,7 +527,7 @@ __global__ void __launch_bounds__(256, BPB200_FINAL_MIN_BLOCKS) level_roots(
 // left_inv[s / 2] = inv[s - 1] >> 1.  A thread takes two output pairs, which
 // make one output pair of each child: one 16-byte load of inv, one 8-byte
 // store per child inverse, and, for a child level coloured by walks
-// (`child_edge`), that pair's edges; for one coloured by union-find
+// (`child_edge`), that pair's edges and a cleared stamp (`child_stamp`); for one coloured by union-find
 // (`child_uf`), its pair-node's root.  An odd child's tail is stored with
 // its virtual partner.  The edges are the only random writes (their node
 // fits L2); xbits gathers one bit per output pair.  A value out of range
@@ -537,7 +537,8 @@ __global__ void __launch_bounds__(256, BPB200_FINAL_MIN_BLOCKS) level_roots(
 __device__ __forceinline__ void level_outputs_run(Grid grid, const Plan* __restrict__ plan,
     uint32_t level, const uint32_t* __restrict__ inv, const uint32_t* __restrict__ xbits,
     uint32_t* __restrict__ ybits, uint32_t* __restrict__ child_inv,
-    uint32_t* __restrict__ child_edge, uint32_t* __restrict__ child_uf, uint32_t* claims) {
+    uint32_t* __restrict__ child_edge, uint32_t* __restrict__ child_stamp,
+    uint32_t* __restrict__ child_uf, uint32_t* claims) {
     const LevelInfo& lv = plan->levels[level];
     const LevelInfo& cl = plan->levels[level + 1];
     const uint32_t ps = (uint32_t)lv.pcap;
@@ -590,13 +591,14 @@ __device__ __forceinline__ void level_outputs_run(Grid grid, const Plan* __restr
                     const uint64_t at = 2ull * node * cps;
                     const uint32_t w = k0 + 1 < cs ? v[1] : cs; // virtual partner
                     __stcs(reinterpret_cast<uint2*>(child_inv + at + k0), make_uint2(v[0], w));
+                    const uint32_t id = node * cps + (k0 >> 1);
                     if (child_edge != nullptr) {
+                        child_stamp[id] = 0;
                         if (v[0] < cs && w < cs + (cs & 1u)) {
                             child_edge[at + v[0]] = w;
                             child_edge[at + w] = v[0];
                         }
                     } else if (child_uf != nullptr) {
-                        const uint32_t id = node * cps + (k0 >> 1);
                         child_uf[id] = id << 1;
                     }
                 };
@@ -617,9 +619,10 @@ __device__ __forceinline__ void level_outputs_run(Grid grid, const Plan* __restr
 __global__ void __launch_bounds__(256) level_outputs(const Plan* __restrict__ plan,
     uint32_t level, const uint32_t* __restrict__ inv, const uint32_t* __restrict__ xbits,
     uint32_t* __restrict__ ybits, uint32_t* __restrict__ child_inv,
-    uint32_t* __restrict__ child_edge, uint32_t* __restrict__ child_uf, uint32_t* claims) {
+    uint32_t* __restrict__ child_edge, uint32_t* __restrict__ child_stamp,
+    uint32_t* __restrict__ child_uf, uint32_t* claims) {
     level_outputs_run(launch_grid(), plan, level, inv, xbits, ybits, child_inv, child_edge,
-        child_uf, claims);
+        child_stamp, child_uf, claims);
 }
 
 // Switch bits of one section at one level, packet-major: thread t maps to

@@ -194,9 +194,6 @@ BP_HD uint64_t packet_path_bits(uint64_t root, uint32_t depth, uint32_t rel,
             share[big] = pairs - first < span ? pairs - first : span;
         }
     }
-    if (share[0] == share[1]) { // every packet but a short tail: no node sizes needed
-        return paths * share[0];
-    }
     const uint64_t nl = count_large(paths, rel, large);
     return nl * share[1] + (paths - nl) * share[0];
 }

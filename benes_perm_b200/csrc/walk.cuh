@@ -21,13 +21,16 @@
 // List 0 is the pair-nodes.  One element of a list in 8, at a hashed place
 // (ruler_slot), is an element of the next list.  Two walks leave it, one per
 // direction, each up to the next such element or to an element stamped by a
-// walk that came the other way, so every element is passed about once: that
-// is half the steps of one-way walks, and the stamp overwrites edge words
-// that nobody needs again, so the walks touch 4 bytes per entry and make one
-// dependent access per step.  A stamp names the walk that passed: kStamp |
+// walk that came the other way, so every element is passed about once, half
+// the steps of one-way walks.  A stamp names the walk that passed: kStamp |
 // ruler << 1 | (direction ^ side of entry); a walk that enters a stamped
-// element at side b goes on as directed ruler (stamp ^ b).  Walks that cross
-// may both stamp the elements where they cross, with stamps that say the
+// element at side b goes on as directed ruler (stamp ^ b).  One atomic
+// exchange leaves the stamp and fetches what was there: the stamps are then
+// only ever touched by atomics and the edges only read.  (Plain loads and
+// stores to the same words, whether stamps in the place of edges or in an
+// array of their own, cost 13 and 18 ms per level at 2^30 entries against
+// 5.6 ms: every sector moved between the two L2 halves at each change.)  A
+// walk that meets another replaces the stamp it finds by one that says the
 // same.  Each directed ruler keeps its successor and the smallest key its
 // own walk saw; a ruler's two walks together cover the stretches around it,
 // so folding min(m0, m1 ^ 1) over the rulers of a cycle (^ 1 mirrors a key
@@ -61,9 +64,10 @@ namespace bpb200 {
 constexpr uint64_t kWalkMaxNode = 1ull << BPB200_WALK_MAX_LOG2; // larger: union-find
 static_assert(BPB200_WALK_MAX_LOG2 >= 13 && BPB200_WALK_MAX_LOG2 <= 28, "walk limit out of range");
 constexpr uint32_t kRulerLog2 = 3;          // elements per element of the next list (log2)
+constexpr uint32_t kRankRulerLog2 = 3;      // the same inside list_rank
 constexpr uint32_t kWalkCap = 1u << 16;     // longest walk between rulers
 constexpr uint32_t kShortCap = 1u << 10;    // longest cycle without rulers
-constexpr uint32_t kStamp = 0x80000000u;
+constexpr uint32_t kStamp = 0x80000000u;    // an element's stamp starts as 0
 constexpr uint32_t kNone = 0xffffffffu;     // successor of an absent element
 constexpr uint32_t kMaxLists = 5;           // lists of rulers: 1..kMaxLists
 constexpr uint32_t kRankMaxLog2 = 14;       // most elements of a node list_rank takes (log2)
@@ -97,30 +101,22 @@ __device__ __forceinline__ uint32_t pair_of(uint32_t i, uint32_t e) {
     return i;
 }
 
-// Words other blocks rewrite while the walks run: read past L1.
-__device__ __forceinline__ uint2 load_live(const uint2* p) {
-    uint2 v;
-    asm volatile("ld.volatile.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ uint32_t load_live(const uint32_t* p) {
-    return *(const volatile uint32_t*)p;
-}
-
 // Smallest key of the stretches around a ruler, for paths that enter it in
 // direction 0 (direction 1: ^ 1).
 __device__ __forceinline__ uint32_t around(uint4 state) { return min(state.y, state.w ^ 1u); }
 
 // The edges of level 0, from its inverse: one thread per output pair.  Every
-// later level's edges are written by its parent's output pass.  A slot no
-// value was routed to means a repeated value.
+// later level's edges are written by its parent's output pass, which clears
+// the stamps as well.  A slot no value was routed to means a repeated value.
 __device__ __forceinline__ void level_edges_run(Grid grid, const Plan* __restrict__ plan,
-    const uint32_t* __restrict__ inv, uint32_t* __restrict__ edge, uint32_t* status) {
+    const uint32_t* __restrict__ inv, uint32_t* __restrict__ edge, uint32_t* __restrict__ stamp,
+    uint32_t* status) {
     const uint32_t s = (uint32_t)plan->levels[0].q;
     const uint32_t np = s - s / 2;
     bool bad = false;
     for (uint32_t k = grid.bid * blockDim.x + threadIdx.x; k < np; k += grid.nblk * blockDim.x) {
         const uint2 both = reinterpret_cast<const uint2*>(inv)[k];
+        stamp[k] = 0;
         const uint32_t u = both.x;
         const uint32_t w = 2 * k + 1 < s ? both.y : s;
         if (u >= s || (2 * k + 1 < s && w >= s)) {
@@ -134,8 +130,9 @@ __device__ __forceinline__ void level_edges_run(Grid grid, const Plan* __restric
 }
 
 __global__ void __launch_bounds__(256) level_edges(const Plan* __restrict__ plan,
-    const uint32_t* __restrict__ inv, uint32_t* __restrict__ edge, uint32_t* status) {
-    level_edges_run(launch_grid(), plan, inv, edge, status);
+    const uint32_t* __restrict__ inv, uint32_t* __restrict__ edge, uint32_t* __restrict__ stamp,
+    uint32_t* status) {
+    level_edges_run(launch_grid(), plan, inv, edge, stamp, status);
 }
 
 // One direction of a walk, advanced one element at a time.  `enter` is the
@@ -153,8 +150,8 @@ struct Walk {
 // entries: the hand-over cost more than the lanes idle behind the longest
 // walk of their warp.)  mark[r] = 0 resets the stamps of list_contract.
 __device__ __forceinline__ void level_walk_run(Grid grid, const Plan* __restrict__ plan,
-    uint32_t level, uint32_t* edge, uint4* __restrict__ state, uint32_t* __restrict__ mark,
-    uint32_t* status) {
+    uint32_t level, const uint32_t* __restrict__ edge, uint32_t* stamp,
+    uint4* __restrict__ state, uint32_t* __restrict__ mark, uint32_t* status) {
     const LevelInfo& lv = plan->levels[level];
     const uint32_t ps = (uint32_t)lv.pcap;
     const NodeRange nr = level_nodes(*plan, level);
@@ -176,31 +173,36 @@ __device__ __forceinline__ void level_walk_run(Grid grid, const Plan* __restrict
             state[r] = make_uint4(kNone, kNone, kNone, kNone);
             continue;
         }
-        uint2* node = reinterpret_cast<uint2*>(edge) + base;
+        const uint2* __restrict__ node = reinterpret_cast<const uint2*>(edge) + base;
         const uint32_t bias = (s & 1u) != 0 ? 0u - (s - 1) : 0u;
-        const uint2 mine = load_live(node + (own >> 1));
+        const uint2 mine = node[own >> 1];
         Walk w[2] = {{mine.y, own + bias, 2 * r, mine.y < limit},
             {mine.x, own + 1 + bias, 2 * r + 1, mine.x < limit}};
         bad |= !w[0].live || !w[1].live;
         for (uint32_t step = 0; (w[0].live || w[1].live) && step < kWalkCap; ++step) {
             bool ruler[2];
             uint2 v[2];
+            uint32_t found[2];
 #pragma unroll
             for (uint32_t d = 0; d < 2; ++d) {
-                ruler[d] = is_ruler(base + (w[d].enter >> 1));
-                v[d] = make_uint2(kStamp, 0u);
-                if (w[d].live && !ruler[d]) v[d] = load_live(node + (w[d].enter >> 1));
+                const uint32_t at = base + (w[d].enter >> 1);
+                ruler[d] = is_ruler(at);
+                v[d] = make_uint2(0u, 0u);
+                found[d] = kStamp;
+                if (w[d].live && !ruler[d]) {
+                    v[d] = node[w[d].enter >> 1];
+                    found[d] = atomicExch(stamp + at, kStamp | (r << 1) | (d ^ (w[d].enter & 1u)));
+                }
             }
 #pragma unroll
             for (uint32_t d = 0; d < 2; ++d) {
                 if (!w[d].live) continue;
                 const uint32_t side = w[d].enter & 1u;
-                if ((v[d].x & kStamp) != 0) {
+                if ((found[d] & kStamp) != 0) {
                     w[d].next = side ^ (ruler[d]
-                        ? ((base + (w[d].enter >> 1)) >> kRulerLog2) << 1 : v[d].x & ~kStamp);
+                        ? ((base + (w[d].enter >> 1)) >> kRulerLog2) << 1 : found[d] & ~kStamp);
                     w[d].live = false;
                 } else {
-                    *(volatile uint32_t*)&node[w[d].enter >> 1].x = kStamp | (r << 1) | (d ^ side);
                     w[d].best = min(w[d].best, w[d].enter + bias);
                     w[d].enter = side != 0 ? v[d].x : v[d].y;
                     if (w[d].enter >= limit) {
@@ -217,8 +219,9 @@ __device__ __forceinline__ void level_walk_run(Grid grid, const Plan* __restrict
 }
 
 __global__ void __launch_bounds__(256, 8) level_walk(const Plan* __restrict__ plan, uint32_t level,
-    uint32_t* edge, uint4* __restrict__ state, uint32_t* __restrict__ mark, uint32_t* status) {
-    level_walk_run(launch_grid(), plan, level, edge, state, mark, status);
+    const uint32_t* __restrict__ edge, uint32_t* stamp, uint4* __restrict__ state,
+    uint32_t* __restrict__ mark, uint32_t* status) {
+    level_walk_run(launch_grid(), plan, level, edge, stamp, state, mark, status);
 }
 
 // Walks over list e (state, mark), giving list e + 1 (up_state, up_mark).
@@ -260,11 +263,9 @@ __device__ __forceinline__ void list_contract_run(Grid grid, const Plan* __restr
                 next = ((at >> kRulerLog2) << 1) | (cur & 1u);
             } else {
                 st = state[at];
-                const uint32_t stamp = load_live(mark + at);
-                if ((stamp & kStamp) != 0) {
-                    next = (stamp & ~kStamp) ^ (cur & 1u);
-                } else {
-                    *(volatile uint32_t*)(mark + at) = kStamp | ((uint32_t)unit ^ (cur & 1u));
+                const uint32_t found = atomicExch(mark + at, kStamp | ((uint32_t)unit ^ (cur & 1u)));
+                if ((found & kStamp) != 0) {
+                    next = (found & ~kStamp) ^ (cur & 1u);
                 }
             }
         }
@@ -337,9 +338,14 @@ BP_HD uint32_t list_node_max(uint64_t ps, uint32_t e) {
     return (ps & ((1ull << sh) - 1)) == 0 ? (uint32_t)(ps >> sh) : (uint32_t)((ps - 1) >> sh) + 2;
 }
 
+// Element of a node's list that ruler i of list_rank stands for.
+__device__ __forceinline__ uint32_t rank_slot(uint32_t i) {
+    return (i << kRankRulerLog2) + ((i * 0x9E3779B1u) >> (32 - kRankRulerLog2));
+}
+
 // Dynamic shared memory of list_rank for nodes of `count` elements.
 BP_HD uint32_t rank_smem(uint32_t count) {
-    const uint32_t rulers = ((count - 1) >> kRulerLog2) + 1;
+    const uint32_t rulers = ((count - 1) >> kRankRulerLog2) + 1;
     return count * 8 + rulers * 16;
 }
 constexpr uint32_t kRankThreads = 1024;
@@ -370,7 +376,7 @@ __device__ __forceinline__ void list_rank_run(Grid grid, const Plan* __restrict_
         const uint64_t pair_lo = j * ps;
         const ListRange range = list_range(pair_lo, pair_lo + ps, e);
         const uint32_t count = range.hi - range.lo;
-        const uint32_t rulers = ((count - 1) >> kRulerLog2) + 1;
+        const uint32_t rulers = ((count - 1) >> kRankRulerLog2) + 1;
         volatile uint32_t* link = smem;
         volatile uint16_t* link16 = reinterpret_cast<volatile uint16_t*>(smem);
         uint32_t* key = smem + count;
@@ -399,7 +405,7 @@ __device__ __forceinline__ void list_rank_run(Grid grid, const Plan* __restrict_
         __syncthreads();
         // rulers first: their word moves to the state, a stamp takes its place
         for (uint32_t r = tid; r < rulers; r += blockDim.x) {
-            const uint32_t i = ruler_slot(r);
+            const uint32_t i = rank_slot(r);
             const uint32_t word = i < count ? link[i] : 0x8000u;
             snext[2 * r] = word;
             if ((word & 0x8000u) == 0) link16[2 * i] = (uint16_t)(0x8000u | (r << 1));
@@ -413,7 +419,7 @@ __device__ __forceinline__ void list_rank_run(Grid grid, const Plan* __restrict_
                 smin[2 * r] = smin[2 * r + 1] = ~0u;
                 continue;
             }
-            const uint32_t own = key[ruler_slot(r)];
+            const uint32_t own = key[rank_slot(r)];
             uint32_t wa = word >> 16, wb = word & 0xffffu;
             uint32_t ma = own, mb = own ^ 1u;
             bool ga = true, gb = true;
@@ -502,8 +508,8 @@ __global__ void __launch_bounds__(kRankThreads, 1) list_rank(const Plan* __restr
 // pair-node k, from the stamp of the walk that passed it and that ruler's
 // colour.  One thread per pair-node, in address order.
 __device__ __forceinline__ void level_colours_run(Grid grid, const Plan* __restrict__ plan,
-    uint32_t level, const uint32_t* __restrict__ edge, const uint8_t* __restrict__ colour,
-    uint32_t* __restrict__ xbits, uint32_t* status) {
+    uint32_t level, const uint32_t* __restrict__ edge, const uint32_t* __restrict__ stamp,
+    const uint8_t* __restrict__ colour, uint32_t* __restrict__ xbits, uint32_t* status) {
     const LevelInfo& lv = plan->levels[level];
     const uint32_t ps = (uint32_t)lv.pcap;
     // this call's pair-nodes; the loop starts at a 32-pair boundary so each
@@ -519,13 +525,13 @@ __device__ __forceinline__ void level_colours_run(Grid grid, const Plan* __restr
         uint32_t x = 0;
         if (p >= first && p < end) {
             const uint32_t q = (uint32_t)p;
-            const uint2 v = pairs[q];
+            const uint32_t v = __ldcs(stamp + q);
             if (is_ruler(q)) {
                 x = colour[q >> kRulerLog2];
-            } else if ((v.x & kStamp) != 0) {
-                const uint32_t r = (v.x & ~kStamp) >> 1;
+            } else if ((v & kStamp) != 0) {
+                const uint32_t r = (v & ~kStamp) >> 1;
                 // padding pair-nodes hold anything; their bits are not used
-                if (r >= rr.lo && r < rr.hi) x = colour[r] ^ v.x;
+                if (r >= rr.lo && r < rr.hi) x = colour[r] ^ v;
             } else {
                 const uint32_t j = q / ps;
                 const uint32_t k = q - j * ps;
@@ -535,7 +541,7 @@ __device__ __forceinline__ void level_colours_run(Grid grid, const Plan* __restr
                     const uint2* node = pairs + (uint64_t)j * ps;
                     const uint32_t bias = (s & 1u) != 0 ? 0u - (s - 1) : 0u;
                     uint32_t cur = 2 * k, step = 0;
-                    uint2 word = v;
+                    uint2 word = node[k];
                     x = ~0u;
                     do {
                         x = min(x, cur + bias);
@@ -558,9 +564,9 @@ __device__ __forceinline__ void level_colours_run(Grid grid, const Plan* __restr
 }
 
 __global__ void __launch_bounds__(256) level_colours(const Plan* __restrict__ plan,
-    uint32_t level, const uint32_t* __restrict__ edge, const uint8_t* __restrict__ colour,
-    uint32_t* __restrict__ xbits, uint32_t* status) {
-    level_colours_run(launch_grid(), plan, level, edge, colour, xbits, status);
+    uint32_t level, const uint32_t* __restrict__ edge, const uint32_t* __restrict__ stamp,
+    const uint8_t* __restrict__ colour, uint32_t* __restrict__ xbits, uint32_t* status) {
+    level_colours_run(launch_grid(), plan, level, edge, stamp, colour, xbits, status);
 }
 
 } // namespace bpb200
