@@ -28,11 +28,10 @@ constexpr uint32_t kErrIterationCap = 2u;    // a bounded retry loop gave up
 constexpr uint32_t kErrInconsistent = 4u;    // colouring constraint violated
 constexpr uint32_t kErrGaveUp = 8u;          // a walk ran too long: encode again with union-find
 
-// Retry bound for every lock-free loop; far above what a valid input needs.
-// Parents strictly decrease along every union-find chain (links go to the
-// smaller root, halving jumps to the grandparent), so loops end anyway; the
-// bound only caps the cost of a pathological chain.
-constexpr uint32_t kSpinCap = 1u << 20;
+// Bound of every walk along a union-find chain.  Parents strictly decrease
+// along a chain, so the walks end anyway; the bound only caps the cost of a
+// pathological one.
+constexpr uint32_t kChainCap = 1u << 20;
 
 // ------------------------------------------------------------------------
 // Parity union-find over pair-nodes.
@@ -40,12 +39,13 @@ constexpr uint32_t kSpinCap = 1u << 20;
 // Word layout: (parent << 1) | bit.  For a non-root the bit is the colour
 // difference between the node and its parent; a root points to itself and
 // its bit is the orientation flag set after all unions (it flips the colour
-// of the whole component so that the odd tail ends up colour 0).  Linking
-// always hangs the larger root under the smaller, so a root is the smallest
-// pair-node of its component and parents strictly decrease along any chain.
-// Path halving stores (grandparent, accumulated bit); the colour difference
-// between a node and any ancestor is fixed by the constraint graph, so such
-// racy plain stores can only ever write true facts.
+// of the whole component so that the odd tail ends up colour 0).  A link
+// hangs a root under a smaller node, so a root is the smallest pair-node of
+// its component and parents strictly decrease along any chain.  The unions
+// write nothing but links and the resolving pass nothing but each node's own
+// root: compressing paths on the way costs more than the shorter paths save,
+// because the words near the roots then move between the two L2 halves all
+// the time.
 // ------------------------------------------------------------------------
 
 struct Found {
@@ -53,184 +53,117 @@ struct Found {
     uint32_t bit;
 };
 
-template <typename Word>
-__device__ __forceinline__ Word uf_load(Word* uf, uint32_t i) {
-    return *((volatile Word*)(uf + i));
-}
-
-template <typename Word>
-__device__ __forceinline__ Found uf_find(Word* uf, uint32_t x, uint32_t* err) {
-    uint32_t acc = 0;
-    uint32_t cur = x;
-    for (uint32_t it = 0; it < kSpinCap; ++it) {
-        const uint32_t w = (uint32_t)uf_load(uf, cur);
-        const uint32_t p = w >> 1;
-        if (p == cur) {
-            return {cur, acc};
-        }
-        const uint32_t wp = (uint32_t)uf_load(uf, p);
-        const uint32_t pp = wp >> 1;
-        if (pp == p) {
-            return {p, acc ^ (w & 1u)};
-        }
-        const uint32_t nb = (w ^ wp) & 1u;
-        uf[cur] = (Word)((pp << 1) | nb);
-        acc ^= nb;
-        cur = pp;
+// A walk that has come kLongChain steps (random inputs: none does) halves
+// the rest of its path after all: x, whose word is w, goes to its
+// grandparent; both are true facts, so the racy store can only write a true
+// one.  Returns the word that leads from x to where the walk goes on.
+constexpr uint32_t kLongChain = 128;
+__device__ __forceinline__ uint32_t uf_halve(uint32_t* uf, uint32_t x, uint32_t w) {
+    const uint32_t up = *(volatile uint32_t*)(uf + (w >> 1));
+    if ((up >> 1) == (w >> 1)) {
+        return w; // the parent is a root
     }
-    atomicOr(err, kErrIterationCap);
-    return {cur, acc};
+    const uint32_t over = (up & ~1u) | ((w ^ up) & 1u);
+    uf[x] = over;
+    return over;
 }
 
-__device__ __forceinline__ uint32_t cas_word(uint32_t* a, uint32_t e, uint32_t v) {
-    return atomicCAS(a, e, v);
-}
-
-// Record x(a) ^ x(b) == rel.
-template <typename Word>
-__device__ __forceinline__ void uf_union(Word* uf, uint32_t a, uint32_t b, uint32_t rel,
-    uint32_t* err) {
-    for (uint32_t it = 0; it < kSpinCap; ++it) {
-        const Found fa = uf_find(uf, a, err);
-        const Found fb = uf_find(uf, b, err);
-        rel ^= fa.bit ^ fb.bit;
-        a = fa.root;
-        b = fb.root;
-        if (a == b) {
-            if (rel != 0) {
-                atomicOr(err, kErrInconsistent);
-            }
-            return;
-        }
-        const uint32_t lo = a < b ? a : b;
-        const uint32_t hi = a < b ? b : a;
-        if (cas_word((uint32_t*)(uf + hi), hi << 1, (lo << 1) | rel) == (hi << 1)) {
-            return;
-        }
-    }
-    atomicOr(err, kErrIterationCap);
-}
-
-// K finds advanced in lockstep: every round issues the loads of all
-// unfinished finds before using any of them, so one thread keeps up to 2K
-// independent loads in flight.  Bits of `pending` name the finds to run.
-// `cached`: plain (L1-cached) loads, for finds that run after every union
-// of the level is done.  Every find of a big component reads its root's
-// word; through L1 those reads stop queueing at the one L2 slice that holds
-// it.  No root changes any more, and a stale cached word is an older parent
-// pointer, i.e. still an ancestor with its true parity, so cached finds end
-// at the same roots with the same bits.  (During the unions a stale word
-// could name a former root; the union kernel keeps uncached loads.)
-template <typename Word>
-__device__ __forceinline__ Word uf_word(Word* uf, uint32_t i, bool cached) {
-    return cached ? uf[i] : uf_load(uf, i);
-}
-
-template <int K, typename Word>
-__device__ __forceinline__ void uf_find_many(Word* uf, const uint32_t (&x)[K], Found (&out)[K],
-    uint32_t pending, uint32_t* err, bool cached = false) {
-    uint32_t cur[K], acc[K];
+// K finds advanced in lockstep, K loads in flight; bits of `pending` name
+// the finds to run.
+template <int K>
+__device__ __forceinline__ void uf_find_many(uint32_t* uf, const uint32_t (&x)[K],
+    Found (&out)[K], uint32_t pending, uint32_t* err) {
 #pragma unroll
-    for (int i = 0; i < K; ++i) {
-        cur[i] = x[i];
-        acc[i] = 0;
-    }
+    for (int i = 0; i < K; ++i) out[i] = {x[i], 0u};
     for (uint32_t it = 0; pending != 0; ++it) {
-        if (it == kSpinCap) {
-            atomicOr(err, kErrIterationCap);
-#pragma unroll
-            for (int i = 0; i < K; ++i) {
-                if (pending & (1u << i)) out[i] = {cur[i], acc[i]};
-            }
-            return;
-        }
-        uint32_t w[K], wp[K];
-#pragma unroll
-        for (int i = 0; i < K; ++i) {
-            if (pending & (1u << i)) w[i] = (uint32_t)uf_word(uf, cur[i], cached);
-        }
-#pragma unroll
-        for (int i = 0; i < K; ++i) {
-            if (pending & (1u << i)) {
-                const uint32_t p = w[i] >> 1;
-                if (p == cur[i]) {
-                    out[i] = {cur[i], acc[i]};
-                    pending &= ~(1u << i);
-                } else {
-                    wp[i] = (uint32_t)uf_word(uf, p, cached);
-                }
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < K; ++i) {
-            if (pending & (1u << i)) {
-                const uint32_t p = w[i] >> 1;
-                const uint32_t pp = wp[i] >> 1;
-                if (pp == p) {
-                    out[i] = {p, acc[i] ^ (w[i] & 1u)};
-                    pending &= ~(1u << i);
-                } else {
-                    const uint32_t nb = (w[i] ^ wp[i]) & 1u;
-                    uf[cur[i]] = (Word)((pp << 1) | nb);
-                    acc[i] ^= nb;
-                    cur[i] = pp;
-                }
-            }
-        }
-    }
-}
-
-// K unions x(a[i]) ^ x(b[i]) == rel[i], with all 2K finds of a round in
-// lockstep.  A failed link retries from the two roots it saw.
-//
-// The first round's finds use L1-cached loads.  Once a component is large,
-// most finds end at its root, and uncached they all queue at the one L2
-// slice holding that word.  A cached word may be stale, but it still names
-// a true ancestor with its true parity, so a find ends at a node X of the
-// right component with the right relative colour; X may have stopped being
-// a root.  That is harmless: when both finds reach the same X the two nodes
-// share a component; otherwise the link is a CAS that requires the larger
-// end `hi` to be a root at that moment (it fails on a stale root, and the
-// retry rounds then read L2), and hanging a true root hi under any smaller
-// node `lo` joins two different components (a root is its component's
-// minimum, so lo < hi lies outside hi's component) while keeping parents
-// strictly decreasing.
-template <int K, typename Word>
-__device__ __forceinline__ void uf_union_many(Word* uf, uint32_t (&a)[K], uint32_t (&b)[K],
-    uint32_t (&rel)[K], uint32_t pending, uint32_t* err) {
-    for (uint32_t it = 0; pending != 0; ++it) {
-        if (it == kSpinCap) {
+        if (it == kChainCap) {
             atomicOr(err, kErrIterationCap);
             return;
         }
-        uint32_t x[2 * K];
-        Found f[2 * K];
+        uint32_t w[K];
 #pragma unroll
         for (int i = 0; i < K; ++i) {
-            x[i] = a[i];
-            x[K + i] = b[i];
+            if (pending & (1u << i)) w[i] = uf[out[i].root];
         }
-        uint32_t both = 0;
-#pragma unroll
-        for (int i = 0; i < K; ++i) {
-            if (pending & (1u << i)) both |= (1u << i) | (1u << (K + i));
-        }
-        uf_find_many<2 * K>(uf, x, f, both, err, it == 0);
 #pragma unroll
         for (int i = 0; i < K; ++i) {
             if (!(pending & (1u << i))) continue;
-            rel[i] ^= f[i].bit ^ f[K + i].bit;
-            a[i] = f[i].root;
-            b[i] = f[K + i].root;
-            if (a[i] == b[i]) {
-                if (rel[i] != 0) atomicOr(err, kErrInconsistent);
+            if ((w[i] >> 1) == out[i].root) {
                 pending &= ~(1u << i);
-                continue;
+            } else {
+                const uint32_t over = it < kLongChain ? w[i] : uf_halve(uf, out[i].root, w[i]);
+                out[i].bit ^= over & 1u;
+                out[i].root = over >> 1;
             }
-            const uint32_t lo = a[i] < b[i] ? a[i] : b[i];
-            const uint32_t hi = a[i] < b[i] ? b[i] : a[i];
-            if (cas_word((uint32_t*)(uf + hi), hi << 1, (lo << 1) | rel[i]) == (hi << 1)) {
-                pending &= ~(1u << i);
+        }
+    }
+}
+
+// Root of x and their colour difference.
+__device__ __forceinline__ Found uf_find(uint32_t* uf, uint32_t x, uint32_t* err) {
+    const uint32_t from[1] = {x};
+    Found out[1];
+    uf_find_many<1>(uf, from, out, 1u, err);
+    return out[0];
+}
+
+// K unions x(a[i]) ^ x(b[i]) == rel[i] in lockstep.  Only the larger of the
+// two nodes is looked at: while it has a parent it is replaced by that; once
+// it is a root it is hung under the smaller node, which need not be a root
+// (it lies in another component: a root is the smallest node of its own).
+// Two thirds of a random graph's unions find their larger end still alone
+// and touch one word (finding both roots, with path halving, took 251 ms per
+// compress at 2^30 entries, this 162 ms).
+//
+// A plain load may return an older word, which still names a true ancestor
+// with its true parity; the link is a compare-and-swap on a root, and a
+// failed one returns the word as it is.  `kSwap`: every look is a
+// compare-and-swap that expects a root, so that words are only touched by
+// atomics, faster while a node's words fit L2 (see level_union).
+template <int K, bool kSwap>
+__device__ __forceinline__ void uf_unite_many(uint32_t* uf, uint32_t (&a)[K], uint32_t (&b)[K],
+    uint32_t (&rel)[K], uint32_t pending, uint32_t* err) {
+    uint32_t w[K];
+    auto look = [&](int i) {
+        if (kSwap) {
+            w[i] = atomicCAS(uf + a[i], a[i] << 1, (b[i] << 1) | rel[i]);
+            if (w[i] == a[i] << 1) pending &= ~(1u << i); // linked
+        } else {
+            w[i] = uf[a[i]];
+        }
+    };
+    auto settle = [&](int i) { // a above b; both the same: nothing left to do
+        const uint32_t hi = max(a[i], b[i]);
+        b[i] = min(a[i], b[i]);
+        a[i] = hi;
+        if (a[i] == b[i]) {
+            if (rel[i] != 0) atomicOr(err, kErrInconsistent);
+            pending &= ~(1u << i);
+        }
+    };
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+        if (pending & (1u << i)) settle(i);
+        if (pending & (1u << i)) look(i);
+    }
+    for (uint32_t it = 0; pending != 0; ++it) {
+        if (it == kChainCap) {
+            atomicOr(err, kErrIterationCap);
+            return;
+        }
+#pragma unroll
+        for (int i = 0; i < K; ++i) {
+            if (!(pending & (1u << i))) continue;
+            const uint32_t up = w[i] >> 1;
+            if (!kSwap && up == a[i]) {
+                w[i] = atomicCAS(uf + up, up << 1, (b[i] << 1) | rel[i]);
+                if (w[i] == up << 1) pending &= ~(1u << i);
+            } else {
+                const uint32_t over = it < kLongChain ? w[i] : uf_halve(uf, a[i], w[i]);
+                rel[i] ^= over & 1u;
+                a[i] = over >> 1;
+                settle(i);
+                if (pending & (1u << i)) look(i);
             }
         }
     }

@@ -46,23 +46,26 @@ constexpr uint32_t kTileThreads = 512;
 #define BPB200_INVERSE_ITEMS 4
 #endif
 constexpr int kInverseItems = BPB200_INVERSE_ITEMS; // slots per thread in level_inverse
-// level_union shape: 2 output pairs per thread with at most 64 registers (4
-// blocks of 256 per SM) measured fastest on B200 at 2^30 uniform entries
-// (union kernels 253 ms per compress; 4 pairs at 100 registers: 304 ms;
-// 8 pairs: 420 ms).  More resident warps hide more of the random latency.
+// level_union shape: 2 output pairs per thread at 6 blocks of 256 per SM
+// measured fastest on B200 at 2^30 uniform entries (169 ms per compress with
+// loads on every level; 1 at 8 blocks: 169, 2 at 4: 172, 4 at 4: 181).
 #ifndef BPB200_UNION_ITEMS
 #define BPB200_UNION_ITEMS 2
 #endif
 #ifndef BPB200_UNION_MIN_BLOCKS
-#define BPB200_UNION_MIN_BLOCKS 4
+#define BPB200_UNION_MIN_BLOCKS 6
 #endif
+// Nodes of up to this many entries (64 MB of union-find words) are united by
+// compare-and-swaps alone, larger ones by loads first: at 2^30 entries the
+// levels of 2^24, 2^25 and 2^26-entry nodes took 10.6, 11.6 and 23.2 ms with
+// swaps, 14.0, 14.4 and 16.8 ms with loads.
+constexpr uint64_t kSwapMaxNode = 1ull << 25;
 constexpr int kUnionItems = BPB200_UNION_ITEMS; // output pairs per thread in level_union
 // level_roots shape: pair-nodes per thread (1, 2, 4 or 8; 32 / items lanes
 // assemble one colour word) and the minimum resident blocks of 256 per SM.
-// 2 pair-nodes at 8 blocks measured fastest on B200 at 2^30 uniform entries
-// (115 ms per compress while the pass also moved values; 2 at 6 blocks: 120;
-// 4 at 6 blocks: 144; 8: 286): the finds are latency-bound, so more resident
-// warps beat more finds per thread.
+// The finds are latency-bound, so more resident warps beat more finds per
+// thread (2^30 uniform entries, first seven levels, before the claims below:
+// 1 pair-node at 8 blocks 55 ms, 2 at 8 57 ms, 4 at 4 61 ms).
 #ifndef BPB200_RESOLVE_ITEMS
 #define BPB200_RESOLVE_ITEMS 2
 #endif
@@ -72,14 +75,6 @@ constexpr int kUnionItems = BPB200_UNION_ITEMS; // output pairs per thread in le
 constexpr int kResolveItems = BPB200_RESOLVE_ITEMS;
 static_assert(kResolveItems == 1 || kResolveItems == 2 || kResolveItems == 4 ||
     kResolveItems == 8, "level_roots assembles colour words from 1, 2, 4 or 8 bits per lane");
-// Levels whose nodes have at most 2^BPB200_FINAL_STRIDE_LOG2 entries resolve
-// in grid-stride order, larger ones in claimed order (see level_roots);
-// measured on B200 at 2^30 uniform entries (105 ms per compress with values;
-// limit 2^24: 110 ms; 2^23: 119 ms).
-#ifndef BPB200_FINAL_STRIDE_LOG2
-#define BPB200_FINAL_STRIDE_LOG2 26
-#endif
-
 // Control words of a level: work counters of its claiming kernels, zeroed
 // for every level at once before the first launch.
 enum : int {
@@ -366,7 +361,11 @@ __device__ __forceinline__ void level_union_run(Grid grid, const Plan* __restric
                 rel[q] = 1u ^ (u[q] & 1u) ^ (w[q] & 1u);
             }
         }
-        uf_union_many<kUnionItems>(uf, a, b, rel, pending, status);
+        if (lv.cap <= kSwapMaxNode) {
+            uf_unite_many<kUnionItems, true>(uf, a, b, rel, pending, status);
+        } else {
+            uf_unite_many<kUnionItems, false>(uf, a, b, rel, pending, status);
+        }
     }
 }
 
@@ -428,7 +427,9 @@ __global__ void __launch_bounds__(256) level_descriptors(const Plan* __restrict_
 
 // Input switch bits of a union-find level: bit k = colour of input 2k = the
 // pair-node's parity to its root, flipped by the root's orientation flag;
-// kResolveItems pair-nodes per thread.
+// kResolveItems pair-nodes per thread.  Finds that shortened paths as they
+// went, in grid-stride order on nodes up to 2^26 entries, took 58 ms per
+// compress at 2^30 entries, these 44 ms.
 __device__ __forceinline__ void level_roots_run(Grid grid, const Plan* __restrict__ plan,
     uint32_t level, uint32_t* uf, uint32_t* __restrict__ xbits, uint32_t* claims,
     uint32_t* status) {
@@ -443,27 +444,11 @@ __device__ __forceinline__ void level_roots_run(Grid grid, const Plan* __restric
     const uint64_t total = end - begin;
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t chunk = (uint64_t)blockDim.x * kResolveItems;
-    // Levels with nodes far above L2 size claim chunks in order (the finds of
-    // neighbouring chunks share the top of their trees).  With nodes near L2
-    // size, claimed chunks would crowd every find in flight onto the root
-    // chains of one or two nodes' large components, which then serialise:
-    // those stride over the whole level (at 2^30 uniform entries, claimed
-    // order took 18.5 -> 12.5 ms on the 2^30-slot level but 14 -> 19 ms on
-    // 2^24-slot nodes).
-    uint64_t first = (uint64_t)grid.bid * chunk;
-    bool started = false;
-    const bool claimed = lv.cap > (1ull << BPB200_FINAL_STRIDE_LOG2);
-    auto next_chunk = [&]() -> bool {
-        if (claimed) {
-            return claim_chunk(claims, chunk, total, &first);
-        }
-        if (started) {
-            first += (uint64_t)grid.nblk * chunk;
-        }
-        started = true;
-        return first < total;
-    };
-    while (next_chunk()) {
+    // Chunks are claimed in address order and every pair-node's root goes
+    // back into its word: parents are smaller than their children, so most
+    // finds end at a parent that was resolved before them.
+    uint64_t first;
+    while (claim_chunk(claims, chunk, total, &first)) {
         const uint64_t p0 = begin + first + (uint64_t)threadIdx.x * kResolveItems;
         uint32_t j = (uint32_t)(p0 / pcap);
         uint32_t k = (uint32_t)(p0 - (uint64_t)j * pcap);
@@ -481,15 +466,12 @@ __device__ __forceinline__ void level_roots_run(Grid grid, const Plan* __restric
             }
         }
         Found f[kResolveItems];
-        uf_find_many<kResolveItems>(uf, x, f, live, status, true);
+        uf_find_many<kResolveItems>(uf, x, f, live, status);
         uint32_t mine = 0; // this lane's kResolveItems colour bits
 #pragma unroll
         for (int q = 0; q < kResolveItems; ++q) {
             if (!(live & (1u << q))) continue;
             mine |= (f[q].bit ^ (uf[f[q].root] & 1u)) << q;
-            // point the pair-node at its root (a true fact), so the finds of
-            // the pair-nodes below it end one step later (105.0 ms per
-            // compress at 2^30 entries against 106.2 without)
             if (f[q].root != x[q]) {
                 uf[x[q]] = (f[q].root << 1) | f[q].bit;
             }
