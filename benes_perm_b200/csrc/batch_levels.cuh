@@ -79,8 +79,10 @@ struct EmitJob {
     uint64_t full;           // full packets (block forms) or first packet (per-bit form)
     uint32_t level;
     int32_t side;
+    int32_t form;
     uint32_t first;
     uint32_t blocks;
+    uint32_t pad_;
 };
 
 // Word fills (blob clearing, validation sentinels, super-ruler marks).
@@ -231,31 +233,15 @@ __global__ void __launch_bounds__(256) batch_outputs(const LevelJob* jobs, uint3
         j->control + kCtlClaimOutputs);
 }
 
-// Emission forms (kernels.cuh), one launch per form over every (permutation,
-// section) that uses it at this level.
-enum EmitForm : int { kEmitWords = 0, kEmitTranspose, kEmitBlocks, kEmitBits, kEmitForms };
-
-__global__ void __launch_bounds__(256) batch_emit(const EmitJob* jobs, uint32_t n, int form) {
+// Switch emission: every (permutation, section, form) of the level in one
+// launch.
+__global__ void __launch_bounds__(256) batch_emit(const EmitJob* jobs, uint32_t n) {
     Grid g;
     const EmitJob* j = batch_job(jobs, n, [](const EmitJob& x) { return x.first; }, &g);
     g.bid = blockIdx.x - j->first;
     g.nblk = j->blocks;
     if (g.bid >= g.nblk) return;
-    switch (form) {
-    case kEmitWords:
-        level_emit_words_run(g, j->plan, j->level, j->side, j->bits, j->addr, j->blob);
-        break;
-    case kEmitTranspose:
-        level_emit_transpose_run(g, j->plan, j->level, j->side, j->bits, j->addr, j->blob,
-            j->full);
-        break;
-    case kEmitBlocks:
-        level_emit_blocks_run(g, j->plan, j->level, j->side, j->bits, j->addr, j->blob, j->full);
-        break;
-    default:
-        level_emit_run(g, j->plan, j->level, j->side, j->bits, j->addr, j->blob, j->full);
-        break;
-    }
+    level_emit_form(g, j->form, j->plan, j->level, j->side, j->bits, j->addr, j->blob, j->full);
 }
 
 } // namespace bpb200

@@ -22,6 +22,17 @@ struct Grid {
 
 __device__ __forceinline__ Grid launch_grid() { return Grid{blockIdx.x, gridDim.x}; }
 
+// Start of every kernel of an encode's launch sequence, which is launched
+// with programmatic stream serialisation (launch_next, encode.cu): its
+// blocks may be resident before the kernel ahead of it has ended, and wait
+// here until it has, with its writes visible.  The next kernel may be made
+// resident as soon as this one's blocks all have started.  A kernel launched
+// without the attribute passes through.
+__device__ __forceinline__ void wait_for_previous() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Device status word bits (read by the host after each call).
 constexpr uint32_t kErrNotPermutation = 1u;  // value out of range or duplicated
 constexpr uint32_t kErrIterationCap = 2u;    // a bounded retry loop gave up

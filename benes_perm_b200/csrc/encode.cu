@@ -256,21 +256,52 @@ void ensure_scratch(Workspace& w, const Plan& p) {
 
 // ------------------------------------------------------------ prologue
 
-struct Header {
-    uint32_t bytes;
-    uint8_t data[84];
+struct Prologue {
+    Plan plan;
+    Header header;
 };
 
-__global__ void prologue(uint32_t* status, uint32_t* blob, Header h) {
-    if (threadIdx.x == 0) {
-        *status = 0;
+// First launch of an encode with global levels: places the plan, clears the
+// blob but for its header, the status word and the level counters, fills
+// level 0's inverse with 0xffffffff (a repeated value leaves such a slot
+// behind) and works out the switch addresses of every global level.  One
+// launch in the place of an upload, three memsets and two kernels.
+__global__ void __launch_bounds__(256) prologue(const __grid_constant__ Prologue p, Plan* plan,
+    uint32_t* status, uint32_t* __restrict__ blob, uint64_t blob_words,
+    uint32_t* __restrict__ control, uint32_t control_words, uint32_t* __restrict__ inv,
+    uint64_t inv_words, NodeAddress* __restrict__ in_addr, NodeAddress* __restrict__ out_addr) {
+    const uint64_t id = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    const uint32_t* from = reinterpret_cast<const uint32_t*>(&p.plan);
+    for (uint64_t i = id; i < sizeof(Plan) / 4; i += stride) {
+        reinterpret_cast<uint32_t*>(plan)[i] = from[i];
     }
-    // the header ends before the first section bit; only whole header bytes
-    // are written, so it cannot clobber section bits sharing its last word
-    uint8_t* b = reinterpret_cast<uint8_t*>(blob);
-    for (uint32_t i = threadIdx.x; i < h.bytes; i += blockDim.x) {
-        b[i] = h.data[i];
+    if (id == 0) *status = 0;
+    for (uint64_t i = id; i < control_words; i += stride) control[i] = 0;
+    for (uint64_t i = id; i < blob_words; i += stride) {
+        blob[i] = i < sizeof(Header) / 4 ? header_word(p.header, i) : 0u;
     }
+    for (uint64_t i = id; i < inv_words; i += stride) inv[i] = ~0u;
+    level_descriptors_run(launch_grid(), &p.plan, in_addr, out_addr);
+}
+
+// Launches the next kernel of an encode's sequence: with programmatic stream
+// serialisation, so its launch and the start of its blocks overlap the end
+// of the kernel ahead, on which it waits itself (wait_for_previous).
+template <typename... Params, typename... Args>
+void launch_next(void (*kernel)(Params...), uint64_t blocks, uint32_t threads, uint32_t smem,
+    cudaStream_t st, Args&&... args) {
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3((unsigned)blocks);
+    config.blockDim = dim3(threads);
+    config.dynamicSmemBytes = smem;
+    config.stream = st;
+    cudaLaunchAttribute attribute{};
+    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    check(cudaLaunchKernelEx(&config, kernel, Params(args)...), "kernel launch");
 }
 
 // ------------------------------------------------------------ tile sizing
@@ -298,6 +329,13 @@ TileShape tile_shape(const Plan& p, uint32_t t0) {
 // 512 (8192 entries: 107 us against 140 us).  Wide tiles fill an SM each.
 unsigned tile_threads(uint64_t tiles, bool wide) {
     return wide ? 2 * kTileThreads : (tiles > 2 * 148 ? kTileThreads / 2 : kTileThreads);
+}
+
+// Threads of a permutation that is a single tile: 8 entries each.
+unsigned single_threads(uint64_t n) {
+    unsigned t = 128;
+    while (t < 2 * kTileThreads && (uint64_t)t * 8 < n) t *= 2;
+    return t;
 }
 
 // Picks the tile level: the first level whose nodes fit `tile_max` entries
@@ -643,9 +681,9 @@ void run_level(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p, cons
             for (uint32_t k = 0; k < (uint32_t)input->ends.size(); ++k) input->wait(k);
         }
         rec.launch(kKindInverse, [&] {
-            level_inverse<T><<<grid_for((lv.cap + kInverseItems - 1) / kInverseItems, kLevelThreads),
-                kLevelThreads, 0, st>>>(dp, src, inv, walks ? nullptr : w.edge,
-                ctl + kCtlClaimInverse, w.d_status);
+            launch_next(level_inverse<T>,
+                grid_for((lv.cap + kInverseItems - 1) / kInverseItems, kLevelThreads), kLevelThreads,
+                0, st, dp, src, inv, walks ? nullptr : w.edge, ctl + kCtlClaimInverse, w.d_status);
         });
     }
     if (walks) {
@@ -653,47 +691,48 @@ void run_level(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p, cons
         const ListRange rr = list_range(pair_lo, pair_lo + prs, 1);
         if (l == 0) {
             rec.launch(kKindInverse, [&] {
-                level_edges<<<gp, kLevelThreads, 0, st>>>(dp, inv, w.edge, w.stamp, w.d_status);
+                launch_next(level_edges, gp, kLevelThreads, 0, st, dp, inv, w.edge, w.stamp,
+                    w.d_status);
             });
         }
         rec.launch(kKindWalk, [&] {
-            level_walk<<<(rr.hi - rr.lo + kLevelThreads - 1) / kLevelThreads, kLevelThreads, 0,
-                st>>>(dp, l, w.edge, w.stamp, w.lists.state[1], w.lists.mark[1], w.d_status);
+            launch_next(level_walk, (rr.hi - rr.lo + kLevelThreads - 1) / kLevelThreads,
+                kLevelThreads, 0, st, dp, l, w.edge, w.stamp, w.lists.state[1], w.lists.mark[1],
+                w.d_status);
         });
         rec.launch(kKindJump, [&] {
             for (uint32_t e = 1; e < shape.top; ++e) {
                 const ListRange to = list_range(pair_lo, pair_lo + prs, e + 1);
-                list_contract<<<grid_for(2ull * (to.hi - to.lo), kLevelThreads), kLevelThreads, 0,
-                    st>>>(dp, l, e, w.lists.state[e], w.lists.mark[e], w.lists.state[e + 1],
-                    w.lists.mark[e + 1], w.d_status);
+                launch_next(list_contract, grid_for(2ull * (to.hi - to.lo), kLevelThreads),
+                    kLevelThreads, 0, st, dp, l, e, w.lists.state[e], w.lists.mark[e],
+                    w.lists.state[e + 1], w.lists.mark[e + 1], w.d_status);
             }
             allow_smem((const void*)list_rank);
-            list_rank<<<(unsigned)std::min<uint64_t>(nodes, 1u << 20), shape.threads, shape.smem,
-                st>>>(dp, l, shape.top, w.lists.state[shape.top], w.lists.colour[shape.top],
-                w.d_status);
+            launch_next(list_rank, std::min<uint64_t>(nodes, 1u << 20), shape.threads, shape.smem, st,
+                dp, l, shape.top, w.lists.state[shape.top], w.lists.colour[shape.top], w.d_status);
             for (uint32_t e = shape.top; e-- > 1;) {
                 const ListRange to = list_range(pair_lo, pair_lo + prs, e);
-                list_expand<<<grid_for(to.hi - to.lo, kLevelThreads), kLevelThreads, 0, st>>>(dp, l,
-                    e, w.lists.state[e], w.lists.mark[e], w.lists.colour[e + 1],
+                launch_next(list_expand, grid_for(to.hi - to.lo, kLevelThreads), kLevelThreads, 0, st,
+                    dp, l, e, w.lists.state[e], w.lists.mark[e], w.lists.colour[e + 1],
                     w.lists.colour[e], w.d_status);
             }
         }, 2 * shape.top - 1);
         rec.launch(kKindResolve, [&] {
-            level_colours<<<gp, kLevelThreads, 0, st>>>(dp, l, w.edge, w.stamp, w.lists.colour[1],
-                w.xbits, w.d_status);
+            launch_next(level_colours, gp, kLevelThreads, 0, st, dp, l, w.edge, w.stamp,
+                w.lists.colour[1], w.xbits, w.d_status);
         });
     } else {
         rec.launch(kKindUnion, [&] {
-            level_union<<<grid_for((prs + kUnionItems - 1) / kUnionItems, kLevelThreads),
-                kLevelThreads, 0, st>>>(dp, l, inv, w.edge, ctl + kCtlClaimUnion, w.d_status);
+            launch_next(level_union, grid_for((prs + kUnionItems - 1) / kUnionItems, kLevelThreads),
+                kLevelThreads, 0, st, dp, l, inv, w.edge, ctl + kCtlClaimUnion, w.d_status);
         });
         rec.launch(kKindOrient, [&] {
-            level_orient<<<grid_for(nodes, kLevelThreads), kLevelThreads, 0, st>>>(dp, l, inv, w.edge,
-                w.d_status);
+            launch_next(level_orient, grid_for(nodes, kLevelThreads), kLevelThreads, 0, st, dp, l, inv,
+                w.edge, w.d_status);
         });
         rec.launch(kKindResolve, [&] {
-            level_roots<<<grid_for((prs + kResolveItems - 1) / kResolveItems, kLevelThreads),
-                kLevelThreads, 0, st>>>(dp, l, w.edge, w.xbits, ctl + kCtlClaimRoots, w.d_status);
+            launch_next(level_roots, grid_for((prs + kResolveItems - 1) / kResolveItems, kLevelThreads),
+                kLevelThreads, 0, st, dp, l, w.edge, w.xbits, ctl + kCtlClaimRoots, w.d_status);
         });
     }
     rec.launch(kKindOutputBits, [&] {
@@ -701,37 +740,24 @@ void run_level(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p, cons
         // words take the place of this level's; the tile builds its own
         const bool global_child = l + 1 < p.tile_level;
         const bool child_walks = global_child && walk_level(p.levels[l + 1], tune, union_find_only);
-        level_outputs<<<grid_for(prs / 2, kLevelThreads), kLevelThreads, 0, st>>>(dp, l, inv,
+        launch_next(level_outputs, grid_for(prs / 2, kLevelThreads), kLevelThreads, 0, st, dp, l, inv,
             w.xbits, w.ybits, child_inv, child_walks ? w.edge : nullptr, w.stamp,
             global_child && !child_walks ? w.edge : nullptr, ctl + kCtlClaimOutputs);
     });
     // above the shard level every shard computes the level, shard 0 alone
     // writes its switches
     const bool emit = p.shards <= 1 || l >= p.shard_level || p.shard == 0;
-    for (int side = 0; side < 2 && emit; ++side) {
-        const uint32_t* bits = side == 0 ? w.xbits : w.ybits;
-        const NodeAddress* addr = w.addr[side] + (1ull << l);
-        emission_launches(p, l, side, [&](int form, uint64_t full, int blocks) {
-            rec.launch(kKindEmit, [&] {
-                switch (form) {
-                case kEmitWords:
-                    level_emit_words<<<blocks, kLevelThreads, 0, st>>>(dp, l, side, bits, addr,
-                        d_blob);
-                    break;
-                case kEmitTranspose:
-                    level_emit_transpose<<<blocks, kLevelThreads, 0, st>>>(dp, l, side, bits,
-                        addr, d_blob, full);
-                    break;
-                case kEmitBlocks:
-                    level_emit_blocks<<<blocks, kLevelThreads, 0, st>>>(dp, l, side, bits, addr,
-                        d_blob, full);
-                    break;
-                default:
-                    level_emit<<<blocks, kLevelThreads, 0, st>>>(dp, l, side, bits, addr, d_blob,
-                        full);
-                    break;
-                }
+    if (emit) {
+        EmitParts parts{};
+        for (int side = 0; side < 2; ++side) {
+            emission_launches(p, l, side, [&](int form, uint64_t full, int blocks) {
+                parts.part[parts.count++] = EmitPart{form, side, parts.blocks, (uint32_t)blocks, full};
+                parts.blocks += (uint32_t)blocks;
             });
+        }
+        rec.launch(kKindEmit, [&] {
+            launch_next(level_emit, parts.blocks, kLevelThreads, 0, st, dp, l, parts, w.xbits,
+                w.ybits, w.addr[0] + (1ull << l), w.addr[1] + (1ull << l), d_blob);
         });
     }
     check(cudaGetLastError(), "level kernel launch");
@@ -770,21 +796,41 @@ struct TileParts {
 
 template <typename T>
 void launch_levels(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p,
-    const TileShape& shape, const Tuning& tune, const T* d_in, uint32_t* d_blob,
-    bool union_find_only, const LevelHook* after_level = nullptr,
+    const TileShape& shape, const Tuning& tune, const Header& header, const T* d_in,
+    uint32_t* d_blob, uint32_t* status_out, bool union_find_only, const LevelHook* after_level = nullptr,
     const TileParts* parts = nullptr, const InputParts* input = nullptr) {
     const Plan* dp = w.d_plan;
     const uint32_t t0 = p.tile_level;
-    if (t0 > 0) {
-        // level 0 validation: inverse slots start as 0xffffffff so a
-        // duplicated value leaves a never-written slot behind
-        check(cudaMemsetAsync(w.inv[0], 0xff, p.levels[0].cap * 4, st), "cudaMemsetAsync");
-        check(cudaMemsetAsync(w.control, 0, t0 * kCtlWords * 4, st), "cudaMemsetAsync(control)");
-        rec.launch(kKindDescriptors, [&] {
-            level_descriptors<<<grid_for(1ull << t0, kLevelThreads), kLevelThreads, 0, st>>>(dp,
-                w.addr[0], w.addr[1]);
+    const uint64_t blob_words = (p.end_offset + 3) / 4;
+    if (t0 == 0) {
+        // the tile reads the input directly: all of it first
+        for (uint32_t k = 0; input != nullptr && k < (uint32_t)input->ends.size(); ++k) {
+            input->wait(k);
+        }
+        rec.level = 0;
+        rec.launch(kKindTile, [&] {
+            auto one = std::make_unique<TileSingle>();
+            one->plan = p;
+            one->header = header;
+            allow_smem((const void*)tile_encode_single<T>);
+            const uint32_t plan_at = (shape.smem + 15) / 16 * 16;
+            const bool near = plan_at + sizeof(Plan) <= kTileSmemBudget;
+            tile_encode_single<T><<<1, single_threads(p.n),
+                near ? plan_at + sizeof(Plan) : shape.smem, st>>>(*one, d_in, d_blob,
+                (uint32_t)blob_words, status_out, shape.slots, near ? plan_at : 0u);
         });
+        check(cudaGetLastError(), "tile kernel launch");
+        return;
     }
+    rec.launch(kKindPrologue, [&] {
+        auto first = std::make_unique<Prologue>();
+        first->plan = p;
+        first->header = header;
+        const uint64_t inv_words = p.levels[0].cap;
+        prologue<<<grid_for((blob_words + inv_words) / 8, 256), 256, 0, st>>>(*first, w.d_plan,
+            w.d_status, d_blob, blob_words, w.control, t0 * kCtlWords, w.inv[0], inv_words,
+            w.addr[0], w.addr[1]);
+    });
     for (uint32_t l = 0; l < t0; ++l) {
         rec.level = (int)l;
         uint32_t* inv = w.inv[l & 1];
@@ -795,10 +841,6 @@ void launch_levels(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p,
         }
     }
     const uint32_t* tile_inv = w.inv[t0 & 1];
-    if (t0 == 0 && input != nullptr) {
-        // the tile reads the input directly: all of it first
-        for (uint32_t k = 0; k < (uint32_t)input->ends.size(); ++k) input->wait(k);
-    }
     rec.level = (int)t0;
     const uint64_t tiles = 1ull << level_nodes(p, t0).shift;
     if (tiles > 0x7fffffffull) {
@@ -814,7 +856,7 @@ void launch_levels(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p,
             const uint64_t hi = parts != nullptr ? parts->cuts[k] : tiles;
             if (hi > lo) {
                 rec.launch(kKindTile, [&] {
-                    kernel<<<(unsigned)(hi - lo), threads, shape.smem, st>>>(dp, src, d_blob,
+                    launch_next(kernel, hi - lo, threads, shape.smem, st, dp, src, d_blob,
                         w.d_status, shape.slots, (uint32_t)lo);
                 });
             }
@@ -824,19 +866,12 @@ void launch_levels(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p,
             lo = hi;
         }
     };
-    if (t0 == 0) {
-        if (wide) {
-            launch_tile(tile_encode_wide<T>, d_in);
-        } else {
-            launch_tile(tile_encode<T>, d_in);
-        }
+    if (wide) {
+        launch_tile(tile_encode_wide<uint32_t>, tile_inv);
     } else {
-        if (wide) {
-            launch_tile(tile_encode_wide<uint32_t>, tile_inv);
-        } else {
-            launch_tile(tile_encode<uint32_t>, tile_inv);
-        }
+        launch_tile(tile_encode<uint32_t>, tile_inv);
     }
+    check(cudaMemcpyAsync(status_out, w.d_status, 4, cudaMemcpyDefault, st), "status");
     check(cudaGetLastError(), "tile kernel launch");
 }
 
@@ -966,8 +1001,6 @@ int run(Workspace& w, Call& call, cudaStream_t st, const void* d_in, uint32_t en
     rec.enabled = g_profiling.load() != 0;
     rec.pool = &w.events;
     rec.st = st;
-    check(cudaMemcpyAsync(w.d_plan, w.h_plan, sizeof(Plan), cudaMemcpyHostToDevice, st),
-        "plan upload");
     Header h{};
     // of the shards of one permutation only shard 0 writes the header
     h.bytes = p.shards > 1 && p.shard != 0 ? 0u : (uint32_t)call.layout.header_bytes;
@@ -977,17 +1010,14 @@ int run(Workspace& w, Call& call, cudaStream_t st, const void* d_in, uint32_t en
     bool union_find_only = colouring == 1;
     uint32_t status = 0;
     for (int pass = 0; pass < 2; ++pass) {
-        check(cudaMemsetAsync(d_blob, 0, (p.end_offset + 3) / 4 * 4, st), "cudaMemsetAsync(blob)");
-        rec.launch(kKindPrologue, [&] { prologue<<<1, 128, 0, st>>>(w.d_status, d_blob, h); });
         if (entry_bytes == 4) {
-            launch_levels<uint32_t>(w, rec, st, p, call.shape, call.tune, (const uint32_t*)d_in,
-                d_blob, union_find_only, after_level, parts, input);
+            launch_levels<uint32_t>(w, rec, st, p, call.shape, call.tune, h, (const uint32_t*)d_in,
+                d_blob, w.h_status, union_find_only, after_level, parts, input);
         } else {
-            launch_levels<uint64_t>(w, rec, st, p, call.shape, call.tune, (const uint64_t*)d_in,
-                d_blob, union_find_only, after_level, parts, input);
+            launch_levels<uint64_t>(w, rec, st, p, call.shape, call.tune, h, (const uint64_t*)d_in,
+                d_blob, w.h_status, union_find_only, after_level, parts, input);
         }
         check(cudaEventRecord(w.stop, st), "cudaEventRecord");
-        check(cudaMemcpyAsync(w.h_status, w.d_status, 4, cudaMemcpyDeviceToHost, st), "status");
         check(cudaStreamSynchronize(st), "cudaStreamSynchronize");
         status = *w.h_status;
         if (union_find_only || p.tile_level == 0 ||
@@ -1843,33 +1873,28 @@ extern "C" int bpb200_compress_device_noalloc(const void* d_entries, uint64_t co
         w.addr[1] = reinterpret_cast<NodeAddress*>(base + noalloc::kOffAddr1);
         place_lists(noalloc::kPairs, base + noalloc::kOffLists, &w.lists);
         cudaStream_t st = (cudaStream_t)stream;
-        // The plan source is ordinary host memory: the copy is staged before
-        // cudaMemcpyAsync returns, so g_plan can be reused by the next call.
-        check(cudaMemcpyAsync(w.d_plan, &noalloc::g_plan, sizeof(Plan), cudaMemcpyHostToDevice, st),
-            "plan upload");
         Header h{};
         h.bytes = (uint32_t)call.layout.header_bytes;
         write_header(call.layout, h.data);
-        // Everything that must start cleared is cleared by the call itself:
-        // the blob (memset), the status word (prologue) and, when level
-        // kernels run, their counters and the inverse sentinels used for
-        // validation.  A second pass as in run().
+        // Everything that must start cleared is cleared by the call's first
+        // kernel.  A second pass as in run().
         const int colouring = g_force_union_find.load();
         bool union_find_only = colouring == 1;
         uint32_t status = 0;
         for (int pass = 0; pass < 2; ++pass) {
-            check(cudaMemsetAsync(d_blob, 0, (p.end_offset + 3) / 4 * 4, st), "cudaMemsetAsync(blob)");
             Recorder rec; // timing disabled: no events are created
             rec.st = st;
-            rec.launch(kKindPrologue, [&] { prologue<<<1, 128, 0, st>>>(w.d_status, (uint32_t*)d_blob, h); });
+            // one tile leaves its status in device memory, level kernels
+            // have it copied there from where they gather it
+            uint32_t* status_out = w.d_status + 1;
             if (entry_bytes == 4) {
-                launch_levels<uint32_t>(w, rec, st, p, call.shape, call.tune,
-                    (const uint32_t*)d_entries, (uint32_t*)d_blob, union_find_only);
+                launch_levels<uint32_t>(w, rec, st, p, call.shape, call.tune, h,
+                    (const uint32_t*)d_entries, (uint32_t*)d_blob, status_out, union_find_only);
             } else {
-                launch_levels<uint64_t>(w, rec, st, p, call.shape, call.tune,
-                    (const uint64_t*)d_entries, (uint32_t*)d_blob, union_find_only);
+                launch_levels<uint64_t>(w, rec, st, p, call.shape, call.tune, h,
+                    (const uint64_t*)d_entries, (uint32_t*)d_blob, status_out, union_find_only);
             }
-            check(cudaMemcpyAsync(&status, w.d_status, 4, cudaMemcpyDeviceToHost, st), "status");
+            check(cudaMemcpyAsync(&status, status_out, 4, cudaMemcpyDeviceToHost, st), "status");
             check(cudaStreamSynchronize(st), "cudaStreamSynchronize");
             if (union_find_only || p.tile_level == 0 ||
                 ((status & kErrGaveUp) == 0 && colouring != 2)) {

@@ -152,6 +152,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) level_inverse(const Plan* __restrict__ plan,
     const T* __restrict__ src, uint32_t* __restrict__ inv, uint32_t* __restrict__ uf,
     uint32_t* claims, uint32_t* status) {
+    wait_for_previous();
     level_inverse_run<T>(launch_grid(), plan, src, inv, uf, claims, status);
 }
 
@@ -273,6 +274,7 @@ __global__ void __launch_bounds__(BPB200_BUCKET_THREADS) level_bucket(const Plan
     uint32_t level, const T* __restrict__ src, uint2* __restrict__ records,
     uint32_t* __restrict__ cursor, uint32_t* __restrict__ uf, uint32_t* status,
     uint64_t e_lo, uint64_t e_hi) {
+    wait_for_previous();
     level_bucket_run<T>(launch_grid(), plan, level, src, records, cursor, uf, status, e_lo, e_hi);
 }
 
@@ -302,6 +304,7 @@ __device__ __forceinline__ void level_place_run(Grid grid, const Plan* __restric
 __global__ void __launch_bounds__(256) level_place(const Plan* __restrict__ plan,
     uint32_t level, const uint2* __restrict__ records, const uint32_t* __restrict__ cursor,
     uint32_t* __restrict__ inv, uint32_t* claims) {
+    wait_for_previous();
     level_place_run(launch_grid(), plan, level, records, cursor, inv, claims);
 }
 
@@ -372,6 +375,7 @@ __device__ __forceinline__ void level_union_run(Grid grid, const Plan* __restric
 __global__ void __launch_bounds__(256, BPB200_UNION_MIN_BLOCKS) level_union(const Plan* __restrict__ plan,
     uint32_t level, const uint32_t* __restrict__ inv, uint32_t* uf, uint32_t* claims,
     uint32_t* status) {
+    wait_for_previous();
     level_union_run(launch_grid(), plan, level, inv, uf, claims, status);
 }
 
@@ -400,6 +404,7 @@ __device__ __forceinline__ void level_orient_run(Grid grid, const Plan* __restri
 
 __global__ void level_orient(const Plan* __restrict__ plan, uint32_t level,
     const uint32_t* __restrict__ inv, uint32_t* uf, uint32_t* status) {
+    wait_for_previous();
     level_orient_run(launch_grid(), plan, level, inv, uf, status);
 }
 
@@ -418,11 +423,6 @@ __device__ __forceinline__ void level_descriptors_run(Grid grid, const Plan* __r
             out_addr[i] = node_address(*plan, 1, level, j);
         }
     }
-}
-
-__global__ void __launch_bounds__(256) level_descriptors(const Plan* __restrict__ plan,
-    NodeAddress* __restrict__ in_addr, NodeAddress* __restrict__ out_addr) {
-    level_descriptors_run(launch_grid(), plan, in_addr, out_addr);
 }
 
 // Input switch bits of a union-find level: bit k = colour of input 2k = the
@@ -492,6 +492,7 @@ __device__ __forceinline__ void level_roots_run(Grid grid, const Plan* __restric
 __global__ void __launch_bounds__(256, BPB200_FINAL_MIN_BLOCKS) level_roots(
     const Plan* __restrict__ plan, uint32_t level, uint32_t* uf, uint32_t* __restrict__ xbits,
     uint32_t* claims, uint32_t* status) {
+    wait_for_previous();
     level_roots_run(launch_grid(), plan, level, uf, xbits, claims, status);
 }
 
@@ -603,6 +604,7 @@ __global__ void __launch_bounds__(256) level_outputs(const Plan* __restrict__ pl
     uint32_t* __restrict__ ybits, uint32_t* __restrict__ child_inv,
     uint32_t* __restrict__ child_edge, uint32_t* __restrict__ child_stamp,
     uint32_t* __restrict__ child_uf, uint32_t* claims) {
+    wait_for_previous();
     level_outputs_run(launch_grid(), plan, level, inv, xbits, ybits, child_inv, child_edge,
         child_stamp, child_uf, claims);
 }
@@ -646,12 +648,6 @@ __device__ __forceinline__ void level_emit_run(Grid grid, const Plan* __restrict
         }
         emit_bit(blob, dest, set, 0xffffffffu);
     }
-}
-
-__global__ void __launch_bounds__(256) level_emit(const Plan* __restrict__ plan,
-    uint32_t level, int side, const uint32_t* __restrict__ bits,
-    const NodeAddress* __restrict__ addr, uint32_t* __restrict__ blob, uint64_t first_packet) {
-    level_emit_run(launch_grid(), plan, level, side, bits, addr, blob, first_packet);
 }
 
 // Block form of level_emit for short runs (span_log2 < 5), on the packets
@@ -708,12 +704,6 @@ __device__ __forceinline__ void level_emit_blocks_run(Grid grid, const Plan* __r
             atomicOr(blob + (dest >> 5) + 1, v >> (32 - off));
         }
     }
-}
-
-__global__ void __launch_bounds__(256) level_emit_blocks(const Plan* __restrict__ plan,
-    uint32_t level, int side, const uint32_t* __restrict__ bits,
-    const NodeAddress* __restrict__ addr, uint32_t* __restrict__ blob, uint64_t full_packets) {
-    level_emit_blocks_run(launch_grid(), plan, level, side, bits, addr, blob, full_packets);
 }
 
 // Transposed form of level_emit_blocks for cluster roots of at least 32
@@ -779,12 +769,6 @@ __device__ __forceinline__ void level_emit_transpose_run(Grid grid, const Plan* 
     }
 }
 
-__global__ void __launch_bounds__(256) level_emit_transpose(const Plan* __restrict__ plan,
-    uint32_t level, int side, const uint32_t* __restrict__ bits,
-    const NodeAddress* __restrict__ addr, uint32_t* __restrict__ blob, uint64_t full_packets) {
-    level_emit_transpose_run(launch_grid(), plan, level, side, bits, addr, blob, full_packets);
-}
-
 // Word-wise form of level_emit for levels whose packets carry at least 32
 // switches of each node (span_log2 >= 5).  The switches of one node inside
 // one packet are a contiguous run of the node's bits and land on a
@@ -837,10 +821,54 @@ __device__ __forceinline__ void level_emit_words_run(Grid grid, const Plan* __re
     }
 }
 
-__global__ void __launch_bounds__(256) level_emit_words(const Plan* __restrict__ plan,
+// Emission forms: the launches of one section at one level (see
+// emission_launches, encode.cu).
+enum EmitForm : int { kEmitWords = 0, kEmitTranspose, kEmitBlocks, kEmitBits, kEmitForms };
+
+// Both sections' switch bits of one level in one launch: part k owns blocks
+// [first, first + blocks).
+struct EmitPart {
+    int32_t form;
+    int32_t side;
+    uint32_t first;
+    uint32_t blocks;
+    uint64_t full; // full packets (block forms) or first packet (per-bit form)
+};
+struct EmitParts {
+    uint32_t count;
+    uint32_t blocks;
+    EmitPart part[4];
+};
+
+__device__ __forceinline__ void level_emit_form(Grid g, int form, const Plan* __restrict__ plan,
     uint32_t level, int side, const uint32_t* __restrict__ bits,
-    const NodeAddress* __restrict__ addr, uint32_t* __restrict__ blob) {
-    level_emit_words_run(launch_grid(), plan, level, side, bits, addr, blob);
+    const NodeAddress* __restrict__ addr, uint32_t* __restrict__ blob, uint64_t full) {
+    switch (form) {
+    case kEmitWords:
+        level_emit_words_run(g, plan, level, side, bits, addr, blob);
+        break;
+    case kEmitTranspose:
+        level_emit_transpose_run(g, plan, level, side, bits, addr, blob, full);
+        break;
+    case kEmitBlocks:
+        level_emit_blocks_run(g, plan, level, side, bits, addr, blob, full);
+        break;
+    default:
+        level_emit_run(g, plan, level, side, bits, addr, blob, full);
+        break;
+    }
+}
+
+__global__ void __launch_bounds__(256) level_emit(const Plan* __restrict__ plan, uint32_t level,
+    const __grid_constant__ EmitParts parts, const uint32_t* __restrict__ xbits,
+    const uint32_t* __restrict__ ybits, const NodeAddress* __restrict__ in_addr,
+    const NodeAddress* __restrict__ out_addr, uint32_t* __restrict__ blob) {
+    wait_for_previous();
+    uint32_t k = 0;
+    while (k + 1 < parts.count && parts.part[k + 1].first <= blockIdx.x) ++k;
+    const EmitPart& p = parts.part[k];
+    level_emit_form(Grid{blockIdx.x - p.first, p.blocks}, p.form, plan, level, p.side,
+        p.side == 0 ? xbits : ybits, p.side == 0 ? in_addr : out_addr, blob, p.full);
 }
 
 } // namespace bpb200

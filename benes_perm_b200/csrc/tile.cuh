@@ -125,7 +125,8 @@ __device__ __forceinline__ Mask tile_colour_node(const uint32_t* edge, uint32_t 
     return x;
 }
 
-template <typename T>
+// kPlanNear: the plan is already in shared memory.
+template <typename T, bool kPlanNear = false>
 __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
     const T* __restrict__ src, uint32_t* __restrict__ blob, uint32_t* status, uint32_t slots,
     uint32_t tile, unsigned char* smem) {
@@ -155,7 +156,7 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
     }
     // The levels and groups the tile works on, into L1: their first uses would
     // otherwise be chains of dependent L2 reads at every level.
-    {
+    if (!kPlanNear) {
         uint32_t sum = 0;
         const char* lo = reinterpret_cast<const char*>(&plan);
         auto touch = [&](const void* from, const void* to) {
@@ -660,6 +661,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_encode(const Plan* __res
     const T* __restrict__ src, uint32_t* __restrict__ blob, uint32_t* status, uint32_t slots,
     uint32_t part_first) {
     extern __shared__ __align__(16) unsigned char smem[];
+    wait_for_previous();
     // a sharded call encodes only its own tiles (level_nodes); a launch may
     // cover a part of them, from tile part_first on
     const uint32_t first = (uint32_t)level_nodes(*plan, plan->tile_level).lo + part_first;
@@ -674,8 +676,59 @@ __global__ void __launch_bounds__(2 * kTileThreads, 1) tile_encode_wide(
     const Plan* __restrict__ plan, const T* __restrict__ src, uint32_t* __restrict__ blob,
     uint32_t* status, uint32_t slots, uint32_t part_first) {
     extern __shared__ __align__(16) unsigned char smem[];
+    wait_for_previous();
     const uint32_t first = (uint32_t)level_nodes(*plan, plan->tile_level).lo + part_first;
     tile_body<T>(plan, src, blob, status, slots, first + blockIdx.x, smem);
+}
+
+struct Header {
+    uint32_t bytes;
+    uint8_t data[84];
+};
+
+// Word i of a blob that holds its header and nothing else.  The header ends
+// before the first section bit.
+__device__ __forceinline__ uint32_t header_word(const Header& h, uint64_t i) {
+    uint32_t v = 0;
+    for (uint32_t k = 0; k < 4; ++k) {
+        if (4 * i + k < h.bytes) v |= (uint32_t)h.data[4 * i + k] << (8 * k);
+    }
+    return v;
+}
+
+// A permutation that is one tile, as a single launch: the plan and the
+// header come as kernel parameters, the block keeps the plan in shared
+// memory at byte `plan_at` (0: no room, it stays a parameter), clears the blob and leaves the status word at `status_out`
+// (device or pinned host memory).  A plan upload, a memset, a header kernel
+// and a status download around the tile took 40 of the 90 us of a 1000-entry
+// call.
+struct TileSingle {
+    Plan plan;
+    Header header;
+};
+
+template <typename T>
+__global__ void __launch_bounds__(2 * kTileThreads, 1) tile_encode_single(
+    const __grid_constant__ TileSingle one, const T* __restrict__ src,
+    uint32_t* __restrict__ blob, uint32_t blob_words, uint32_t* status_out, uint32_t slots,
+    uint32_t plan_at) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ uint32_t status;
+    const Plan* plan = &one.plan;
+    if (plan_at != 0) {
+        uint32_t* near = reinterpret_cast<uint32_t*>(smem + plan_at);
+        const uint32_t* from = reinterpret_cast<const uint32_t*>(&one.plan);
+        for (uint32_t i = threadIdx.x; i < sizeof(Plan) / 4; i += blockDim.x) near[i] = from[i];
+        plan = reinterpret_cast<const Plan*>(near);
+    }
+    for (uint32_t i = threadIdx.x; i < blob_words; i += blockDim.x) {
+        blob[i] = header_word(one.header, i);
+    }
+    if (threadIdx.x == 0) status = 0;
+    __syncthreads();
+    tile_body<T, true>(plan, src, blob, &status, slots, 0, smem);
+    __syncthreads();
+    if (threadIdx.x == 0) *(volatile uint32_t*)status_out = status;
 }
 
 // Tiles of many permutations in one launch (the batched and serving forms):

@@ -132,6 +132,7 @@ __device__ __forceinline__ void level_edges_run(Grid grid, const Plan* __restric
 __global__ void __launch_bounds__(256) level_edges(const Plan* __restrict__ plan,
     const uint32_t* __restrict__ inv, uint32_t* __restrict__ edge, uint32_t* __restrict__ stamp,
     uint32_t* status) {
+    wait_for_previous();
     level_edges_run(launch_grid(), plan, inv, edge, stamp, status);
 }
 
@@ -221,6 +222,7 @@ __device__ __forceinline__ void level_walk_run(Grid grid, const Plan* __restrict
 __global__ void __launch_bounds__(256, 8) level_walk(const Plan* __restrict__ plan, uint32_t level,
     const uint32_t* __restrict__ edge, uint32_t* stamp, uint4* __restrict__ state,
     uint32_t* __restrict__ mark, uint32_t* status) {
+    wait_for_previous();
     level_walk_run(launch_grid(), plan, level, edge, stamp, state, mark, status);
 }
 
@@ -277,6 +279,7 @@ __device__ __forceinline__ void list_contract_run(Grid grid, const Plan* __restr
 __global__ void __launch_bounds__(256) list_contract(const Plan* __restrict__ plan,
     uint32_t level, uint32_t e, const uint4* __restrict__ state, uint32_t* mark,
     uint4* __restrict__ up_state, uint32_t* __restrict__ up_mark, uint32_t* status) {
+    wait_for_previous();
     list_contract_run(launch_grid(), plan, level, e, state, mark, up_state, up_mark, status);
 }
 
@@ -328,6 +331,7 @@ __device__ __forceinline__ void list_expand_run(Grid grid, const Plan* __restric
 __global__ void __launch_bounds__(256) list_expand(const Plan* __restrict__ plan, uint32_t level,
     uint32_t e, const uint4* __restrict__ state, const uint32_t* __restrict__ mark,
     const uint8_t* __restrict__ up_colour, uint8_t* __restrict__ colour, uint32_t* status) {
+    wait_for_previous();
     list_expand_run(launch_grid(), plan, level, e, state, mark, up_colour, colour, status);
 }
 
@@ -501,6 +505,7 @@ __global__ void __launch_bounds__(kRankThreads, 1) list_rank(const Plan* __restr
     uint32_t level, uint32_t e, const uint4* __restrict__ state, uint8_t* __restrict__ colour,
     uint32_t* status) {
     extern __shared__ __align__(16) uint32_t rank_shared[];
+    wait_for_previous();
     list_rank_run(launch_grid(), plan, level, e, state, colour, status, rank_shared);
 }
 
@@ -566,6 +571,7 @@ __device__ __forceinline__ void level_colours_run(Grid grid, const Plan* __restr
 __global__ void __launch_bounds__(256) level_colours(const Plan* __restrict__ plan,
     uint32_t level, const uint32_t* __restrict__ edge, const uint32_t* __restrict__ stamp,
     const uint8_t* __restrict__ colour, uint32_t* __restrict__ xbits, uint32_t* status) {
+    wait_for_previous();
     level_colours_run(launch_grid(), plan, level, edge, stamp, colour, xbits, status);
 }
 
