@@ -309,13 +309,13 @@ void launch_next(void (*kernel)(Params...), uint64_t blocks, uint32_t threads, u
 TileShape tile_shape(const Plan& p, uint32_t t0) {
     uint64_t slots = 0;
     for (uint32_t l = t0; l <= p.depth; ++l) {
-        const uint64_t stride = 2 * ((p.levels[l].pcap + 1) / 2 * 2);
-        slots = std::max<uint64_t>(slots, stride << (l - t0));
+        slots = std::max<uint64_t>(slots,
+            (uint64_t)tile_node_slots(p.levels[l].pcap, l == p.depth, p.leaf) << (l - t0));
     }
     TileShape s;
-    s.slots = (uint32_t)std::min<uint64_t>(slots, 1u << 30);
-    uint32_t off[7];
-    s.smem = tile_smem_layout(s.slots, off);
+    s.slots = (uint32_t)std::min<uint64_t>((slots + 3) & ~3ull, 1u << 30);
+    uint32_t off[5];
+    s.smem = tile_smem_layout(s.slots, p.depth - t0, off);
     if (slots >= 65536) {
         s.smem = UINT32_MAX;
     }

@@ -77,27 +77,29 @@ __device__ __forceinline__ void shared_store16_if(bool yes, uint32_t addr, uint3
                  :: "r"((uint32_t)yes), "r"(addr), "h"((uint16_t)v) : "memory");
 }
 
-// Where one node's switches of one section go: first bits of its run in
-// packet 0 and in its tail packet, packets of the section's cluster apart.
-struct TileAddress {
-    uint64_t full; // top bit: the cluster root is a large node
-    uint64_t tail;
-};
-constexpr uint64_t kTileRootLarge = 1ull << 63;
+// Slots per node in the tile's arrays: two per pair-node of the stride, or,
+// at the leaf level, a leaf's entries if those are fewer.
+__host__ __device__ inline uint32_t tile_node_slots(uint64_t pcap, bool leaf_level, uint32_t leaf) {
+    const uint32_t slots = 2 * tile_pair_stride(pcap);
+    return leaf_level && leaf < slots ? leaf : slots;
+}
+
+// Words of one section's switch bits at one level, with a spare word.
+__host__ __device__ inline uint32_t tile_bit_words(uint32_t slots) { return slots / 64 + 2; }
 
 // Byte offsets of the smem arrays; identical on host (sizing) and device.
-// `slots`: 2 * tile_pair_stride * nodes at the level that needs most.
-__host__ __device__ inline uint32_t tile_smem_layout(uint32_t slots, uint32_t* off) {
-    const uint32_t words = slots / 64 + 2;
+// `slots`: nodes * tile_node_slots at the level that needs most; `levels`:
+// routing levels in the tile.
+__host__ __device__ inline uint32_t tile_smem_layout(uint32_t slots, uint32_t levels,
+    uint32_t* off) {
     const uint32_t rulers = (slots >> (kTileRulerLog2 + 1)) + 1;
     uint32_t o = 0;
     off[0] = o; o = align_up(o + slots * 2, 16);           // inverse, even levels
     off[1] = o; o = align_up(o + slots * 2, 16);           // inverse, odd levels
     off[2] = o; o = align_up(o + slots * 2, 16);           // edges, one word per pair-node
     off[3] = o; o = align_up(o + rulers * 8, 16);          // directed ruler states
-    off[4] = o; o = align_up(o + words * 4, 16);           // xbits (input switches)
-    off[5] = o; o = align_up(o + words * 4, 16);           // ybits (output switches)
-    off[6] = o; o = align_up(o + 2 * kNodeWave * (uint32_t)sizeof(TileAddress), 16);
+    off[4] = o; // switch bits of every level, input and output section
+    o = align_up(o + 2 * levels * tile_bit_words(slots) * 4, 16);
     return o;
 }
 
@@ -130,16 +132,15 @@ template <typename T, bool kPlanNear = false>
 __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
     const T* __restrict__ src, uint32_t* __restrict__ blob, uint32_t* status, uint32_t slots,
     uint32_t tile, unsigned char* smem) {
-    uint32_t off[7];
-    tile_smem_layout(slots, off);
+    uint32_t off[5];
+    tile_smem_layout(slots, plan_ptr->depth - plan_ptr->tile_level, off);
     uint16_t* invs[2] = {(uint16_t*)(smem + off[0]), (uint16_t*)(smem + off[1])};
     uint32_t* edge = (uint32_t*)(smem + off[2]);
     uint16_t* edge16 = (uint16_t*)edge;
     uint32_t* state = (uint32_t*)(smem + off[3]);
     volatile uint32_t* vstate = state;
-    uint32_t* xbits = (uint32_t*)(smem + off[4]);
-    uint32_t* ybits = (uint32_t*)(smem + off[5]);
-    TileAddress* desc = (TileAddress*)(smem + off[6]);
+    uint32_t* level_bits = (uint32_t*)(smem + off[4]);
+    const uint32_t bit_words = tile_bit_words(slots);
 
     const Plan& plan = *plan_ptr;
     const uint32_t tid = threadIdx.x;
@@ -263,7 +264,7 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
         }
     }
 
-    for (uint32_t t = 0;; ++t) {
+    for (uint32_t t = 0; T0 + t < D; ++t) {
         const uint32_t level = T0 + t;
         const LevelInfo& lv = plan.levels[level];
         const uint32_t nodes = 1u << t;
@@ -273,8 +274,10 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
         const uint32_t ps = tile_pair_stride(lv.pcap);
         const uint32_t stride = 2 * ps;
         const FastDiv by_ps(ps);
-        uint16_t* cur = invs[t & 1]; // this level's inverse (values, for leaves)
-        uint16_t* nxt = invs[(t + 1) & 1];
+        const uint16_t* cur = invs[t & 1]; // this level's inverse
+        uint16_t* nxt = invs[(t + 1) & 1]; // the children's (values, for leaves)
+        uint32_t* xbits = level_bits + 2 * t * bit_words;
+        uint32_t* ybits = xbits + bit_words;
         // uniform per level: whether every node here exists / is internal
         const bool all_exist = level == 0 || plan.levels[level - 1].q > leaf;
         const bool all_internal = q32 > leaf && all_exist;
@@ -294,7 +297,7 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
         // key(w) = (w + bias) mod 2^16 (see the top of this file)
         auto key_bias = [](uint32_t s) { return (s & 1u) != 0 ? 0u - (s - 1u) : 0u; };
 
-        if (level < D) {
+        {
             // ---- input switch bits: the colour of input 2k of every pair-node
             if (ps <= kTileSerialPairs) {
                 for (uint32_t e = tid; e < (nodes * ps + 31) / 32 + 1; e += blockDim.x) xbits[e] = 0;
@@ -441,7 +444,7 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
             // of its edges, or a leaf child's values.
             {
                 const LevelInfo& cl = plan.levels[level + 1];
-                const uint32_t cstride = 2 * tile_pair_stride(cl.pcap);
+                const uint32_t cstride = tile_node_slots(cl.pcap, level + 1 == D, leaf);
                 const uint32_t hs = ps / 2;
                 const FastDiv by_hs(hs);
                 const uint32_t total = nodes * hs;
@@ -496,161 +499,188 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
                     }
                 }
             }
-            // ---- switch bits out, packet-major over a wave of node addresses
-            const uint32_t wave_log2 = t < kNodeWaveLog2 ? t : kNodeWaveLog2; // log2(min(nodes, kNodeWave))
-            const uint32_t wn = 1u << wave_log2;
-            for (uint32_t w0 = 0; w0 < nodes; w0 += wn) {
-                for (uint32_t e = tid; e < 2 * wn; e += blockDim.x) {
-                    const uint32_t slot = e >> 1;
-                    const int side = (int)(e & 1);
-                    const uint32_t s = node_size(w0 + slot);
-                    if (internal_node(w0 + slot, s)) {
-                        const NodeAddress a = node_address(plan, side, level, first + w0 + slot);
-                        const GroupInfo& gi = plan.groups[side][lv.side[side].group];
-                        const bool large = a.packet_bits == gi.packet_bits[1] &&
-                            gi.packet_bits[0] != gi.packet_bits[1];
-                        const uint64_t at = plan.section_offset[side] * 8 + a.base;
-                        desc[side * kNodeWave + slot] = TileAddress{
-                            (at + a.full_prefix) | (large ? kTileRootLarge : 0ull),
-                            at + a.tail_prefix};
-                    }
-                }
-                __syncthreads();
-                for (int side = 0; side < 2; ++side) {
-                    const LevelSide& ls = lv.side[side];
-                    const GroupInfo& gi = plan.groups[side][ls.group];
-                    const uint32_t span_log2 = gi.depth - ls.rel - 1;
-                    const uint32_t shift = wave_log2 + span_log2;
-                    const uint32_t packets =
-                        ((uint32_t)lv.cap / 2 + (1u << span_log2) - 1) >> span_log2;
-                    const uint32_t* bits = side == 0 ? xbits : ybits;
-                    const uint64_t packet_bits[2] = {gi.packet_bits[0], gi.packet_bits[1]};
-                    // blob bit of switch `pair` of a node with `half` switches
-                    auto bit_of = [&](uint32_t slot, uint32_t pair, uint32_t half) {
-                        const TileAddress& a = desc[side * kNodeWave + slot];
-                        const uint32_t packet = pair >> span_log2;
-                        const uint64_t full = a.full;
-                        return (packet == (half - 1) >> span_log2 ? a.tail : full & ~kTileRootLarge) +
-                            packet * packet_bits[full >> 63] + (pair & ((1u << span_log2) - 1));
-                    };
-                    auto put = [&](uint64_t dest, uint32_t v) {
-                        const uint32_t sh = (uint32_t)(dest & 31);
-                        atomicOr(blob + (dest >> 5), v << sh);
-                        if (sh != 0 && (v >> (32 - sh)) != 0) {
-                            atomicOr(blob + (dest >> 5) + 1, v >> (32 - sh));
-                        }
-                    };
-                    if (span_log2 >= 5) {
-                        // runs of at least 32 switches: word-wise copies as in
-                        // level_emit_words (the bit arrays keep a spare word)
-                        const uint32_t cshift = span_log2 - 5;
-                        const uint32_t cs = wave_log2 + cshift;
-                        const uint32_t chunks = packets << cs;
-                        for (uint32_t c = tid; c < chunks; c += blockDim.x) {
-                            const uint32_t packet = c >> cs;
-                            const uint32_t rem = c & ((1u << cs) - 1);
-                            const uint32_t slot = rem >> cshift;
-                            const uint32_t pair0 =
-                                (packet << span_log2) + ((rem & ((1u << cshift) - 1)) << 5);
-                            const uint32_t path = w0 + slot;
-                            const uint32_t s = node_size(path);
-                            if (pair0 >= s / 2 || !internal_node(path, s)) {
-                                continue;
-                            }
-                            const uint32_t q = path * ps + pair0;
-                            uint32_t v = __funnelshift_r(bits[q >> 5], bits[(q >> 5) + 1], q & 31);
-                            if (s / 2 - pair0 < 32) {
-                                v &= (1u << (s / 2 - pair0)) - 1u;
-                            }
-                            if (v != 0) {
-                                put(bit_of(slot, pair0, s / 2), v);
-                            }
-                        }
-                        continue;
-                    }
-                    // short runs: the packets every node fills go out as
-                    // word blocks (see level_emit_blocks), the rest bit by bit
-                    uint32_t full = 0;
-                    if (all_internal && q32 / 2 >= 1) {
-                        full = ((q32 / 2) - 1) >> span_log2;
-                    }
-                    if (full > packets) {
-                        full = packets;
-                    }
-                    if (full > 0) {
-                        const uint32_t rel = ls.rel;
-                        // nodes per word: within a word, a cluster root and the wave
-                        uint32_t g_log2 = 5 - span_log2;
-                        g_log2 = g_log2 < rel ? g_log2 : rel;
-                        g_log2 = g_log2 < wave_log2 ? g_log2 : wave_log2;
-                        const uint32_t span_mask = (1u << (1u << span_log2)) - 1u;
-                        const uint32_t groups_log2 = wave_log2 - g_log2;
-                        const uint32_t work = full << groups_log2;
-                        for (uint32_t c = tid; c < work; c += blockDim.x) {
-                            const uint32_t packet = c >> groups_log2;
-                            const uint32_t slot0 = (c & ((1u << groups_log2) - 1)) << g_log2;
-                            uint32_t v = 0;
-                            for (uint32_t i = 0; i < (1u << g_log2); ++i) {
-                                const uint32_t q = (w0 + slot0 + i) * ps + (packet << span_log2);
-                                const uint32_t field =
-                                    __funnelshift_r(bits[q >> 5], bits[(q >> 5) + 1], q & 31) &
-                                    span_mask;
-                                v |= field << (i << span_log2);
-                            }
-                            if (v != 0) { // below every node's tail packet
-                                put(bit_of(slot0, packet << span_log2, node_size(w0 + slot0) / 2), v);
-                            }
-                        }
-                    }
-                    const uint32_t rest = (packets - full) << shift;
-                    for (uint32_t base = warp * 32; base < rest; base += nwarps * 32) {
-                        const uint32_t tt = base + lane;
-                        bool set = false;
-                        uint64_t dest = 0;
-                        if (tt < rest) {
-                            const uint32_t packet = full + (tt >> shift);
-                            const uint32_t rem = tt & ((1u << shift) - 1);
-                            const uint32_t slot = rem >> span_log2;
-                            const uint32_t pair = (packet << span_log2) + (rem & ((1u << span_log2) - 1));
-                            const uint32_t path = w0 + slot;
-                            const uint32_t s = node_size(path);
-                            if (pair < s / 2 && internal_node(path, s)) {
-                                const uint32_t q = path * ps + pair;
-                                set = ((bits[q >> 5] >> (q & 31)) & 1u) != 0;
-                                if (set) {
-                                    dest = bit_of(slot, pair, s / 2);
-                                }
-                            }
-                        }
-                        emit_bit(blob, dest, set, 0xffffffffu);
-                    }
-                }
-                __syncthreads();
-            }
         }
+        __syncthreads();
+    }
 
-        // leaves at this level (all of level D, and the size-`leaf` nodes of a
-        // mixed level D - 1): one thread per leaf (see thread_factoradic_rank)
-        if (q32 <= leaf) {
-            for (uint32_t path = tid; path < nodes; path += blockDim.x) {
-                const uint32_t s = node_size(path);
-                if (s > leaf || !exists(path)) {
-                    continue;
-                }
+    // ---- switch bits and middle-group ranks out, all levels at once: a warp
+    // task is one section of up to 32 nodes of a level, or the ranks of up to
+    // 32 leaves.  Keeping every level's bits until here costs 1/32 of the
+    // tile's memory per level; going out level by level, with two barriers
+    // and a wave of node addresses each time, took a third of a small tile's
+    // time.
+    const uint32_t levels = D - T0;
+    uint32_t tasks = 0;
+    for (uint32_t t = 0; t < levels; ++t) tasks += t < 5 ? 2u : 2u << (t - 5);
+    const uint32_t leaf_tasks = levels < 5 ? 1u : 1u << (levels - 5);
+    const bool mixed = levels > 0 && plan.levels[D - 1].q <= leaf; // leaves at level D - 1 too
+    tasks += leaf_tasks + (mixed ? (levels < 6 ? 1u : 1u << (levels - 6)) : 0u);
+    for (uint32_t task = warp; task < tasks; task += nwarps) {
+        uint32_t t = 0, at = task;
+        for (; t < levels; ++t) {
+            const uint32_t here = t < 5 ? 2u : 2u << (t - 5);
+            if (at < here) break;
+            at -= here;
+        }
+        const bool is_leaf = t == levels;
+        if (is_leaf && at >= leaf_tasks) { // level D - 1's leaves
+            at -= leaf_tasks;
+            --t;
+        }
+        const uint32_t level = T0 + t;
+        const LevelInfo& lv = plan.levels[level];
+        const uint32_t first = J << t;
+        const uint32_t q32 = (uint32_t)lv.q;
+        const uint32_t r32 = (uint32_t)lv.r;
+        const bool all_exist = level == 0 || plan.levels[level - 1].q > leaf;
+        auto node_size = [&](uint32_t path) {
+            if (r32 == 0) return q32;
+            return q32 + ((__brev(first + path) >> (32 - level)) < r32 ? 1u : 0u);
+        };
+        auto exists = [&](uint32_t path) {
+            return all_exist ||
+                size_at(plan.levels[level - 1], level - 1, (first + path) >> 1) > leaf;
+        };
+        const uint32_t wave_log2 = t < 5 ? t : 5; // log2 of the task's nodes
+        const uint32_t slot_mask = (1u << wave_log2) - 1;
+        if (is_leaf) {
+            const uint32_t path = (at << 5) + lane;
+            const uint32_t s = lane <= slot_mask ? node_size(path) : leaf + 1;
+            if (s <= leaf && exists(path)) {
                 int section = 0;
                 const uint64_t bit = leaf_rank_bit(plan, level, first + path, &section);
                 bool valid = true;
-                const U128 rank = thread_factoradic_rank(cur + path * stride, s, &valid);
-                if (!valid) {
+                const U128 rank = thread_factoradic_rank(
+                    invs[t & 1] + path * tile_node_slots(lv.pcap, level == D, leaf), s, &valid);
+                if (valid) {
+                    thread_emit_rank(blob, plan.section_offset[section] * 8 + bit,
+                        plan.fact_bits[s], rank);
+                } else {
                     atomicOr(status, kErrNotPermutation);
-                    continue;
                 }
-                thread_emit_rank(blob, plan.section_offset[section] * 8 + bit,
-                    plan.fact_bits[s], rank);
+            }
+            continue;
+        }
+        const int side = (int)(at & 1);
+        const uint32_t w0 = (at >> 1) << 5;
+        const uint32_t ps = tile_pair_stride(lv.pcap);
+        const uint32_t* bits = level_bits + (2 * t + side) * bit_words;
+        const LevelSide& ls = lv.side[side];
+        const GroupInfo& gi = plan.groups[side][ls.group];
+        const uint32_t span_log2 = gi.depth - ls.rel - 1;
+        const uint64_t packet_bits[2] = {gi.packet_bits[0], gi.packet_bits[1]};
+        // this lane's node: its switches (0: not an internal node) and the
+        // blob bits of its run in packet 0 and in its tail packet
+        uint32_t my_half = 0, my_large = 0;
+        uint64_t my_full = 0, my_tail = 0;
+        {
+            const uint32_t path = w0 + (lane & slot_mask);
+            const uint32_t s = node_size(path);
+            if (s > leaf && exists(path)) {
+                const NodeAddress a = node_address(plan, side, level, first + path);
+                const uint64_t start = plan.section_offset[side] * 8 + a.base;
+                my_half = s / 2;
+                my_large = a.packet_bits != packet_bits[0] ? 1u : 0u;
+                my_full = start + a.full_prefix;
+                my_tail = start + a.tail_prefix;
             }
         }
-        if (level >= D) {
-            break;
+        // blob bit of switch `pair` of node `slot`; all lanes call
+        auto bit_of = [&](uint32_t slot, uint32_t pair, uint32_t half) {
+            const uint32_t packet = pair >> span_log2;
+            const uint64_t full = __shfl_sync(0xffffffffu, my_full, slot);
+            const uint64_t tail = __shfl_sync(0xffffffffu, my_tail, slot);
+            const uint32_t large = __shfl_sync(0xffffffffu, my_large, slot);
+            return (packet == (half - 1) >> span_log2 ? tail : full) +
+                packet * (large != 0 ? packet_bits[1] : packet_bits[0]) +
+                (pair & ((1u << span_log2) - 1));
+        };
+        auto put = [&](uint64_t dest, uint32_t v) {
+            if (v == 0) return;
+            const uint32_t sh = (uint32_t)(dest & 31);
+            atomicOr(blob + (dest >> 5), v << sh);
+            if (sh != 0 && (v >> (32 - sh)) != 0) {
+                atomicOr(blob + (dest >> 5) + 1, v >> (32 - sh));
+            }
+        };
+        const uint32_t packets = ((uint32_t)lv.cap / 2 + (1u << span_log2) - 1) >> span_log2;
+        if (span_log2 >= 5) {
+            // runs of at least 32 switches: word-wise copies as in
+            // level_emit_words
+            const uint32_t cshift = span_log2 - 5;
+            const uint32_t cs = wave_log2 + cshift;
+            const uint32_t chunks = packets << cs;
+            for (uint32_t base = 0; base < chunks; base += 32) {
+                const uint32_t c = base + lane;
+                const uint32_t packet = c >> cs;
+                const uint32_t rem = c & ((1u << cs) - 1);
+                const uint32_t slot = rem >> cshift;
+                const uint32_t pair0 =
+                    (packet << span_log2) + ((rem & ((1u << cshift) - 1)) << 5);
+                const uint32_t half = __shfl_sync(0xffffffffu, my_half, slot);
+                const uint64_t dest = bit_of(slot, pair0, half);
+                if (c < chunks && pair0 < half) {
+                    const uint32_t q = (w0 + slot) * ps + pair0;
+                    uint32_t v = __funnelshift_r(bits[q >> 5], bits[(q >> 5) + 1], q & 31);
+                    if (half - pair0 < 32) {
+                        v &= (1u << (half - pair0)) - 1u;
+                    }
+                    put(dest, v);
+                }
+            }
+            continue;
+        }
+        // short runs: the packets every node fills go out as word blocks
+        // (see level_emit_blocks_run), the rest bit by bit
+        uint32_t full = 0;
+        if (q32 > leaf && all_exist && q32 / 2 >= 1) {
+            full = ((q32 / 2) - 1) >> span_log2;
+        }
+        if (full > packets) {
+            full = packets;
+        }
+        if (full > 0) {
+            // nodes per word: within a word, a cluster root and the task
+            uint32_t g_log2 = 5 - span_log2;
+            g_log2 = g_log2 < ls.rel ? g_log2 : ls.rel;
+            g_log2 = g_log2 < wave_log2 ? g_log2 : wave_log2;
+            const uint32_t span_mask = (1u << (1u << span_log2)) - 1u;
+            const uint32_t groups_log2 = wave_log2 - g_log2;
+            const uint32_t work = full << groups_log2;
+            for (uint32_t base = 0; base < work; base += 32) {
+                const uint32_t c = base + lane;
+                const uint32_t packet = c >> groups_log2;
+                const uint32_t slot0 = (c & ((1u << groups_log2) - 1)) << g_log2;
+                // below every node's tail packet: any half past it will do
+                const uint64_t dest = bit_of(slot0, packet << span_log2, 0u);
+                if (c < work) {
+                    uint32_t v = 0;
+                    for (uint32_t i = 0; i < (1u << g_log2); ++i) {
+                        const uint32_t q = (w0 + slot0 + i) * ps + (packet << span_log2);
+                        const uint32_t field =
+                            __funnelshift_r(bits[q >> 5], bits[(q >> 5) + 1], q & 31) & span_mask;
+                        v |= field << (i << span_log2);
+                    }
+                    put(dest, v);
+                }
+            }
+        }
+        const uint32_t shift = wave_log2 + span_log2;
+        const uint32_t rest = (packets - full) << shift;
+        for (uint32_t base = 0; base < rest; base += 32) {
+            const uint32_t c = base + lane;
+            const uint32_t packet = full + (c >> shift);
+            const uint32_t rem = c & ((1u << shift) - 1);
+            const uint32_t slot = rem >> span_log2;
+            const uint32_t pair = (packet << span_log2) + (rem & ((1u << span_log2) - 1));
+            const uint32_t half = __shfl_sync(0xffffffffu, my_half, slot);
+            const uint64_t dest = bit_of(slot, pair, half);
+            bool set = false;
+            if (c < rest && pair < half) {
+                const uint32_t q = (w0 + slot) * ps + pair;
+                set = ((bits[q >> 5] >> (q & 31)) & 1u) != 0;
+            }
+            emit_bit(blob, dest, set, 0xffffffffu);
         }
     }
 }
