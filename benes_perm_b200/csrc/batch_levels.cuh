@@ -229,8 +229,7 @@ __global__ void __launch_bounds__(256) batch_outputs(const LevelJob* jobs, uint3
     const LevelJob* j = level_job(jobs, n, kBOutputs, &g);
     if (g.bid >= g.nblk) return;
     level_outputs_run(g, j->plan, j->level, j->inv, j->xbits, j->ybits, j->child_inv,
-        j->child_walks == 1 ? j->edge : nullptr, j->stamp, j->child_walks == 0 ? j->edge : nullptr,
-        j->control + kCtlClaimOutputs);
+        j->child_walks == 1 ? j->edge : nullptr, j->stamp, j->child_walks == 0 ? j->edge : nullptr);
 }
 
 // Switch emission: every (permutation, section, form) of the level in one

@@ -213,14 +213,17 @@ struct Lease {
     ~Lease() { release(w); }
 };
 
+bool single_launch(const Plan& p);
+
 // Grows the level scratch to fit `p`.  Growth at least doubles the previous
 // capacities: freeing device memory synchronises the whole device, so a
 // workspace that serves requests of varying sizes (the batched and serving
 // forms) must reach its final size after a few calls, not one per call.
 void ensure_scratch(Workspace& w, const Plan& p) {
-    uint64_t slots = p.tile_level > 0 ? p.max_slots : 0;
-    uint64_t pairs = p.tile_level > 0 ? p.max_pairs : 0;
-    uint64_t nodes = p.tile_level > 0 ? (1ull << p.tile_level) : 0;
+    const bool levels = !single_launch(p);
+    uint64_t slots = levels ? p.max_slots : 0;
+    uint64_t pairs = levels ? p.max_pairs : 0;
+    uint64_t nodes = levels ? (1ull << p.tile_level) : 0;
     const bool need_records = p.levels[0].cap > kWalkMaxNode;
     if (slots <= w.slot_cap && pairs <= w.pair_cap && nodes <= w.node_cap &&
         (w.records != nullptr || !need_records)) {
@@ -306,20 +309,65 @@ void launch_next(void (*kernel)(Params...), uint64_t blocks, uint32_t threads, u
 
 // ------------------------------------------------------------ tile sizing
 
-TileShape tile_shape(const Plan& p, uint32_t t0) {
+// Shared memory of levels [t0, stop) of one node of level t0.
+TileShape tile_shape(const Plan& p, uint32_t t0, uint32_t stop) {
     uint64_t slots = 0;
-    for (uint32_t l = t0; l <= p.depth; ++l) {
+    const uint32_t end = stop == p.depth ? stop + 1 : stop; // the leaves, too
+    for (uint32_t l = t0; l < end; ++l) {
         slots = std::max<uint64_t>(slots,
             (uint64_t)tile_node_slots(p.levels[l].pcap, l == p.depth, p.leaf) << (l - t0));
     }
     TileShape s;
     s.slots = (uint32_t)std::min<uint64_t>((slots + 3) & ~3ull, 1u << 30);
     uint32_t off[5];
-    s.smem = tile_smem_layout(s.slots, p.depth - t0, off);
+    s.smem = tile_smem_layout(s.slots, stop - t0, off);
     if (slots >= 65536) {
         s.smem = UINT32_MAX;
     }
     return s;
+}
+
+TileShape tile_shape(const Plan& p, uint32_t t0) { return tile_shape(p, t0, p.depth); }
+
+// Stages.  Nodes of up to 2^15 entries fit an SM for a level or two even
+// when they are above the tile size: the levels from there to the tile level
+// run as one launch of tile_encode_wide over [l, stop) instead of level
+// kernels, which for so small nodes are all launches and latency (2^20
+// entries: 672 -> 648 us) or random L2 accesses (2^30 entries, levels 15 and
+// 16: 27 ms as level kernels, 15 ms as a stage).
+// A launch of few tiles hands the subtree over after two levels to four
+// times as many CTAs: a lone CTA takes 12 us for a level of 16384 entries,
+// four take 6 (16384 entries: 187 -> 141 us, 2^16: 285 -> 230 us; tiles of
+// 4096 entries lose more by the hand-over than they gain, 93 -> 103 us).
+constexpr uint64_t kStageMaxNode = 1ull << 15;
+constexpr uint32_t kStageLevels = 2;
+constexpr uint64_t kFewTiles = 4 * 148;          // CTAs after the hand-over, at most
+constexpr uint64_t kFewTilesMinNode = 4096;      // larger tiles only
+
+// Level at which a stage from level l on stops, at or before `last`; 0: no
+// stage.
+uint32_t stage_stop(const Plan& p, uint32_t l, uint32_t last) {
+    if (l >= last || p.levels[l].cap > kStageMaxNode || (p.shards > 1 && l < p.shard_level)) {
+        return 0;
+    }
+    for (uint32_t stop = std::min(last, l + kStageLevels); stop > l; --stop) {
+        // every node handed over has to be internal
+        if (stop < p.depth && p.levels[stop].q > p.leaf &&
+            tile_shape(p, l, stop).smem <= kTileSmemBudget) {
+            return stop;
+        }
+    }
+    return 0;
+}
+
+// Level at which a launch of the tiles of level l hands over, or 0: whole
+// subtrees.
+uint32_t few_tiles_stop(const Plan& p, uint32_t l) {
+    const uint64_t tiles = 1ull << level_nodes(p, l).shift;
+    if (tiles * 4 > kFewTiles || p.levels[l].cap <= kFewTilesMinNode) {
+        return 0;
+    }
+    return stage_stop(p, l, p.depth);
 }
 
 // Threads per tile.  With more tiles than two per SM, 256: the tile is bound
@@ -327,16 +375,18 @@ TileShape tile_shape(const Plan& p, uint32_t t0) {
 // less at theirs (tiles of 100,000,007 entries: 6.1 ms against 7.7 ms with
 // 512).  Fewer tiles than that leave SMs idle, and one tile ends sooner with
 // 512 (8192 entries: 107 us against 140 us).  Wide tiles fill an SM each.
-unsigned tile_threads(uint64_t tiles, bool wide) {
-    return wide ? 2 * kTileThreads : (tiles > 2 * 148 ? kTileThreads / 2 : kTileThreads);
-}
-
-// Threads of a permutation that is a single tile: 8 entries each.
-unsigned single_threads(uint64_t n) {
+unsigned tile_threads(uint64_t tiles, bool wide, uint64_t entries) {
+    if (tiles > 2 * 148 && !wide) return kTileThreads / 2;
     unsigned t = 128;
-    while (t < 2 * kTileThreads && (uint64_t)t * 8 < n) t *= 2;
+    while (t < (wide ? 2 : 1) * kTileThreads && (uint64_t)t * 8 < entries) t *= 2;
     return t;
 }
+
+// Threads of a stage: 8 entries each, up to 1024.
+unsigned stage_threads(uint64_t entries) { return tile_threads(1, true, entries); }
+
+// Whether the whole permutation is one launch of one CTA.
+bool single_launch(const Plan& p) { return p.tile_level == 0 && few_tiles_stop(p, 0) == 0; }
 
 // Picks the tile level: the first level whose nodes fit `tile_max` entries
 // and whose deepest padded tile level also fits the shared-memory budget.
@@ -352,7 +402,9 @@ void choose_tile(Plan& p, TileShape* shape, uint64_t tile_max = kTileMaxEntries)
     }
     p.tile_level = t0;
     uint64_t slots = 0, pairs = 0;
-    for (uint32_t l = 0; l <= t0; ++l) {
+    // level arrays: the global levels, the tiles' and those a launch of few
+    // tiles may be handed over at
+    for (uint32_t l = 0; l <= t0 || (l <= p.depth && l < 10); ++l) {
         slots = std::max<uint64_t>(slots, (1ull << l) * 2 * p.levels[l].pcap);
         pairs = std::max<uint64_t>(pairs, (1ull << l) * p.levels[l].pcap);
     }
@@ -677,9 +729,6 @@ void run_level(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p, cons
                 w.records, w.cursor, inv, ctl + kCtlClaimPlace);
         }, parts == 0 ? 2 : parts + 1);
     } else if (l == 0) {
-        if (input != nullptr) {
-            for (uint32_t k = 0; k < (uint32_t)input->ends.size(); ++k) input->wait(k);
-        }
         rec.launch(kKindInverse, [&] {
             launch_next(level_inverse<T>,
                 grid_for((lv.cap + kInverseItems - 1) / kInverseItems, kLevelThreads), kLevelThreads,
@@ -737,12 +786,13 @@ void run_level(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p, cons
     }
     rec.launch(kKindOutputBits, [&] {
         // the colours are all in xbits: the child level's edges or union-find
-        // words take the place of this level's; the tile builds its own
-        const bool global_child = l + 1 < p.tile_level;
+        // words take the place of this level's; tiles and stages build their own
+        const bool global_child = l + 1 < p.tile_level &&
+            (union_find_only || stage_stop(p, l + 1, p.tile_level) == 0);
         const bool child_walks = global_child && walk_level(p.levels[l + 1], tune, union_find_only);
-        launch_next(level_outputs, grid_for(prs / 2, kLevelThreads), kLevelThreads, 0, st, dp, l, inv,
+        launch_next(level_outputs, (prs / 2 + 32 + kLevelThreads - 1) / kLevelThreads, kLevelThreads, 0, st, dp, l, inv,
             w.xbits, w.ybits, child_inv, child_walks ? w.edge : nullptr, w.stamp,
-            global_child && !child_walks ? w.edge : nullptr, ctl + kCtlClaimOutputs);
+            global_child && !child_walks ? w.edge : nullptr);
     });
     // above the shard level every shard computes the level, shard 0 alone
     // writes its switches
@@ -802,11 +852,12 @@ void launch_levels(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p,
     const Plan* dp = w.d_plan;
     const uint32_t t0 = p.tile_level;
     const uint64_t blob_words = (p.end_offset + 3) / 4;
-    if (t0 == 0) {
-        // the tile reads the input directly: all of it first
-        for (uint32_t k = 0; input != nullptr && k < (uint32_t)input->ends.size(); ++k) {
-            input->wait(k);
-        }
+    // level 0 reads the input at once unless it is bucketed part by part
+    const bool by_parts = t0 > 0 && p.levels[0].cap > kWalkMaxNode && w.records != nullptr;
+    for (uint32_t k = 0; input != nullptr && !by_parts && k < (uint32_t)input->ends.size(); ++k) {
+        input->wait(k);
+    }
+    if (single_launch(p)) {
         rec.level = 0;
         rec.launch(kKindTile, [&] {
             auto one = std::make_unique<TileSingle>();
@@ -815,7 +866,7 @@ void launch_levels(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p,
             allow_smem((const void*)tile_encode_single<T>);
             const uint32_t plan_at = (shape.smem + 15) / 16 * 16;
             const bool near = plan_at + sizeof(Plan) <= kTileSmemBudget;
-            tile_encode_single<T><<<1, single_threads(p.n),
+            tile_encode_single<T><<<1, stage_threads(p.n),
                 near ? plan_at + sizeof(Plan) : shape.smem, st>>>(*one, d_in, d_blob,
                 (uint32_t)blob_words, status_out, shape.slots, near ? plan_at : 0u);
         });
@@ -826,50 +877,80 @@ void launch_levels(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p,
         auto first = std::make_unique<Prologue>();
         first->plan = p;
         first->header = header;
-        const uint64_t inv_words = p.levels[0].cap;
+        // (a stage from level 0 checks its input itself)
+        const bool scatter = t0 > 0 && (union_find_only || stage_stop(p, 0, t0) == 0);
+        const uint64_t inv_words = scatter ? p.levels[0].cap : 0;
         prologue<<<grid_for((blob_words + inv_words) / 8, 256), 256, 0, st>>>(*first, w.d_plan,
             w.d_status, d_blob, blob_words, w.control, t0 * kCtlWords, w.inv[0], inv_words,
             w.addr[0], w.addr[1]);
     });
-    for (uint32_t l = 0; l < t0; ++l) {
+    // inv[cur] holds the inverse of the level reached, from level 1 on
+    uint32_t cur = 0;
+    auto stage = [&](uint32_t l, uint32_t stop) {
         rec.level = (int)l;
-        uint32_t* inv = w.inv[l & 1];
-        uint32_t* child_inv = w.inv[(l + 1) & 1];
-        run_level<T>(w, rec, st, p, tune, l, d_in, d_blob, inv, child_inv, union_find_only, input);
-        if (after_level != nullptr) {
-            (*after_level)(l);
+        const TileShape part = tile_shape(p, l, stop);
+        const uint64_t nodes = 1ull << level_nodes(p, l).shift;
+        const unsigned threads = stage_threads(p.levels[l].cap);
+        rec.launch(kKindTile, [&] {
+            if (l == 0) {
+                allow_smem((const void*)tile_encode_wide<T>);
+                launch_next(tile_encode_wide<T>, nodes, threads, part.smem, st, dp, d_in, d_blob,
+                    w.d_status, part.slots, 0u, l, stop, w.inv[cur ^ 1]);
+            } else {
+                allow_smem((const void*)tile_encode_wide<uint32_t>);
+                launch_next(tile_encode_wide<uint32_t>, nodes, threads, part.smem, st, dp,
+                    w.inv[cur], d_blob, w.d_status, part.slots, 0u, l, stop, w.inv[cur ^ 1]);
+            }
+        });
+        cur ^= 1;
+    };
+    for (uint32_t l = 0; l < t0;) {
+        const uint32_t stop = union_find_only ? 0 : stage_stop(p, l, t0);
+        if (stop != 0) {
+            stage(l, stop);
+        } else {
+            rec.level = (int)l;
+            run_level<T>(w, rec, st, p, tune, l, d_in, d_blob, w.inv[cur], w.inv[cur ^ 1],
+                union_find_only, by_parts ? input : nullptr);
+            cur ^= 1;
+        }
+        const uint32_t next = stop != 0 ? stop : l + 1;
+        for (; l < next; ++l) {
+            if (after_level != nullptr) {
+                (*after_level)(l);
+            }
         }
     }
-    const uint32_t* tile_inv = w.inv[t0 & 1];
-    rec.level = (int)t0;
-    const uint64_t tiles = 1ull << level_nodes(p, t0).shift;
+    uint32_t last = t0;
+    TileShape last_shape = shape;
+    while (const uint32_t stop = few_tiles_stop(p, last)) {
+        stage(last, stop);
+        last = stop;
+        last_shape = tile_shape(p, last);
+    }
+    rec.level = (int)last;
+    const uint64_t tiles = 1ull << level_nodes(p, last).shift;
     if (tiles > 0x7fffffffull) {
         throw CudaFail{cudaErrorInvalidValue, "too many tiles"};
     }
-    const bool wide = shape.smem > kTileSmemTwoPerSm;
-    const unsigned threads = tile_threads(tiles, wide);
-    auto launch_tile = [&](auto kernel, const auto* src) {
-        allow_smem((const void*)kernel);
-        uint64_t lo = 0;
-        const size_t count = parts != nullptr ? parts->cuts.size() : 1;
-        for (size_t k = 0; k < count; ++k) {
-            const uint64_t hi = parts != nullptr ? parts->cuts[k] : tiles;
-            if (hi > lo) {
-                rec.launch(kKindTile, [&] {
-                    launch_next(kernel, hi - lo, threads, shape.smem, st, dp, src, d_blob,
-                        w.d_status, shape.slots, (uint32_t)lo);
-                });
-            }
-            if (parts != nullptr && parts->after_part) {
-                parts->after_part((uint32_t)k);
-            }
-            lo = hi;
+    const bool wide = last_shape.smem > kTileSmemTwoPerSm;
+    const unsigned threads = tile_threads(tiles, wide, p.levels[last].cap);
+    auto kernel = wide ? tile_encode_wide<uint32_t> : tile_encode<uint32_t>;
+    allow_smem((const void*)kernel);
+    uint64_t lo = 0;
+    const size_t count = parts != nullptr ? parts->cuts.size() : 1;
+    for (size_t k = 0; k < count; ++k) {
+        const uint64_t hi = parts != nullptr ? parts->cuts[k] : tiles;
+        if (hi > lo) {
+            rec.launch(kKindTile, [&] {
+                launch_next(kernel, hi - lo, threads, last_shape.smem, st, dp, w.inv[cur], d_blob,
+                    w.d_status, last_shape.slots, (uint32_t)lo, last, p.depth, nullptr);
+            });
         }
-    };
-    if (wide) {
-        launch_tile(tile_encode_wide<uint32_t>, tile_inv);
-    } else {
-        launch_tile(tile_encode<uint32_t>, tile_inv);
+        if (parts != nullptr && parts->after_part) {
+            parts->after_part((uint32_t)k);
+        }
+        lo = hi;
     }
     check(cudaMemcpyAsync(status_out, w.d_status, 4, cudaMemcpyDefault, st), "status");
     check(cudaGetLastError(), "tile kernel launch");

@@ -80,7 +80,6 @@ enum : int {
     kCtlClaimPlace = 1,   // level_place
     kCtlClaimUnion = 3,   // level_union
     kCtlClaimRoots = 4,   // level_roots
-    kCtlClaimOutputs = 5, // level_outputs
     kCtlWords = 8
 };
 
@@ -519,7 +518,7 @@ __device__ __forceinline__ void level_outputs_run(Grid grid, const Plan* __restr
     uint32_t level, const uint32_t* __restrict__ inv, const uint32_t* __restrict__ xbits,
     uint32_t* __restrict__ ybits, uint32_t* __restrict__ child_inv,
     uint32_t* __restrict__ child_edge, uint32_t* __restrict__ child_stamp,
-    uint32_t* __restrict__ child_uf, uint32_t* claims) {
+    uint32_t* __restrict__ child_uf) {
     const LevelInfo& lv = plan->levels[level];
     const LevelInfo& cl = plan->levels[level + 1];
     const uint32_t ps = (uint32_t)lv.pcap;
@@ -532,14 +531,12 @@ __device__ __forceinline__ void level_outputs_run(Grid grid, const Plan* __restr
     const uint64_t end = first + ((uint64_t)hs << nr.shift);
     const uint64_t begin = first & ~31ull;
     const uint32_t lane = threadIdx.x & 31;
-    uint64_t chunk = 0;
-    // claimed in address order (claim_chunk), 4 outputs a thread: the child
-    // nodes being scattered to at any time fit L2 (in grid-stride order the
-    // output pass took 407 ms per compress at 2^30 entries, claimed 100 ms;
-    // 4 and 16 quads a claim 111 and 152 ms)
-    while (claim_chunk(claims, blockDim.x, end - begin, &chunk)) {
-        const uint64_t g = begin + chunk + threadIdx.x;
-        if (g - lane >= end) continue;
+    // one quad a thread, blocks starting in address order, so the child nodes
+    // being scattered to at any time fit L2 (in grid-stride order the output
+    // pass took 407 ms per compress at 2^30 entries)
+    const uint64_t stride = (uint64_t)grid.nblk * blockDim.x;
+    for (uint64_t g = begin + (uint64_t)grid.bid * blockDim.x + threadIdx.x; g - lane < end;
+         g += stride) {
         uint32_t ys = 0;
         if (g >= first && g < end) {
             const uint32_t j = (uint32_t)g / hs;
@@ -601,10 +598,10 @@ __global__ void __launch_bounds__(256) level_outputs(const Plan* __restrict__ pl
     uint32_t level, const uint32_t* __restrict__ inv, const uint32_t* __restrict__ xbits,
     uint32_t* __restrict__ ybits, uint32_t* __restrict__ child_inv,
     uint32_t* __restrict__ child_edge, uint32_t* __restrict__ child_stamp,
-    uint32_t* __restrict__ child_uf, uint32_t* claims) {
+    uint32_t* __restrict__ child_uf) {
     wait_for_previous();
     level_outputs_run(launch_grid(), plan, level, inv, xbits, ybits, child_inv, child_edge,
-        child_stamp, child_uf, claims);
+        child_stamp, child_uf);
 }
 
 // Switch bits of one section at one level, packet-major: thread t maps to

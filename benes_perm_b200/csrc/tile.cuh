@@ -127,13 +127,18 @@ __device__ __forceinline__ Mask tile_colour_node(const uint32_t* edge, uint32_t 
     return x;
 }
 
+// Levels [T0, stop) of one node of level T0.  stop = the routing depth: the
+// whole subtree, down to the ranks.  An earlier stop leaves the inverses of
+// the nodes of level `stop` (all of them internal) in next_inv, laid out as
+// level_outputs does: a stage of the subtree, after which more CTAs go on.
 // kPlanNear: the plan is already in shared memory.
 template <typename T, bool kPlanNear = false>
 __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
     const T* __restrict__ src, uint32_t* __restrict__ blob, uint32_t* status, uint32_t slots,
-    uint32_t tile, unsigned char* smem) {
+    uint32_t tile, unsigned char* smem, uint32_t T0, uint32_t stop,
+    uint32_t* __restrict__ next_inv) {
     uint32_t off[5];
-    tile_smem_layout(slots, plan_ptr->depth - plan_ptr->tile_level, off);
+    tile_smem_layout(slots, stop - T0, off);
     uint16_t* invs[2] = {(uint16_t*)(smem + off[0]), (uint16_t*)(smem + off[1])};
     uint32_t* edge = (uint32_t*)(smem + off[2]);
     uint16_t* edge16 = (uint16_t*)edge;
@@ -147,7 +152,6 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
     const uint32_t lane = tid & 31;
     const uint32_t warp = tid >> 5;
     const uint32_t nwarps = blockDim.x >> 5;
-    const uint32_t T0 = plan.tile_level;
     const uint32_t D = plan.depth;
     const uint32_t leaf = plan.leaf;
     const uint32_t J = tile;
@@ -264,7 +268,7 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
         }
     }
 
-    for (uint32_t t = 0; T0 + t < D; ++t) {
+    for (uint32_t t = 0; T0 + t < stop; ++t) {
         const uint32_t level = T0 + t;
         const LevelInfo& lv = plan.levels[level];
         const uint32_t nodes = 1u << t;
@@ -445,6 +449,7 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
             {
                 const LevelInfo& cl = plan.levels[level + 1];
                 const uint32_t cstride = tile_node_slots(cl.pcap, level + 1 == D, leaf);
+                const bool hand_over = level + 1 == stop && stop < D;
                 const uint32_t hs = ps / 2;
                 const FastDiv by_hs(hs);
                 const uint32_t total = nodes * hs;
@@ -476,8 +481,12 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
                                 if (k0 >= cs) return;
                                 uint16_t* to = nxt + cpath * cstride;
                                 const bool two = k0 + 1 < cs;
-                                if (cs > leaf) {
-                                    const uint32_t w = two ? v[1] : cs; // virtual partner
+                                const uint32_t w = two ? v[1] : cs; // virtual partner
+                                if (hand_over) {
+                                    reinterpret_cast<uint2*>(next_inv)[
+                                        (uint64_t)(2 * first + cpath) * cl.pcap + (k0 >> 1)] =
+                                        make_uint2(v[0], w);
+                                } else if (cs > leaf) {
                                     *reinterpret_cast<uint32_t*>(to + k0) = v[0] | (w << 16);
                                     edge16[cpath * cstride + v[0]] = (uint16_t)w;
                                     edge16[cpath * cstride + w] = (uint16_t)v[0];
@@ -504,21 +513,29 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
     }
 
     // ---- switch bits and middle-group ranks out, all levels at once: a warp
-    // task is one section of up to 32 nodes of a level, or the ranks of up to
-    // 32 leaves.  Keeping every level's bits until here costs 1/32 of the
+    // task is one section of up to 32 nodes of a level (in large tiles one of
+    // several parts of that), or the ranks of up to 32 leaves.  Keeping every level's bits until here costs 1/32 of the
     // tile's memory per level; going out level by level, with two barriers
     // and a wave of node addresses each time, took a third of a small tile's
     // time.
-    const uint32_t levels = D - T0;
+    const uint32_t levels = stop - T0;
+    const bool leaves = stop == D;
     uint32_t tasks = 0;
-    for (uint32_t t = 0; t < levels; ++t) tasks += t < 5 ? 2u : 2u << (t - 5);
+    auto parts_of = [&](uint32_t t) { // 128 words of bits a part
+        const uint32_t parts = (slots >> 13) >> (t < 5 ? 0 : t - 5);
+        return parts > 1 ? parts : 1u;
+    };
+    auto tasks_of = [&](uint32_t t) { return (t < 5 ? 2u : 2u << (t - 5)) * parts_of(t); };
+    for (uint32_t t = 0; t < levels; ++t) tasks += tasks_of(t);
     const uint32_t leaf_tasks = levels < 5 ? 1u : 1u << (levels - 5);
     const bool mixed = levels > 0 && plan.levels[D - 1].q <= leaf; // leaves at level D - 1 too
-    tasks += leaf_tasks + (mixed ? (levels < 6 ? 1u : 1u << (levels - 6)) : 0u);
+    if (leaves) {
+        tasks += leaf_tasks + (mixed ? (levels < 6 ? 1u : 1u << (levels - 6)) : 0u);
+    }
     for (uint32_t task = warp; task < tasks; task += nwarps) {
         uint32_t t = 0, at = task;
         for (; t < levels; ++t) {
-            const uint32_t here = t < 5 ? 2u : 2u << (t - 5);
+            const uint32_t here = tasks_of(t);
             if (at < here) break;
             at -= here;
         }
@@ -561,6 +578,9 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
             }
             continue;
         }
+        const uint32_t parts = parts_of(t);
+        const uint32_t part = at % parts;
+        at /= parts;
         const int side = (int)(at & 1);
         const uint32_t w0 = (at >> 1) << 5;
         const uint32_t ps = tile_pair_stride(lv.pcap);
@@ -610,7 +630,7 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
             const uint32_t cshift = span_log2 - 5;
             const uint32_t cs = wave_log2 + cshift;
             const uint32_t chunks = packets << cs;
-            for (uint32_t base = 0; base < chunks; base += 32) {
+            for (uint32_t base = part * 32; base < chunks; base += parts * 32) {
                 const uint32_t c = base + lane;
                 const uint32_t packet = c >> cs;
                 const uint32_t rem = c & ((1u << cs) - 1);
@@ -647,7 +667,7 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
             const uint32_t span_mask = (1u << (1u << span_log2)) - 1u;
             const uint32_t groups_log2 = wave_log2 - g_log2;
             const uint32_t work = full << groups_log2;
-            for (uint32_t base = 0; base < work; base += 32) {
+            for (uint32_t base = part * 32; base < work; base += parts * 32) {
                 const uint32_t c = base + lane;
                 const uint32_t packet = c >> groups_log2;
                 const uint32_t slot0 = (c & ((1u << groups_log2) - 1)) << g_log2;
@@ -667,7 +687,7 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
         }
         const uint32_t shift = wave_log2 + span_log2;
         const uint32_t rest = (packets - full) << shift;
-        for (uint32_t base = 0; base < rest; base += 32) {
+        for (uint32_t base = part * 32; base < rest; base += parts * 32) {
             const uint32_t c = base + lane;
             const uint32_t packet = full + (c >> shift);
             const uint32_t rem = c & ((1u << shift) - 1);
@@ -689,13 +709,13 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
 template <typename T>
 __global__ void __launch_bounds__(kTileThreads, 2) tile_encode(const Plan* __restrict__ plan,
     const T* __restrict__ src, uint32_t* __restrict__ blob, uint32_t* status, uint32_t slots,
-    uint32_t part_first) {
+    uint32_t part_first, uint32_t level, uint32_t stop, uint32_t* __restrict__ next_inv) {
     extern __shared__ __align__(16) unsigned char smem[];
     wait_for_previous();
-    // a sharded call encodes only its own tiles (level_nodes); a launch may
-    // cover a part of them, from tile part_first on
-    const uint32_t first = (uint32_t)level_nodes(*plan, plan->tile_level).lo + part_first;
-    tile_body<T>(plan, src, blob, status, slots, first + blockIdx.x, smem);
+    // a sharded call encodes only its own nodes (level_nodes); a launch may
+    // cover a part of them, from part_first on
+    const uint32_t first = (uint32_t)level_nodes(*plan, level).lo + part_first;
+    tile_body<T>(plan, src, blob, status, slots, first + blockIdx.x, smem, level, stop, next_inv);
 }
 
 // Tiles too large for two CTAs per SM (nodes of 16384 entries, up to about
@@ -704,11 +724,12 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_encode(const Plan* __res
 template <typename T>
 __global__ void __launch_bounds__(2 * kTileThreads, 1) tile_encode_wide(
     const Plan* __restrict__ plan, const T* __restrict__ src, uint32_t* __restrict__ blob,
-    uint32_t* status, uint32_t slots, uint32_t part_first) {
+    uint32_t* status, uint32_t slots, uint32_t part_first, uint32_t level, uint32_t stop,
+    uint32_t* __restrict__ next_inv) {
     extern __shared__ __align__(16) unsigned char smem[];
     wait_for_previous();
-    const uint32_t first = (uint32_t)level_nodes(*plan, plan->tile_level).lo + part_first;
-    tile_body<T>(plan, src, blob, status, slots, first + blockIdx.x, smem);
+    const uint32_t first = (uint32_t)level_nodes(*plan, level).lo + part_first;
+    tile_body<T>(plan, src, blob, status, slots, first + blockIdx.x, smem, level, stop, next_inv);
 }
 
 struct Header {
@@ -756,7 +777,7 @@ __global__ void __launch_bounds__(2 * kTileThreads, 1) tile_encode_single(
     }
     if (threadIdx.x == 0) status = 0;
     __syncthreads();
-    tile_body<T, true>(plan, src, blob, &status, slots, 0, smem);
+    tile_body<T, true>(plan, src, blob, &status, slots, 0, smem, 0, plan->depth, nullptr);
     __syncthreads();
     if (threadIdx.x == 0) *(volatile uint32_t*)status_out = status;
 }
@@ -772,8 +793,10 @@ struct TileJob {
     const void* src;
     uint32_t* blob;
     uint32_t* status;
+    uint32_t* next_inv;    // a stage's output (tile_body), null for whole subtrees
     uint32_t slots;
-    uint32_t pad_;
+    uint32_t level;
+    uint32_t stop;
     uint32_t first_block;
     uint32_t tiles;
     uint32_t blob_words;   // words to clear (single-tile jobs)
@@ -782,9 +805,8 @@ struct TileJob {
 };
 
 template <typename T>
-__global__ void __launch_bounds__(kTileThreads, 2) tile_encode_batch(
-    const TileJob* __restrict__ jobs, uint32_t njobs) {
-    extern __shared__ __align__(16) unsigned char smem[];
+__device__ __forceinline__ void tile_batch_body(const TileJob* __restrict__ jobs, uint32_t njobs,
+    unsigned char* smem) {
     uint32_t lo = 0, hi = njobs;
     while (hi - lo > 1) { // last job whose first block is <= blockIdx.x
         const uint32_t mid = (lo + hi) / 2;
@@ -800,7 +822,22 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_encode_batch(
         __syncthreads();
     }
     tile_body<T>(job.plan, (const T*)job.src, job.blob, job.status, job.slots,
-        blockIdx.x - job.first_block, smem);
+        blockIdx.x - job.first_block, smem, job.level, job.stop, job.next_inv);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kTileThreads, 2) tile_encode_batch(
+    const TileJob* __restrict__ jobs, uint32_t njobs) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    tile_batch_body<T>(jobs, njobs, smem);
+}
+
+// Stages of many permutations: one large node per SM.
+template <typename T>
+__global__ void __launch_bounds__(2 * kTileThreads, 1) tile_encode_batch_wide(
+    const TileJob* __restrict__ jobs, uint32_t njobs) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    tile_batch_body<T>(jobs, njobs, smem);
 }
 
 } // namespace bpb200

@@ -387,24 +387,37 @@ __device__ __forceinline__ void list_rank_run(Grid grid, const Plan* __restrict_
         uint32_t* smin = key + count;      // 2 * rulers
         uint32_t* snext = smin + 2 * rulers;
         __syncthreads(); // the previous node's arrays are free
-        for (uint32_t i = tid; i < count; i += blockDim.x) {
-            const uint32_t q = pair_of(range.lo + i, e);
-            const bool mine = q >= pair_lo && q < pair_lo + ps;
-            const uint4 st = mine ? state[range.lo + i] : make_uint4(kNone, 0, 0, 0);
-            uint32_t word = 0x8000u; // not here: nothing leads to it
-            uint32_t k = ~0u;
-            if (st.x != kNone) {
-                uint32_t a = st.x - 2 * range.lo, b = st.z - 2 * range.lo;
-                if (a >= 2 * count || b >= 2 * count) {
-                    bad = true;
-                    a = 2 * i;
-                    b = 2 * i + 1;
+        constexpr uint32_t kBatch = 8; // states in flight per thread
+        for (uint32_t i0 = tid; i0 < count; i0 += kBatch * blockDim.x) {
+            uint4 st[kBatch];
+#pragma unroll
+            for (uint32_t b = 0; b < kBatch; ++b) {
+                const uint32_t i = i0 + b * blockDim.x;
+                st[b] = make_uint4(kNone, 0u, 0u, 0u);
+                if (i < count) {
+                    const uint32_t q = pair_of(range.lo + i, e);
+                    if (q >= pair_lo && q < pair_lo + ps) st[b] = state[range.lo + i];
                 }
-                word = b | (a << 16);
-                k = around(st);
             }
-            key[i] = k;
-            link[i] = word;
+#pragma unroll
+            for (uint32_t b = 0; b < kBatch; ++b) {
+                const uint32_t i = i0 + b * blockDim.x;
+                if (i >= count) break;
+                uint32_t word = 0x8000u; // not here: nothing leads to it
+                uint32_t k = ~0u;
+                if (st[b].x != kNone) {
+                    uint32_t x = st[b].x - 2 * range.lo, z = st[b].z - 2 * range.lo;
+                    if (x >= 2 * count || z >= 2 * count) {
+                        bad = true;
+                        x = 2 * i;
+                        z = 2 * i + 1;
+                    }
+                    word = z | (x << 16);
+                    k = around(st[b]);
+                }
+                key[i] = k;
+                link[i] = word;
+            }
         }
         __syncthreads();
         // rulers first: their word moves to the state, a stamp takes its place

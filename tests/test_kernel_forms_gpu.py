@@ -71,3 +71,44 @@ def test_lookup_words(gpu, oracle, n, m, placement, shift):
         gpu.lookup_device(room.data_ptr() + shift, len(blob), n, b200_format(gpu, kw),
                           out.data_ptr(), n, inverse=inverse)
         assert torch.equal(out.cpu(), torch.argsort(want) if inverse else want)
+
+
+@pytest.mark.parametrize("n", [4097, 8193, 16383, 16385, 24577, 32767, 32768, 32769, 65535, 65537,
+                               131073])
+@pytest.mark.parametrize("m", [1, 4, 5])
+def test_stages(gpu, oracle, n, m):
+    """Nodes around the stage limit (2^15 entries) and launches of few tiles,
+    which hand their subtrees over to more CTAs; the batched form runs the
+    same stages from job lists."""
+    import torch
+    kinds = gpu.PermutationKind
+    items, keep = [], []
+    for i, kind in enumerate((kinds.uniform, kinds.single_cycle, kinds.reverse)):
+        kw = dict(middle_group_log2=m, middle_placement=i)
+        dtype = np.uint64 if i == 1 else np.uint32
+        check(gpu, oracle, n, n + i, kind, dtype, **kw)
+        perm = gpu.fill_permutation(kind, n + i, n, dtype)
+        want = oracle.compress(perm, oracle_format(kw))
+        src = torch.from_numpy(perm.view(np.int64 if i == 1 else np.int32)).cuda()
+        blob = torch.zeros((len(want) + 3) // 4 * 4, dtype=torch.uint8, device="cuda")
+        keep.append((src, blob, want))
+        items.append((src.data_ptr(), n, perm.dtype.itemsize, b200_format(gpu, kw),
+                      blob.data_ptr(), len(want)))
+    torch.cuda.synchronize()
+    gpu.compress_batch_device(items)
+    for _, blob, want in keep:
+        assert blob.cpu().numpy()[:len(want)].tobytes() == want
+
+
+def test_stage_rejects_repeats(gpu):
+    """A stage reads the caller's values itself: out of range and repeated
+    values are reported, and the next call is right again."""
+    for n in (12289, 30000):
+        perm = gpu.fill_permutation(gpu.PermutationKind.uniform, n, n, np.uint32)
+        good = gpu.compress(perm)
+        for bad in (n, int(perm[1])):
+            wrong = perm.copy()
+            wrong[0] = bad
+            with pytest.raises(ValueError):
+                gpu.compress(wrong)
+            assert gpu.compress(perm) == good
