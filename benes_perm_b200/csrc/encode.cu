@@ -860,7 +860,7 @@ void launch_levels(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p,
     if (single_launch(p)) {
         rec.level = 0;
         rec.launch(kKindTile, [&] {
-            auto one = std::make_unique<TileSingle>();
+            const std::unique_ptr<TileSingle> one(new TileSingle); // not cleared: set at once
             one->plan = p;
             one->header = header;
             allow_smem((const void*)tile_encode_single<T>);
@@ -874,7 +874,7 @@ void launch_levels(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p,
         return;
     }
     rec.launch(kKindPrologue, [&] {
-        auto first = std::make_unique<Prologue>();
+        const std::unique_ptr<Prologue> first(new Prologue); // not cleared: set at once
         first->plan = p;
         first->header = header;
         // (a stage from level 0 checks its input itself)

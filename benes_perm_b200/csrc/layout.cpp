@@ -1,9 +1,8 @@
 // SPDX-License-Identifier: Apache-2.0
 #include "layout.hpp"
 
+#include <algorithm>
 #include <cstring>
-#include <map>
-#include <utility>
 
 namespace bpb200 {
 namespace {
@@ -35,49 +34,111 @@ uint32_t factoradic_bits(uint32_t c) {
     return bits;
 }
 
-// Memoised subtree sizes (FormatSizeCache, src/internal.hpp:225-313).
+const uint32_t* factoradic_table() {
+    static const struct Table {
+        uint32_t bits[33];
+        Table() {
+            for (uint32_t c = 0; c <= 32; ++c) bits[c] = factoradic_bits(c);
+        }
+    } table;
+    return table.bits;
+}
+
+struct DigitTables {
+    uint32_t reciprocal[33] = {};
+    DigitGroup groups[33] = {};
+};
+
+const DigitTables& digit_tables() {
+    static const DigitTables tables = [] {
+        DigitTables t;
+        for (uint32_t i = 1; i <= 32; ++i) {
+            t.reciprocal[i] = i > 1 ? 0xffffffffu / i + 1u : 0u;
+            uint32_t product = i, digits = 1;
+            while (digits < i && (uint64_t)product * (i - digits) < (1u << 27)) {
+                product *= i - digits;
+                ++digits;
+            }
+            t.groups[i] = {~0ull / product, product, digits};
+        }
+        return t;
+    }();
+    return tables;
+}
+
+// Switches and middle bits of the subtrees of every level's two node sizes,
+// q_l = floor(n / 2^l) and q_l + 1 (FormatSizeCache, src/internal.hpp:225-313,
+// memoises the same recursion).  Both halves of either size are one of the
+// next level's two, so the tables fill from the leaves up in a few steps per
+// level.  Level 0's second size belongs to no node and may wrap around.
 class Sizes {
 public:
-    explicit Sizes(uint32_t leaf) : leaf_(leaf) {}
-
-    std::pair<uint64_t, uint64_t> subtree(uint64_t c) {
-        if (c <= leaf_) {
-            return {0, factoradic_bits((uint32_t)c)};
+    Sizes(uint64_t n, uint32_t leaf, uint32_t depth) : n_(n), leaf_(leaf) {
+        for (uint32_t l = depth + 2; l-- > 0;) {
+            for (uint32_t big = 0; big < 2; ++big) {
+                const uint64_t c = small(l) + big;
+                if (c <= leaf_) {
+                    switches_[l][big] = 0;
+                    middle_[l][big] = factoradic_table()[c];
+                    continue;
+                }
+                const uint32_t lo = (uint32_t)(c / 2 - small(l + 1));
+                const uint32_t hi = (uint32_t)(c - c / 2 - small(l + 1));
+                if (l == 0 && big == 1) {
+                    switches_[l][big] = c / 2 + switches_[l + 1][hi] + switches_[l + 1][lo];
+                    middle_[l][big] = middle_[l + 1][hi] + middle_[l + 1][lo];
+                } else {
+                    switches_[l][big] = add(c / 2, add(switches_[l + 1][hi], switches_[l + 1][lo]));
+                    middle_[l][big] = add(middle_[l + 1][hi], middle_[l + 1][lo]);
+                }
+            }
         }
-        auto it = subtree_.find(c);
-        if (it != subtree_.end()) {
-            return it->second;
-        }
-        const auto l = subtree(c - c / 2);
-        const auto r = subtree(c / 2);
-        const std::pair<uint64_t, uint64_t> v{
-            add(c / 2, add(l.first, r.first)), add(l.second, r.second)};
-        subtree_.emplace(c, v);
-        return v;
     }
-    uint64_t switches(uint64_t c) { return subtree(c).first; }
-    uint64_t middle(uint64_t c) { return subtree(c).second; }
 
-    uint64_t top_switches(uint64_t c, uint32_t depth) {
-        if (c <= leaf_ || depth == 0) {
-            return 0;
+    uint64_t switches(uint32_t level, uint32_t big) const { return switches_[level][big]; }
+    uint64_t middle(uint32_t level, uint32_t big) const { return middle_[level][big]; }
+
+    // Switches of the first `depth` levels of the subtrees of the two sizes
+    // of level `start`.
+    void top_switches(uint32_t start, uint32_t depth, uint64_t (&out)[2]) const {
+        uint64_t below[2] = {0, 0};
+        for (uint32_t l = start + depth; l-- > start;) {
+            uint64_t here[2];
+            for (uint32_t big = 0; big < 2; ++big) {
+                const uint64_t c = small(l) + big;
+                here[big] = c <= leaf_ ? 0
+                    : c / 2 + below[c - c / 2 - small(l + 1)] + below[c / 2 - small(l + 1)];
+            }
+            below[0] = here[0];
+            below[1] = here[1];
         }
-        const auto key = std::make_pair(c, depth);
-        auto it = top_.find(key);
-        if (it != top_.end()) {
-            return it->second;
-        }
-        const uint64_t v = add(c / 2,
-            add(top_switches(c - c / 2, depth - 1), top_switches(c / 2, depth - 1)));
-        top_.emplace(key, v);
-        return v;
+        out[0] = below[0];
+        out[1] = below[1];
     }
 
 private:
+    uint64_t small(uint32_t l) const { return l < 64 ? n_ >> l : 0; }
+
+    uint64_t n_;
     uint32_t leaf_;
-    std::map<uint64_t, std::pair<uint64_t, uint64_t>> subtree_;
-    std::map<std::pair<uint64_t, uint32_t>, uint64_t> top_;
+    uint64_t switches_[66][2];
+    uint64_t middle_[66][2];
 };
+
+// packet_path_bits over all 2^rel nodes of a level of a cluster: of those
+// exactly root mod 2^rel are large.
+uint64_t packet_level_bits(uint64_t root, uint32_t depth, uint32_t rel, uint64_t packet,
+    uint32_t leaf) {
+    const uint64_t small = root >> rel;
+    const uint64_t nodes = 1ull << rel;
+    const uint64_t large = root & (nodes - 1);
+    const uint64_t span = 1ull << (depth - rel - 1);
+    const uint64_t first = packet * span;
+    auto share = [&](uint64_t count) {
+        return count <= leaf || first >= count / 2 ? 0 : std::min(count / 2 - first, span);
+    };
+    return large * share(small + 1) + (nodes - large) * share(small);
+}
 
 uint32_t routing_depth(uint64_t count, uint32_t leaf) {
     uint32_t d = 0;
@@ -140,13 +201,13 @@ void layout_or_throw(uint64_t count, const Format& in, Layout* out) {
     if (depth == 0) {
         f.middle_placement = 0;
     }
-    Sizes sizes(leaf);
+    const Sizes sizes(count, leaf, depth);
     Layout L;
     L.format = f;
     L.size = count;
     L.depth = depth;
-    L.switch_bits = sizes.switches(count);
-    L.middle_bits = sizes.middle(count);
+    L.switch_bits = sizes.switches(0, 0);
+    L.middle_bits = sizes.middle(0, 0);
     L.header_bytes = add(20, (uint64_t)f.input_cluster_count + f.output_cluster_count);
     const uint64_t in_bytes = add(bytes_of(L.switch_bits),
         f.middle_placement == 1 ? bytes_of(L.middle_bits) : 0);
@@ -203,7 +264,7 @@ Error make_plan(const Layout& L, uint64_t tile_max, Plan* out) {
         if (L.depth > kMaxLevels - 1) {
             throw Fail{kLength, "permutation is too large for the B200 backend"};
         }
-        Sizes sizes(leaf);
+        const Sizes sizes(n, leaf, L.depth);
         p.n = n;
         p.leaf = leaf;
         p.depth = L.depth;
@@ -222,11 +283,11 @@ Error make_plan(const Layout& L, uint64_t tile_max, Plan* out) {
             lv.cap = lv.q + (lv.r != 0 ? 1 : 0);
             lv.pcap = ((lv.cap + 1) / 2 + 1) & ~1ull;
             for (int big = 0; big < 2; ++big) {
-                const uint64_t c = lv.q + (uint64_t)big;
-                lv.middle[big] = sizes.middle(c);
+                lv.middle[big] = sizes.middle(l, big);
                 for (int side = 0; side < 2; ++side) {
                     const bool embeds = L.format.middle_placement == (uint8_t)(side + 1);
-                    lv.section[side][big] = sizes.switches(c) + (embeds ? sizes.middle(c) : 0);
+                    lv.section[side][big] =
+                        sizes.switches(l, big) + (embeds ? lv.middle[big] : 0);
                 }
             }
         }
@@ -240,12 +301,12 @@ Error make_plan(const Layout& L, uint64_t tile_max, Plan* out) {
                 GroupInfo& gi = p.groups[side][g];
                 gi.start = start;
                 gi.depth = cl[g];
+                sizes.top_switches(start, gi.depth, gi.group_bits);
                 for (int big = 0; big < 2; ++big) {
                     const uint64_t root = p.levels[start].q + (uint64_t)big;
-                    gi.group_bits[big] = sizes.top_switches(root, gi.depth);
                     uint64_t bits = 0;
                     for (uint32_t l = 0; l < gi.depth; ++l) {
-                        bits += packet_path_bits(root, gi.depth, l, 0, 1ull << l, leaf);
+                        bits += packet_level_bits(root, gi.depth, l, 0, leaf);
                     }
                     gi.packet_bits[big] = bits;
                 }
@@ -267,7 +328,7 @@ Error make_plan(const Layout& L, uint64_t tile_max, Plan* out) {
                     const uint64_t root = p.levels[gi.start].q + (uint64_t)rb;
                     uint64_t f0 = 0;
                     for (uint32_t up = 0; up < ls.rel; ++up) {
-                        f0 += packet_path_bits(root, gi.depth, up, 0, 1ull << up, leaf);
+                        f0 += packet_level_bits(root, gi.depth, up, 0, leaf);
                     }
                     ls.prefix0[rb] = f0;
                     for (int nb = 0; nb < 2; ++nb) {
@@ -275,7 +336,7 @@ Error make_plan(const Layout& L, uint64_t tile_max, Plan* out) {
                         const uint64_t tail = pairs == 0 ? 0 : (pairs - 1) >> (gi.depth - ls.rel - 1);
                         uint64_t ft = 0;
                         for (uint32_t up = 0; up < ls.rel; ++up) {
-                            ft += packet_path_bits(root, gi.depth, up, tail, 1ull << up, leaf);
+                            ft += packet_level_bits(root, gi.depth, up, tail, leaf);
                         }
                         ls.prefix_tail[rb][nb] = ft;
                     }
@@ -298,17 +359,10 @@ Error make_plan(const Layout& L, uint64_t tile_max, Plan* out) {
         p.max_slots = slots;
         p.max_pairs = pairs;
         for (uint32_t c = 0; c <= 32; ++c) {
-            p.fact_bits[c] = factoradic_bits(c);
+            p.fact_bits[c] = factoradic_table()[c];
         }
-        for (uint32_t i = 1; i <= 32; ++i) {
-            p.digit_reciprocal[i] = i > 1 ? 0xffffffffu / i + 1u : 0u;
-            uint32_t product = i, digits = 1;
-            while (digits < i && (uint64_t)product * (i - digits) < (1u << 27)) {
-                product *= i - digits;
-                ++digits;
-            }
-            p.digit_groups[i] = {~0ull / product, product, digits};
-        }
+        std::memcpy(p.digit_reciprocal, digit_tables().reciprocal, sizeof p.digit_reciprocal);
+        std::memcpy(p.digit_groups, digit_tables().groups, sizeof p.digit_groups);
         return {};
     } catch (const Fail& f) {
         return {f.code, f.message};
