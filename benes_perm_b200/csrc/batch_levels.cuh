@@ -118,6 +118,7 @@ __device__ __forceinline__ const LevelJob* level_job(const LevelJob* jobs, uint3
 }
 
 __global__ void __launch_bounds__(256) batch_fill(const FillJob* jobs, uint32_t n) {
+    wait_for_previous();
     Grid g;
     const FillJob* j = batch_job(jobs, n, [](const FillJob& x) { return x.first; }, &g);
     g.bid = blockIdx.x - j->first;
@@ -132,6 +133,7 @@ __global__ void __launch_bounds__(256) batch_fill(const FillJob* jobs, uint32_t 
 // Status word, blob header (after the blob was cleared by batch_fill) and
 // switch addresses of every level.
 __global__ void __launch_bounds__(256) batch_init(const LevelJob* jobs, uint32_t n) {
+    wait_for_previous();
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBInit, &g);
     if (g.bid >= g.nblk) return;
@@ -144,6 +146,7 @@ __global__ void __launch_bounds__(256) batch_init(const LevelJob* jobs, uint32_t
 }
 
 __global__ void __launch_bounds__(256) batch_inverse(const LevelJob* jobs, uint32_t n) {
+    wait_for_previous();
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBInverse, &g);
     if (g.bid >= g.nblk) return;
@@ -157,6 +160,7 @@ __global__ void __launch_bounds__(256) batch_inverse(const LevelJob* jobs, uint3
 }
 
 __global__ void __launch_bounds__(256) batch_edges(const LevelJob* jobs, uint32_t n) {
+    wait_for_previous();
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBEdges, &g);
     if (g.bid >= g.nblk) return;
@@ -164,6 +168,7 @@ __global__ void __launch_bounds__(256) batch_edges(const LevelJob* jobs, uint32_
 }
 
 __global__ void __launch_bounds__(256) batch_walk(const LevelJob* jobs, uint32_t n) {
+    wait_for_previous();
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBWalk, &g);
     if (g.bid >= g.nblk) return;
@@ -171,6 +176,7 @@ __global__ void __launch_bounds__(256) batch_walk(const LevelJob* jobs, uint32_t
 }
 
 __global__ void __launch_bounds__(256) batch_contract(const LevelJob* jobs, uint32_t n, uint32_t e) {
+    wait_for_previous();
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBContract + (int)e - 1, &g);
     if (g.bid >= g.nblk) return;
@@ -180,6 +186,7 @@ __global__ void __launch_bounds__(256) batch_contract(const LevelJob* jobs, uint
 
 __global__ void __launch_bounds__(kRankThreads, 1) batch_rank(const LevelJob* jobs, uint32_t n) {
     extern __shared__ __align__(16) uint32_t rank_shared[];
+    wait_for_previous();
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBRank, &g);
     if (g.bid >= g.nblk) return;
@@ -188,6 +195,7 @@ __global__ void __launch_bounds__(kRankThreads, 1) batch_rank(const LevelJob* jo
 }
 
 __global__ void __launch_bounds__(256) batch_expand(const LevelJob* jobs, uint32_t n, uint32_t e) {
+    wait_for_previous();
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBExpand + (int)e - 1, &g);
     if (g.bid >= g.nblk) return;
@@ -196,6 +204,7 @@ __global__ void __launch_bounds__(256) batch_expand(const LevelJob* jobs, uint32
 }
 
 __global__ void __launch_bounds__(256) batch_colours(const LevelJob* jobs, uint32_t n) {
+    wait_for_previous();
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBColours, &g);
     if (g.bid >= g.nblk) return;
@@ -204,6 +213,7 @@ __global__ void __launch_bounds__(256) batch_colours(const LevelJob* jobs, uint3
 
 __global__ void __launch_bounds__(256, BPB200_UNION_MIN_BLOCKS) batch_union(const LevelJob* jobs,
     uint32_t n) {
+    wait_for_previous();
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBUnion, &g);
     if (g.bid >= g.nblk) return;
@@ -211,6 +221,7 @@ __global__ void __launch_bounds__(256, BPB200_UNION_MIN_BLOCKS) batch_union(cons
 }
 
 __global__ void __launch_bounds__(256) batch_orient(const LevelJob* jobs, uint32_t n) {
+    wait_for_previous();
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBOrient, &g);
     if (g.bid >= g.nblk) return;
@@ -218,6 +229,7 @@ __global__ void __launch_bounds__(256) batch_orient(const LevelJob* jobs, uint32
 }
 
 __global__ void __launch_bounds__(256, 4) batch_roots(const LevelJob* jobs, uint32_t n) {
+    wait_for_previous();
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBRoots, &g);
     if (g.bid >= g.nblk) return;
@@ -225,6 +237,7 @@ __global__ void __launch_bounds__(256, 4) batch_roots(const LevelJob* jobs, uint
 }
 
 __global__ void __launch_bounds__(256) batch_outputs(const LevelJob* jobs, uint32_t n) {
+    wait_for_previous();
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBOutputs, &g);
     if (g.bid >= g.nblk) return;
@@ -235,6 +248,7 @@ __global__ void __launch_bounds__(256) batch_outputs(const LevelJob* jobs, uint3
 // Switch emission: every (permutation, section, form) of the level in one
 // launch.
 __global__ void __launch_bounds__(256) batch_emit(const EmitJob* jobs, uint32_t n) {
+    wait_for_previous();
     Grid g;
     const EmitJob* j = batch_job(jobs, n, [](const EmitJob& x) { return x.first; }, &g);
     g.bid = blockIdx.x - j->first;

@@ -829,6 +829,7 @@ template <typename T>
 __global__ void __launch_bounds__(kTileThreads, 2) tile_encode_batch(
     const TileJob* __restrict__ jobs, uint32_t njobs) {
     extern __shared__ __align__(16) unsigned char smem[];
+    wait_for_previous();
     tile_batch_body<T>(jobs, njobs, smem);
 }
 
@@ -837,6 +838,7 @@ template <typename T>
 __global__ void __launch_bounds__(2 * kTileThreads, 1) tile_encode_batch_wide(
     const TileJob* __restrict__ jobs, uint32_t njobs) {
     extern __shared__ __align__(16) unsigned char smem[];
+    wait_for_previous();
     tile_batch_body<T>(jobs, njobs, smem);
 }
 
