@@ -166,6 +166,45 @@ BP_HD uint32_t leaf_apply(const Plan& p, uint32_t (&rank)[4], uint32_t size,
     return 0; // unreachable for index < size
 }
 
+// What a path needs of one level and section, gathered from the plan: the
+// device kernel keeps the table of its call in shared memory.
+struct PathLevel {
+    uint64_t prefix0[2];        // by cluster root size
+    uint64_t prefix_tail[2][2]; // by root and node size
+    uint64_t packet_bits[2];
+    uint32_t q, r;              // node sizes of the level (low words; see path_node_size)
+    uint32_t group;
+    uint32_t start;             // first level of the group
+    uint32_t rel;
+    uint32_t span_log2;
+};
+
+BP_HD PathLevel path_level(const Plan& p, int side, uint32_t level) {
+    const LevelInfo& lv = p.levels[level];
+    const LevelSide& ls = lv.side[side];
+    const GroupInfo& gi = p.groups[side][ls.group];
+    PathLevel t;
+    for (int rs = 0; rs < 2; ++rs) {
+        t.prefix0[rs] = ls.prefix0[rs];
+        t.prefix_tail[rs][0] = ls.prefix_tail[rs][0];
+        t.prefix_tail[rs][1] = ls.prefix_tail[rs][1];
+        t.packet_bits[rs] = gi.packet_bits[rs];
+    }
+    t.q = (uint32_t)lv.q;
+    t.r = (uint32_t)lv.r;
+    t.group = ls.group;
+    t.start = gi.start;
+    t.rel = ls.rel;
+    t.span_log2 = gi.depth - ls.rel - 1; // unused past the last routing level
+    return t;
+}
+
+// The plan itself as the source of path levels (host probe).
+struct PlanLevels {
+    const Plan* plan;
+    BP_HD PathLevel at(int side, uint32_t level) const { return path_level(*plan, side, level); }
+};
+
 // Switch addresses along one query's path through one section.  All nodes of
 // the path inside one cluster group share the cluster root, so its base is
 // worked out once per group; below it only the packet that holds the wanted
@@ -173,61 +212,63 @@ BP_HD uint32_t leaf_apply(const Plan& p, uint32_t (&rank)[4], uint32_t size,
 struct PathAddress {
     uint64_t base = 0;  // blob bit of the cluster's packets
     uint64_t root_count = 0;
-    uint64_t packet_bits = 0;
     uint32_t group = ~0u;
-    uint32_t rs = 0;
+    uint32_t rs = 0;    // 1: the cluster root is a large node
 
     template <typename Int>
-    BP_HD uint64_t bit(const Plan& p, int side, uint32_t level, Int node, Int size, Int pair) {
-        const LevelSide& ls = p.levels[level].side[side];
-        const GroupInfo& gi = p.groups[side][ls.group];
-        const uint32_t rel = ls.rel;
-        if (ls.group != group) {
-            group = ls.group;
+    BP_HD uint64_t bit(const Plan& p, const PathLevel& t, int side, uint32_t level, Int node,
+        Int size, Int pair) {
+        if (t.group != group) {
+            group = t.group;
             base = p.section_offset[side] * 8 + cluster_base(p, side, group, level, node);
-            rs = node_is_large(p.levels[gi.start], gi.start, node >> rel) ? 1u : 0u;
-            root_count = p.levels[gi.start].q + rs;
-            packet_bits = gi.packet_bits[rs];
+            rs = node_is_large(p.levels[t.start], t.start, node >> t.rel) ? 1u : 0u;
+            root_count = p.levels[t.start].q + rs;
         }
-        const Int path = node & (((Int)1 << rel) - 1);
-        const uint32_t span_log2 = gi.depth - rel - 1;
-        const Int packet = pair >> span_log2;
-        const uint64_t at = base + packet * packet_bits + (pair & (((Int)1 << span_log2) - 1));
-        if (packet == (size / 2 - 1) >> span_log2) {
-            return at + ls.prefix_tail[rs][size != (Int)p.levels[level].q ? 1 : 0] +
-                packet_path_bits(root_count, gi.depth, rel, packet, path, p.leaf);
+        const Int path = node & (((Int)1 << t.rel) - 1);
+        const Int span = (Int)1 << t.span_log2;
+        const Int packet = pair >> t.span_log2;
+        const uint64_t at = base + (uint64_t)packet * t.packet_bits[rs] + (pair & (span - 1));
+        const bool tail = packet == (size / 2 - 1) >> t.span_log2;
+        // packet_path_bits in Int arithmetic: switches of the nodes left of
+        // this one in the packet, by the two node sizes of the level
+        const Int small = (Int)(root_count >> t.rel);
+        const Int large = (Int)root_count & (((Int)1 << t.rel) - 1);
+        const Int first = tail ? packet << t.span_log2 : 0;
+        auto share = [&](Int count) -> Int {
+            const Int half = count / 2;
+            return count <= p.leaf || first >= half ? 0 : (half - first < span ? half - first : span);
+        };
+        const Int each = share(small);
+        uint64_t before = (uint64_t)path * each;
+        if (large != 0 && path != 0) {
+            const Int more = share(small + 1) - each;
+            if (more != 0) before += count_large(path, t.rel, large) * more;
         }
-        // a node with a packet after this one fills it, and then so does
-        // every node of the level but for a short tail of the smallest
-        const Int span = (Int)1 << span_log2;
-        const Int small = (Int)(root_count >> rel);
-        if (small > p.leaf && small / 2 >= span) {
-            return at + ls.prefix0[rs] + ((uint64_t)path << span_log2);
-        }
-        return at + ls.prefix0[rs] +
-            packet_path_bits(root_count, gi.depth, rel, 0, path, p.leaf);
+        return at + before +
+            (tail ? t.prefix_tail[rs][size != (Int)p.levels[level].q ? 1 : 0] : t.prefix0[rs]);
     }
 };
 
 // node_size, in 32 bits where those hold every index.
-BP_HD uint64_t path_node_size(const LevelInfo& lv, uint32_t level, uint64_t node) {
-    return node_size(lv, level, node);
+BP_HD uint64_t path_node_size(const Plan& p, const PathLevel&, uint32_t level, uint64_t node) {
+    return node_size(p.levels[level], level, node);
 }
-BP_HD uint32_t path_node_size(const LevelInfo& lv, uint32_t level, uint32_t node) {
+BP_HD uint32_t path_node_size(const Plan&, const PathLevel& t, uint32_t level, uint32_t node) {
 #if defined(__CUDA_ARCH__)
     const uint32_t reversed = level == 0 ? 0u : __brev(node) >> (32 - level);
 #else
     const uint32_t reversed = (uint32_t)reverse_bits(node, level);
 #endif
-    return (uint32_t)lv.q + (reversed < (uint32_t)lv.r ? 1u : 0u);
+    return t.q + (reversed < t.r ? 1u : 0u);
 }
 
 // Forward (p[value]) or inverse (p^-1[value]) lookup.  Returns a
 // LookupStatus; *out is valid when it is kLookupOk.  Int holds every index
 // and node of the permutation: 32 bits up to 2^31 entries, else 64.
-template <typename Int>
-BP_HD uint32_t lookup_path(const Plan& p, const BlobBits& blob, uint64_t value, bool inverse,
-    uint64_t* out) {
+// `levels` gives the path levels of a section (PlanLevels, or a table).
+template <typename Int, typename Levels>
+BP_HD uint32_t lookup_path(const Plan& p, const Levels& levels, const BlobBits& blob,
+    uint64_t value, bool inverse, uint64_t* out) {
     if (value >= p.n) {
         return kLookupOutOfRange;
     }
@@ -245,13 +286,14 @@ BP_HD uint32_t lookup_path(const Plan& p, const BlobBits& blob, uint64_t value, 
         }
         bool right = false;
         if ((size & 1) == 0 || index != size - 1) { // the odd tail passes straight left
-            const uint64_t bit = way_down.bit(p, down, level, node, size, index >> 1);
+            const uint64_t bit =
+                way_down.bit(p, levels.at(down, level), down, level, node, size, (Int)(index >> 1));
             right = blob_bit(blob, 0, bit, &status) != (uint32_t)(index & 1);
         }
         index >>= 1;
         node = 2 * node + (right ? 1 : 0);
         ++level;
-        size = path_node_size(p.levels[level], level, node);
+        size = path_node_size(p, levels.at(down, level), level, node);
     }
     int section = 0;
     const uint64_t rank_bit = leaf_rank_bit(p, level, node, &section);
@@ -262,12 +304,13 @@ BP_HD uint32_t lookup_path(const Plan& p, const BlobBits& blob, uint64_t value, 
     for (uint32_t l = level; l-- > 0;) {
         const Int at = node >> (level - l);
         const uint32_t right = (uint32_t)(node >> (level - 1 - l)) & 1u;
-        const Int count = path_node_size(p.levels[l], l, at);
+        const auto& here = levels.at(up, l);
+        const Int count = path_node_size(p, here, l, at);
         if (right == 0 && (count & 1) != 0 && index == count / 2) {
             index = count - 1; // back out through the odd tail
             continue;
         }
-        const uint64_t bit = way_up.bit(p, up, l, at, count, index);
+        const uint64_t bit = way_up.bit(p, here, up, l, at, count, index);
         index = 2 * index + (right ^ blob_bit(blob, 0, bit, &status));
     }
     *out = index;
@@ -276,8 +319,9 @@ BP_HD uint32_t lookup_path(const Plan& p, const BlobBits& blob, uint64_t value, 
 
 BP_HD uint32_t lookup_one(const Plan& p, const BlobBits& blob, uint64_t value, bool inverse,
     uint64_t* out) {
-    return p.n <= (1ull << 31) ? lookup_path<uint32_t>(p, blob, value, inverse, out)
-                               : lookup_path<uint64_t>(p, blob, value, inverse, out);
+    const PlanLevels levels{&p};
+    return p.n <= (1ull << 31) ? lookup_path<uint32_t>(p, levels, blob, value, inverse, out)
+                               : lookup_path<uint64_t>(p, levels, blob, value, inverse, out);
 }
 
 } // namespace bpb200

@@ -54,10 +54,21 @@ __host__ __device__ inline uint32_t tile_pair_stride(uint64_t pcap) {
     return ((uint32_t)pcap + 1u) & ~1u;
 }
 
-// One pair-node in 2^kTileRulerLog2 is a ruler (see the walk below).
-constexpr uint32_t kTileRulerLog2 = 3;
-// Nodes of at most this many pair-nodes are coloured by one thread each.
-constexpr uint32_t kTileSerialPairs = 64;
+// One pair-node in 2^tile_ruler_log2 is a ruler (see the walk below), and
+// nodes of at most tile_serial_pairs pair-nodes are coloured by one thread
+// each.  Large tiles are bound by instruction issue: few rulers, and serial
+// nodes of up to 64 pair-nodes (8192 entries: 2^26 entries' tiles 3.47 ms
+// against 3.67 with a ruler per 4).  Tiles of up to 4096 slots leave most of
+// their SM idle and wait for their longest walk: a ruler per 4 and fewer
+// serial nodes (1000 entries: 68.4 -> 63.2 us a call, 4096: 85.3 -> 81.5; a
+// ruler per 2: 67.3 and 88.6).
+constexpr uint32_t kSmallTileSlots = 4096;
+__host__ __device__ inline uint32_t tile_ruler_log2(uint32_t slots) {
+    return slots <= kSmallTileSlots ? 2u : 3u;
+}
+__host__ __device__ inline uint32_t tile_serial_pairs(uint32_t slots) {
+    return slots <= kSmallTileSlots ? 32u : 64u;
+}
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
@@ -92,7 +103,7 @@ __host__ __device__ inline uint32_t tile_bit_words(uint32_t slots) { return slot
 // routing levels in the tile.
 __host__ __device__ inline uint32_t tile_smem_layout(uint32_t slots, uint32_t levels,
     uint32_t* off) {
-    const uint32_t rulers = (slots >> (kTileRulerLog2 + 1)) + 1;
+    const uint32_t rulers = (slots >> (tile_ruler_log2(slots) + 1)) + 1;
     uint32_t o = 0;
     off[0] = o; o = align_up(o + slots * 2, 16);           // inverse, even levels
     off[1] = o; o = align_up(o + slots * 2, 16);           // inverse, odd levels
@@ -146,6 +157,8 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
     volatile uint32_t* vstate = state;
     uint32_t* level_bits = (uint32_t*)(smem + off[4]);
     const uint32_t bit_words = tile_bit_words(slots);
+    const uint32_t ruler_log2 = tile_ruler_log2(slots);
+    const uint32_t serial_pairs = tile_serial_pairs(slots);
 
     const Plan& plan = *plan_ptr;
     const uint32_t tid = threadIdx.x;
@@ -303,7 +316,7 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
 
         {
             // ---- input switch bits: the colour of input 2k of every pair-node
-            if (ps <= kTileSerialPairs) {
+            if (ps <= serial_pairs) {
                 for (uint32_t e = tid; e < (nodes * ps + 31) / 32 + 1; e += blockDim.x) xbits[e] = 0;
                 __syncthreads();
                 for (uint32_t path = tid; path < nodes; path += blockDim.x) {
@@ -328,7 +341,7 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
                     }
                 }
             } else {
-                // Ruler walks.  One pair-node in 8 (at a hashed position) is
+                // Ruler walks.  One pair-node in 2^ruler_log2 (hashed) is
                 // a ruler; a thread walks both directions away from it until
                 // each meets a ruler or a pair-node stamped by a walk coming
                 // the other way, so every pair-node is passed about once.  A
@@ -339,11 +352,11 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
                 // stamped pair-node at input w goes on as directed ruler
                 // stamp ^ (w & 1); two walks crossing may both stamp the
                 // pair-nodes where they cross, with stamps that say the same.
-                const uint32_t rulers = (nodes * ps + (1u << kTileRulerLog2) - 1) >> kTileRulerLog2;
+                const uint32_t rulers = (nodes * ps + (1u << ruler_log2) - 1) >> ruler_log2;
                 const uint32_t edge_addr = smem_addr(edge);
                 for (uint32_t r = tid; r < rulers; r += blockDim.x) {
-                    const uint32_t at = (r << kTileRulerLog2) +
-                        ((r * 0x9E3779B1u) >> (32 - kTileRulerLog2));
+                    const uint32_t at = (r << ruler_log2) +
+                        ((r * 0x9E3779B1u) >> (32 - ruler_log2));
                     const uint32_t path = by_ps(at);
                     const uint32_t s = path < nodes ? node_size(path) : 0;
                     const bool real = at - path * ps < s - s / 2 && internal_node(path, s);
@@ -358,8 +371,8 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
                         state[2 * r + 1] = 0xffff0000u | (2 * r + 1);
                         continue;
                     }
-                    const uint32_t at = (r << kTileRulerLog2) +
-                        ((r * 0x9E3779B1u) >> (32 - kTileRulerLog2));
+                    const uint32_t at = (r << ruler_log2) +
+                        ((r * 0x9E3779B1u) >> (32 - ruler_log2));
                     const uint32_t path = by_ps(at);
                     const uint32_t base = path * ps;
                     const uint32_t bias = key_bias(node_size(path));
@@ -398,7 +411,7 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
                 // it): three hops a round at least quadruple the stretch.
                 // States change in place: a state read early or late is a
                 // shorter or a longer stretch, both true.
-                for (uint32_t reach = 1; reach < (ps >> kTileRulerLog2) + 2; reach *= 4) {
+                for (uint32_t reach = 1; reach < (ps >> ruler_log2) + 2; reach *= 4) {
                     for (uint32_t i = tid; i < 2 * rulers; i += blockDim.x) {
                         uint32_t me = vstate[i];
 #pragma unroll

@@ -439,23 +439,24 @@ __device__ __forceinline__ void list_rank_run(Grid grid, const Plan* __restrict_
             const uint32_t own = key[rank_slot(r)];
             uint32_t wa = word >> 16, wb = word & 0xffffu;
             uint32_t ma = own, mb = own ^ 1u;
+            uint32_t va, vb;
             bool ga = true, gb = true;
-            uint32_t va = 0, vb = 0;
-            for (uint32_t step = 0; (ga || gb) && step <= count; ++step) {
+            for (uint32_t step = 0; step <= count; ++step) {
+                // both walks and their keys in flight together; a walk that
+                // has ended reads its last word again
                 va = link[wa >> 1];
                 vb = link[wb >> 1];
+                const uint32_t ka = key[wa >> 1] ^ (wa & 1u);
+                const uint32_t kb = key[wb >> 1] ^ (wb & 1u);
                 ga = (va & 0x8000u) == 0;
                 gb = (vb & 0x8000u) == 0;
-                if (ga) {
-                    link16[wa & ~1u] = (uint16_t)(0x8000u | (r << 1) | (wa & 1u));
-                    ma = min(ma, key[wa >> 1] ^ (wa & 1u));
-                    wa = (wa & 1u) != 0 ? va & 0xffffu : va >> 16;
-                }
-                if (gb) {
-                    link16[wb & ~1u] = (uint16_t)(0x8000u | (r << 1) | (~wb & 1u));
-                    mb = min(mb, key[wb >> 1] ^ (wb & 1u));
-                    wb = (wb & 1u) != 0 ? vb & 0xffffu : vb >> 16;
-                }
+                if (ga) link16[wa & ~1u] = (uint16_t)(0x8000u | (r << 1) | (wa & 1u));
+                if (gb) link16[wb & ~1u] = (uint16_t)(0x8000u | (r << 1) | (~wb & 1u));
+                if (!ga && !gb) break;
+                ma = ga ? min(ma, ka) : ma;
+                mb = gb ? min(mb, kb) : mb;
+                wa = ga ? (va >> ((~wa & 1u) << 4)) & 0xffffu : wa;
+                wb = gb ? (vb >> ((~wb & 1u) << 4)) & 0xffffu : wb;
             }
             const uint32_t na = ga ? 2 * r : (va & 0x7fffu) ^ (wa & 1u);
             const uint32_t nb = gb ? 2 * r + 1 : (vb & 0x7fffu) ^ (wb & 1u);
