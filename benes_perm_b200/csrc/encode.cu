@@ -771,7 +771,22 @@ void run_level(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p, cons
                 w.lists.colour[1], w.xbits, w.d_status);
         });
     } else {
-        rec.launch(kKindUnion, [&] {
+        const bool by_windows = lv.cap > kSwapMaxNode && w.records != nullptr;
+        if (by_windows) {
+            const uint32_t low = (uint32_t)(pair_lo >> kUnionWindowLog2);
+            const uint32_t high = (uint32_t)((pair_lo + prs - 1) >> kUnionWindowLog2);
+            check(cudaMemsetAsync(w.cursor, 0, kUnionWindows * 4, st), "cudaMemsetAsync(cursors)");
+            rec.launch(kKindUnion, [&] {
+                launch_next(union_bucket, grid_for(prs / kUnionBucketItems, kLevelThreads),
+                    kLevelThreads, 0, st, dp, l, inv, w.edge, w.records, w.cursor, w.slot_cap,
+                    w.d_status);
+                for (uint32_t v = high + 1; v-- > low;) {
+                    launch_next(union_window, device_sms() * 6, kLevelThreads, 0, st, v, w.edge,
+                        w.records, w.cursor, w.slot_cap, w.d_status);
+                }
+            }, 2 + high - low);
+        }
+        if (!by_windows) rec.launch(kKindUnion, [&] {
             launch_next(level_union, grid_for((prs + kUnionItems - 1) / kUnionItems, kLevelThreads),
                 kLevelThreads, 0, st, dp, l, inv, w.edge, ctl + kCtlClaimUnion, w.d_status);
         });
