@@ -112,3 +112,13 @@ def test_stage_rejects_repeats(gpu):
             with pytest.raises(ValueError):
                 gpu.compress(wrong)
             assert gpu.compress(perm) == good
+
+
+@pytest.mark.slow
+@pytest.mark.parametrize("n,kind", [((1 << 25) + 3, 1), ((1 << 25) + 2, 0)])
+def test_union_windows(gpu, oracle, n, kind):
+    """The smallest nodes whose unions go by windows: the upper window holds
+    one or two pair-nodes, the odd tail among them.  (The 100,000,007 and 2^30
+    entry digests cover several windows.)"""
+    kinds = gpu.PermutationKind
+    check(gpu, oracle, n, n, (kinds.uniform, kinds.single_cycle)[kind])
