@@ -707,7 +707,7 @@ void run_level(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p, cons
         check(cudaMemsetAsync(w.cursor, 0, windows * 4, st), "cudaMemsetAsync(cursors)");
         auto bucket = [&](uint64_t lo, uint64_t hi) {
             const int gb = grid_for((hi - lo + kBucketItems - 1) / kBucketItems, kBucketThreads);
-            level_bucket<T><<<gb, kBucketThreads, 0, st>>>(dp, l, src, w.records, w.cursor, w.edge,
+            level_bucket<T><<<gb, kBucketThreads, 0, st>>>(dp, src, w.records, w.cursor, w.edge,
                 w.d_status, lo, hi);
         };
         const uint32_t parts = input != nullptr ? (uint32_t)input->ends.size() : 0;

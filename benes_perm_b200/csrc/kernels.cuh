@@ -159,120 +159,133 @@ __global__ void __launch_bounds__(256) level_inverse(const Plan* __restrict__ pl
 // sector per entry (about 21 G entries/s on B200).  Instead:
 //   level_bucket  streams the values once and appends (destination, i)
 //                 records to the 2^kPlaceLog2-slot destination window they
-//                 land in (block-local counts in shared memory, one global
-//                 reservation per block and window);
+//                 land in.  A block sorts its 4096 records by window in
+//                 shared memory (counts, a scan, one global reservation per
+//                 window) and writes them out in that order, so a window's
+//                 records leave as runs of whole sectors;
 //   level_place   replays each window's records; the writes of one window
 //                 stay inside an L2-resident 32 MB range.
-// Windows of 2^23 slots measured fastest on B200 at 2^30 uniform entries
-// (2^21: 256 ms of inverse per compress, 2^22: 240, 2^23: 226): larger
-// windows give each block longer runs of records per window.
+// Bound by HBM for the bucket pass (8 + 8 + 2 bytes per uint64 entry) and by
+// L2's random writes for the replay (2^30 at 220 G/s: 4.9 ms).  2^30 uniform
+// uint64 entries, both kernels: 13.5 ms; 28.5 ms with every thread writing
+// its records where they fell, 8 bytes to a sector.  Windows of 2^24 slots
+// (64 MB, half of L2): 14.8 ms; 2^25: 29.5 ms, the window no longer fits.
+// 2^24 entries: 0.236 ms against 0.273 before and 0.275 with 2^24 slots.
 // A window receives at most as many records as it has slots when the input
 // is a permutation; an overfull window means a repeated value.
 // ---------------------------------------------------------------------------
 #ifndef BPB200_PLACE_LOG2
-#define BPB200_PLACE_LOG2 24
+#define BPB200_PLACE_LOG2 23
 #endif
 constexpr uint32_t kPlaceLog2 = BPB200_PLACE_LOG2; // slots per destination window (log2)
-constexpr uint32_t kMaxWindows = 2048;
+constexpr uint32_t kMaxWindows = 256;
 static_assert((1ull << 31) >> kPlaceLog2 <= kMaxWindows, "windows must cover 2^31 slots");
 constexpr int kBucketItems = 16;
+constexpr int kBucketThreads = 256; // block size of level_bucket: a thread per window
+static_assert(kMaxWindows <= kBucketThreads, "one window per thread in the scan");
 
-#ifndef BPB200_BUCKET_THREADS
-#define BPB200_BUCKET_THREADS 256
-#endif
-constexpr int kBucketThreads = BPB200_BUCKET_THREADS; // block size of level_bucket
-
+// Slots [e_lo, e_hi) of level 0 (all of it, or one part of an input still
+// being uploaded; e_lo a multiple of 4 so vector loads stay aligned).
 template <typename T>
-// Slots [e_lo, e_hi) of the level (the whole level, or one part of an input
-// still being uploaded; e_lo a multiple of 4 so vector loads stay aligned).
-__device__ __forceinline__ void level_bucket_run(Grid grid, const Plan* __restrict__ plan,
-    uint32_t level, const T* __restrict__ src, uint2* __restrict__ records,
-    uint32_t* __restrict__ cursor, uint32_t* __restrict__ uf, uint32_t* status,
-    uint64_t e_lo, uint64_t e_hi) {
+__global__ void __launch_bounds__(kBucketThreads, 4) level_bucket(const Plan* __restrict__ plan,
+    const T* __restrict__ src, uint2* __restrict__ records, uint32_t* __restrict__ cursor,
+    uint32_t* __restrict__ uf, uint32_t* status, uint64_t e_lo, uint64_t e_hi) {
+    __shared__ uint2 sorted[kBucketThreads * kBucketItems];
     __shared__ uint32_t count[kMaxWindows];
-    __shared__ uint32_t start[kMaxWindows];
-    const LevelInfo& lv = plan->levels[level];
-    const uint32_t cap = (uint32_t)lv.cap;
-    const uint32_t pcap = (uint32_t)lv.pcap;
-    const uint64_t slots = cap;
-    const uint64_t total = e_hi < slots ? e_hi : slots;
-    const uint32_t windows = (uint32_t)((slots + (1ull << kPlaceLog2) - 1) >> kPlaceLog2);
-    const uint64_t chunk = (uint64_t)blockDim.x * kBucketItems;
+    __shared__ uint32_t local[kMaxWindows]; // the window's first record in `sorted`
+    __shared__ uint32_t start[kMaxWindows]; // and in its region of `records`
+    __shared__ uint32_t sums[kBucketThreads / 32];
+    constexpr int kVec = 16 / sizeof(T);
+    constexpr uint32_t kChunk = kBucketThreads * kBucketItems;
+    wait_for_previous();
+    const uint64_t n = plan->levels[0].cap;
+    const uint64_t total = e_hi < n ? e_hi : n;
     const bool aligned = ((uintptr_t)src & 15u) == 0 && (e_lo & 3u) == 0;
-    for (uint64_t c0 = e_lo + (uint64_t)grid.bid * chunk; c0 < total;
-         c0 += (uint64_t)grid.nblk * chunk) {
-        for (uint32_t b = threadIdx.x; b < windows; b += blockDim.x) count[b] = 0;
+    const uint32_t t = threadIdx.x;
+    for (uint64_t c0 = e_lo + (uint64_t)blockIdx.x * kChunk; c0 < total;
+         c0 += (uint64_t)gridDim.x * kChunk) {
+        const bool whole = aligned && c0 + kChunk <= total;
+        if (t < kMaxWindows) count[t] = 0;
         __syncthreads();
-        const uint64_t e0 = c0 + (uint64_t)threadIdx.x * kBucketItems;
-        uint32_t dest[kBucketItems], idx[kBucketItems];
+        auto item = [&](int q) -> uint32_t { // offset in the chunk of this thread's value q
+            return whole ? (t + kBucketThreads * (q / kVec)) * kVec + q % kVec
+                         : t + kBucketThreads * q;
+        };
         T v[kBucketItems];
-        if (aligned && e0 + kBucketItems <= total) {
-            constexpr int kVec = 16 / sizeof(T);
+        if (whole) {
 #pragma unroll
             for (int q = 0; q < kBucketItems / kVec; ++q) {
-                const uint4 part = __ldcs(reinterpret_cast<const uint4*>(src + e0) + q);
+                const uint4 part = __ldcs(reinterpret_cast<const uint4*>(src + c0) + t +
+                    kBucketThreads * q);
                 const T* parts = reinterpret_cast<const T*>(&part);
 #pragma unroll
                 for (int r = 0; r < kVec; ++r) v[q * kVec + r] = parts[r];
             }
         } else {
 #pragma unroll
-            for (int q = 0; q < kBucketItems; ++q) v[q] = e0 + q < total ? src[e0 + q] : (T)0;
+            for (int q = 0; q < kBucketItems; ++q) {
+                v[q] = c0 + item(q) < total ? src[c0 + item(q)] : (T)0;
+            }
         }
-        uint32_t j = (uint32_t)(e0 < total ? e0 / cap : 0);
-        uint32_t i = (uint32_t)(e0 < total ? e0 - (uint64_t)j * cap : 0);
-        uint32_t s = size_at(lv, level, j);
+        uint32_t dest[kBucketItems], rank[kBucketItems];
 #pragma unroll
         for (int q = 0; q < kBucketItems; ++q) {
             dest[q] = ~0u;
-            if (e0 + q < total && i < s) {
-                if ((i & 1u) == 0) { // unconditional: see level_inverse
-                    const uint32_t id = j * pcap + (i >> 1);
-                    uf[id] = id << 1;
-                }
-                const uint64_t val = (uint64_t)v[q];
-                if (val >= s) {
+            if (c0 + item(q) < total) {
+                if ((uint64_t)v[q] >= n) {
                     atomicOr(status, kErrNotPermutation);
                 } else {
-                    dest[q] = j * cap + (uint32_t)val;
-                    idx[q] = i;
-                    atomicAdd(&count[dest[q] >> kPlaceLog2], 1u);
+                    dest[q] = (uint32_t)v[q];
+                    rank[q] = atomicAdd(&count[dest[q] >> kPlaceLog2], 1u);
                 }
             }
-            if (++i == cap) {
-                i = 0;
-                ++j;
-                s = size_at(lv, level, j);
-            }
+        }
+        // union-find roots of the chunk's pair-nodes (unconditional: see
+        // level_inverse)
+        const uint64_t pairs = ((c0 + kChunk < total ? c0 + kChunk : total) + 1) / 2;
+#pragma unroll
+        for (int q = 0; q < kBucketItems / 2; ++q) {
+            const uint64_t id = c0 / 2 + t + kBucketThreads * q;
+            if (id < pairs) uf[id] = (uint32_t)id << 1;
         }
         __syncthreads();
-        for (uint32_t b = threadIdx.x; b < windows; b += blockDim.x) {
-            if (count[b] != 0) start[b] = atomicAdd(cursor + b, count[b]);
-            count[b] = 0;
+        const uint32_t mine = t < kMaxWindows ? count[t] : 0;
+        uint32_t upto = mine;
+#pragma unroll
+        for (int d = 1; d < 32; d *= 2) {
+            const uint32_t o = __shfl_up_sync(0xffffffffu, upto, d);
+            if ((t & 31u) >= (uint32_t)d) upto += o;
         }
+        if ((t & 31u) == 31u) sums[t / 32] = upto;
+        if (mine != 0) start[t] = atomicAdd(cursor + t, mine);
+        __syncthreads();
+        uint32_t all = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < kBucketThreads / 32; ++k) {
+            if (k < t / 32) upto += sums[k];
+            all += sums[k];
+        }
+        if (t < kMaxWindows) local[t] = upto - mine;
         __syncthreads();
 #pragma unroll
         for (int q = 0; q < kBucketItems; ++q) {
             if (dest[q] == ~0u) continue;
-            const uint32_t b = dest[q] >> kPlaceLog2;
-            const uint64_t at = ((uint64_t)b << kPlaceLog2) + start[b] + atomicAdd(&count[b], 1u);
-            if (at < slots && at < ((uint64_t)(b + 1) << kPlaceLog2)) {
-                records[at] = make_uint2(dest[q], idx[q]);
+            sorted[local[dest[q] >> kPlaceLog2] + rank[q]] =
+                make_uint2(dest[q], (uint32_t)c0 + item(q));
+        }
+        __syncthreads();
+        for (uint32_t k = t; k < all; k += kBucketThreads) {
+            const uint2 r = sorted[k];
+            const uint32_t b = r.x >> kPlaceLog2;
+            const uint64_t at = ((uint64_t)b << kPlaceLog2) + start[b] + (k - local[b]);
+            if (at < n && at < ((uint64_t)(b + 1) << kPlaceLog2)) {
+                records[at] = r;
             } else {
                 atomicOr(status, kErrNotPermutation); // more values than slots: a repeat
             }
         }
         __syncthreads();
     }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(BPB200_BUCKET_THREADS) level_bucket(const Plan* __restrict__ plan,
-    uint32_t level, const T* __restrict__ src, uint2* __restrict__ records,
-    uint32_t* __restrict__ cursor, uint32_t* __restrict__ uf, uint32_t* status,
-    uint64_t e_lo, uint64_t e_hi) {
-    wait_for_previous();
-    level_bucket_run<T>(launch_grid(), plan, level, src, records, cursor, uf, status, e_lo, e_hi);
 }
 
 constexpr int kPlaceItems = 16;

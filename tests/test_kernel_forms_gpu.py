@@ -122,3 +122,23 @@ def test_union_windows(gpu, oracle, n, kind):
     entry digests cover several windows.)"""
     kinds = gpu.PermutationKind
     check(gpu, oracle, n, n, (kinds.uniform, kinds.single_cycle)[kind])
+
+
+@pytest.mark.parametrize("n", [(1 << 23) + 1, 3 * (1 << 22) + 4093])
+def test_bucket_pass(gpu, oracle, n):
+    """The smallest partitioned inverses: a last window of one slot, a last
+    chunk that is not whole, inputs on and off 16-byte boundaries."""
+    import torch
+    perm = gpu.fill_permutation(gpu.PermutationKind.uniform, n, n, np.uint32)
+    want = oracle.compress(perm, oracle_format({}))
+    stream = torch.cuda.current_stream().cuda_stream
+    blob = torch.empty((len(want) + 3) // 4 * 4, dtype=torch.uint8, device="cuda")
+    for dtype, as_torch in ((np.uint32, np.int32), (np.uint64, np.int64)):
+        for shift in (0, 1):
+            src = np.zeros(n + 1, dtype=dtype)
+            src[shift:shift + n] = perm
+            d = torch.from_numpy(src.view(as_torch)).cuda()
+            blob.zero_()
+            gpu.compress_device(d.data_ptr() + shift * src.itemsize, n, src.itemsize,
+                                blob.data_ptr(), len(want), b200_format(gpu, {}), stream)
+            assert blob.cpu().numpy()[:len(want)].tobytes() == want, (dtype, shift)
