@@ -6,10 +6,15 @@ compresses of a seeded uniform permutation on the current GPU while forcing
 one setting at a time (bpb200_set_tuning), walking the knobs one after
 another (coordinate descent from the compiled defaults):
 
-  walk_blocks_per_sm  persistent orbit-walk blocks per SM
-  walk_max_log2       largest node coloured by orbit walks (else union-find)
-  jump_block_log2     largest super-ruler count jumped inside one CTA
+  jump_block_log2     largest list of a node's rulers ranked inside one CTA
   tile_max_log2       largest node encoded by the shared-memory tile
+
+walk_max_log2, the largest node coloured by ruler walks (else union-find),
+stays at its compiled 2^23: on the uniform inputs timed here union-find is up
+to 5 % faster below that, but on inputs made of long runs its chains reach
+the cap on their length, which the walks' do not.  walk_blocks_per_sm is part
+of every setting but no kernel reads it: the walks take one ruler per thread,
+so the list's length sizes their grid.
 
 None of them may change a byte: every setting's blob is hashed and the run
 fails unless all hashes of a class agree.  The winners go to tuning.json
@@ -17,7 +22,7 @@ beside the library, which the library reads at load; the per-class timings
 of the defaults and of the table go to the same file ("measured") and, with
 --summary, to a markdown table.
 
-Usage: python -m benes_perm_b200.tune [--classes 14,16,...] [--reps 5]
+Usage: python -m benes_perm_b200.tune [--classes 14,16,...] [--reps 21]
            [--out benes_perm_b200/tuning.json] [--summary FILE]
 """
 from __future__ import annotations
@@ -34,9 +39,7 @@ import numpy as np
 HERE = os.path.dirname(os.path.abspath(__file__))
 
 CANDIDATES = {
-    "walk_blocks_per_sm": [2, 3, 4, 6],
-    "walk_max_log2": [16, 18, 20, 22, 23],
-    "jump_block_log2": [10, 12, 14, 16],
+    "jump_block_log2": [10, 12, 14],
     "tile_max_log2": [11, 12, 13, 14],
 }
 
@@ -104,8 +107,8 @@ def tune_class(bp, torch, log2n, reps):
 
 def main(argv=None) -> None:
     ap = argparse.ArgumentParser()
-    ap.add_argument("--classes", default="14,16,18,20,22,24,26,28,30")
-    ap.add_argument("--reps", type=int, default=5)
+    ap.add_argument("--classes", default="14,16,18,20,21,22,24,26,28,30")
+    ap.add_argument("--reps", type=int, default=21)
     ap.add_argument("--out", default=os.path.join(HERE, "tuning.json"))
     ap.add_argument("--summary", default=None)
     args = ap.parse_args(argv)
@@ -136,7 +139,7 @@ def main(argv=None) -> None:
                 f.write(f"| 2^{c} | {rec['entries']} | {rec['entry_bytes']} B | "
                         f"{rec['default_ms']:.3f} | {rec['tuned_ms']:.3f} | "
                         f"{rec['default_ms'] / rec['tuned_ms']:.3f}x | "
-                        f"walk blocks/SM {s['walk_blocks_per_sm']}, walk max 2^{s['walk_max_log2']}, "
+                        f"walk max 2^{s['walk_max_log2']}, "
                         f"one-CTA jump 2^{s['jump_block_log2']}, tile 2^{s['tile_max_log2']} |\n")
 
 
