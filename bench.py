@@ -200,11 +200,12 @@ def algorithmic_bytes(n, depth, tile, entry_bytes, switch_bits, middle_bits, wal
                       place_levels=()):
     """Compulsory HBM bytes per kernel kind for one compress: every array a
     kernel must touch, read once and written once at its minimal width.
-    Levels in `walk_levels` are coloured by orbit walks (walk + jump), the
+    Levels in `walk_levels` are coloured by ruler walks (walk + jump), the
     other global levels by union-find (union).  Only level 0 builds an
     inverse from its values (partitioned, kind "place", on the levels in
-    `place_levels`; else "inverse"); every later level's inverse is written
-    by its parent's output pass ("output_bits")."""
+    `place_levels`; else "inverse") and, when it is a walk level, its edges;
+    every later level's inverse and edges are written by its parent's output
+    pass ("output_bits")."""
     kinds = ("inverse", "place", "union", "walk", "jump", "resolve", "output_bits", "emit",
              "tile")
     per = {k: 0.0 for k in kinds}
@@ -213,14 +214,18 @@ def algorithmic_bytes(n, depth, tile, entry_bytes, switch_bits, middle_bits, wal
         if lvl == 0:
             per["place" if lvl in place_levels else "inverse"] += (w + 4) * n
         if lvl in walk_levels:
-            per["walk"] += 12 * n                  # values, inverse, owner stamp per vertex
+            if lvl == 0:
+                per["inverse"] += (4 + 4 + 2) * n  # inverse read, edges and stamps written
+            per["walk"] += (4 + 4) * n             # edges; one stamp per pair-node, exchanged
             per["jump"] += 2 * n                   # ruler states (16 B per 16 slots) read+written
-            per["resolve"] += (4 + w + 4) * n + n / 8  # owners, values, children, bits
         else:
             per["union"] += 8 * n                  # inverse, one word per pair read+written
-            per["resolve"] += (2 + w + 4) * n + n / 8  # union-find words, values, children, bits
-        # this level's inverse, the children's inverse (when they are global), output bits
-        per["output_bits"] += 4 * n + (4 * n if lvl + 1 < tile else 0) + n / 8
+        per["resolve"] += 2 * n + n / 16           # words or stamps of the pair-nodes, bits
+        # this level's inverse, the children's inverse (when they are global),
+        # the edges and stamps of children coloured by walks, output bits
+        per["output_bits"] += 4 * n + (4 * n if lvl + 1 < tile else 0) + n / 16
+        if lvl + 1 in walk_levels:
+            per["output_bits"] += (4 + 2) * n
         per["emit"] += n / 4                       # bits of both sides, read and placed
     w = entry_bytes if tile == 0 else 4
     per["tile"] = w * n + 2 * (depth - tile) * n / 16 + middle_bits / 8
@@ -233,22 +238,20 @@ def random_accesses(n, tile, walk_levels, place_levels):
     """Random 4-byte accesses per step by kernel kind and level, the least
     each kind's algorithm needs (reads, writes): the inverse scatter one
     write per entry (level 0 only; later inverses are written in order); a
-    union per output pair at least two finds and a link (a read per entry,
-    a write per pair); an orbit-walk step two gathers and an owner stamp
-    (two reads and a write per entry); finalize one lookup per pair-node
-    (find or owner-to-colour); the output pass one colour bit per output
-    pair."""
+    union per output pair one look at its larger end and one link; a walk
+    step the edges of a pair-node (one read) and its stamp's exchange (one
+    write); the resolving pass one lookup per pair-node (its root or its
+    ruler's colour); the output pass one colour bit per output pair and, for
+    children coloured by walks, one edge written per entry."""
     acc = {}
     half = n / 2
     for lvl in range(tile):
         if lvl == 0:
-            acc[("place" if lvl in place_levels else "inverse", lvl)] = (0.0, float(n))
-        if lvl in walk_levels:
-            acc[("walk", lvl)] = (2.0 * n, float(n))
-        else:
-            acc[("union", lvl)] = (float(n), half)
+            edges = float(n) if lvl in walk_levels else 0.0
+            acc[("place" if lvl in place_levels else "inverse", lvl)] = (0.0, n + edges)
+        acc[("walk" if lvl in walk_levels else "union", lvl)] = (half, half)
         acc[("resolve", lvl)] = (half, 0.0)
-        acc[("output_bits", lvl)] = (half, 0.0)
+        acc[("output_bits", lvl)] = (half, float(n) if lvl + 1 in walk_levels else 0.0)
     return acc
 
 
@@ -262,7 +265,7 @@ def random_access_roofline(n, depth, tile, walk_levels, place_levels, node_log2,
     bound on the time, hence ``frac`` <= 1.  ``bound_dram_s`` takes the DRAM
     rates for levels whose nodes exceed 2^23 entries (their arrays do not
     fit L2); a kind can beat it where its access order keeps them in L2
-    (claim-ordered work, the partitioned inverse)."""
+    (claim-ordered work, the partitioned inverse, unions by windows)."""
     bound_l2, bound_dram = {}, {}
     l2, dram = probe["l2_32MB"], probe["dram_4GB"]
     for (kind, lvl), (reads, writes) in random_accesses(n, tile, walk_levels,

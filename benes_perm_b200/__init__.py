@@ -287,9 +287,9 @@ def set_profiling(enabled: bool) -> None:
 
 
 def set_union_find_only(enabled) -> None:
-    """Test hook: colour global levels with union-find instead of orbit walks
-    (True), or run the walks and colour their levels with the union-find
-    fallback anyway ("fallback"); False restores the default."""
+    """Test hook: colour global levels with union-find instead of ruler walks
+    (True), or run the walks and then the union-find second pass anyway
+    ("fallback"); False restores the default."""
     library().bpb200_set_colouring(2 if enabled == "fallback" else (1 if enabled else 0))
 
 

@@ -85,7 +85,7 @@ struct EmitJob {
     uint32_t pad_;
 };
 
-// Word fills (blob clearing, validation sentinels, super-ruler marks).
+// Word fills (blob clearing, validation sentinels).
 struct FillJob {
     uint32_t* ptr;
     uint64_t words;

@@ -3,10 +3,12 @@
 // Host orchestration and C ABI of the B200 compact encoder.
 //
 // One call: plan on the host (closed-form layout, a few KB) -> prologue
-// kernel (zero status, header bytes) -> level kernels for the levels whose
-// nodes exceed a tile -> one tile kernel finishing every subtree in shared
-// memory.  Everything runs on one stream; scratch lives in a pooled
-// per-device workspace so repeated calls allocate nothing.
+// kernel (places the plan, clears blob and status, header bytes) -> level
+// kernels for the levels whose nodes exceed a tile -> tile kernels (a stage
+// of two levels where nodes or launches are small, then the rest of every
+// subtree) in shared memory.  A permutation of one tile is one launch.
+// Everything runs on one stream; scratch lives in a pooled per-device
+// workspace so repeated calls allocate nothing.
 #include "../../include/benes_b200.h"
 #include "batch_levels.cuh"
 #include "kernels.cuh"
@@ -419,20 +421,17 @@ std::atomic<int> g_force_union_find{0};
 //
 // Launch choices that change speed but never bytes, per size class (the
 // class of a permutation of n entries is ceil(log2 n)):
-//   walk_blocks_per_sm  persistent level_walk blocks per SM; resident
-//                       walkers times the slots per ruler is the address
-//                       window the walks keep live, which must stay in L2
-//   walk_max_log2       largest node coloured by orbit walks (larger nodes
+//   walk_blocks_per_sm  kept in the setting's layout; no kernel reads it
+//                       (the walks take one ruler per thread)
+//   walk_max_log2       largest node coloured by ruler walks (larger nodes
 //                       by union-find); at most the compiled walk limit
-//   jump_block_log2     largest super-ruler count whose pointer-jumping
-//                       rounds run inside one CTA (else one launch pair per
-//                       round)
+//   jump_block_log2     largest list of a node's rulers ranked inside one
+//                       CTA (2^10 to 2^14), longer ones are contracted first
 //   tile_max_log2       largest node handed to the shared-memory tile
 // The table comes from tuning.json beside this library (written by
 // benes_perm_b200/tune.py; BPB200_TUNING_FILE names another file, "none"
 // disables it), loaded once; classes it lacks take the nearest class it
 // has, and without a table the compiled defaults apply.
-// BPB200_WALK_BLOCKS_PER_SM overrides the default walk blocks per SM.
 struct Tuning {
     uint32_t walk_blocks_per_sm;
     uint32_t walk_max_log2;
@@ -441,13 +440,7 @@ struct Tuning {
 };
 
 Tuning default_tuning() {
-    static const Tuning t = [] {
-        const char* env = std::getenv("BPB200_WALK_BLOCKS_PER_SM");
-        const int v = env ? std::atoi(env) : 4;
-        return Tuning{(uint32_t)(v < 1 ? 1 : (v > 8 ? 8 : v)), BPB200_WALK_MAX_LOG2,
-            kRankMaxLog2, 13};
-    }();
-    return t;
+    return Tuning{4, BPB200_WALK_MAX_LOG2, kRankMaxLog2, 13};
 }
 
 Tuning clamp_tuning(Tuning t) {
@@ -1857,8 +1850,8 @@ int bpb200_probe_rank_bit(uint64_t count, const bpb200_format* format, uint32_t 
 // latency-critical paths that cannot afford the device-wide synchronisation
 // cudaMalloc/cudaFree can imply.  For them,
 // bpb200_compress_device_noalloc runs the same encode with all of its
-// scratch (plan, status word, level arrays, inverse, union-find words,
-// colour bits, node descriptors) carved out of one file-scope device array
+// scratch (plan, status word, inverses, edges, stamps, ruler lists, colour
+// bits, node descriptors) carved out of one file-scope device array
 // of fixed size.  The array exists on every GPU that loads this library and
 // stays allocated until the process exits.
 // ---------------------------------------------------------------------------

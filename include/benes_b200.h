@@ -110,9 +110,9 @@ int bpb200_compress_device_shard(const void* d_entries, uint64_t count, uint32_t
  * 8 MB, present on every GPU that loads the library until the process
  * exits), so it accepts at most 262144 (2^18) entries and returns
  * BPB200_LENGTH above that.  It calls no cudaMalloc/cudaFree.  Like
- * bpb200_compress_device, each call uploads its plan from host memory,
- * waits for `stream` to finish the work and reads the device status word
- * back before it returns.  The first call on each device looks up the
+ * bpb200_compress_device, each call passes its plan as a parameter of its
+ * first kernel, waits for `stream` to finish the work and reads the device
+ * status word back before it returns.  The first call on each device looks up the
  * array's device address (cudaGetSymbolAddress); make that first call
  * before capturing any stream.  All calls share the one array: calls whose
  * GPU work overlaps (different streams or host threads without ordering)
@@ -224,9 +224,9 @@ void bpb200_set_profiling(int enabled);
  * BPB200_TUNING_FILE names another file, "none" disables it); a class of
  * ceil(log2 count) the table lacks takes its nearest class. */
 typedef struct bpb200_tuning {
-    uint32_t walk_blocks_per_sm; /* persistent orbit-walk blocks per SM, 1..8 */
-    uint32_t walk_max_log2;      /* largest node coloured by orbit walks (log2 entries) */
-    uint32_t jump_block_log2;    /* largest super-ruler count jumped inside one CTA (log2) */
+    uint32_t walk_blocks_per_sm; /* 1..8; kept for the layout, without effect */
+    uint32_t walk_max_log2;      /* largest node coloured by ruler walks (log2 entries) */
+    uint32_t jump_block_log2;    /* longest list of rulers ranked inside one CTA (log2), 10..14 */
     uint32_t tile_max_log2;      /* largest node encoded by the shared-memory tile (log2), 9..14 */
 } bpb200_tuning;
 
@@ -238,9 +238,9 @@ int bpb200_get_tuning(uint64_t count, bpb200_tuning* out);
 int bpb200_set_tuning(const bpb200_tuning* forced);
 
 /* Test hook: 1 makes later calls colour every global level with the
- * union-find kernels instead of the orbit walks (the path the walks fall
- * back to on contrived inputs); 2 runs the walks and then colours each walk
- * level with that fallback anyway, as if a walk had given up (single-call
+ * union-find kernels instead of the ruler walks (what a call does in a
+ * second pass when a walk gives up on contrived inputs); 2 runs the walks
+ * and then that second pass anyway, as if a walk had given up (single-call
  * paths; the batched groups treat 2 as 0); 0 restores the default.  Output
  * bytes are identical in every mode. */
 void bpb200_set_colouring(int union_find_only);
