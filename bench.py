@@ -351,6 +351,11 @@ def _cpu_setup(n_sample):
     return ref, ref.hardware_threads(), perm, fmt, out
 
 
+def _not_built(missing):
+    return (f"{os.path.relpath(str(missing), ROOT)} is not there: it is built from the "
+            "reference's sources (oracle/Makefile)")
+
+
 def reference_arm(args, world, rank):
     """portable_cpu of the reference on the host cores: each step compresses
     a bounded sample (2^24 entries by default) of the headline workload with
@@ -358,7 +363,11 @@ def reference_arm(args, world, rank):
     if rank != 0:
         return
     n_sample = 1 << args.cpu_log2n
-    ref, threads, perm, fmt, out = _cpu_setup(n_sample)
+    try:
+        ref, threads, perm, fmt, out = _cpu_setup(n_sample)
+    except FileNotFoundError as missing:
+        print(json.dumps({"impl": "reference", "unavailable": _not_built(missing)}), flush=True)
+        return
     for _ in range(args.warmup):
         ref.compress(perm, fmt, threads=threads, out=out)
     t0 = time.perf_counter()
@@ -386,7 +395,10 @@ def reference_arm(args, world, rank):
 
 def cpu_baseline(args):
     n_sample = 1 << args.cpu_log2n
-    ref, threads, perm, fmt, out = _cpu_setup(n_sample)
+    try:
+        ref, threads, perm, fmt, out = _cpu_setup(n_sample)
+    except FileNotFoundError as missing:
+        return {"unavailable": _not_built(missing)}
     ref.compress(perm, fmt, threads=threads, out=out)
     times = []
     for _ in range(3):
