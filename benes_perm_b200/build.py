@@ -17,7 +17,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libbenes_b200.so")
 SOURCES = ["encode.cu", "layout.cpp", "permgen.cpp"]
-HEADERS = ["plan.hpp", "layout.hpp", "device.cuh", "kernels.cuh", "tile.cuh", "walk.cuh",
+HEADERS = ["plan.hpp", "layout.hpp", "device.cuh", "kernels.cuh", "settle.cuh", "tile.cuh", "walk.cuh",
            "batch_levels.cuh", "group.inc", "serve.inc", "file.inc", "staging.inc", "lookup.hpp",
            "lookup.inc", "probe.inc"]
 

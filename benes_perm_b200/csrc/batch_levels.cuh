@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(256, BPB200_UNION_MIN_BLOCKS) batch_union(cons
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBUnion, &g);
     if (g.bid >= g.nblk) return;
-    level_union_run(g, j->plan, j->level, j->inv, j->edge, j->control + kCtlClaimUnion, j->status);
+    level_union_run(g, j->plan, j->level, j->inv, j->edge, j->control, j->status, j->status);
 }
 
 __global__ void __launch_bounds__(256) batch_orient(const LevelJob* jobs, uint32_t n) {
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(256) batch_orient(const LevelJob* jobs, uint32
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBOrient, &g);
     if (g.bid >= g.nblk) return;
-    level_orient_run(g, j->plan, j->level, j->inv, j->edge, j->status);
+    level_orient_run(g, j->plan, j->level, j->inv, j->edge, j->control, j->status, j->status);
 }
 
 __global__ void __launch_bounds__(256, 4) batch_roots(const LevelJob* jobs, uint32_t n) {
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(256, 4) batch_roots(const LevelJob* jobs, uint
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBRoots, &g);
     if (g.bid >= g.nblk) return;
-    level_roots_run(g, j->plan, j->level, j->edge, j->xbits, j->control + kCtlClaimRoots, j->status);
+    level_roots_run(g, j->plan, j->level, j->edge, j->xbits, j->control, j->status);
 }
 
 __global__ void __launch_bounds__(256) batch_outputs(const LevelJob* jobs, uint32_t n) {

@@ -35,14 +35,17 @@ __device__ __forceinline__ void wait_for_previous() {
 
 // Device status word bits (read by the host after each call).
 constexpr uint32_t kErrNotPermutation = 1u;  // value out of range or duplicated
-constexpr uint32_t kErrIterationCap = 2u;    // a bounded retry loop gave up
+constexpr uint32_t kErrIterationCap = 2u;    // a bounded loop ran out (no input reaches it)
 constexpr uint32_t kErrInconsistent = 4u;    // colouring constraint violated
 constexpr uint32_t kErrGaveUp = 8u;          // a walk ran too long: encode again with union-find
 
-// Bound of every walk along a union-find chain.  Parents strictly decrease
-// along a chain, so the walks end anyway; the bound only caps the cost of a
-// pathological one.
-constexpr uint32_t kChainCap = 1u << 20;
+// Longest walk along a union-find chain.  Uniform inputs and single cycles
+// stay below 45 steps (2^26 entries), but inputs that keep neighbours
+// together can hang every pair-node under its predecessor, a chain as long
+// as the node.  A walk that gets this far stops and gives its level up
+// (give_up, kernels.cuh): level_settle (settle.cuh) then shortens every chain
+// and finishes the unions.
+constexpr uint32_t kLongChain = 256;
 
 // ------------------------------------------------------------------------
 // Parity union-find over pair-nodes.
@@ -56,7 +59,8 @@ constexpr uint32_t kChainCap = 1u << 20;
 // write nothing but links and the resolving pass nothing but each node's own
 // root: compressing paths on the way costs more than the shorter paths save,
 // because the words near the roots then move between the two L2 halves all
-// the time.
+// the time.  Chains that are long all the same are compressed afterwards
+// (settle.cuh).
 // ------------------------------------------------------------------------
 
 struct Found {
@@ -64,33 +68,15 @@ struct Found {
     uint32_t bit;
 };
 
-// A walk that has come kLongChain steps (random inputs: none does) halves
-// the rest of its path after all: x, whose word is w, goes to its
-// grandparent; both are true facts, so the racy store can only write a true
-// one.  Returns the word that leads from x to where the walk goes on.
-constexpr uint32_t kLongChain = 128;
-__device__ __forceinline__ uint32_t uf_halve(uint32_t* uf, uint32_t x, uint32_t w) {
-    const uint32_t up = *(volatile uint32_t*)(uf + (w >> 1));
-    if ((up >> 1) == (w >> 1)) {
-        return w; // the parent is a root
-    }
-    const uint32_t over = (up & ~1u) | ((w ^ up) & 1u);
-    uf[x] = over;
-    return over;
-}
-
 // K finds advanced in lockstep, K loads in flight; bits of `pending` name
-// the finds to run.
+// the finds to run.  Returns the finds that met a long chain: their `out` is
+// an ancestor, not the root.
 template <int K>
-__device__ __forceinline__ void uf_find_many(uint32_t* uf, const uint32_t (&x)[K],
-    Found (&out)[K], uint32_t pending, uint32_t* err) {
+__device__ __forceinline__ uint32_t uf_find_many(const uint32_t* uf, const uint32_t (&x)[K],
+    Found (&out)[K], uint32_t pending) {
 #pragma unroll
     for (int i = 0; i < K; ++i) out[i] = {x[i], 0u};
-    for (uint32_t it = 0; pending != 0; ++it) {
-        if (it == kChainCap) {
-            atomicOr(err, kErrIterationCap);
-            return;
-        }
+    for (uint32_t it = 0; pending != 0 && it < kLongChain; ++it) {
         uint32_t w[K];
 #pragma unroll
         for (int i = 0; i < K; ++i) {
@@ -102,20 +88,12 @@ __device__ __forceinline__ void uf_find_many(uint32_t* uf, const uint32_t (&x)[K
             if ((w[i] >> 1) == out[i].root) {
                 pending &= ~(1u << i);
             } else {
-                const uint32_t over = it < kLongChain ? w[i] : uf_halve(uf, out[i].root, w[i]);
-                out[i].bit ^= over & 1u;
-                out[i].root = over >> 1;
+                out[i].bit ^= w[i] & 1u;
+                out[i].root = w[i] >> 1;
             }
         }
     }
-}
-
-// Root of x and their colour difference.
-__device__ __forceinline__ Found uf_find(uint32_t* uf, uint32_t x, uint32_t* err) {
-    const uint32_t from[1] = {x};
-    Found out[1];
-    uf_find_many<1>(uf, from, out, 1u, err);
-    return out[0];
+    return pending;
 }
 
 // K unions x(a[i]) ^ x(b[i]) == rel[i] in lockstep.  Only the larger of the
@@ -124,7 +102,8 @@ __device__ __forceinline__ Found uf_find(uint32_t* uf, uint32_t x, uint32_t* err
 // (it lies in another component: a root is the smallest node of its own).
 // Two thirds of a random graph's unions find their larger end still alone
 // and touch one word (finding both roots, with path halving, took 251 ms per
-// compress at 2^30 entries, this 162 ms).
+// compress at 2^30 entries, this 162 ms).  Returns the unions that met a long
+// chain and are not done.
 //
 // A plain load may return an older word, which still names a true ancestor
 // with its true parity; the link is a compare-and-swap on a root, and a
@@ -132,8 +111,8 @@ __device__ __forceinline__ Found uf_find(uint32_t* uf, uint32_t x, uint32_t* err
 // compare-and-swap that expects a root, so that words are only touched by
 // atomics, faster while a node's words fit L2 (see level_union).
 template <int K, bool kSwap>
-__device__ __forceinline__ void uf_unite_many(uint32_t* uf, uint32_t (&a)[K], uint32_t (&b)[K],
-    uint32_t (&rel)[K], uint32_t pending, uint32_t* err) {
+__device__ __forceinline__ uint32_t uf_unite_many(uint32_t* uf, uint32_t (&a)[K],
+    uint32_t (&b)[K], uint32_t (&rel)[K], uint32_t pending, uint32_t* err) {
     uint32_t w[K];
     auto look = [&](int i) {
         if (kSwap) {
@@ -157,11 +136,7 @@ __device__ __forceinline__ void uf_unite_many(uint32_t* uf, uint32_t (&a)[K], ui
         if (pending & (1u << i)) settle(i);
         if (pending & (1u << i)) look(i);
     }
-    for (uint32_t it = 0; pending != 0; ++it) {
-        if (it == kChainCap) {
-            atomicOr(err, kErrIterationCap);
-            return;
-        }
+    for (uint32_t it = 0; pending != 0 && it < kLongChain; ++it) {
 #pragma unroll
         for (int i = 0; i < K; ++i) {
             if (!(pending & (1u << i))) continue;
@@ -170,14 +145,14 @@ __device__ __forceinline__ void uf_unite_many(uint32_t* uf, uint32_t (&a)[K], ui
                 w[i] = atomicCAS(uf + up, up << 1, (b[i] << 1) | rel[i]);
                 if (w[i] == up << 1) pending &= ~(1u << i);
             } else {
-                const uint32_t over = it < kLongChain ? w[i] : uf_halve(uf, a[i], w[i]);
-                rel[i] ^= over & 1u;
-                a[i] = over >> 1;
+                rel[i] ^= w[i] & 1u;
+                a[i] = up;
                 settle(i);
                 if (pending & (1u << i)) look(i);
             }
         }
     }
+    return pending;
 }
 
 // Blocks take chunks of `chunk` consecutive items in increasing order from

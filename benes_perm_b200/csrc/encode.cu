@@ -14,6 +14,7 @@
 #include "kernels.cuh"
 #include "layout.hpp"
 #include "plan.hpp"
+#include "settle.cuh"
 #include "tile.cuh"
 #include "walk.cuh"
 
@@ -290,23 +291,35 @@ __global__ void __launch_bounds__(256) prologue(const __grid_constant__ Prologue
     level_descriptors_run(launch_grid(), &p.plan, in_addr, out_addr);
 }
 
-// Launches the next kernel of an encode's sequence: with programmatic stream
-// serialisation, so its launch and the start of its blocks overlap the end
-// of the kernel ahead, on which it waits itself (wait_for_previous).
+// Launches a kernel with one launch attribute set.
 template <typename... Params, typename... Args>
-void launch_next(void (*kernel)(Params...), uint64_t blocks, uint32_t threads, uint32_t smem,
-    cudaStream_t st, Args&&... args) {
+void launch_with(cudaLaunchAttributeID id, void (*kernel)(Params...), uint64_t blocks,
+    uint32_t threads, uint32_t smem, cudaStream_t st, Args&&... args) {
     cudaLaunchConfig_t config{};
     config.gridDim = dim3((unsigned)blocks);
     config.blockDim = dim3(threads);
     config.dynamicSmemBytes = smem;
     config.stream = st;
     cudaLaunchAttribute attribute{};
-    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attribute.val.programmaticStreamSerializationAllowed = 1;
+    attribute.id = id;
+    if (id == cudaLaunchAttributeCooperative) {
+        attribute.val.cooperative = 1;
+    } else {
+        attribute.val.programmaticStreamSerializationAllowed = 1;
+    }
     config.attrs = &attribute;
     config.numAttrs = 1;
     check(cudaLaunchKernelEx(&config, kernel, Params(args)...), "kernel launch");
+}
+
+// Launches the next kernel of an encode's sequence: with programmatic stream
+// serialisation, so its launch and the start of its blocks overlap the end
+// of the kernel ahead, on which it waits itself (wait_for_previous).
+template <typename... Params, typename... Args>
+void launch_next(void (*kernel)(Params...), uint64_t blocks, uint32_t threads, uint32_t smem,
+    cudaStream_t st, Args&&... args) {
+    launch_with(cudaLaunchAttributeProgrammaticStreamSerialization, kernel, blocks, threads, smem,
+        st, args...);
 }
 
 // ------------------------------------------------------------ tile sizing
@@ -771,26 +784,28 @@ void run_level(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p, cons
             check(cudaMemsetAsync(w.cursor, 0, kUnionWindows * 4, st), "cudaMemsetAsync(cursors)");
             rec.launch(kKindUnion, [&] {
                 launch_next(union_bucket, grid_for(prs / kUnionBucketItems, kLevelThreads),
-                    kLevelThreads, 0, st, dp, l, inv, w.edge, w.records, w.cursor, w.slot_cap,
+                    kLevelThreads, 0, st, dp, l, inv, w.edge, w.records, w.cursor, w.slot_cap, ctl,
                     w.d_status);
                 for (uint32_t v = high + 1; v-- > low;) {
                     launch_next(union_window, device_sms() * 6, kLevelThreads, 0, st, v, w.edge,
-                        w.records, w.cursor, w.slot_cap, w.d_status);
+                        w.records, w.cursor, w.slot_cap, ctl, w.d_status);
                 }
             }, 2 + high - low);
         }
         if (!by_windows) rec.launch(kKindUnion, [&] {
             launch_next(level_union, grid_for((prs + kUnionItems - 1) / kUnionItems, kLevelThreads),
-                kLevelThreads, 0, st, dp, l, inv, w.edge, ctl + kCtlClaimUnion, w.d_status);
+                kLevelThreads, 0, st, dp, l, inv, w.edge, ctl, w.d_status);
         });
         rec.launch(kKindOrient, [&] {
             launch_next(level_orient, grid_for(nodes, kLevelThreads), kLevelThreads, 0, st, dp, l, inv,
-                w.edge, w.d_status);
+                w.edge, ctl, w.d_status);
         });
         rec.launch(kKindResolve, [&] {
             launch_next(level_roots, grid_for((prs + kResolveItems - 1) / kResolveItems, kLevelThreads),
-                kLevelThreads, 0, st, dp, l, w.edge, w.xbits, ctl + kCtlClaimRoots, w.d_status);
-        });
+                kLevelThreads, 0, st, dp, l, w.edge, w.xbits, ctl);
+            launch_with(cudaLaunchAttributeCooperative, level_settle, device_sms(), kSettleThreads,
+                0, st, dp, l, inv, w.edge, w.xbits, ctl, w.d_status);
+        }, 2);
     }
     rec.launch(kKindOutputBits, [&] {
         // the colours are all in xbits: the child level's edges or union-find

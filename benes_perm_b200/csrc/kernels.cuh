@@ -78,10 +78,25 @@ static_assert(kResolveItems == 1 || kResolveItems == 2 || kResolveItems == 4 ||
 enum : int {
     kCtlClaimInverse = 0, // level_inverse
     kCtlClaimPlace = 1,   // level_place
+    kCtlChains = 2,       // kErrGaveUp: a union-find walk met a long chain (give_up)
     kCtlClaimUnion = 3,   // level_union
     kCtlClaimRoots = 4,   // level_roots
+    kCtlArrived = 5,      // level_settle: blocks at its barriers
+    kCtlChanged = 6,      // level_settle: two words, last pass with work left
     kCtlWords = 8
 };
+
+// Gives a union-find level up: kErrGaveUp in *chains, which is the level's
+// kCtlChains word or, in a batched launch, the permutation's status word;
+// level_union and level_roots get no more work from the level's counters.
+__device__ __forceinline__ void give_up(uint32_t* ctl, uint32_t* chains) {
+    atomicOr(chains, kErrGaveUp);
+    atomicOr(ctl + kCtlClaimUnion, 0x80000000u);
+    atomicOr(ctl + kCtlClaimRoots, 0x80000000u);
+}
+__device__ __forceinline__ bool given_up(const uint32_t* chains) {
+    return (*(const volatile uint32_t*)chains & kErrGaveUp) != 0;
+}
 
 struct TileShape {
     uint32_t slots;   // padded entry slots needed at the deepest level
@@ -318,75 +333,79 @@ __global__ void __launch_bounds__(256) level_place(const Plan* __restrict__ plan
     level_place_run(launch_grid(), plan, level, records, cursor, inv, claims);
 }
 
+// Unions of output pairs [p0, p0 + kUnionItems) below `end`; returns whether
+// one met a long chain.  `swap`: see uf_unite_many.
+__device__ __forceinline__ bool unite_outputs(const LevelInfo& lv, uint32_t level,
+    const uint32_t* __restrict__ inv, uint32_t* uf, uint64_t p0, uint64_t end, bool swap,
+    uint32_t* status) {
+    const uint32_t pcap = (uint32_t)lv.pcap;
+    uint32_t j = (uint32_t)(p0 / pcap);
+    uint32_t k = (uint32_t)(p0 - (uint64_t)j * pcap);
+    uint32_t s = size_at(lv, level, j);
+    uint32_t a[kUnionItems], b[kUnionItems], rel[kUnionItems];
+    uint32_t u[kUnionItems], w[kUnionItems], base[kUnionItems];
+    uint32_t pending = 0;
+#pragma unroll
+    for (int q = 0; q < kUnionItems; ++q) {
+        if (p0 + q < end && k < s / 2) {
+            pending |= 1u << q;
+            const uint2 both = *reinterpret_cast<const uint2*>(inv + 2 * ((uint64_t)j * pcap + k));
+            u[q] = both.x;
+            w[q] = both.y;
+            base[q] = j * pcap;
+            rel[q] = s; // stash the node size for the range check below
+        }
+        if (++k == pcap) {
+            k = 0;
+            ++j;
+            s = size_at(lv, level, j);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < kUnionItems; ++q) {
+        if (pending & (1u << q)) {
+            if (u[q] >= rel[q] || w[q] >= rel[q]) {
+                atomicOr(status, kErrNotPermutation);
+                pending &= ~(1u << q);
+                continue;
+            }
+            a[q] = base[q] + (u[q] >> 1);
+            b[q] = base[q] + (w[q] >> 1);
+            rel[q] = 1u ^ (u[q] & 1u) ^ (w[q] & 1u);
+        }
+    }
+    pending = swap ? uf_unite_many<kUnionItems, true>(uf, a, b, rel, pending, status)
+                   : uf_unite_many<kUnionItems, false>(uf, a, b, rel, pending, status);
+    return pending != 0;
+}
+
 // Blocks claim chunks of output pairs in address order (claim_chunk), so the
 // union-find words being linked at any time belong to the few nodes those
 // chunks cover: once a node's words fit in L2 the random finds hit there.
 __device__ __forceinline__ void level_union_run(Grid grid, const Plan* __restrict__ plan,
-    uint32_t level, const uint32_t* __restrict__ inv, uint32_t* uf, uint32_t* claims,
-    uint32_t* status) {
+    uint32_t level, const uint32_t* __restrict__ inv, uint32_t* uf, uint32_t* ctl,
+    uint32_t* chains, uint32_t* status) {
     const LevelInfo& lv = plan->levels[level];
-    const uint32_t pcap = (uint32_t)lv.pcap;
     const NodeRange nr = level_nodes(*plan, level);
-    const uint64_t begin = nr.lo * pcap;
-    const uint64_t total = (uint64_t)pcap << nr.shift;
-    const uint64_t end = begin + total;
+    const uint64_t begin = nr.lo * lv.pcap;
+    const uint64_t total = lv.pcap << nr.shift;
     uint64_t first;
-    auto next = [&]() -> bool {
-        return claim_chunk(claims, (uint64_t)blockDim.x * kUnionItems, total, &first);
-    };
-    while (next()) {
+    while (claim_chunk(ctl + kCtlClaimUnion, (uint64_t)blockDim.x * kUnionItems, total, &first)) {
         const uint64_t p0 = begin + first + (uint64_t)threadIdx.x * kUnionItems;
-        if (p0 >= end) {
+        if (p0 >= begin + total) {
             continue;
         }
-        uint32_t j = (uint32_t)(p0 / pcap);
-        uint32_t k = (uint32_t)(p0 - (uint64_t)j * pcap);
-        uint32_t s = size_at(lv, level, j);
-        uint32_t a[kUnionItems], b[kUnionItems], rel[kUnionItems];
-        uint32_t u[kUnionItems], w[kUnionItems], base[kUnionItems];
-        uint32_t pending = 0;
-#pragma unroll
-        for (int q = 0; q < kUnionItems; ++q) {
-            if (p0 + q < end && k < s / 2) {
-                pending |= 1u << q;
-                const uint2 both = *reinterpret_cast<const uint2*>(inv + 2 * ((uint64_t)j * pcap + k));
-                u[q] = both.x;
-                w[q] = both.y;
-                base[q] = j * pcap;
-                rel[q] = s; // stash the node size for the range check below
-            }
-            if (++k == pcap) {
-                k = 0;
-                ++j;
-                s = size_at(lv, level, j);
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < kUnionItems; ++q) {
-            if (pending & (1u << q)) {
-                if (u[q] >= rel[q] || w[q] >= rel[q]) {
-                    atomicOr(status, kErrNotPermutation);
-                    pending &= ~(1u << q);
-                    continue;
-                }
-                a[q] = base[q] + (u[q] >> 1);
-                b[q] = base[q] + (w[q] >> 1);
-                rel[q] = 1u ^ (u[q] & 1u) ^ (w[q] & 1u);
-            }
-        }
-        if (lv.cap <= kSwapMaxNode) {
-            uf_unite_many<kUnionItems, true>(uf, a, b, rel, pending, status);
-        } else {
-            uf_unite_many<kUnionItems, false>(uf, a, b, rel, pending, status);
+        if (unite_outputs(lv, level, inv, uf, p0, begin + total, lv.cap <= kSwapMaxNode, status)) {
+            give_up(ctl, chains);
         }
     }
 }
 
 __global__ void __launch_bounds__(256, BPB200_UNION_MIN_BLOCKS) level_union(const Plan* __restrict__ plan,
-    uint32_t level, const uint32_t* __restrict__ inv, uint32_t* uf, uint32_t* claims,
+    uint32_t level, const uint32_t* __restrict__ inv, uint32_t* uf, uint32_t* ctl,
     uint32_t* status) {
     wait_for_previous();
-    level_union_run(launch_grid(), plan, level, inv, uf, claims, status);
+    level_union_run(launch_grid(), plan, level, inv, uf, ctl, ctl + kCtlChains, status);
 }
 
 // ---------------------------------------------------------------------------
@@ -449,7 +468,7 @@ __device__ __forceinline__ uint32_t union_append(uint2* __restrict__ records,
 // Finishes the unions that found no room.
 template <int K>
 __device__ __forceinline__ void union_finish(uint32_t* uf, const uint2 (&rec)[K], uint32_t left,
-    uint32_t* status) {
+    uint32_t* ctl, uint32_t* status) {
     uint32_t a[K], b[K], rel[K];
 #pragma unroll
     for (int i = 0; i < K; ++i) {
@@ -457,12 +476,14 @@ __device__ __forceinline__ void union_finish(uint32_t* uf, const uint2 (&rec)[K]
         b[i] = rec[i].y >> 1;
         rel[i] = rec[i].y & 1u;
     }
-    uf_unite_many<K, false>(uf, a, b, rel, left, status);
+    if (uf_unite_many<K, false>(uf, a, b, rel, left, status) != 0) {
+        give_up(ctl, ctl + kCtlChains);
+    }
 }
 
 __global__ void __launch_bounds__(256) union_bucket(const Plan* __restrict__ plan, uint32_t level,
     const uint32_t* __restrict__ inv, uint32_t* uf, uint2* __restrict__ records,
-    uint32_t* __restrict__ cursor, uint64_t capacity, uint32_t* status) {
+    uint32_t* __restrict__ cursor, uint64_t capacity, uint32_t* ctl, uint32_t* status) {
     wait_for_previous();
     __shared__ uint32_t count[kUnionWindows];
     __shared__ uint32_t start[kUnionWindows];
@@ -504,14 +525,31 @@ __global__ void __launch_bounds__(256) union_bucket(const Plan* __restrict__ pla
         }
         const uint32_t left = union_append<kUnionBucketItems>(records, cursor, capacity, rec,
             pending, count, start);
-        if (left != 0) union_finish<kUnionBucketItems>(uf, rec, left, status);
+        if (left != 0) union_finish<kUnionBucketItems>(uf, rec, left, ctl, status);
     }
+}
+
+// A union that has come half of kLongChain halves the rest of its path: x,
+// whose word is w, goes to its grandparent; both are true facts, so the racy
+// store can only write a true one.  Returns the word that leads from x to
+// where the walk goes on.  (Uniform inputs never get here, but the branch
+// keeps the two unions of a thread apart in the code: without it the windows
+// of 100,000,007 entries' top two levels take 3.09 ms, with it 2.90.)
+__device__ __forceinline__ uint32_t uf_halve(uint32_t* uf, uint32_t x, uint32_t w) {
+    const uint32_t up = *(volatile uint32_t*)(uf + (w >> 1));
+    if ((up >> 1) == (w >> 1)) {
+        return w; // the parent is a root
+    }
+    const uint32_t over = (up & ~1u) | ((w ^ up) & 1u);
+    uf[x] = over;
+    return over;
 }
 
 __global__ void __launch_bounds__(256, 6) union_window(uint32_t window, uint32_t* uf,
     uint2* __restrict__ records, uint32_t* __restrict__ cursor, uint64_t capacity,
-    uint32_t* status) {
+    uint32_t* ctl, uint32_t* status) {
     wait_for_previous();
+    if (__syncthreads_or(given_up(ctl + kCtlChains))) return; // mostly by a higher window
     __shared__ uint32_t count[kUnionWindows];
     __shared__ uint32_t start[kUnionWindows];
     const uint64_t base = (uint64_t)window << (kUnionWindowLog2 + 1);
@@ -545,7 +583,7 @@ __global__ void __launch_bounds__(256, 6) union_window(uint32_t window, uint32_t
                     live &= ~(1u << i);
                     continue;
                 }
-                const uint32_t over = it < kLongChain ? w[i] : uf_halve(uf, rec[i].x, w[i]);
+                const uint32_t over = it < kLongChain / 2 ? w[i] : uf_halve(uf, rec[i].x, w[i]);
                 const uint32_t up = over >> 1, b = rec[i].y >> 1;
                 const uint32_t rel = (rec[i].y ^ over) & 1u;
                 rec[i] = make_uint2(max(up, b), (min(up, b) << 1) | rel);
@@ -555,19 +593,21 @@ __global__ void __launch_bounds__(256, 6) union_window(uint32_t window, uint32_t
                 } else if (rec[i].x >> kUnionWindowLog2 != window) {
                     live &= ~(1u << i); // on to a lower window
                     pending |= 1u << i;
-                } else if (it == kChainCap) {
-                    atomicOr(status, kErrIterationCap);
+                } else if (it == kLongChain) {
+                    give_up(ctl, ctl + kCtlChains);
                     live &= ~(1u << i);
                 }
             }
         }
         const uint32_t left = union_append<K>(records, cursor, capacity, rec, pending, count, start);
-        if (left != 0) union_finish<K>(uf, rec, left, status);
+        if (left != 0) union_finish<K>(uf, rec, left, ctl, status);
     }
 }
 
 __device__ __forceinline__ void level_orient_run(Grid grid, const Plan* __restrict__ plan, uint32_t level,
-    const uint32_t* __restrict__ inv, uint32_t* uf, uint32_t* status) {
+    const uint32_t* __restrict__ inv, uint32_t* uf, uint32_t* ctl, uint32_t* chains,
+    uint32_t* status) {
+    if (given_up(chains)) return;
     const LevelInfo& lv = plan->levels[level];
     const uint32_t pcap = (uint32_t)lv.pcap;
     const NodeRange nr = level_nodes(*plan, level);
@@ -582,17 +622,20 @@ __device__ __forceinline__ void level_orient_run(Grid grid, const Plan* __restri
             atomicOr(status, kErrNotPermutation);
             continue;
         }
-        const Found f = uf_find(uf, (uint32_t)j * pcap + (s >> 1), status);
-        if (f.bit) {
-            atomicOr(uf + f.root, 1u);
+        const uint32_t x[1] = {(uint32_t)j * pcap + (s >> 1)};
+        Found f[1];
+        if (uf_find_many<1>(uf, x, f, 1u) != 0) {
+            give_up(ctl, chains);
+        } else if (f[0].bit) {
+            atomicOr(uf + f[0].root, 1u);
         }
     }
 }
 
 __global__ void level_orient(const Plan* __restrict__ plan, uint32_t level,
-    const uint32_t* __restrict__ inv, uint32_t* uf, uint32_t* status) {
+    const uint32_t* __restrict__ inv, uint32_t* uf, uint32_t* ctl, uint32_t* status) {
     wait_for_previous();
-    level_orient_run(launch_grid(), plan, level, inv, uf, status);
+    level_orient_run(launch_grid(), plan, level, inv, uf, ctl, ctl + kCtlChains, status);
 }
 
 // Switch addresses of every node of the levels above the tile's: level l's
@@ -618,8 +661,8 @@ __device__ __forceinline__ void level_descriptors_run(Grid grid, const Plan* __r
 // went, in grid-stride order on nodes up to 2^26 entries, took 58 ms per
 // compress at 2^30 entries, these 44 ms.
 __device__ __forceinline__ void level_roots_run(Grid grid, const Plan* __restrict__ plan,
-    uint32_t level, uint32_t* uf, uint32_t* __restrict__ xbits, uint32_t* claims,
-    uint32_t* status) {
+    uint32_t level, uint32_t* uf, uint32_t* __restrict__ xbits, uint32_t* ctl,
+    uint32_t* chains) {
     const LevelInfo& lv = plan->levels[level];
     const uint32_t pcap = (uint32_t)lv.pcap;
     // this call's pair-nodes [lo_pair, end); chunks start at a 32-pair
@@ -635,7 +678,7 @@ __device__ __forceinline__ void level_roots_run(Grid grid, const Plan* __restric
     // back into its word: parents are smaller than their children, so most
     // finds end at a parent that was resolved before them.
     uint64_t first;
-    while (claim_chunk(claims, chunk, total, &first)) {
+    while (claim_chunk(ctl + kCtlClaimRoots, chunk, total, &first)) {
         const uint64_t p0 = begin + first + (uint64_t)threadIdx.x * kResolveItems;
         uint32_t j = (uint32_t)(p0 / pcap);
         uint32_t k = (uint32_t)(p0 - (uint64_t)j * pcap);
@@ -653,7 +696,10 @@ __device__ __forceinline__ void level_roots_run(Grid grid, const Plan* __restric
             }
         }
         Found f[kResolveItems];
-        uf_find_many<kResolveItems>(uf, x, f, live, status);
+        if (uf_find_many<kResolveItems>(uf, x, f, live) != 0) {
+            give_up(ctl, chains);
+            live = 0;
+        }
         uint32_t mine = 0; // this lane's kResolveItems colour bits
 #pragma unroll
         for (int q = 0; q < kResolveItems; ++q) {
@@ -678,9 +724,9 @@ __device__ __forceinline__ void level_roots_run(Grid grid, const Plan* __restric
 
 __global__ void __launch_bounds__(256, BPB200_FINAL_MIN_BLOCKS) level_roots(
     const Plan* __restrict__ plan, uint32_t level, uint32_t* uf, uint32_t* __restrict__ xbits,
-    uint32_t* claims, uint32_t* status) {
+    uint32_t* ctl) {
     wait_for_previous();
-    level_roots_run(launch_grid(), plan, level, uf, xbits, claims, status);
+    level_roots_run(launch_grid(), plan, level, uf, xbits, ctl, ctl + kCtlChains);
 }
 
 // Output side of a level, in natural (node, output pair) order: the output
