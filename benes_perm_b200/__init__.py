@@ -586,6 +586,19 @@ def probe_switch_bit(count: int, fmt: FormatOptions, side: int, level: int, node
     return out.value
 
 
+def probe_scratch(count: int, fmt: Optional[FormatOptions], shard: int = 0, shards: int = 1):
+    """(levels at which a call hands its nodes over in device memory, slots its
+    level arrays hold): bpb200_probe_scratch, a test hook."""
+    cf = to_c_format(fmt)
+    levels = (ctypes.c_uint32 * 64)()
+    slots = ctypes.c_uint64(0)
+    n = library().bpb200_probe_scratch(ctypes.c_uint64(count), ctypes.byref(cf),
+                                       ctypes.c_uint32(shard), ctypes.c_uint32(shards), levels,
+                                       ctypes.c_uint32(64), ctypes.byref(slots))
+    raise_for(max(0, -n), "invalid scratch query")
+    return list(levels[:n]), slots.value
+
+
 def probe_rank_bit(count: int, fmt: FormatOptions, level: int, node: int):
     cf = to_c_format(fmt)
     sec = ctypes.c_int(0)

@@ -403,6 +403,19 @@ unsigned stage_threads(uint64_t entries) { return tile_threads(1, true, entries)
 // Whether the whole permutation is one launch of one CTA.
 bool single_launch(const Plan& p) { return p.tile_level == 0 && few_tiles_stop(p, 0) == 0; }
 
+// Slots and pair-nodes of the largest level the launches keep in device
+// memory: those down to the tile level and those that launches of few tiles
+// hand over at, which a shard, having fewer tiles, does further down.
+void size_levels(Plan& p) {
+    p.max_slots = p.max_pairs = 0;
+    auto hold = [&](uint32_t l) {
+        p.max_slots = std::max<uint64_t>(p.max_slots, (2 * p.levels[l].pcap) << l);
+        p.max_pairs = std::max<uint64_t>(p.max_pairs, p.levels[l].pcap << l);
+    };
+    for (uint32_t l = 0; l <= p.tile_level; ++l) hold(l);
+    for (uint32_t l = p.tile_level; (l = few_tiles_stop(p, l)) != 0;) hold(l);
+}
+
 // Picks the tile level: the first level whose nodes fit `tile_max` entries
 // and whose deepest padded tile level also fits the shared-memory budget.
 void choose_tile(Plan& p, TileShape* shape, uint64_t tile_max = kTileMaxEntries) {
@@ -416,16 +429,25 @@ void choose_tile(Plan& p, TileShape* shape, uint64_t tile_max = kTileMaxEntries)
         s = tile_shape(p, t0);
     }
     p.tile_level = t0;
-    uint64_t slots = 0, pairs = 0;
-    // level arrays: the global levels, the tiles' and those a launch of few
-    // tiles may be handed over at
-    for (uint32_t l = 0; l <= t0 || (l <= p.depth && l < 10); ++l) {
-        slots = std::max<uint64_t>(slots, (1ull << l) * 2 * p.levels[l].pcap);
-        pairs = std::max<uint64_t>(pairs, (1ull << l) * p.levels[l].pcap);
-    }
-    p.max_slots = slots;
-    p.max_pairs = pairs;
+    size_levels(p);
     *shape = s;
+}
+
+bool valid_shard(uint32_t shard, uint32_t shards) {
+    return shards != 0 && (shards & (shards - 1)) == 0 && shard < shards;
+}
+
+// Restricts a plan whose tile level is chosen to one shard; false when the
+// permutation is too small for that many.
+bool set_shard(Plan& p, uint32_t shard, uint32_t shards) {
+    uint32_t k = 0;
+    while ((1u << k) < shards) ++k;
+    if (!valid_shard(shard, shards) || k > p.tile_level) return false;
+    p.shards = shards;
+    p.shard = shard;
+    p.shard_level = k;
+    size_levels(p);
+    return true;
 }
 
 std::atomic<int> g_force_union_find{0};
@@ -913,6 +935,9 @@ void launch_levels(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p,
         rec.level = (int)l;
         const TileShape part = tile_shape(p, l, stop);
         const uint64_t nodes = 1ull << level_nodes(p, l).shift;
+        if ((2 * p.levels[stop].pcap) << stop > p.max_slots) { // see size_levels
+            throw CudaFail{cudaErrorInvalidValue, "level scratch"};
+        }
         const unsigned threads = stage_threads(p.levels[l].cap);
         rec.launch(kKindTile, [&] {
             if (l == 0) {
@@ -1708,7 +1733,7 @@ int bpb200_compress_device_shard(const void* d_entries, uint64_t count, uint32_t
             set_error(err, err_len, "b200 backend is unavailable");
             return kUnavailable;
         }
-        if (shards == 0 || (shards & (shards - 1)) != 0 || shard >= shards) {
+        if (!valid_shard(shard, shards)) {
             set_error(err, err_len, "shards must be a power of two and shard below it");
             return kInvalidArgument;
         }
@@ -1722,15 +1747,10 @@ int bpb200_compress_device_shard(const void* d_entries, uint64_t count, uint32_t
         if (rc != kOk) {
             return rc;
         }
-        uint32_t k = 0;
-        while ((1u << k) < shards) ++k;
-        if (k > call.plan->tile_level) {
+        if (!set_shard(*call.plan, shard, shards)) {
             set_error(err, err_len, "permutation too small for that many shards");
             return kInvalidArgument;
         }
-        call.plan->shards = shards;
-        call.plan->shard = shard;
-        call.plan->shard_level = k;
         return run(w, call, (cudaStream_t)stream, d_entries, entry_bytes, (uint32_t*)d_blob,
             device_seconds, err, err_len);
     });
@@ -1833,6 +1853,41 @@ int bpb200_probe_switch_bit(uint64_t count, const bpb200_format* format, int sid
     }
     *bit = switch_bit(node_address(*p, side, level, node), pair);
     return kOk;
+}
+
+int bpb200_probe_scratch(uint64_t count, const bpb200_format* format, uint32_t shard,
+    uint32_t shards, uint32_t* levels, uint32_t capacity, uint64_t* slots) {
+    Layout L;
+    if (!make_layout(count, to_format(format), &L).ok()) {
+        return -kInvalidArgument;
+    }
+    std::unique_ptr<Plan> p(new Plan);
+    const uint64_t tile_max = 1ull << tuning_for(count).tile_max_log2;
+    if (!make_plan(L, tile_max, p.get()).ok()) {
+        return -kInvalidArgument;
+    }
+    TileShape shape;
+    choose_tile(*p, &shape, tile_max);
+    if (!set_shard(*p, shard, shards)) {
+        return -kInvalidArgument;
+    }
+    // as launch_levels
+    uint32_t n = 0;
+    auto reach = [&](uint32_t l) {
+        if (n < capacity) levels[n] = l;
+        ++n;
+        return l;
+    };
+    uint32_t l = 0;
+    while (l < p->tile_level) {
+        const uint32_t stop = stage_stop(*p, l, p->tile_level);
+        l = reach(stop != 0 ? stop : l + 1);
+    }
+    while (const uint32_t stop = few_tiles_stop(*p, l)) {
+        l = reach(stop);
+    }
+    *slots = p->max_slots;
+    return n <= capacity ? (int)n : -kLength;
 }
 
 int bpb200_probe_rank_bit(uint64_t count, const bpb200_format* format, uint32_t level,

@@ -82,8 +82,8 @@ struct Plan {
     uint64_t end_offset;
     uint64_t switch_bits;
     uint64_t middle_bits;
-    uint64_t max_slots;         // max over levels of 2^l * 2 * pcap_l
-    uint64_t max_pairs;         // max over levels of 2^l * pcap_l
+    uint64_t max_slots;         // max over the levels kept in memory of 2^l * 2 * pcap_l
+    uint64_t max_pairs;         // max over the levels kept in memory of 2^l * pcap_l
     uint32_t fact_bits[33];     // ceil(log2(c!)) for c = 0..32
     uint32_t digit_reciprocal[33]; // ceil(2^32 / r) for r = 2..32
     DigitGroup digit_groups[33];   // from radix i down, i = 1..32

@@ -268,6 +268,14 @@ int bpb200_probe_switch_bit(uint64_t count, const bpb200_format* format, int sid
 int bpb200_probe_rank_bit(uint64_t count, const bpb200_format* format, uint32_t level,
     uint64_t node, int* section, uint64_t* bit);
 
+/* Scratch probe (test hook, no device work): the levels at which one call (or
+ * one of `shards` shards of it; 0 of 1: the whole permutation) hands its
+ * nodes over in device memory, in order, and the slots its level arrays
+ * hold.  Returns the number of levels (at most `capacity`), or an error as a
+ * negative of the status code. */
+int bpb200_probe_scratch(uint64_t count, const bpb200_format* format, uint32_t shard,
+    uint32_t shards, uint32_t* levels, uint32_t capacity, uint64_t* slots);
+
 /* Batch lookup verifier: a read-only device twin of the reference's lookup
  * (src/internal.hpp:1035-1124, behind CompressedPermutationView::forward /
  * inverse), for checking every entry of blobs too large to re-encode on the
