@@ -38,6 +38,14 @@ constexpr uint32_t kErrNotPermutation = 1u;  // value out of range or duplicated
 constexpr uint32_t kErrIterationCap = 2u;    // a bounded loop ran out (no input reaches it)
 constexpr uint32_t kErrInconsistent = 4u;    // colouring constraint violated
 constexpr uint32_t kErrGaveUp = 8u;          // a walk ran too long: encode again with union-find
+constexpr uint32_t kErrBelow = 16u;          // a node below level 0 is not a permutation
+
+// What a node of `level` that is not a permutation says.  Level 0 checks
+// every value of the input, so its finding is final; below it, the cause may
+// also be a walk that gave up.
+__device__ __forceinline__ uint32_t not_permutation(uint32_t level) {
+    return level == 0 ? kErrNotPermutation : kErrBelow;
+}
 
 // Longest walk along a union-find chain.  Uniform inputs and single cycles
 // stay below 45 steps (2^26 entries), but inputs that keep neighbours

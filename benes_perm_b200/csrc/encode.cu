@@ -1103,9 +1103,15 @@ thread_local std::vector<Recorder::Mark> t_marks;
 thread_local std::vector<double> t_mark_seconds;
 std::atomic<int> g_profiling{0};
 
+// Whether a permutation has to be encoded again with union-find: a walk gave
+// up, and not because the input is no permutation.
+bool gave_up(uint32_t status) {
+    return (status & kErrGaveUp) != 0 && (status & kErrNotPermutation) == 0;
+}
+
 // Return code of a finished encode's status word.
 int status_code(uint32_t status, char* err, size_t err_len) {
-    if (status & kErrNotPermutation) {
+    if (status & (kErrNotPermutation | kErrBelow)) {
         set_error(err, err_len, "input must contain every value from zero through size minus one");
         return kInvalidArgument;
     }
@@ -1149,8 +1155,7 @@ int run(Workspace& w, Call& call, cudaStream_t st, const void* d_in, uint32_t en
         check(cudaEventRecord(w.stop, st), "cudaEventRecord");
         check(cudaStreamSynchronize(st), "cudaStreamSynchronize");
         status = *w.h_status;
-        if (union_find_only || p.tile_level == 0 ||
-            ((status & kErrGaveUp) == 0 && colouring != 2)) {
+        if (union_find_only || p.tile_level == 0 || (!gave_up(status) && colouring != 2)) {
             break;
         }
         union_find_only = true;
@@ -2055,8 +2060,7 @@ extern "C" int bpb200_compress_device_noalloc(const void* d_entries, uint64_t co
             }
             check(cudaMemcpyAsync(&status, status_out, 4, cudaMemcpyDeviceToHost, st), "status");
             check(cudaStreamSynchronize(st), "cudaStreamSynchronize");
-            if (union_find_only || p.tile_level == 0 ||
-                ((status & kErrGaveUp) == 0 && colouring != 2)) {
+            if (union_find_only || p.tile_level == 0 || (!gave_up(status) && colouring != 2)) {
                 break;
             }
             union_find_only = true;

@@ -365,7 +365,7 @@ __device__ __forceinline__ bool unite_outputs(const LevelInfo& lv, uint32_t leve
     for (int q = 0; q < kUnionItems; ++q) {
         if (pending & (1u << q)) {
             if (u[q] >= rel[q] || w[q] >= rel[q]) {
-                atomicOr(status, kErrNotPermutation);
+                atomicOr(status, not_permutation(level));
                 pending &= ~(1u << q);
                 continue;
             }
@@ -511,7 +511,7 @@ __global__ void __launch_bounds__(256) union_bucket(const Plan* __restrict__ pla
             if (k >= s / 2) continue;
             const uint32_t u = both[i].x, w = both[i].y;
             if (u >= s || w >= s) {
-                atomicOr(status, kErrNotPermutation);
+                atomicOr(status, not_permutation(level));
                 continue;
             }
             const uint32_t a = j * ps + (u >> 1), b = j * ps + (w >> 1);
@@ -619,7 +619,7 @@ __device__ __forceinline__ void level_orient_run(Grid grid, const Plan* __restri
             continue;
         }
         if (inv[2 * j * pcap + s - 1] >= s) {
-            atomicOr(status, kErrNotPermutation);
+            atomicOr(status, not_permutation(level));
             continue;
         }
         const uint32_t x[1] = {(uint32_t)j * pcap + (s >> 1)};

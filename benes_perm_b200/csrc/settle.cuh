@@ -171,6 +171,7 @@ __global__ void __launch_bounds__(kSettleThreads, 1) level_settle(const Plan* __
     for (uint64_t j = nr.lo + id; j < nr.lo + (1ull << nr.shift); j += stride) {
         const uint32_t s = size_at(lv, level, (uint32_t)j);
         if ((s & 1u) == 0) continue;
+        if (inv[2 * j * ps + s - 1] >= s) atomicOr(status, not_permutation(level));
         const uint32_t x = (uint32_t)j * ps + (s >> 1);
         const uint32_t w = __ldcg(uf + x);
         if ((w >> 1) != x && (w & 1u) != 0) atomicOr(uf + (w >> 1), 1u);

@@ -276,7 +276,7 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
             }
         }
         if (__syncthreads_or(bad)) {
-            if (tid == 0) atomicOr(status, kErrNotPermutation);
+            if (tid == 0) atomicOr(status, not_permutation(T0));
             return;
         }
     }
@@ -586,7 +586,7 @@ __device__ __forceinline__ void tile_body(const Plan* __restrict__ plan_ptr,
                     thread_emit_rank(blob, plan.section_offset[section] * 8 + bit,
                         plan.fact_bits[s], rank);
                 } else {
-                    atomicOr(status, kErrNotPermutation);
+                    atomicOr(status, not_permutation(T0));
                 }
             }
             continue;
