@@ -117,6 +117,12 @@ __device__ __forceinline__ const LevelJob* level_job(const LevelJob* jobs, uint3
     return j;
 }
 
+// A member that meets a long chain gives up as a whole: the host encodes it
+// again by itself.
+__device__ __forceinline__ Chains batch_chains(const LevelJob* j) {
+    return Chains{j->control, j->status, nullptr, 0};
+}
+
 __global__ void __launch_bounds__(256) batch_fill(const FillJob* jobs, uint32_t n) {
     wait_for_previous();
     Grid g;
@@ -217,7 +223,7 @@ __global__ void __launch_bounds__(256, BPB200_UNION_MIN_BLOCKS) batch_union(cons
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBUnion, &g);
     if (g.bid >= g.nblk) return;
-    level_union_run(g, j->plan, j->level, j->inv, j->edge, j->control, j->status, j->status);
+    level_union_run(g, j->plan, j->level, j->inv, j->edge, batch_chains(j), j->status);
 }
 
 __global__ void __launch_bounds__(256) batch_orient(const LevelJob* jobs, uint32_t n) {
@@ -225,7 +231,7 @@ __global__ void __launch_bounds__(256) batch_orient(const LevelJob* jobs, uint32
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBOrient, &g);
     if (g.bid >= g.nblk) return;
-    level_orient_run(g, j->plan, j->level, j->inv, j->edge, j->control, j->status, j->status);
+    level_orient_run(g, j->plan, j->level, j->inv, j->edge, batch_chains(j), j->status);
 }
 
 __global__ void __launch_bounds__(256, 4) batch_roots(const LevelJob* jobs, uint32_t n) {
@@ -233,7 +239,7 @@ __global__ void __launch_bounds__(256, 4) batch_roots(const LevelJob* jobs, uint
     Grid g;
     const LevelJob* j = level_job(jobs, n, kBRoots, &g);
     if (g.bid >= g.nblk) return;
-    level_roots_run(g, j->plan, j->level, j->edge, j->xbits, j->control, j->status);
+    level_roots_run(g, j->plan, j->level, j->edge, j->xbits, batch_chains(j));
 }
 
 __global__ void __launch_bounds__(256) batch_outputs(const LevelJob* jobs, uint32_t n) {

@@ -51,8 +51,8 @@ __device__ __forceinline__ uint32_t not_permutation(uint32_t level) {
 // stay below 45 steps (2^26 entries), but inputs that keep neighbours
 // together can hang every pair-node under its predecessor, a chain as long
 // as the node.  A walk that gets this far stops and gives its level up
-// (give_up, kernels.cuh): level_settle (settle.cuh) then shortens every chain
-// and finishes the unions.
+// (give_up, defer; kernels.cuh): level_settle (settle.cuh) then shortens
+// every chain and finishes the unions.
 constexpr uint32_t kLongChain = 256;
 
 // ------------------------------------------------------------------------
@@ -111,7 +111,7 @@ __device__ __forceinline__ uint32_t uf_find_many(const uint32_t* uf, const uint3
 // Two thirds of a random graph's unions find their larger end still alone
 // and touch one word (finding both roots, with path halving, took 251 ms per
 // compress at 2^30 entries, this 162 ms).  Returns the unions that met a long
-// chain and are not done.
+// chain and are not done: a, b and rel are as far as they came.
 //
 // A plain load may return an older word, which still names a true ancestor
 // with its true parity; the link is a compare-and-swap on a root, and a

@@ -728,6 +728,7 @@ void run_level(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p, cons
     const uint64_t nodes = 1ull << nr.shift;
     const int gp = grid_for(prs, kLevelThreads);
     uint32_t* ctl = w.control + l * kCtlWords;
+    const Chains chains = level_chains(ctl, w.ybits, (uint32_t)(prs / 64));
     const bool walks = walk_level(lv, tune, union_find_only);
     if (l == 0 && lv.cap > kWalkMaxNode && w.records != nullptr) {
         const uint64_t slots = lv.cap;
@@ -806,27 +807,27 @@ void run_level(Workspace& w, Recorder& rec, cudaStream_t st, const Plan& p, cons
             check(cudaMemsetAsync(w.cursor, 0, kUnionWindows * 4, st), "cudaMemsetAsync(cursors)");
             rec.launch(kKindUnion, [&] {
                 launch_next(union_bucket, grid_for(prs / kUnionBucketItems, kLevelThreads),
-                    kLevelThreads, 0, st, dp, l, inv, w.edge, w.records, w.cursor, w.slot_cap, ctl,
+                    kLevelThreads, 0, st, dp, l, inv, w.edge, w.records, w.cursor, w.slot_cap, chains,
                     w.d_status);
                 for (uint32_t v = high + 1; v-- > low;) {
                     launch_next(union_window, device_sms() * 6, kLevelThreads, 0, st, v, w.edge,
-                        w.records, w.cursor, w.slot_cap, ctl, w.d_status);
+                        w.records, w.cursor, w.slot_cap, chains, w.d_status);
                 }
             }, 2 + high - low);
         }
         if (!by_windows) rec.launch(kKindUnion, [&] {
             launch_next(level_union, grid_for((prs + kUnionItems - 1) / kUnionItems, kLevelThreads),
-                kLevelThreads, 0, st, dp, l, inv, w.edge, ctl, w.d_status);
+                kLevelThreads, 0, st, dp, l, inv, w.edge, chains, w.d_status);
         });
         rec.launch(kKindOrient, [&] {
             launch_next(level_orient, grid_for(nodes, kLevelThreads), kLevelThreads, 0, st, dp, l, inv,
-                w.edge, ctl, w.d_status);
+                w.edge, chains, w.d_status);
         });
         rec.launch(kKindResolve, [&] {
             launch_next(level_roots, grid_for((prs + kResolveItems - 1) / kResolveItems, kLevelThreads),
-                kLevelThreads, 0, st, dp, l, w.edge, w.xbits, ctl);
+                kLevelThreads, 0, st, dp, l, w.edge, w.xbits, chains);
             launch_with(cudaLaunchAttributeCooperative, level_settle, device_sms(), kSettleThreads,
-                0, st, dp, l, inv, w.edge, w.xbits, ctl, w.d_status);
+                0, st, dp, l, inv, w.edge, w.xbits, chains, w.d_status);
         }, 2);
     }
     rec.launch(kKindOutputBits, [&] {

@@ -83,19 +83,46 @@ enum : int {
     kCtlClaimRoots = 4,   // level_roots
     kCtlArrived = 5,      // level_settle: blocks at its barriers
     kCtlChanged = 6,      // level_settle: two words, last pass with work left
-    kCtlWords = 8
+    kCtlDeferred = 8,     // unions put off
+    kCtlWords = 12
 };
 
-// Gives a union-find level up: kErrGaveUp in *chains, which is the level's
-// kCtlChains word or, in a batched launch, the permutation's status word;
-// level_union and level_roots get no more work from the level's counters.
-__device__ __forceinline__ void give_up(uint32_t* ctl, uint32_t* chains) {
-    atomicOr(chains, kErrGaveUp);
-    atomicOr(ctl + kCtlClaimUnion, 0x80000000u);
-    atomicOr(ctl + kCtlClaimRoots, 0x80000000u);
+// What a union-find level's kernels share about its long chains: the level's
+// control words, the word that says it is given up (kErrGaveUp in its
+// kCtlChains word or, in a batched launch, in the permutation's status word)
+// and the list of unions put off (in the memory of the output switch bits,
+// which are written later; no list in a batched launch).
+struct Chains {
+    uint32_t* ctl;
+    uint32_t* flag;
+    uint2* list;
+    uint32_t room;
+};
+constexpr uint32_t kStopClaims = 0x80000000u;
+__host__ __device__ __forceinline__ Chains level_chains(uint32_t* ctl, uint32_t* ybits,
+    uint32_t room) {
+    return Chains{ctl, ctl + kCtlChains, reinterpret_cast<uint2*>(ybits), room};
 }
-__device__ __forceinline__ bool given_up(const uint32_t* chains) {
-    return (*(const volatile uint32_t*)chains & kErrGaveUp) != 0;
+
+// Gives a union-find level up: its roots are left to level_settle.
+__device__ __forceinline__ void give_up(const Chains& c) {
+    atomicOr(c.flag, kErrGaveUp);
+    atomicOr(c.ctl + kCtlClaimRoots, kStopClaims);
+}
+__device__ __forceinline__ bool given_up(const Chains& c) {
+    return (*(volatile uint32_t*)c.flag & kErrGaveUp) != 0;
+}
+
+// Gives the level up and puts a union off.  Once the list is full the others
+// stop too: level_settle then does all of them again.
+__device__ __forceinline__ void defer(const Chains& c, uint2 rec) {
+    give_up(c);
+    const uint32_t at = c.list != nullptr ? atomicAdd(c.ctl + kCtlDeferred, 1u) : 0u;
+    if (at < c.room) {
+        c.list[at] = rec;
+    } else {
+        atomicOr(c.ctl + kCtlClaimUnion, kStopClaims);
+    }
 }
 
 struct TileShape {
@@ -334,10 +361,11 @@ __global__ void __launch_bounds__(256) level_place(const Plan* __restrict__ plan
 }
 
 // Unions of output pairs [p0, p0 + kUnionItems) below `end`; returns whether
-// one met a long chain.  `swap`: see uf_unite_many.
+// one met a long chain and puts those off (with `chains`).  `swap`: see
+// uf_unite_many.
 __device__ __forceinline__ bool unite_outputs(const LevelInfo& lv, uint32_t level,
     const uint32_t* __restrict__ inv, uint32_t* uf, uint64_t p0, uint64_t end, bool swap,
-    uint32_t* status) {
+    const Chains* chains, uint32_t* status) {
     const uint32_t pcap = (uint32_t)lv.pcap;
     uint32_t j = (uint32_t)(p0 / pcap);
     uint32_t k = (uint32_t)(p0 - (uint64_t)j * pcap);
@@ -376,6 +404,12 @@ __device__ __forceinline__ bool unite_outputs(const LevelInfo& lv, uint32_t leve
     }
     pending = swap ? uf_unite_many<kUnionItems, true>(uf, a, b, rel, pending, status)
                    : uf_unite_many<kUnionItems, false>(uf, a, b, rel, pending, status);
+    if (chains != nullptr) {
+#pragma unroll
+        for (int q = 0; q < kUnionItems; ++q) {
+            if (pending & (1u << q)) defer(*chains, make_uint2(a[q], (b[q] << 1) | rel[q]));
+        }
+    }
     return pending != 0;
 }
 
@@ -383,29 +417,29 @@ __device__ __forceinline__ bool unite_outputs(const LevelInfo& lv, uint32_t leve
 // union-find words being linked at any time belong to the few nodes those
 // chunks cover: once a node's words fit in L2 the random finds hit there.
 __device__ __forceinline__ void level_union_run(Grid grid, const Plan* __restrict__ plan,
-    uint32_t level, const uint32_t* __restrict__ inv, uint32_t* uf, uint32_t* ctl,
-    uint32_t* chains, uint32_t* status) {
+    uint32_t level, const uint32_t* __restrict__ inv, uint32_t* uf, const Chains& chains,
+    uint32_t* status) {
     const LevelInfo& lv = plan->levels[level];
     const NodeRange nr = level_nodes(*plan, level);
     const uint64_t begin = nr.lo * lv.pcap;
     const uint64_t total = lv.pcap << nr.shift;
     uint64_t first;
-    while (claim_chunk(ctl + kCtlClaimUnion, (uint64_t)blockDim.x * kUnionItems, total, &first)) {
+    while (claim_chunk(chains.ctl + kCtlClaimUnion, (uint64_t)blockDim.x * kUnionItems, total,
+        &first)) {
         const uint64_t p0 = begin + first + (uint64_t)threadIdx.x * kUnionItems;
         if (p0 >= begin + total) {
             continue;
         }
-        if (unite_outputs(lv, level, inv, uf, p0, begin + total, lv.cap <= kSwapMaxNode, status)) {
-            give_up(ctl, chains);
-        }
+        unite_outputs(lv, level, inv, uf, p0, begin + total, lv.cap <= kSwapMaxNode, &chains,
+            status);
     }
 }
 
 __global__ void __launch_bounds__(256, BPB200_UNION_MIN_BLOCKS) level_union(const Plan* __restrict__ plan,
-    uint32_t level, const uint32_t* __restrict__ inv, uint32_t* uf, uint32_t* ctl,
+    uint32_t level, const uint32_t* __restrict__ inv, uint32_t* uf, const __grid_constant__ Chains chains,
     uint32_t* status) {
     wait_for_previous();
-    level_union_run(launch_grid(), plan, level, inv, uf, ctl, ctl + kCtlChains, status);
+    level_union_run(launch_grid(), plan, level, inv, uf, chains, status);
 }
 
 // ---------------------------------------------------------------------------
@@ -468,7 +502,7 @@ __device__ __forceinline__ uint32_t union_append(uint2* __restrict__ records,
 // Finishes the unions that found no room.
 template <int K>
 __device__ __forceinline__ void union_finish(uint32_t* uf, const uint2 (&rec)[K], uint32_t left,
-    uint32_t* ctl, uint32_t* status) {
+    const Chains& chains, uint32_t* status) {
     uint32_t a[K], b[K], rel[K];
 #pragma unroll
     for (int i = 0; i < K; ++i) {
@@ -476,14 +510,16 @@ __device__ __forceinline__ void union_finish(uint32_t* uf, const uint2 (&rec)[K]
         b[i] = rec[i].y >> 1;
         rel[i] = rec[i].y & 1u;
     }
-    if (uf_unite_many<K, false>(uf, a, b, rel, left, status) != 0) {
-        give_up(ctl, ctl + kCtlChains);
+    left = uf_unite_many<K, false>(uf, a, b, rel, left, status);
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+        if (left & (1u << i)) defer(chains, make_uint2(a[i], (b[i] << 1) | rel[i]));
     }
 }
 
 __global__ void __launch_bounds__(256) union_bucket(const Plan* __restrict__ plan, uint32_t level,
     const uint32_t* __restrict__ inv, uint32_t* uf, uint2* __restrict__ records,
-    uint32_t* __restrict__ cursor, uint64_t capacity, uint32_t* ctl, uint32_t* status) {
+    uint32_t* __restrict__ cursor, uint64_t capacity, const __grid_constant__ Chains chains, uint32_t* status) {
     wait_for_previous();
     __shared__ uint32_t count[kUnionWindows];
     __shared__ uint32_t start[kUnionWindows];
@@ -525,16 +561,17 @@ __global__ void __launch_bounds__(256) union_bucket(const Plan* __restrict__ pla
         }
         const uint32_t left = union_append<kUnionBucketItems>(records, cursor, capacity, rec,
             pending, count, start);
-        if (left != 0) union_finish<kUnionBucketItems>(uf, rec, left, ctl, status);
+        if (left != 0) union_finish<kUnionBucketItems>(uf, rec, left, chains, status);
     }
 }
 
 // A union that has come half of kLongChain halves the rest of its path: x,
 // whose word is w, goes to its grandparent; both are true facts, so the racy
 // store can only write a true one.  Returns the word that leads from x to
-// where the walk goes on.  (Uniform inputs never get here, but the branch
-// keeps the two unions of a thread apart in the code: without it the windows
-// of 100,000,007 entries' top two levels take 3.09 ms, with it 2.90.)
+// where the walk goes on.  Uniform inputs never get here, but the compiler
+// makes a slower loop of union_window without the branch: 3.07 ms for the
+// windows of 100,000,007 entries' top two levels, 2.84 with it (and 3.08
+// where `chains` is a __grid_constant__).
 __device__ __forceinline__ uint32_t uf_halve(uint32_t* uf, uint32_t x, uint32_t w) {
     const uint32_t up = *(volatile uint32_t*)(uf + (w >> 1));
     if ((up >> 1) == (w >> 1)) {
@@ -547,9 +584,10 @@ __device__ __forceinline__ uint32_t uf_halve(uint32_t* uf, uint32_t x, uint32_t 
 
 __global__ void __launch_bounds__(256, 6) union_window(uint32_t window, uint32_t* uf,
     uint2* __restrict__ records, uint32_t* __restrict__ cursor, uint64_t capacity,
-    uint32_t* ctl, uint32_t* status) {
+    const Chains chains, uint32_t* status) {
     wait_for_previous();
-    if (__syncthreads_or(given_up(ctl + kCtlChains))) return; // mostly by a higher window
+    const volatile uint32_t* stop = chains.ctl + kCtlClaimUnion;
+    if (__syncthreads_or((*stop & kStopClaims) != 0)) return; // too many unions put off
     __shared__ uint32_t count[kUnionWindows];
     __shared__ uint32_t start[kUnionWindows];
     const uint64_t base = (uint64_t)window << (kUnionWindowLog2 + 1);
@@ -594,18 +632,18 @@ __global__ void __launch_bounds__(256, 6) union_window(uint32_t window, uint32_t
                     live &= ~(1u << i); // on to a lower window
                     pending |= 1u << i;
                 } else if (it == kLongChain) {
-                    give_up(ctl, ctl + kCtlChains);
+                    defer(chains, rec[i]);
                     live &= ~(1u << i);
                 }
             }
         }
         const uint32_t left = union_append<K>(records, cursor, capacity, rec, pending, count, start);
-        if (left != 0) union_finish<K>(uf, rec, left, ctl, status);
+        if (left != 0) union_finish<K>(uf, rec, left, chains, status);
     }
 }
 
 __device__ __forceinline__ void level_orient_run(Grid grid, const Plan* __restrict__ plan, uint32_t level,
-    const uint32_t* __restrict__ inv, uint32_t* uf, uint32_t* ctl, uint32_t* chains,
+    const uint32_t* __restrict__ inv, uint32_t* uf, const Chains& chains,
     uint32_t* status) {
     if (given_up(chains)) return;
     const LevelInfo& lv = plan->levels[level];
@@ -625,7 +663,7 @@ __device__ __forceinline__ void level_orient_run(Grid grid, const Plan* __restri
         const uint32_t x[1] = {(uint32_t)j * pcap + (s >> 1)};
         Found f[1];
         if (uf_find_many<1>(uf, x, f, 1u) != 0) {
-            give_up(ctl, chains);
+            give_up(chains);
         } else if (f[0].bit) {
             atomicOr(uf + f[0].root, 1u);
         }
@@ -633,9 +671,9 @@ __device__ __forceinline__ void level_orient_run(Grid grid, const Plan* __restri
 }
 
 __global__ void level_orient(const Plan* __restrict__ plan, uint32_t level,
-    const uint32_t* __restrict__ inv, uint32_t* uf, uint32_t* ctl, uint32_t* status) {
+    const uint32_t* __restrict__ inv, uint32_t* uf, const __grid_constant__ Chains chains, uint32_t* status) {
     wait_for_previous();
-    level_orient_run(launch_grid(), plan, level, inv, uf, ctl, ctl + kCtlChains, status);
+    level_orient_run(launch_grid(), plan, level, inv, uf, chains, status);
 }
 
 // Switch addresses of every node of the levels above the tile's: level l's
@@ -661,8 +699,8 @@ __device__ __forceinline__ void level_descriptors_run(Grid grid, const Plan* __r
 // went, in grid-stride order on nodes up to 2^26 entries, took 58 ms per
 // compress at 2^30 entries, these 44 ms.
 __device__ __forceinline__ void level_roots_run(Grid grid, const Plan* __restrict__ plan,
-    uint32_t level, uint32_t* uf, uint32_t* __restrict__ xbits, uint32_t* ctl,
-    uint32_t* chains) {
+    uint32_t level, uint32_t* uf, uint32_t* __restrict__ xbits,
+    const Chains& chains) {
     const LevelInfo& lv = plan->levels[level];
     const uint32_t pcap = (uint32_t)lv.pcap;
     // this call's pair-nodes [lo_pair, end); chunks start at a 32-pair
@@ -678,7 +716,7 @@ __device__ __forceinline__ void level_roots_run(Grid grid, const Plan* __restric
     // back into its word: parents are smaller than their children, so most
     // finds end at a parent that was resolved before them.
     uint64_t first;
-    while (claim_chunk(ctl + kCtlClaimRoots, chunk, total, &first)) {
+    while (claim_chunk(chains.ctl + kCtlClaimRoots, chunk, total, &first)) {
         const uint64_t p0 = begin + first + (uint64_t)threadIdx.x * kResolveItems;
         uint32_t j = (uint32_t)(p0 / pcap);
         uint32_t k = (uint32_t)(p0 - (uint64_t)j * pcap);
@@ -697,7 +735,7 @@ __device__ __forceinline__ void level_roots_run(Grid grid, const Plan* __restric
         }
         Found f[kResolveItems];
         if (uf_find_many<kResolveItems>(uf, x, f, live) != 0) {
-            give_up(ctl, chains);
+            give_up(chains);
             live = 0;
         }
         uint32_t mine = 0; // this lane's kResolveItems colour bits
@@ -724,9 +762,9 @@ __device__ __forceinline__ void level_roots_run(Grid grid, const Plan* __restric
 
 __global__ void __launch_bounds__(256, BPB200_FINAL_MIN_BLOCKS) level_roots(
     const Plan* __restrict__ plan, uint32_t level, uint32_t* uf, uint32_t* __restrict__ xbits,
-    uint32_t* ctl) {
+    const __grid_constant__ Chains chains) {
     wait_for_previous();
-    level_roots_run(launch_grid(), plan, level, uf, xbits, ctl, ctl + kCtlChains);
+    level_roots_run(launch_grid(), plan, level, uf, xbits, chains);
 }
 
 // Output side of a level, in natural (node, output pair) order: the output

@@ -13,20 +13,27 @@
 //   flatten  every pair-node takes its ancestor's word over until it points
 //            at its root; a pass multiplies the stretch a word covers by at
 //            least kSettleHops + 1, so a chain of 2^29 takes ten passes;
-//   unite    all output pairs' unions again, most of them found done.  Of
-//            two roots that a pair still joins one is linked each time, so
-//            the roots left to join at least halve from round to round;
+//   unite    the unions put off or, when there were more than their list
+//            holds, all output pairs' again.  Of two roots that a union still
+//            joins one is linked each time, so the roots left to join at
+//            least halve from round to round;
 // and, once a round leaves nothing undone, orients the odd tails'
 // components and writes the colours.  No input makes it fail.
 //
 // Its blocks wait on one another between the passes, so it is launched
 // cooperatively, one block per SM, and returns at once where no walk gave
 // up.  What bounds it: the words' dependent reads, at one block's warps per
-// SM.  Device time of the whole call: 2^24 + 5 entries 5.9 ms for neighbours
-// kept in pairs and 4.5 ms for blocks of 100,001 entries (uniform 5.1 ms;
-// walks without a limit took 234 ms for the blocks), 2^25 + 2 entries 11.6
-// and 10.3 ms (uniform 9.9; 700 ms), 100,000,007 entries 36.2 and 46 ms
-// (uniform 30.6; 2470 ms).  3, 5 or 16 hops a pass: within 5 % of 8.
+// SM.  Device time of the whole call, ms, for uniform inputs, neighbours kept
+// in pairs and blocks of 100,001 entries (in brackets: walks without a limit,
+// which ran into a cap on the pairs):
+//   2^24 + 2 entries     5.1, 5.9 (failed), 4.5 (320)
+//   2^25 + 2 entries     9.9, 11.4 (failed), 10.0 (700)
+//   100,000,007 entries  30.4, 33.7 (failed), 36.8 (2470)
+// Doing all unions again in place of the listed ones took 6.0 and 4.7, 11.6
+// and 10.3, 36.2 and 46 ms.  A limit of 1024 steps for the unions suits some
+// inputs (p = 1,048,583 i mod 2^28: 77 ms, 122 with 256, uniform 86), and
+// costs others more (2^28 in blocks: 184 ms, 119 with 256).  3, 5 or 16 hops a
+// pass: within 5 % of 8.
 #pragma once
 
 #include "device.cuh"
@@ -142,9 +149,10 @@ __device__ __forceinline__ bool settle_flatten(SettleBarrier& barrier, const Lev
 
 __global__ void __launch_bounds__(kSettleThreads, 1) level_settle(const Plan* __restrict__ plan,
     uint32_t level, const uint32_t* __restrict__ inv, uint32_t* uf, uint32_t* __restrict__ xbits,
-    uint32_t* ctl, uint32_t* status) {
+    const __grid_constant__ Chains chains, uint32_t* status) {
     wait_for_previous();
-    if (!given_up(ctl + kCtlChains)) return; // the same for all blocks: nothing here sets it
+    if (!given_up(chains)) return; // the same for all blocks: nothing here sets it
+    const uint32_t deferred = chains.ctl[kCtlDeferred];
     const LevelInfo& lv = plan->levels[level];
     const uint32_t ps = (uint32_t)lv.pcap;
     const NodeRange nr = level_nodes(*plan, level);
@@ -152,8 +160,8 @@ __global__ void __launch_bounds__(kSettleThreads, 1) level_settle(const Plan* __
     const uint64_t end = lo + ((uint64_t)ps << nr.shift);
     const uint64_t id = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    SettleBarrier barrier{ctl, status};
-    bool again = true;
+    SettleBarrier barrier{chains.ctl, status};
+    bool again = deferred != 0;
     for (uint32_t round = 0; again; ++round) {
         if (!settle_flatten(barrier, lv, level, uf, lo, end)) return;
         if (round == kSettleRounds) {
@@ -161,8 +169,16 @@ __global__ void __launch_bounds__(kSettleThreads, 1) level_settle(const Plan* __
             return;
         }
         bool undone = false;
-        for (uint64_t p0 = lo + id * kUnionItems; p0 < end; p0 += stride * kUnionItems) {
-            undone |= unite_outputs(lv, level, inv, uf, p0, end, true, status);
+        if (deferred > chains.room) {
+            for (uint64_t p0 = lo + id * kUnionItems; p0 < end; p0 += stride * kUnionItems) {
+                undone |= unite_outputs(lv, level, inv, uf, p0, end, true, nullptr, status);
+            }
+        } else {
+            for (uint64_t i = id; i < deferred; i += stride) {
+                const uint2 r = chains.list[i];
+                uint32_t a[1] = {r.x}, b[1] = {r.y >> 1}, rel[1] = {r.y & 1u};
+                undone |= uf_unite_many<1, true>(uf, a, b, rel, 1u, status) != 0;
+            }
         }
         if (!barrier.wait(undone, &again)) return;
     }
