@@ -3,8 +3,8 @@
 
 Produces ``benes_perm_b200/libbenes_b200.so`` next to this file with one nvcc
 invocation.  nvcc cross-compiles, so this runs on machines without a GPU.
-``defines`` (e.g. ``["BPB200_RULER_LOG2=5"]``) and ``out`` build a variant
-library elsewhere, for tuning the compile-time knobs of the walk colouring.
+``defines`` (e.g. ``["BPB200_PLACE_LOG2=24"]``) and ``out`` build a variant
+library elsewhere, for tuning the compile-time knobs.
 """
 from __future__ import annotations
 

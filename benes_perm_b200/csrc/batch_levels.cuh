@@ -14,8 +14,8 @@
 // the work in flight at any moment still covers a few nodes of one or two
 // permutations.  A group of R permutations therefore needs one launch per
 // kernel step per level instead of R, and the steps of short, latency-bound
-// levels of different permutations (pointer-jumping rounds, small walks)
-// run side by side on different SMs.
+// levels of different permutations (list contraction and ranking, small
+// walks) run side by side on different SMs.
 #pragma once
 
 #include "kernels.cuh"

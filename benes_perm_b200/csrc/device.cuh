@@ -1,8 +1,8 @@
 // SPDX-License-Identifier: Apache-2.0
 //
 // Device building blocks shared by the level kernels and the tile kernel:
-// parity union-find, warp-aggregated bit emission and the warp factoradic
-// rank.
+// parity union-find, warp-aggregated bit emission and the factoradic rank of
+// a middle group.
 #pragma once
 
 #include "plan.hpp"

@@ -48,7 +48,7 @@ constexpr int kLevelThreads = 256;
 enum KernelKind : int {
     kKindPrologue = 0,
     kKindInverse,
-    kKindDescriptors,
+    kKindDescriptors, // part of the prologue: never recorded, kept in the numbering
     kKindUnion,
     kKindOrient,
     kKindResolve,

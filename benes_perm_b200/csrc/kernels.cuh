@@ -17,6 +17,7 @@
 //                colouring: each component's smallest vertex gets colour
 //                0); the input switch of pair k is x(k).  Nodes that fit L2
 //                are coloured by walks instead (walk.cuh)
+//   settle       a level whose union-find chains get long (settle.cuh)
 //   outputs      output switch of output pair k is colour(inv[2k]); the
 //                children's inverses follow from the same two reads (the
 //                values p are read at level 0 only)
@@ -37,9 +38,10 @@
 namespace bpb200 {
 
 constexpr uint32_t kTileThreads = 512;
-// 4 slots per thread measured fastest on B200 at 2^30 uniform entries
-// (inverse kernels 207 ms per compress; 8: 227 ms; 16: 243 ms): more
-// threads keep more of the scattered inverse stores in flight.
+// 4 slots per thread: more threads keep more of the scattered inverse stores
+// in flight (measured on B200 when every level of 2^30 uniform entries had
+// its own inverse: 207 ms per compress, 8 slots 227, 16 slots 243; it now
+// runs on level 0 of inputs of up to 2^23 entries only).
 #ifndef BPB200_INVERSE_ITEMS
 #define BPB200_INVERSE_ITEMS 4
 #endif

@@ -11,8 +11,9 @@ another (coordinate descent from the compiled defaults):
 
 walk_max_log2, the largest node coloured by ruler walks (else union-find),
 stays at its compiled 2^23: on the uniform inputs timed here union-find is up
-to 5 % faster below that, but on inputs made of long runs its chains reach
-the cap on their length, which the walks' do not.  walk_blocks_per_sm is part
+to 5 % faster below that, but inputs made of long runs give it long chains,
+which cost a second colouring of the level (level_settle) and the walks
+nothing.  walk_blocks_per_sm is part
 of every setting but no kernel reads it: the walks take one ruler per thread,
 so the list's length sizes their grid.
 
