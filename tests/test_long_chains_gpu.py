@@ -117,3 +117,15 @@ def test_batch_allocation_free_and_shards(gpu, oracle):
         assert total.max() <= 255 and total.astype(np.uint8).tobytes() == want
     finally:
         gpu.set_union_find_only(False)
+
+
+def test_calls_at_once(gpu, oracle):
+    """Several host threads' calls at once, on streams of their own: the
+    launches of one wait for their own blocks only."""
+    from concurrent.futures import ThreadPoolExecutor
+    n = (1 << 23) + 5
+    perms = [structured(kind, n) for kind in ("pairs", "riffle", "reverse", "rotation")]
+    with ThreadPoolExecutor(4) as pool:
+        wants = list(pool.map(lambda p: oracle.compress(p, oracle_format({})), perms))
+        for _ in range(5):
+            assert list(pool.map(gpu.compress, perms)) == wants
