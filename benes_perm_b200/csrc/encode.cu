@@ -291,7 +291,9 @@ __global__ void __launch_bounds__(256) prologue(const __grid_constant__ Prologue
     level_descriptors_run(launch_grid(), &p.plan, in_addr, out_addr);
 }
 
-// Launches a kernel with one launch attribute set.
+// Launches a kernel with one launch attribute set.  A cooperative launch of
+// more blocks than the stream's context can hold at once (one that owns only
+// a part of the SMs) is tried again with half of them.
 template <typename... Params, typename... Args>
 void launch_with(cudaLaunchAttributeID id, void (*kernel)(Params...), uint64_t blocks,
     uint32_t threads, uint32_t smem, cudaStream_t st, Args&&... args) {
@@ -309,7 +311,13 @@ void launch_with(cudaLaunchAttributeID id, void (*kernel)(Params...), uint64_t b
     }
     config.attrs = &attribute;
     config.numAttrs = 1;
-    check(cudaLaunchKernelEx(&config, kernel, Params(args)...), "kernel launch");
+    cudaError_t e = cudaLaunchKernelEx(&config, kernel, Params(args)...);
+    while (e == cudaErrorCooperativeLaunchTooLarge && config.gridDim.x > 1) {
+        cudaGetLastError(); // the error is not sticky
+        config.gridDim.x /= 2;
+        e = cudaLaunchKernelEx(&config, kernel, Params(args)...);
+    }
+    check(e, "kernel launch");
 }
 
 // Launches the next kernel of an encode's sequence: with programmatic stream
